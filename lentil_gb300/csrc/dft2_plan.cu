@@ -102,6 +102,9 @@ struct lgb_dft2_plan_s {
   PhaseAxis* axes = nullptr;     // [2] rows, cols
   double* unit2 = nullptr;       // [1] = 1 (the scale is applied by the epilogue)
   double2 *E1 = nullptr, *E2 = nullptr;
+  bool sliced = false;           // FP64 on the tensor cores: digit matrices in place of E1, E2
+  uint16_t *d1 = nullptr, *d2 = nullptr;
+  PhaseAxis ar{}, ac{};
   uint16_t *e1h = nullptr, *e1l = nullptr, *e2h = nullptr, *e2l = nullptr;
   int* host_err = nullptr;       // pinned copy of *err (a status-pool word)
   cudaEvent_t copied = nullptr;  // recorded after that copy
@@ -123,6 +126,9 @@ size_t plan_carve(lgb_dft2_plan_s* P, void* base) {
     P->e1l = c.take<uint16_t>(mrows1 * 2 * P->kp1);
     P->e2h = c.take<uint16_t>(nrows2 * 2 * P->kp2);
     P->e2l = c.take<uint16_t>(nrows2 * 2 * P->kp2);
+  } else if (P->sliced) {
+    P->d1 = c.take<uint16_t>(sliced_matrix_entries(P->m, P->M, true));
+    P->d2 = c.take<uint16_t>(sliced_matrix_entries(P->n, P->N, !P->left));
   } else {
     P->E1 = c.take<double2>((size_t)P->M * P->m);
     P->E2 = c.take<double2>((size_t)P->n * P->N);
@@ -137,6 +143,7 @@ struct ExecSpace {
 };
 
 size_t exec_carve(const lgb_dft2_plan_s* P, int count, void* base, ExecSpace* s) {
+  if (P->sliced) return sliced_dft2_workspace(count, P->m, P->n, P->M, P->N);
   PlanCarve c(base);
   ExecSpace t{};
   if (split_precision(P->precision)) {
@@ -183,6 +190,9 @@ int plan_setup(lgb_dft2_plan_s* P, int m, int n, int M, int N, double alpha_r, d
   P->kp2 = round_up(n, 32);
   P->scale = unitary ? std::sqrt(std::fabs(alpha_r * alpha_c)) : 1.0;
   P->left = (double)M * m * n + (double)M * n * N <= (double)m * n * N + (double)M * m * N;
+  P->sliced = precision == LGB_FP64 && sliced_applies(m, n, M, N);
+  P->ar = ax[0];
+  P->ac = ax[1];
   P->bytes = plan_carve(P, nullptr);
   return LGB_OK;
 }
@@ -240,6 +250,10 @@ int plan_build(lgb_dft2_plan_s* P, const PhaseAxis* ax, cudaStream_t s) {
     if (!st) st = launch_e2_block_split(P->axes + 1, 1, P->n, P->N, P->kp2,
                                         cdiv(P->N, 128) * 256, bf16, P->e2h, P->e2l, s);
     return st;
+  }
+  if (P->sliced) {
+    int st = launch_matrix_digits(ax[0], P->m, P->M, true, P->d1, s);
+    return st ? st : launch_matrix_digits(ax[1], P->n, P->N, !P->left, P->d2, s);
   }
   int st = launch_dft_matrix_c128(ax[0], P->m, P->M, P->E1, true, s);
   if (!st) st = launch_dft_matrix_c128(ax[1], P->n, P->N, P->E2, false, s);
@@ -357,6 +371,9 @@ extern "C" int lgb_dft2_plan_execute(lgb_dft2_plan P, const lgb_c128* f, int cou
   double2* Fout = reinterpret_cast<double2*>(F);
   const int m = P->m, n = P->n, M = P->M, N = P->N;
   int st;
+  if (P->sliced)
+    return launch_sliced_dft2({count, m, n, M, N, P->d1, P->d2, P->ar, P->ac, P->scale, fin, Fout},
+                              workspace, s);
   if (!split) {
     const long long sf = (long long)m * n, sF = (long long)M * N;
     if (P->left) {

@@ -127,12 +127,33 @@ struct ZgemmScratch {
 int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2* C, int ldc, long long sC,
                  int batch, double alpha, cudaStream_t s, const ZgemmScratch* scratch = nullptr);
+// Bytes of lgb_dft2's workspace on the plain FP64 path (plan.cu)
+size_t plain_dft2_workspace(int m, int n, int M, int N);
 // lgb_dft2_batch's body (plan.cu), with the FP64 GEMMs' split-K partials
 // taken from `zs` when it is given (nothing is allocated then)
 int dft2_batch(const double2* f, int count, int m, int n, double2* F, int M, int N,
                double alpha_r, double alpha_c, double shift_r, double shift_c, double offset_r,
                double offset_c, int unitary, int precision, void* workspace,
                size_t workspace_bytes, cudaStream_t s, const ZgemmScratch* zs);
+// mft_sliced.cu ----------------------------------------------------------
+// complex128 dft2 on the tensor cores by error-free slicing
+struct SlicedDft2 {
+  int count, m, n, M, N;
+  const uint16_t *e1, *e2;   // launch_matrix_digits of the row axis (m -> M) and the column axis (n -> N)
+  PhaseAxis ar, ac;
+  double scale;
+  const double2* f;          // [count][m][n]
+  double2* F;                // [count][M][N]
+};
+bool sliced_applies(int m, int n, int M, int N);
+// Product order; E1 is an operand B, E2 an operand A when left, else B.
+bool sliced_left(int m, int n, int M, int N);
+size_t sliced_matrix_entries(int len_in, int len_out, bool operand_b);    // 16-bit entries
+int launch_matrix_digits(const PhaseAxis& ax, int len_in, int len_out, bool operand_b, uint16_t* out,
+                         cudaStream_t s);
+size_t sliced_dft2_workspace(int count, int m, int n, int M, int N);
+int launch_sliced_dft2(const SlicedDft2& q, void* workspace, cudaStream_t s);
+
 // out[b] += sum_l weights[b][l] * unit2[l] * |F[b][l]|^2 into a window (FP64)
 int launch_intensity_accum_c128(const double2* F, int M, int N, long long sF, int batch_inner,
                                 const double* weights, const double* unit2, double* out,

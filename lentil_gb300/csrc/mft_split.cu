@@ -49,9 +49,6 @@
 // the epilogue warps of both.
 // Every mbarrier wait is bounded in time; on expiry the kernel records
 // LGB_ETIMEOUT in a device flag, drains what it issued and returns.
-#include <cuda.h>
-#include <cudaTypedefs.h>
-
 #include <algorithm>
 #include <array>
 #include <atomic>
@@ -60,6 +57,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "tcgen05.cuh"
 
 namespace lgb {
 namespace tc {
@@ -146,192 +144,6 @@ __device__ __forceinline__ int tile_n(const Params& p, int tn) {
 
 __device__ __forceinline__ int matrix_slot(const Params& p, int lam) {
   return p.lam_idx ? p.lam_idx[lam] : lam;
-}
-
-// ------------------------------------------------------------------ PTX ---
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ uint64_t gtimer() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait: true when the phase completed, false on time-out (recorded
-// as LGB_ETIMEOUT) or when another role already flagged an error.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* err,
-                                          unsigned long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = gtimer();
-  for (uint32_t n = 1;; ++n) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((n & 63) == 0) {
-      if (*(volatile int*)err != 0) return false;
-      if (gtimer() - t0 > limit_ns) {
-        atomicCAS(err, 0, LGB_ETIMEOUT);
-        return false;
-      }
-    }
-  }
-}
-// Wait for work this CTA already issued (TMA loads in flight, MMAs) before
-// leaving: bounded in time only, whatever the error flag says, so that a
-// launch that gave up still retires its copies and MMAs before its shared
-// memory and TMEM are released.  Copies and MMAs that were issued complete
-// on their own; only a barrier whose loads were never issued (the stall
-// test) runs out, after limit_ns.
-__device__ __forceinline__ void mbar_wait_issued(uint32_t bar, uint32_t parity,
-                                                 unsigned long long limit_ns) {
-  if (mbar_try_wait(bar, parity)) return;
-  const uint64_t t0 = gtimer();
-  for (uint32_t n = 1;; ++n) {
-    if (mbar_try_wait(bar, parity)) return;
-    if ((n & 63) == 0 && gtimer() - t0 > limit_ns) return;
-  }
-}
-// Shared-memory address of the same variable in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
-               "barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// arrive (+ expected bytes) on a barrier given by its cluster address.
-// Default (CTA-scope release) semantics: what these arrivals publish needs no
-// cluster-wide fence -- the producer has written nothing the consumer reads,
-// and an epilogue's TMEM reads are complete at tcgen05.wait::ld, ordered
-// against the next MMA by the tcgen05 fences around the barrier.  (A
-// cluster-scope release here stalled every epilogue warp on a memory barrier
-// once per K block: measured 11 % of the whole step.)
-__device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cluster.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-// TMA tile load into this CTA's shared memory, completion counted on a
-// barrier of either CTA of the pair (cluster address).
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar,
-                                            int x, int y, int z) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
-      : "memory");
-}
-// Bulk tensor store / FP32 reduce-add of a swizzled shared-memory tile
-// (async proxy; completion tracked by bulk groups of the issuing thread).
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(src), "r"(x), "r"(y), "r"(z)
-               : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, uint32_t src, int x, int y,
-                                                  int z) {
-  asm volatile(
-      "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-          reinterpret_cast<uint64_t>(map)),
-      "r"(src), "r"(x), "r"(y), "r"(z)
-      : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// the shared-memory sources of this thread's bulk groups may be overwritten
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-// this thread's bulk groups have completed their global writes
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-// K-major operand tile with the 128-byte swizzle TMA writes: rows of 64
-// 16-bit elements (128 B), 8-row groups 1024 B apart.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                             // leading byte offset (unused, SW128 K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                   // stride byte offset: 8-row group pitch
-  d |= (uint64_t)1 << 46;                             // descriptor version
-  d |= (uint64_t)2 << 61;                             // 128-byte swizzle
-  return d;
-}
-// D[256 x 256] (+)= A[256 x 16] . B[256 x 16]^T over the CTA pair: each CTA
-// supplies 128 rows of A and 128 rows of B at the same shared-memory offset.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-// arrive once on the barrier at this offset in both CTAs when the MMAs
-// issued so far have completed
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
-  const uint16_t both = 3;
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], %1;" ::"r"(bar), "h"(both)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]),
-        "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]),
-        "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b),
-               "f"(c), "f"(d)
-               : "memory");
 }
 
 // ------------------------------------------------------------ schedule ---
@@ -726,40 +538,6 @@ split_mft_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_consta
 }
 
 // ------------------------------------------------------------------ host ---
-static PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaDriverEntryPointQueryResult q;
-    void* f = nullptr;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault,
-                                         &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-  });
-  return fn;
-}
-
-// 3-D row-major map: dims {K, rows, batch} of elem_bytes-wide elements, box
-// {box_k, box_rows, 1}.
-static int make_map_any(CUtensorMap* map, const void* ptr, CUtensorMapDataType dtype, int elem_bytes,
-                        int K, int rows, int batch, int box_k, int box_rows, CUtensorMapSwizzle swz) {
-  auto enc = encode_fn();
-  LGB_REQUIRE(enc, LGB_ECUDA, "cuTensorMapEncodeTiled is unavailable");
-  LGB_REQUIRE(((uintptr_t)ptr & 15) == 0, LGB_EINVAL, "tensor map base must be 16-byte aligned");
-  LGB_REQUIRE(((size_t)K * elem_bytes) % 16 == 0, LGB_EINVAL, "tensor map row pitch must be a multiple of 16 bytes");
-  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)batch};
-  cuuint64_t strides[2] = {(cuuint64_t)K * elem_bytes, (cuuint64_t)K * elem_bytes * rows};
-  cuuint32_t box[3] = {(cuuint32_t)box_k, (cuuint32_t)box_rows, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult res = enc(map, dtype, 3, const_cast<void*>(ptr), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (res != CUDA_SUCCESS)
-    return set_error(LGB_ECUDA, "cuTensorMapEncodeTiled failed with code " + std::to_string((int)res));
-  return LGB_OK;
-}
-
 static CUtensorMapDataType half_type(bool bf16) {
   return bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
 }

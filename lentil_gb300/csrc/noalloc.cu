@@ -59,7 +59,7 @@ extern "C" int lgb_dft2_noalloc(const lgb_c128* f, int m, int n, lgb_c128* F, in
   LGB_RANGE("lgb_dft2_noalloc");
   using namespace lgb;
   LGB_REQUIRE(m > 0 && n > 0 && M > 0 && N > 0, LGB_EINVAL, "dft2_noalloc: sizes must be positive");
-  const size_t need = lgb_dft2_workspace_size(m, n, M, N, LGB_FP64);
+  const size_t need = plain_dft2_workspace(m, n, M, N);
   if (need > (size_t)LGB_NOALLOC_SCRATCH_BYTES)
     return set_error(LGB_EINVAL,
                      "dft2_noalloc: this transform needs " + std::to_string(need) +

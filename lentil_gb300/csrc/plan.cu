@@ -36,6 +36,10 @@ struct Dft2Fp64Space {
   int* err;
   double2 *E1, *E2, *T;
 };
+struct Dft2SlicedSpace {
+  void* ws;             // launch_sliced_dft2's workspace (its status word first)
+  uint16_t *e1, *e2;
+};
 struct Dft2SplitSpace {
   int* err;
   PhaseAxis* axes;      // [2]
@@ -53,6 +57,20 @@ static size_t carve_fp64(void* ws, int count, int m, int n, int M, int N, Dft2Fp
   t.T = c.take<double2>((size_t)count * std::max((size_t)M * n, (size_t)m * N));
   if (s) *s = t;
   return c.used;
+}
+
+static size_t carve_sliced(void* ws, int count, int m, int n, int M, int N, Dft2SlicedSpace* s) {
+  Carve c(ws);
+  Dft2SlicedSpace t;
+  t.ws = c.take<char>(sliced_dft2_workspace(count, m, n, M, N));
+  t.e1 = c.take<uint16_t>(sliced_matrix_entries(m, M, true));
+  t.e2 = c.take<uint16_t>(sliced_matrix_entries(n, N, !sliced_left(m, n, M, N)));
+  if (s) *s = t;
+  return c.used;
+}
+
+size_t plain_dft2_workspace(int m, int n, int M, int N) {
+  return carve_fp64(nullptr, 1, m, n, M, N, nullptr);
 }
 
 static size_t carve_split(void* ws, int count, int m, int n, int M, int N, Dft2SplitSpace* s) {
@@ -90,8 +108,9 @@ using namespace lgb;
 extern "C" size_t lgb_dft2_batch_workspace_size(int count, int m, int n, int M, int N,
                                                 int precision) {
   if (count <= 0 || m <= 0 || n <= 0 || M <= 0 || N <= 0) return 0;
-  return is_split(precision) ? carve_split(nullptr, count, m, n, M, N, nullptr)
-                             : carve_fp64(nullptr, count, m, n, M, N, nullptr);
+  if (is_split(precision)) return carve_split(nullptr, count, m, n, M, N, nullptr);
+  return sliced_applies(m, n, M, N) ? carve_sliced(nullptr, count, m, n, M, N, nullptr)
+                                    : carve_fp64(nullptr, count, m, n, M, N, nullptr);
 }
 
 extern "C" size_t lgb_dft2_workspace_size(int m, int n, int M, int N, int precision) {
@@ -121,13 +140,21 @@ int lgb::dft2_batch(const double2* fin, int count, int m, int n, double2* Fout, 
   LGB_REQUIRE(precision == LGB_FP64 || is_split(precision), LGB_EINVAL, "dft2: unknown precision");
   LGB_REQUIRE(workspace && ((uintptr_t)workspace & 255) == 0, LGB_EWORKSPACE,
               "dft2: workspace must be non-null and 256-byte aligned");
-  LGB_REQUIRE(workspace_bytes >= lgb_dft2_batch_workspace_size(count, m, n, M, N, precision),
+  LGB_REQUIRE(workspace_bytes >= (zs ? plain_dft2_workspace(m, n, M, N)
+                                     : lgb_dft2_batch_workspace_size(count, m, n, M, N, precision)),
               LGB_EWORKSPACE, "dft2: workspace too small");
   PhaseAxis ar, ac;
   if ((st = make_phase_axis(alpha_r, shift_r, offset_r, m, M, &ar))) return st;
   if ((st = make_phase_axis(alpha_c, shift_c, offset_c, n, N, &ac))) return st;
   const double scale = unitary ? std::sqrt(std::fabs(alpha_r * alpha_c)) : 1.0;
 
+  if (precision == LGB_FP64 && !zs && sliced_applies(m, n, M, N)) {
+    Dft2SlicedSpace w;
+    carve_sliced(workspace, count, m, n, M, N, &w);
+    if ((st = launch_matrix_digits(ar, m, M, true, w.e1, s))) return st;
+    if ((st = launch_matrix_digits(ac, n, N, !sliced_left(m, n, M, N), w.e2, s))) return st;
+    return launch_sliced_dft2({count, m, n, M, N, w.e1, w.e2, ar, ac, scale, fin, Fout}, w.ws, s);
+  }
   if (precision == LGB_FP64) {
     Dft2Fp64Space w;
     carve_fp64(workspace, count, m, n, M, N, &w);
