@@ -143,7 +143,7 @@ struct ExecSpace {
 };
 
 size_t exec_carve(const lgb_dft2_plan_s* P, int count, void* base, ExecSpace* s) {
-  if (P->sliced) return sliced_dft2_workspace(count, P->m, P->n, P->M, P->N);
+  if (P->sliced) return sliced_dft2_workspace(count, P->m, P->n, P->M, P->N, P->left);
   PlanCarve c(base);
   ExecSpace t{};
   if (split_precision(P->precision)) {
@@ -252,8 +252,8 @@ int plan_build(lgb_dft2_plan_s* P, const PhaseAxis* ax, cudaStream_t s) {
     return st;
   }
   if (P->sliced) {
-    int st = launch_matrix_digits(ax[0], P->m, P->M, true, P->d1, s);
-    return st ? st : launch_matrix_digits(ax[1], P->n, P->N, !P->left, P->d2, s);
+    int st = launch_matrix_digits(ax[0], nullptr, 1, P->m, P->M, true, P->d1, s);
+    return st ? st : launch_matrix_digits(ax[1], nullptr, 1, P->n, P->N, !P->left, P->d2, s);
   }
   int st = launch_dft_matrix_c128(ax[0], P->m, P->M, P->E1, true, s);
   if (!st) st = launch_dft_matrix_c128(ax[1], P->n, P->N, P->E2, false, s);
@@ -371,9 +371,18 @@ extern "C" int lgb_dft2_plan_execute(lgb_dft2_plan P, const lgb_c128* f, int cou
   double2* Fout = reinterpret_cast<double2*>(F);
   const int m = P->m, n = P->n, M = P->M, N = P->N;
   int st;
-  if (P->sliced)
-    return launch_sliced_dft2({count, m, n, M, N, P->d1, P->d2, P->ar, P->ac, P->scale, fin, Fout},
-                              workspace, s);
+  if (P->sliced) {
+    SlicedDft2 q{};
+    q.count = count;
+    q.m = m; q.n = n; q.M = M; q.N = N;
+    q.left = P->left;
+    q.e1 = P->d1; q.e2 = P->d2;
+    q.ar = P->ar; q.ac = P->ac;
+    q.scale = P->scale;
+    q.f = fin;
+    q.F = Fout;
+    return launch_sliced_dft2(q, workspace, s);
+  }
   if (!split) {
     const long long sf = (long long)m * n, sF = (long long)M * N;
     if (P->left) {

@@ -384,8 +384,12 @@ __device__ __forceinline__ void store_digits(const DigitRows& o, int j, int k, l
     *reinterpret_cast<uint32_t*>(p + i * o.plane() + o.b * o.set()) = __byte_perm(a[i], c[i], 0x7632);
 }
 
-// DFT-matrix digits: vector j < L (output index) over the input index.
-__global__ void __launch_bounds__(128) matrix_digits_kernel(PhaseAxis ax, int len_in, DigitRows out) {
+// DFT-matrix digits: vector j < L (output index) over the input index; matrix
+// z's axis is axes[z], or ax when there is one.
+__global__ void __launch_bounds__(128) matrix_digits_kernel(PhaseAxis ax, const PhaseAxis* __restrict__ axes,
+                                                            int len_in, DigitRows out) {
+  if (axes) ax = axes[blockIdx.z];
+  out.base += (size_t)blockIdx.z * NE * out.plane();
   const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x), j = blockIdx.y;
   if (k >= out.kp) return;
   const double2 zero = make_double2(0.0, 0.0);
@@ -590,6 +594,8 @@ struct FinishParams {
   const double2* f;          // [item][m][n]
   int m, n;
   PhaseAxis ar, ac;
+  const PhaseAxis* axes;     // per item, or null: ar, ac
+  int cols;
   longlong2* scratch;        // P again: the item's intermediate rows
   const int* flags;
   const int* err;
@@ -605,6 +611,7 @@ __device__ __forceinline__ void cfma(double2& c, double2 a, double2 b) {
 // One output row u (left) or column v of a transform in plain FP64, by one
 // block: the intermediate row, then the output from it.
 __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
+  const PhaseAxis ar = p.axes ? p.axes[b] : p.ar, ac = p.axes ? p.axes[p.cols + b] : p.ac;
   const double2* f = p.f + (size_t)b * p.m * p.n;
   double2* F = p.F + (size_t)b * p.M * p.N;
   const int len = p.left ? p.n : p.m, inner = p.left ? p.m : p.n;
@@ -612,8 +619,8 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
   for (int a = threadIdx.x; a < len; a += blockDim.x) {
     double2 t = make_double2(0.0, 0.0);
     for (int k = 0; k < inner; ++k) {
-      if (p.left) cfma(t, expm2pi_fixed_f64(phase_fixed(p.ar, k, q)), f[(size_t)k * p.n + a]);
-      else cfma(t, f[(size_t)a * p.n + k], expm2pi_fixed_f64(phase_fixed(p.ac, k, q)));
+      if (p.left) cfma(t, expm2pi_fixed_f64(phase_fixed(ar, k, q)), f[(size_t)k * p.n + a]);
+      else cfma(t, f[(size_t)a * p.n + k], expm2pi_fixed_f64(phase_fixed(ac, k, q)));
     }
     T[a] = t;
   }
@@ -622,8 +629,8 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
   for (int o = threadIdx.x; o < outs; o += blockDim.x) {
     double2 t = make_double2(0.0, 0.0);
     for (int k = 0; k < len; ++k) {
-      if (p.left) cfma(t, T[k], expm2pi_fixed_f64(phase_fixed(p.ac, k, o)));
-      else cfma(t, expm2pi_fixed_f64(phase_fixed(p.ar, k, o)), T[k]);
+      if (p.left) cfma(t, T[k], expm2pi_fixed_f64(phase_fixed(ac, k, o)));
+      else cfma(t, expm2pi_fixed_f64(phase_fixed(ar, k, o)), T[k]);
     }
     F[p.left ? (size_t)q * p.N + o : (size_t)o * p.N + q] = make_double2(p.scale * t.x, p.scale * t.y);
   }
@@ -704,10 +711,10 @@ int make_digit_map(CUtensorMap* map, const DigitRows& d, int digits, int items, 
 }
 
 // The data operand has ND digits and its own rows for every item, the matrix
-// NE digits shared by the items; A is the data when DATA_A.
+// NE digits, shared by the items unless `own`; A is the data when DATA_A.
 template <bool DATA_A>
-int launch_gemm(const DigitRows& A, const DigitRows& B, int items, const Deal& deal, int S, longlong2* P,
-                long long item_stride, int ld, int* err, cudaStream_t s) {
+int launch_gemm(const DigitRows& A, const DigitRows& B, bool own, int items, const Deal& deal, int S,
+                longlong2* P, long long item_stride, int ld, int* err, cudaStream_t s) {
   constexpr int NA = DATA_A ? ND : NE, NB = DATA_A ? NE : ND;
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
@@ -718,15 +725,15 @@ int launch_gemm(const DigitRows& A, const DigitRows& B, int items, const Deal& d
   LGB_CUDA(attr);
   CUtensorMap a, b;
   int st;
-  if ((st = make_digit_map(&a, A, NA, DATA_A ? items : 1, BM, 1))) return st;
-  if ((st = make_digit_map(&b, B, NB, DATA_A ? 1 : items, BC, 2))) return st;
+  if ((st = make_digit_map(&a, A, NA, DATA_A || own ? items : 1, BM, 1))) return st;
+  if ((st = make_digit_map(&b, B, NB, !DATA_A || own ? items : 1, BC, 2))) return st;
   GemmParams p{};
   p.deal = deal;
   p.total = items * deal.tilesA * deal.tilesB * deal.chains;
   p.rowsB = B.L;
   p.ld = ld;
-  p.dA = DATA_A ? NA : 0;
-  p.dB = DATA_A ? 0 : NB;
+  p.dA = DATA_A || own ? NA : 0;
+  p.dB = !DATA_A || own ? NB : 0;
   p.S = S;
   p.P = P;
   p.item_stride = item_stride;
@@ -754,9 +761,9 @@ struct Layout {
 
 constexpr size_t CHUNK_BYTES = (size_t)512 << 20;
 
-Layout layout(int count, int m, int n, int M, int N, void* ws) {
+Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
   Layout t{};
-  t.left = sliced_left(m, n, M, N);
+  t.left = left;
   t.K1 = t.left ? m : n;
   t.K2 = t.left ? n : m;
   t.vecs1 = t.left ? n : m;
@@ -795,7 +802,6 @@ Layout layout(int count, int m, int n, int M, int N, void* ws) {
 
 }  // namespace
 
-// Product order: (E1 f) E2 as lentil, or E1 (f E2) when that needs fewer flops.
 bool sliced_left(int m, int n, int M, int N) {
   return (double)M * m * n + (double)M * n * N <= (double)m * n * N + (double)M * m * N;
 }
@@ -818,22 +824,23 @@ size_t sliced_matrix_entries(int len_in, int len_out, bool operand_b) {
   return NE * DigitRows{nullptr, len_out, round_up(len_in, BK), operand_b ? 1 : 0}.plane();
 }
 
-int launch_matrix_digits(const PhaseAxis& ax, int len_in, int len_out, bool operand_b, uint16_t* out,
-                         cudaStream_t s) {
+int launch_matrix_digits(const PhaseAxis& ax, const PhaseAxis* axes, int count, int len_in, int len_out,
+                         bool operand_b, uint16_t* out, cudaStream_t s) {
   const DigitRows d{out, len_out, round_up(len_in, BK), operand_b ? 1 : 0};
-  matrix_digits_kernel<<<dim3(cdiv(d.kp, 256), len_out), 128, 0, s>>>(ax, len_in, d);
+  matrix_digits_kernel<<<dim3(cdiv(d.kp, 256), len_out, count), 128, 0, s>>>(ax, axes, len_in, d);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }
 
-size_t sliced_dft2_workspace(int count, int m, int n, int M, int N) {
-  return layout(count, m, n, M, N, nullptr).bytes;
+size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left) {
+  return layout(count, m, n, M, N, left, nullptr).bytes;
 }
 
 int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
-  const Layout t = layout(q.count, q.m, q.n, q.M, q.N, ws);
-  const DigitRows e1{const_cast<uint16_t*>(q.e1), q.M, round_up(q.m, BK), 1};
-  const DigitRows e2{const_cast<uint16_t*>(q.e2), q.N, round_up(q.n, BK), t.left ? 0 : 1};
+  const Layout t = layout(q.count, q.m, q.n, q.M, q.N, q.left, ws);
+  const bool own = q.axes != nullptr;
+  DigitRows e1{const_cast<uint16_t*>(q.e1), q.M, round_up(q.m, BK), 1};
+  DigitRows e2{const_cast<uint16_t*>(q.e2), q.N, round_up(q.n, BK), t.left ? 0 : 1};
   const int S1 = unit_shift(t.K1), S2 = unit_shift(t.K2);
   int st;
   for (int b0 = 0; b0 < q.count; b0 += t.chunk) {
@@ -846,13 +853,13 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     else
       slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.flags);
     LGB_CUDA(cudaGetLastError());
-    if ((st = launch_gemm<true>(t.d1, t.left ? e1 : e2, items, t.deal1, S1, t.P, t.item_stride, t.ld1, t.err, s)))
+    if ((st = launch_gemm<true>(t.d1, t.left ? e1 : e2, own, items, t.deal1, S1, t.P, t.item_stride, t.ld1, t.err, s)))
       return st;
     slice_product_kernel<<<dim3(t.rows1, items), 256, 0, s>>>(
         PartialSums{t.P, t.item_stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2);
     LGB_CUDA(cudaGetLastError());
-    st = t.left ? launch_gemm<false>(e2, t.d2, items, t.deal2, S2, t.P, t.item_stride, t.ld2, t.err, s)
-                : launch_gemm<true>(t.d2, e1, items, t.deal2, S2, t.P, t.item_stride, t.ld2, t.err, s);
+    st = t.left ? launch_gemm<false>(e2, t.d2, own, items, t.deal2, S2, t.P, t.item_stride, t.ld2, t.err, s)
+                : launch_gemm<true>(t.d2, e1, own, items, t.deal2, S2, t.P, t.item_stride, t.ld2, t.err, s);
     if (st) return st;
     FinishParams p{};
     p.q = PartialSums{t.P, t.item_stride, t.ld2, q.M, q.N, t.deal2};
@@ -868,11 +875,17 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     p.n = q.n;
     p.ar = q.ar;
     p.ac = q.ac;
+    p.axes = own ? q.axes + b0 : nullptr;
+    p.cols = q.cols;
     p.scratch = t.P;
     p.flags = t.flags;
     p.err = t.err;
     finish_kernel<<<dim3(cdiv(q.N, 256), q.M, items), 256, 0, s>>>(p);
     LGB_CUDA(cudaGetLastError());
+    if (own) {
+      e1.base += (size_t)items * NE * e1.plane();
+      e2.base += (size_t)items * NE * e2.plane();
+    }
   }
   return LGB_OK;
 }

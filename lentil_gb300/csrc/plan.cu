@@ -62,7 +62,7 @@ static size_t carve_fp64(void* ws, int count, int m, int n, int M, int N, Dft2Fp
 static size_t carve_sliced(void* ws, int count, int m, int n, int M, int N, Dft2SlicedSpace* s) {
   Carve c(ws);
   Dft2SlicedSpace t;
-  t.ws = c.take<char>(sliced_dft2_workspace(count, m, n, M, N));
+  t.ws = c.take<char>(sliced_dft2_workspace(count, m, n, M, N, sliced_left(m, n, M, N)));
   t.e1 = c.take<uint16_t>(sliced_matrix_entries(m, M, true));
   t.e2 = c.take<uint16_t>(sliced_matrix_entries(n, N, !sliced_left(m, n, M, N)));
   if (s) *s = t;
@@ -151,9 +151,18 @@ int lgb::dft2_batch(const double2* fin, int count, int m, int n, double2* Fout, 
   if (precision == LGB_FP64 && !zs && sliced_applies(m, n, M, N)) {
     Dft2SlicedSpace w;
     carve_sliced(workspace, count, m, n, M, N, &w);
-    if ((st = launch_matrix_digits(ar, m, M, true, w.e1, s))) return st;
-    if ((st = launch_matrix_digits(ac, n, N, !sliced_left(m, n, M, N), w.e2, s))) return st;
-    return launch_sliced_dft2({count, m, n, M, N, w.e1, w.e2, ar, ac, scale, fin, Fout}, w.ws, s);
+    SlicedDft2 q{};
+    q.count = count;
+    q.m = m; q.n = n; q.M = M; q.N = N;
+    q.left = sliced_left(m, n, M, N);
+    q.e1 = w.e1; q.e2 = w.e2;
+    q.ar = ar; q.ac = ac;
+    q.scale = scale;
+    q.f = fin;
+    q.F = Fout;
+    if ((st = launch_matrix_digits(ar, nullptr, 1, m, M, true, w.e1, s))) return st;
+    if ((st = launch_matrix_digits(ac, nullptr, 1, n, N, !q.left, w.e2, s))) return st;
+    return launch_sliced_dft2(q, w.ws, s);
   }
   if (precision == LGB_FP64) {
     Dft2Fp64Space w;
@@ -323,6 +332,9 @@ struct lgb_psf_plan_s {
   int kernel_launches[LGB_PROFILE_SLOTS] = {0};
   // fp64
   double2 *E1 = nullptr, *E2 = nullptr, *f = nullptr, *T = nullptr, *F = nullptr;
+  bool sliced = false;             // FP64 on the tensor cores: digit matrices in place of E1, E2
+  uint16_t *d1 = nullptr, *d2 = nullptr;
+  void* sliced_ws = nullptr;       // one PSF's wavelengths
 };
 
 static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
@@ -353,10 +365,16 @@ static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
     }
   } else {
     const size_t Q = (size_t)B * L;
-    P->E1 = c.take<double2>((size_t)L * d.M * d.m);
-    P->E2 = c.take<double2>((size_t)L * d.n * d.N);
+    if (P->sliced) {
+      P->d1 = c.take<uint16_t>(L * sliced_matrix_entries(d.m, d.M, true));
+      P->d2 = c.take<uint16_t>(L * sliced_matrix_entries(d.n, d.N, false));
+      P->sliced_ws = c.take<char>(sliced_dft2_workspace(L, d.m, d.n, d.M, d.N, true));
+    } else {
+      P->E1 = c.take<double2>((size_t)L * d.M * d.m);
+      P->E2 = c.take<double2>((size_t)L * d.n * d.N);
+      P->T = c.take<double2>(Q * d.M * d.n);
+    }
     P->f = c.take<double2>(Q * d.m * d.n);
-    P->T = c.take<double2>(Q * d.M * d.n);
     P->F = c.take<double2>(Q * d.M * d.N);
   }
   return c.used;
@@ -410,6 +428,7 @@ static lgb_psf_plan_s* new_plan(const lgb_psf_desc& d) {
   P->d.wavelengths = P->d.alpha_r = P->d.alpha_c = P->d.shift_r = P->d.shift_c = nullptr;
   P->kp1 = round_up(d.m, 32);
   P->kp2 = round_up(d.n, 32);
+  P->sliced = d.precision == LGB_FP64 && sliced_applies(d.m, d.n, d.M, d.N);
   P->bytes = plan_carve(P, nullptr);
   return P;
 }
@@ -457,6 +476,9 @@ static int build_plan(lgb_psf_plan_s* P, cudaStream_t s, lgb_psf_plan* plan) {
     const bool bf16 = d.precision == LGB_SPLIT_BF16;
     st = launch_e1_block_split(P->axes, L, d.m, d.M, P->kp1, cdiv(d.M, 64) * 128, bf16, P->e1h, P->e1l, s);
     if (!st) st = launch_e2_block_split(P->axes + L, L, d.n, d.N, P->kp2, cdiv(d.N, 128) * 256, bf16, P->e2h, P->e2l, s);
+  } else if (P->sliced) {
+    st = launch_matrix_digits(PhaseAxis{}, P->axes, L, d.m, d.M, true, P->d1, s);
+    if (!st) st = launch_matrix_digits(PhaseAxis{}, P->axes + L, L, d.n, d.N, false, P->d2, s);
   } else {
     for (int l = 0; l < L && !st; ++l) {
       st = launch_dft_matrix_c128(axes[l], d.m, d.M, P->E1 + (size_t)l * d.M * d.m, true, s);
@@ -590,7 +612,7 @@ static int psf_execute_n(lgb_psf_plan P, int B, const int* lam_idx, int n_sel, c
       return st;
     return prof_end(P, LGB_PROFILE_OTHER, s, ev);
   }
-  // plain FP64
+  // FP64
   cudaEvent_t ev[2];
   if ((st = prof_begin(P, LGB_PROFILE_PHASOR, s, ev))) return st;
   if ((st = launch_phasor_batch_c128(amp, opd, d.H, d.W, d.r0, d.c0, d.m, d.n, P->two_over_lambda,
@@ -602,6 +624,21 @@ static int psf_execute_n(lgb_psf_plan P, int B, const int* lam_idx, int n_sel, c
   for (int b = 0; b < B; ++b) {
     const size_t q0 = (size_t)b * L;
     if ((st = prof_begin(P, LGB_PROFILE_MFT1, s, ev))) return st;
+    if (P->sliced) {                        // both products: profiled as the first
+      SlicedDft2 q{};
+      q.count = L;
+      q.m = d.m; q.n = d.n; q.M = d.M; q.N = d.N;
+      q.left = true;
+      q.e1 = P->d1; q.e2 = P->d2;
+      q.axes = P->axes;
+      q.cols = L;
+      q.scale = 1.0;
+      q.f = P->f + q0 * sf;
+      q.F = P->F + q0 * sF;
+      if ((st = launch_sliced_dft2(q, P->sliced_ws, s))) return st;
+      if ((st = prof_end(P, LGB_PROFILE_MFT1, s, ev))) return st;
+      continue;
+    }
     if ((st = launch_zgemm(d.M, d.n, d.m, P->E1, d.m, sE1, P->f + q0 * sf, d.n, sf, P->T + q0 * sT,
                            d.n, sT, L, 1.0, s)))
       return st;
