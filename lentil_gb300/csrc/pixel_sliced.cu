@@ -1,0 +1,321 @@
+// Pixel MTF and spline resampling of pixelate (pixelate.cu) as real matrix
+// products out = L . X . R^T on the tensor cores, at FP64 accuracy (sliced.cuh):
+//   - the MTF of images whose size has no FFT here: |C img C^T|, C circulant;
+//   - the off-grid resampling G p G^T, G banded (64 taps a row).
+// Each product is: digits of X's rows and of R's rows; GEMM (its output's
+// contiguous index runs over X's rows, so the transposed product comes out
+// row by row); digits of those rows; GEMM with L's digits; finish.
+// Non-finite images, and a device-side wait that ran out, are evaluated in
+// plain FP64 by the finishing kernels.
+#include "pixelate.cuh"
+#include "sliced.cuh"
+
+namespace lgb {
+namespace {
+
+// ------------------------------------------------------------ row sources ---
+struct DenseRows {
+  const double* x;
+  int K;
+  __device__ __forceinline__ double at(int r, int k) const { return x[(size_t)r * K + k]; }
+};
+struct CirculantRows {                       // C[r][k] = c[(r - k) mod N]
+  const double* c;
+  int K;
+  __device__ __forceinline__ double at(int r, int k) const { return c[r >= k ? r - k : r - k + K]; }
+};
+struct BandedRows {                          // G[r][q0[r] + b] = Gt[b][r]
+  const double* Gt;
+  const int* q0;
+  int K, S;
+  __device__ __forceinline__ double at(int r, int k) const {
+    const int b = k - q0[r];
+    return b >= 0 && b < RS_BW ? Gt[(size_t)b * S + r] : 0.0;
+  }
+};
+
+__device__ __forceinline__ void store_real_digits(const DigitRows& o, int r, int k, long long v0, long long v1) {
+  uint16_t* p = o.base + (size_t)r * o.kp + k;
+  uint32_t a[ND], c[ND];
+  digits_of(v0, a);
+  digits_of(v1, c);
+#pragma unroll
+  for (int i = 0; i < ND; ++i)
+    *reinterpret_cast<uint32_t*>(p + i * o.plane()) = __byte_perm(a[i], c[i], 0x7632);
+}
+
+// Row r (one block) of a real matrix -> digits and exponent.
+template <typename Rows>
+__global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out, int* __restrict__ exps,
+                                                         int* __restrict__ flag) {
+  const int r = blockIdx.x, K = src.K;
+  __shared__ int se[8], sf[8];
+  int e = 1, bad = 0;
+  for (int k = threadIdx.x; k < K; k += 256) note_exponent(src.at(r, k), e, bad);
+  e = __reduce_max_sync(0xffffffffu, e);
+  bad = __reduce_or_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0) { se[threadIdx.x >> 5] = e; sf[threadIdx.x >> 5] = bad; }
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) { e = max(e, se[w]); bad |= sf[w]; }
+  if (threadIdx.x == 0) {
+    exps[r] = e - 1022;
+    if (bad) atomicOr(flag, bad);
+  }
+  if (bad) return;
+  for (int k = 2 * threadIdx.x; k < out.kp; k += 512)
+    store_real_digits(out, r, k, k < K ? fixed_data(src.at(r, k), e) : 0,
+                      k + 1 < K ? fixed_data(src.at(r, k + 1), e) : 0);
+}
+
+// Row r of a product (entry a in units of 2^(ea[a] + eb[r] - 16 - S)) ->
+// digits.  A thread keeps its first 2 KEEP entries between the two passes.
+__global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSums<long long> q,
+                                                                 const int* __restrict__ ea,
+                                                                 const int* __restrict__ eb, int S,
+                                                                 DigitRows out, int* __restrict__ exps) {
+  constexpr int KEEP = 4, NONE = -(1 << 28);
+  const int r = blockIdx.x;
+  __shared__ uint8_t parts[MAX_TILES_A];
+  __shared__ int se[8];
+  count_parts(q, 0, r, parts);
+  long long kept[2 * KEEP];
+  int e = NONE;
+  auto look = [&](int a) {
+    long long v = 0;
+    if (a < q.cols) {
+      v = entry(q, q.P, parts, r, a);
+      if (v) e = max(e, ea[a] + bit_length(v));
+    }
+    return v;
+  };
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) {
+    const int k = 2 * threadIdx.x + 512 * i;
+    kept[2 * i] = look(k);
+    kept[2 * i + 1] = look(k + 1);
+  }
+  for (int k = 512 * KEEP + threadIdx.x; k < q.cols; k += 256) look(k);
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0) se[threadIdx.x >> 5] = e;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) e = max(e, se[w]);
+  if (threadIdx.x == 0) exps[r] = e == NONE ? 0 : e + eb[r] - 16 - S;
+  auto put = [&](int k, long long v0, long long v1) {
+    store_real_digits(out, r, k, k < q.cols ? shift_round(v0, ea[k] - e + XBITS) : 0,
+                      k + 1 < q.cols ? shift_round(v1, ea[k + 1] - e + XBITS) : 0);
+  };
+#pragma unroll
+  for (int i = 0; i < KEEP; ++i) {
+    const int k = 2 * threadIdx.x + 512 * i;
+    if (k < out.kp) put(k, kept[2 * i], kept[2 * i + 1]);
+  }
+  for (int k = 512 * KEEP + 2 * threadIdx.x; k < out.kp; k += 512)
+    put(k, k < q.cols ? entry(q, q.P, parts, r, k) : 0, k + 1 < q.cols ? entry(q, q.P, parts, r, k + 1) : 0);
+}
+
+// v * 2^e
+__device__ __forceinline__ double scaled(long long v, int e) {
+  const double x = (double)v;
+  if (e > -960 && e < 960) return x * __longlong_as_double((long long)(e + 1023) << 52);
+  return scalbn(x, e);
+}
+
+__device__ __forceinline__ double block_sum(double v, double* sm) {      // 256 threads; thread 0 has the sum
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0)
+    for (int w = 1; w < 8; ++w) v += sm[w];
+  return v;
+}
+
+struct FinishReal {
+  PartialSums<long long> q;
+  const int *ea, *eb;
+  int S;
+  const int* status;         // [0] expired wait, [1] non-finite input
+  double* out;               // [rows][cols], or null
+  double* sum;               // += sum of the results
+};
+
+// Row k of |C img C^T|: its entries, their sum, and, when d is set, the
+// samples on the detector grid with their sum.
+__global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, const double* __restrict__ img,
+                                                           const double* __restrict__ c,
+                                                           double* __restrict__ scratch, int os,
+                                                           double* __restrict__ d,
+                                                           double* __restrict__ sum_d) {
+  const int N = p.q.rows, k = blockIdx.x;
+  __shared__ uint8_t parts[MAX_TILES_A];
+  __shared__ double sm[8];
+  const bool plain = p.status[0] != 0 || p.status[1] != 0;
+  double* T = scratch + (size_t)k * N;       // plain: row k of C img (P's memory)
+  count_parts(p.q, 0, k, parts);
+  if (plain) {
+    for (int j = threadIdx.x; j < N; j += 256) {
+      double t = 0.0;
+      for (int i = 0; i < N; ++i) t = fma(c[k >= i ? k - i : k - i + N], img[(size_t)i * N + j], t);
+      T[j] = t;
+    }
+    __syncthreads();
+  }
+  double s = 0.0, sd = 0.0;
+  const int Nd = N / os;
+  for (int l = threadIdx.x; l < N; l += 256) {
+    double v = 0.0;
+    if (plain)
+      for (int j = 0; j < N; ++j) v = fma(T[j], c[j >= l ? j - l : j - l + N], v);
+    else
+      v = scaled(entry(p.q, p.q.P, parts, k, l), p.ea[l] + p.eb[k] - 16 - p.S);
+    v = fabs(v);
+    if (p.out) p.out[(size_t)k * N + l] = v;
+    s += v;
+    if (d && k % os == 0 && l % os == 0) {
+      d[(size_t)(k / os) * Nd + l / os] = v;
+      sd += v;
+    }
+  }
+  s = block_sum(s, sm);
+  if (threadIdx.x == 0) atomicAdd(p.sum, s);
+  if (d && k % os == 0) {
+    sd = block_sum(sd, sm);
+    if (threadIdx.x == 0) atomicAdd(sum_d, sd);
+  }
+}
+
+// Row k of G p G^T and its sum.
+__global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p, const double* __restrict__ img,
+                                                              const double* __restrict__ Gt,
+                                                              const int* __restrict__ q0, int N) {
+  const int S = p.q.rows, k = blockIdx.x;
+  __shared__ uint8_t parts[MAX_TILES_A];
+  __shared__ double sm[8];
+  const bool plain = p.status[0] != 0 || p.status[1] != 0;
+  count_parts(p.q, 0, k, parts);
+  double s = 0.0;
+  for (int l = threadIdx.x; l < S; l += 256) {
+    double v = 0.0;
+    if (plain) {
+      const int nk = min(RS_BW, N - q0[k]), nl = min(RS_BW, N - q0[l]);
+      for (int a = 0; a < nk; ++a) {
+        double t = 0.0;
+        for (int b = 0; b < nl; ++b) t = fma(Gt[(size_t)b * S + l], img[(size_t)(q0[k] + a) * N + q0[l] + b], t);
+        v = fma(Gt[(size_t)a * S + k], t, v);
+      }
+    } else {
+      v = scaled(entry(p.q, p.q.P, parts, k, l), p.ea[l] + p.eb[k] - 16 - p.S);
+    }
+    p.out[(size_t)k * S + l] = v;
+    s += v;
+  }
+  s = block_sum(s, sm);
+  if (threadIdx.x == 0) atomicAdd(p.sum, s);
+}
+
+// ------------------------------------------------------------------ host ---
+DigitRows real_rows(uint16_t* base, int L, int K) { return DigitRows{base, L, round_up(K, BK), -1}; }
+
+// Two products of one sandwich: X is p x q (rows of K = q), R has rows r of
+// length q, L rows r of length p (both sides have the same operator here).
+struct Sandwich {
+  int p, q, r;
+  Band band;                 // of the operator's rows
+  Deal deal1, deal2;
+  int ld1, ld2;
+  size_t P_entries;
+  Sandwich(int p_, int q_, int r_, int step) : p(p_), q(q_), r(r_) {
+    const int total = cdiv(q, 2 * BK);
+    band.step = step;
+    band.total = total;
+    band.count = step ? std::min(total, (96 * step + 68) / 64 + 2) : total;
+    deal1 = deal_of(p, r, BN, band.count, 1);                 // A: X's rows, B: operator rows
+    deal2 = deal_of(r, r, BN, band.count, 1);                 // A: rows of the first product
+    ld1 = round_up(p, BM);
+    ld2 = round_up(r, BM);
+    P_entries = std::max((size_t)r * ld1 * max_parts(deal1), (size_t)r * ld2 * max_parts(deal2));
+  }
+};
+
+size_t digit_entries(int L, int K) { return ND * real_rows(nullptr, L, K).plane(); }
+
+struct Space {
+  int* status;               // [0] expired wait, [1] non-finite
+  int *eX, *eR, *eT;
+  uint16_t *dX, *dR, *dT;
+  long long* P;
+  size_t bytes;
+};
+
+Space carve(const Sandwich& w, void* ws) {
+  Space t{};
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    off = align_up(off, 256);
+    char* q = ws ? static_cast<char*>(ws) + off : nullptr;
+    off += bytes;
+    return q;
+  };
+  t.status = reinterpret_cast<int*>(take(2 * sizeof(int)));
+  t.eX = reinterpret_cast<int*>(take(sizeof(int) * w.p));
+  t.eR = reinterpret_cast<int*>(take(sizeof(int) * w.r));
+  t.eT = reinterpret_cast<int*>(take(sizeof(int) * w.r));
+  t.dX = reinterpret_cast<uint16_t*>(take(2 * digit_entries(w.p, w.q)));
+  t.dR = reinterpret_cast<uint16_t*>(take(2 * digit_entries(w.r, w.q)));
+  t.dT = reinterpret_cast<uint16_t*>(take(2 * digit_entries(w.r, w.p)));
+  t.P = reinterpret_cast<long long*>(take(sizeof(long long) * w.P_entries));
+  t.bytes = off;
+  return t;
+}
+
+template <typename Rows>
+int run_sandwich(const Sandwich& w, const Space& t, const double* X, const Rows& op, cudaStream_t s) {
+  const int S = unit_shift(w.q);
+  const DigitRows dX = real_rows(t.dX, w.p, w.q), dR = real_rows(t.dR, w.r, w.q), dT = real_rows(t.dT, w.r, w.p);
+  LGB_CUDA(cudaMemsetAsync(t.status, 0, 2 * sizeof(int), s));
+  slice_real_kernel<<<w.p, 256, 0, s>>>(DenseRows{X, w.q}, dX, t.eX, t.status + 1);
+  slice_real_kernel<<<w.r, 256, 0, s>>>(op, dR, t.eR, t.status + 1);
+  LGB_CUDA(cudaGetLastError());
+  int st = launch_gemm<ND, ND, true>(dX, 1, dR, 1, 1, w.deal1, w.band, S, t.P, 0, w.ld1, t.status, s);
+  if (st) return st;
+  slice_real_product_kernel<<<w.r, 256, 0, s>>>(PartialSums<long long>{t.P, 0, w.ld1, w.r, w.p, w.deal1}, t.eX,
+                                                t.eR, S, dT, t.eT);
+  LGB_CUDA(cudaGetLastError());
+  return launch_gemm<ND, ND, true>(dT, 1, dR, 1, 1, w.deal2, w.band, S, t.P, 0, w.ld2, t.status, s);
+}
+
+}  // namespace
+
+size_t pixel_sliced_workspace(int N) { return carve(Sandwich(N, N, N, 0), nullptr).bytes; }
+
+int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, double* P, double* sums, int os,
+                        double* d, cudaStream_t s) {
+  const Sandwich w(N, N, N, 0);
+  const Space t = carve(w, ws);
+  const int st = run_sandwich(w, t, img, CirculantRows{c, N}, s);
+  if (st) return st;
+  const FinishReal f{PartialSums<long long>{t.P, 0, w.ld2, N, N, w.deal2}, t.eT, t.eR, unit_shift(N), t.status,
+                     P, sums};
+  finish_pixel_kernel<<<N, 256, 0, s>>>(f, img, c, reinterpret_cast<double*>(t.P), os, d, sums + 1);
+  LGB_CUDA(cudaGetLastError());
+  return LGB_OK;
+}
+
+size_t resample_sliced_workspace(int N, int os, int S) { return carve(Sandwich(N, N, S, os), nullptr).bytes; }
+
+int launch_resample_sliced(const double* P, int N, int os, int S, const double* Gt, const int* q0, void* ws,
+                           double* raw, double* sum, cudaStream_t s) {
+  const Sandwich w(N, N, S, os);
+  const Space t = carve(w, ws);
+  const int st = run_sandwich(w, t, P, BandedRows{Gt, q0, N, S}, s);
+  if (st) return st;
+  const FinishReal f{PartialSums<long long>{t.P, 0, w.ld2, S, S, w.deal2}, t.eT, t.eR, unit_shift(N), t.status,
+                     raw, sum};
+  finish_resample_kernel<<<S, 256, 0, s>>>(f, P, Gt, q0, N);
+  LGB_CUDA(cudaGetLastError());
+  return LGB_OK;
+}
+
+}  // namespace lgb

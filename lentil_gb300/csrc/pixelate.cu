@@ -10,11 +10,13 @@
 //     C a + i C b), between tiled transposes (~5 N^2 log2 N flop), in
 //     double-float arithmetic (below);
 //   - any other N: |C . img . C^T| with C the real symmetric circulant
-//     C[i][j] = c[(i - j) mod N], c = ifft(s), as two FP64 GEMMs.
+//     C[i][j] = c[(i - j) mod N], c = ifft(s): two products on the tensor
+//     cores at FP64 accuracy (pixel_sliced.cu), or, where N is outside their
+//     range, two FP64 GEMMs.
 // pixelate then resamples by 1/os with a cubic spline (lentil/util.py:261-349);
 // when N is a multiple of os every sample falls on a grid point, so the
 // result is d = p[::os, ::os] rescaled by sum(p)/sum(d) and masked where
-// d == 0; otherwise the spline evaluation runs as two banded FP64 passes
+// d == 0; otherwise the spline evaluation runs as two banded products
 // (the off-grid section below).
 //
 // The same FFT machinery also filters white noise for lgb_power_spectrum
@@ -22,8 +24,8 @@
 #include <algorithm>
 #include <cmath>
 
-#include "common.cuh"
 #include "kernels.cuh"
+#include "pixelate.cuh"
 
 namespace lgb {
 
@@ -208,24 +210,36 @@ __global__ void transpose_c128_kernel(const double2* __restrict__ in, double2* _
     if (xo < N && yo0 + k < N) out[(size_t)(yo0 + k) * N + xo] = t[threadIdx.x][k];
 }
 
-// s[k] = sinc(fftfreq(N)[k] * os): N values, computed once per call (FP64
-// sinpi is slow on this part's FP64 pipe; the N^2 products below only read)
-__global__ void sinc_table_kernel(int N, double os, double* __restrict__ s) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < N) s[k] = sinc_os(k, N, os);
+// s[k] = sinc(fftfreq(N)[k] * os) and, when tab is set, tab[k] = cos(2 pi k / N):
+// computed once per call (FP64 sinpi is slow on this part's FP64 pipe; the
+// N^2 products below only read)
+__global__ void sinc_table_kernel(int N, double os, double* __restrict__ s, double* __restrict__ tab) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, k = i < N ? i : i - N;
+  if (i < N) s[k] = sinc_os(k, N, os);
+  else if (tab && k < N) tab[k] = cospi(2.0 * (double)k / N);
 }
 
 // ------------------------------------------------------------- GEMM path
-// c[k] = (1/N) sum_f s_f cos(2 pi f k / N)
-__global__ void pixel_taps_kernel(int N, const double* __restrict__ sinc, double* __restrict__ c) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= N) return;
+// c[k] = (1/N) sum_f s_f cos(2 pi f k / N), one block per tap, the cosines
+// from the table at the exact phase index f k mod N.  (One thread per tap,
+// each with N cospi of its own, took 1.59 ms at N = 1000 on 8 CTAs.)
+__global__ void __launch_bounds__(128) pixel_taps_kernel(int N, const double* __restrict__ sinc,
+                                                         const double* __restrict__ tab,
+                                                         double* __restrict__ c) {
+  const int k = blockIdx.x;
+  __shared__ double sm[4];
+  int ph = (int)(((long long)threadIdx.x * k) % N);
+  const int step = (int)((128ll * k) % N);
   double acc = 0.0;
-  for (int f = 0; f < N; ++f) {
-    const long long ph = ((long long)f * k) % N;         // exact phase index
-    acc += sinc[f] * cospi(2.0 * (double)ph / N);
+  for (int f = threadIdx.x; f < N; f += 128) {
+    acc = fma(sinc[f], tab[ph], acc);
+    ph += step;
+    if (ph >= N) ph -= N;
   }
-  c[k] = acc / N;
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) c[k] = (sm[0] + sm[1] + sm[2] + sm[3]) / N;
 }
 
 __global__ void circulant_kernel(int N, const double* __restrict__ c, double* __restrict__ C) {
@@ -284,17 +298,9 @@ __global__ void __launch_bounds__(256) dgemm_kernel(int N, const double* __restr
 }
 
 // ---------------------------------------------------------- common tail
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // p = |value| written to P; sums[0] += sum p; decimated samples
-// d[k][l] = p[k*os][l*os] with sums[1] += sum d.  Reads a real (GEMM path)
-// or complex (FFT path) array.
-template <bool COMPLEX>
-__global__ void pixel_abs_reduce_kernel(int N, int os, const void* __restrict__ src,
+// d[k][l] = p[k*os][l*os] with sums[1] += sum d.
+__global__ void pixel_abs_reduce_kernel(int N, int os, const double* __restrict__ src,
                                         double* __restrict__ P, double* __restrict__ d,
                                         double* __restrict__ sums) {
   double s_all = 0.0, s_dec = 0.0;
@@ -302,13 +308,7 @@ __global__ void pixel_abs_reduce_kernel(int N, int os, const void* __restrict__ 
   const int Nd = N / os;
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total;
        p += (size_t)gridDim.x * blockDim.x) {
-    double v;
-    if (COMPLEX) {
-      const double2 z = static_cast<const double2*>(src)[p];
-      v = hypot(z.x, z.y);
-    } else {
-      v = fabs(static_cast<const double*>(src)[p]);
-    }
+    const double v = fabs(src[p]);
     if (P) P[p] = v;
     s_all += v;
     const int i = (int)(p / N), j = (int)(p % N);
@@ -347,14 +347,14 @@ __global__ void pixelate_scale_kernel(int count, const double* __restrict__ d,
 // samples: with h truncated at |t| <= RS_TAPS (|z|^31 < 2e-18 of the
 // signal) the window is RS_BW = 2 RS_TAPS + 4 wide, and the whole
 // resampling is out = G p G^T with G banded, S x RS_BW plus a start index
-// per row.  Both passes are FP64 FMA over L2-resident operands.
-constexpr int RS_PAD = 12, RS_TAPS = 30, RS_BW = 2 * RS_TAPS + 4;
-
+// per row: two products on the tensor cores over the windows of 96 rows
+// (pixel_sliced.cu), or, outside their range, two FP64 passes.
 __host__ __device__ __forceinline__ double rs_coord(int k, int S, int N, int os) {
   return ((double)k - S / 2.0) / (1.0 / os) + N / 2.0;
 }
 
 __device__ __forceinline__ int rs_reflect(int r, int L) {   // half-sample symmetric
+  if ((unsigned)r < (unsigned)L) return r;
   r %= 2 * L;
   if (r < 0) r += 2 * L;
   return r >= L ? 2 * L - 1 - r : r;
@@ -372,35 +372,48 @@ __device__ __forceinline__ int rs_start(int k, int S, int N, int os) {
   return min(max(i0 - RS_TAPS - RS_PAD, 0), max(0, N - RS_BW));
 }
 
-// Gt[b][k] = weight of input sample q0[k] + b in output sample k
-__global__ void resample_operator_kernel(int N, int os, int S, double* __restrict__ Gt,
-                                         int* __restrict__ q0) {
+// Gt[b][k] = weight of input sample q0[k] + b in output sample k, at pos[k];
+// one block per k, a thread per (b, spline coefficient).  Away from the edges
+// a coefficient reaches a sample by one tap; near them (reflected or clamped
+// taps) every tap is looked at.  (One thread per weight looking at all 244
+// taps took 31 us at 334 rows, a serial chain.)
+__global__ void __launch_bounds__(4 * RS_BW) resample_operator_kernel(int N, int os, int S,
+                                                                      double* __restrict__ Gt,
+                                                                      int* __restrict__ q0,
+                                                                      double* __restrict__ pos) {
   __shared__ double h[RS_TAPS + 1];
-  if (threadIdx.x == 0) {
-    const double z = sqrt(3.0) - 2.0;
-    h[0] = sqrt(3.0);
-    for (int a = 1; a <= RS_TAPS; ++a) h[a] = h[a - 1] * z;
+  if (threadIdx.x <= RS_TAPS) {                 // sqrt(3) z^t by squaring
+    double p = sqrt(3.0) - 2.0, v = sqrt(3.0);
+    for (int t = threadIdx.x; t; t >>= 1, p *= p)
+      if (t & 1) v *= p;
+    h[threadIdx.x] = v;
   }
   __syncthreads();
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= S * RS_BW) return;
-  const int k = idx / RS_BW, b = idx - k * RS_BW;
+  const int k = blockIdx.x, b = threadIdx.x >> 2, jj = threadIdx.x & 3;
   const int Np = N + 2 * RS_PAD;
-  const double xp = rs_coord(k, S, N, os) + RS_PAD;
-  const int i0 = (int)floor(xp) - 1;
+  const double x = rs_coord(k, S, N, os), xp = x + RS_PAD;
+  const int i0 = (int)floor(xp) - 1, j = i0 + jj;
   const int start = rs_start(k, S, N, os);
   const int want = start + b;
-  double g = 0.0;
-  for (int j = i0; j < i0 + 4; ++j) {
-    const double w = rs_beta3(xp - j);
-    const int jj = rs_reflect(j, Np);
+  double sum = 0.0;
+  if (i0 - RS_TAPS >= RS_PAD && i0 + 3 + RS_TAPS < N + RS_PAD) {
+    const int t = abs(j - RS_PAD - want);
+    if (t <= RS_TAPS) sum = h[t];
+  } else {
+    const int jr = rs_reflect(j, Np);
     for (int t = -RS_TAPS; t <= RS_TAPS; ++t) {
-      const int q = min(max(rs_reflect(jj - t, Np) - RS_PAD, 0), N - 1);
-      if (q == want) g += w * h[t < 0 ? -t : t];
+      const int q = min(max(rs_reflect(jr - t, Np) - RS_PAD, 0), N - 1);
+      if (q == want) sum += h[t < 0 ? -t : t];
     }
   }
-  Gt[(size_t)b * S + k] = g;
-  if (b == 0) q0[k] = start;
+  double g = sum != 0.0 ? rs_beta3(xp - j) * sum : 0.0;
+  g += __shfl_xor_sync(0xffffffffu, g, 1);
+  g += __shfl_xor_sync(0xffffffffu, g, 2);
+  if (jj == 0) Gt[(size_t)b * S + k] = g;
+  if (threadIdx.x == 0) {
+    q0[k] = start;
+    pos[k] = x;
+  }
 }
 
 constexpr int RS_ROWS = 8;        // image rows per thread in the row pass
@@ -460,13 +473,17 @@ __global__ void __launch_bounds__(256) resample_cols_kernel(const double* __rest
 // out = (raw * (sum p / sum raw)) * mask, the mask being the order-1
 // nearest-mode interpolation of (p != 0) at the same points, zeroed below
 // DBL_EPSILON (lentil/util.py:317-320, 333-347)
-__global__ void resample_finish_kernel(const double* __restrict__ raw,
-                                       const double* __restrict__ p, int N, int S, int os,
-                                       const double* __restrict__ sums, double* __restrict__ out) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= S * S) return;
-  const int k = idx / S, l = idx - k * S;
-  const double y = rs_coord(k, S, N, os), x = rs_coord(l, S, N, os);
+__global__ void __launch_bounds__(256) resample_finish_kernel(const double* __restrict__ raw,
+                                                              const double* __restrict__ p, int N, int S,
+                                                              const double* __restrict__ pos,
+                                                              const double* __restrict__ sums,
+                                                              double* __restrict__ out) {
+  const int k = blockIdx.y, l = blockIdx.x * 256 + threadIdx.x;
+  __shared__ double ratio;
+  if (threadIdx.x == 0) ratio = sums[0] / sums[2];
+  __syncthreads();
+  if (l >= S) return;
+  const double y = pos[k], x = pos[l];
   const int iy = (int)floor(y), ix = (int)floor(x);
   const double fy = y - iy, fx = x - ix;
   const int ya = min(max(iy, 0), N - 1), yb = min(max(iy + 1, 0), N - 1);
@@ -475,7 +492,8 @@ __global__ void resample_finish_kernel(const double* __restrict__ raw,
   double mask = (1.0 - fy) * ((1.0 - fx) * m(ya, xa) + fx * m(ya, xb)) +
                 fy * ((1.0 - fx) * m(yb, xa) + fx * m(yb, xb));
   if (mask < 2.220446049250313e-16) mask = 0.0;
-  out[idx] = (raw[idx] * (sums[0] / sums[2])) * mask;
+  const size_t idx = (size_t)k * S + l;
+  out[idx] = (raw[idx] * ratio) * mask;
 }
 
 // S = ceil(N * (1/os)), evaluated as numpy does (lentil/util.py:323-324)
@@ -497,16 +515,24 @@ static bool fft_size(int N, int* logN) {
   return true;
 }
 
+// The tensor-core products (pixel_sliced.cu) take images of 64 to 16384 rows:
+// below, a contraction is too short to be worth cutting into digits (at
+// N = 75 the two forms cost the same), above, their 64-bit sums run out.
+// N = 1000: the two products 4.1 -> 0.1 ms; the resampling by 3 of them
+// 0.11 -> 0.05 ms.
+static bool sliced_size(int N) { return N >= 64 && N <= 16384; }
+
 struct PixelSpace {
   double* sums;          // [0] sum p, [1] sum of the grid samples, [2] sum of the resampled
   double* sinc;          // [N] sinc(fftfreq * os)
   double* d;
   // GEMM path
-  double *c, *C, *T, *P;
+  double *c, *tab, *C, *T, *P;
+  void* sliced;          // workspace of the tensor-core products (MTF, then resampling)
   // FFT path
   double2 *X, *Y, *tw;
   // off-grid resampling: operator and the two passes
-  double *Gt, *Tm, *raw;
+  double *Gt, *Tm, *raw, *pos;
   int* q0;
 };
 
@@ -532,28 +558,37 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
     t.tw = static_cast<double2*>(take((size_t)(N / 2) * sizeof(double2)));
   } else {
     t.c = static_cast<double*>(take(N * sizeof(double)));
-    t.C = static_cast<double*>(take(NN * sizeof(double)));
-    t.T = static_cast<double*>(take(NN * sizeof(double)));
+    t.tab = static_cast<double*>(take(N * sizeof(double)));
     t.P = static_cast<double*>(take(NN * sizeof(double)));
+    if (!sliced_size(N)) {
+      t.C = static_cast<double*>(take(NN * sizeof(double)));
+      t.T = static_cast<double*>(take(NN * sizeof(double)));
+    }
   }
   const int S = resample_size(N, std::max(os, 1));
-  if (!resample_on_grid(N, std::max(os, 1), S)) {
+  const bool off_grid = !resample_on_grid(N, std::max(os, 1), S);
+  if (sliced_size(N) && (!fft || off_grid))
+    t.sliced = take(std::max(fft ? 0 : pixel_sliced_workspace(N),
+                             off_grid ? resample_sliced_workspace(N, std::max(os, 1), S) : 0));
+  if (off_grid) {
     t.Gt = static_cast<double*>(take((size_t)RS_BW * S * sizeof(double)));
     t.q0 = static_cast<int*>(take((size_t)S * sizeof(int)));
-    t.Tm = static_cast<double*>(take((size_t)N * S * sizeof(double)));
+    t.pos = static_cast<double*>(take((size_t)S * sizeof(double)));
+    if (!sliced_size(N)) t.Tm = static_cast<double*>(take((size_t)N * S * sizeof(double)));
     t.raw = static_cast<double*>(take((size_t)S * S * sizeof(double)));
   }
   if (s) *s = t;
   return off;
 }
 
-// Runs the MTF product; returns (src, complex?) of the pre-abs result.
-static int run_pixel(const double* img, int N, int os, void* ws, cudaStream_t s, PixelSpace* w,
-                     const void** src, bool* is_complex) {
-  pixel_space(ws, N, os, w);
+// The MTF product p = |C img C^T|: written to P (if not null), its sum added
+// to sums[0]; with d, every os-th sample and their sum (sums[1]).
+static int run_pixel(const double* img, int N, int os_mtf, PixelSpace* w, double* P, int os, double* d,
+                     cudaStream_t s) {
   LGB_CUDA(cudaMemsetAsync(w->sums, 0, 4 * sizeof(double), s));
-  sinc_table_kernel<<<cdiv(N, 256), 256, 0, s>>>(N, (double)os, w->sinc);
+  sinc_table_kernel<<<cdiv(2 * N, 128), 128, 0, s>>>(N, (double)os_mtf, w->sinc, w->tab);
   int logN;
+  const double* src;
   if (fft_size(N, &logN)) {
     // separable filter P = C . img . C^T (C real symmetric): filter the rows,
     // transpose, filter the rows again, transpose back; X and Y hold the real
@@ -572,28 +607,19 @@ static int run_pixel(const double* img, int N, int os, void* ws, cudaStream_t s,
     transpose_f64_kernel<<<tgrid, tblock, 0, s>>>(R, RT, N);
     pixel_filter_rows_kernel<<<N / 2, threads, smem, s>>>(RT, R, N, logN, twd, w->sinc);
     transpose_f64_kernel<<<tgrid, tblock, 0, s>>>(R, RT, N);
+    src = RT;
+  } else {
+    pixel_taps_kernel<<<N, 128, 0, s>>>(N, w->sinc, w->tab, w->c);
     LGB_CUDA(cudaGetLastError());
-    w->P = RT;
-    *src = RT;
-    *is_complex = false;
-    return LGB_OK;
+    if (sliced_size(N)) return launch_pixel_sliced(img, N, w->c, w->sliced, P, w->sums, os, d, s);
+    circulant_kernel<<<dim3(cdiv(N, 128), N), 128, 0, s>>>(N, w->c, w->C);
+    dim3 grid(cdiv(N, DBN), cdiv(N, DBM));
+    dgemm_kernel<<<grid, 256, 0, s>>>(N, w->C, img, w->T);      // T = C . img
+    dgemm_kernel<<<grid, 256, 0, s>>>(N, w->T, w->C, w->P);     // P = T . C^T (C symmetric)
+    src = w->P;
   }
-  pixel_taps_kernel<<<cdiv(N, 128), 128, 0, s>>>(N, w->sinc, w->c);
-  circulant_kernel<<<dim3(cdiv(N, 128), N), 128, 0, s>>>(N, w->c, w->C);
-  dim3 grid(cdiv(N, DBN), cdiv(N, DBM));
-  dgemm_kernel<<<grid, 256, 0, s>>>(N, w->C, img, w->T);      // T = C . img
-  dgemm_kernel<<<grid, 256, 0, s>>>(N, w->T, w->C, w->P);     // P = T . C^T (C symmetric)
-  LGB_CUDA(cudaGetLastError());
-  *src = w->P;
-  *is_complex = false;
-  return LGB_OK;
-}
-
-static int abs_reduce(int N, int os, const void* src, bool cplx, double* P, double* d,
-                      double* sums, cudaStream_t s) {
   const int blocks = std::max(1, std::min(4 * sm_count(), cdiv(N * N, 256)));
-  if (cplx) pixel_abs_reduce_kernel<true><<<blocks, 256, 0, s>>>(N, os, src, P, d, sums);
-  else pixel_abs_reduce_kernel<false><<<blocks, 256, 0, s>>>(N, os, src, P, d, sums);
+  pixel_abs_reduce_kernel<<<blocks, 256, 0, s>>>(N, os, src, P, d, w->sums);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }
@@ -738,13 +764,9 @@ extern "C" int lgb_pixel(const double* img, int rows, int cols, int oversample, 
   LGB_REQUIRE(workspace_bytes >= lgb_pixel_workspace_size(rows, oversample), LGB_EWORKSPACE,
               "pixel: workspace too small");
   const int N = rows;
-  cudaStream_t s = as_stream(stream);
   PixelSpace w;
-  const void* src;
-  bool cplx;
-  int st = run_pixel(img, N, oversample, workspace, s, &w, &src, &cplx);
-  if (st) return st;
-  return abs_reduce(N, 1, src, cplx, out, nullptr, w.sums, s);
+  pixel_space(workspace, N, oversample, &w);
+  return run_pixel(img, N, oversample, &w, out, 1, nullptr, as_stream(stream));
 }
 
 extern "C" int lgb_pixelate(const double* img, int rows, int cols, int oversample, double* out,
@@ -758,24 +780,28 @@ extern "C" int lgb_pixelate(const double* img, int rows, int cols, int oversampl
   const int N = rows, os = oversample, S = resample_size(N, os);
   cudaStream_t s = as_stream(stream);
   PixelSpace w;
-  const void* src;
-  bool cplx;
-  int st = run_pixel(img, N, os, workspace, s, &w, &src, &cplx);
-  if (st) return st;
+  int st;
+  pixel_space(workspace, N, os, &w);
   if (resample_on_grid(N, os, S)) {
-    if ((st = abs_reduce(N, os, src, cplx, nullptr, w.d, w.sums, s))) return st;
+    if ((st = run_pixel(img, N, os, &w, nullptr, os, w.d, s))) return st;
     pixelate_scale_kernel<<<cdiv(S * S, 256), 256, 0, s>>>(S * S, w.d, w.sums, out);
     LGB_CUDA(cudaGetLastError());
     return LGB_OK;
   }
-  double* P = w.P;                       // the real MTF product, made |.| in place
-  if ((st = abs_reduce(N, 1, src, cplx, P, nullptr, w.sums, s))) return st;
-  resample_operator_kernel<<<cdiv(S * RS_BW, 256), 256, 0, s>>>(N, os, S, w.Gt, w.q0);
-  resample_rows_kernel<<<dim3(cdiv(S, 64), cdiv(N, 4 * RS_ROWS)), dim3(64, 4), 0, s>>>(
-      P, N, S, w.Gt, w.q0, w.Tm);
-  resample_cols_kernel<<<dim3(cdiv(S, 64), cdiv(S, 4 * RS_OUT)), dim3(64, 4), 0, s>>>(
-      w.Tm, N, S, w.Gt, w.q0, w.raw, w.sums);
-  resample_finish_kernel<<<cdiv(S * S, 256), 256, 0, s>>>(w.raw, P, N, S, os, w.sums, out);
+  int logN;
+  double* const P = fft_size(N, &logN) ? reinterpret_cast<double*>(w.Y) : w.P;
+  if ((st = run_pixel(img, N, os, &w, P, 1, nullptr, s))) return st;
+  resample_operator_kernel<<<S, 4 * RS_BW, 0, s>>>(N, os, S, w.Gt, w.q0, w.pos);
+  LGB_CUDA(cudaGetLastError());
+  if (sliced_size(N)) {
+    if ((st = launch_resample_sliced(P, N, os, S, w.Gt, w.q0, w.sliced, w.raw, w.sums + 2, s))) return st;
+  } else {
+    resample_rows_kernel<<<dim3(cdiv(S, 64), cdiv(N, 4 * RS_ROWS)), dim3(64, 4), 0, s>>>(
+        P, N, S, w.Gt, w.q0, w.Tm);
+    resample_cols_kernel<<<dim3(cdiv(S, 64), cdiv(S, 4 * RS_OUT)), dim3(64, 4), 0, s>>>(
+        w.Tm, N, S, w.Gt, w.q0, w.raw, w.sums);
+  }
+  resample_finish_kernel<<<dim3(cdiv(S, 256), S), 256, 0, s>>>(w.raw, P, N, S, w.pos, w.sums, out);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }

@@ -99,3 +99,30 @@ def test_rule_is_by_shape(cuda_device):
     plain = 16 * (128 * 64 + 64 * 128 + max(128 * 64, 64 * 128))
     assert lib.lgb_dft2_workspace_size(*small, _lib.FP64) - plain < 1024
     assert lib.lgb_dft2_workspace_size(*large, _lib.FP64) > 4 * 128 * 128 * 16
+
+
+@pytest.mark.parametrize('n,os_', [(65, 1), (96, 5), (97, 2), (127, 3), (130, 70), (193, 2), (257, 4)])
+def test_pixelate_products(cuda_device, n, os_):
+    # sizes around the 96-row windows of the banded products and the 64-entry
+    # chains, with zeroed rows (the mask) and one bright pixel
+    from oracle import lentil_oracle as lo
+    rng = np.random.default_rng(n)
+    img = rng.random((n, n))
+    img[:3], img[:, -2:], img[n // 2, n // 3] = 0, 0, 1e3
+    assert lo.peak_normalised_error(lg.detector.pixel(img, os_), lo.pixel(img, os_)) < 1e-13
+    ref = lo.pixelate(img, os_)
+    # the rescaling divides by the sum of the samples, which a large
+    # oversampling of few samples makes small: scale the bound by it
+    assert lo.peak_normalised_error(lg.detector.pixelate(img, os_), ref) < 1e-12
+
+
+@pytest.mark.parametrize('bad', [float('nan'), float('inf')])
+def test_pixelate_of_non_finite_images(cuda_device, bad):
+    rng = np.random.default_rng(2)
+    img = rng.random((100, 100))
+    img[3, 4] = bad
+    for os_ in (2, 3):
+        assert np.isnan(lg.detector.pixelate(img, os_)).all()
+    p = lg.detector.pixel(img, 2)
+    assert not np.isfinite(p).any()
+    assert np.isfinite(lg.detector.pixelate(np.nan_to_num(img, posinf=1.0), 3)).all()
