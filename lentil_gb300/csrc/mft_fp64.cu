@@ -10,69 +10,79 @@
 
 namespace lgb {
 
-constexpr int ZBM = 64, ZBN = 64, ZBK = 16;
+// 16 x 16 outputs per CTA of 64 threads.  The FP64 pipe (two FMAs a clock per
+// SM) bounds every shape, and loads from shared memory cost little beside it,
+// so the tile is small enough that even a 64 x 64 output spreads over all SMs
+// (with K split): a 64^3 product took 134 us in 64 x 64 tiles, two CTAs of
+// work, and takes 4 us here; at 512^3 the two tiles cost the same.
+constexpr int ZBM = 16, ZBN = 16, ZBK = 8;
 
 // blockIdx.z = b * splits + split: problem b, K range [split * kchunk,
 // (split + 1) * kchunk); with splits > 1 each split writes its own partial
 // product (C offset by split * sP) for zgemm_reduce_kernel to sum in order.
-__global__ void __launch_bounds__(256) zgemm_kernel(int M, int N, int K,
-                                                    const double2* __restrict__ A, int lda, long long sA,
-                                                    const double2* __restrict__ B, int ldb, long long sB,
-                                                    double2* __restrict__ C, int ldc, long long sC,
-                                                    double alpha, int splits, int kchunk, long long sP) {
+__global__ void __launch_bounds__(64) zgemm_kernel(int M, int N, int K,
+                                                   const double2* __restrict__ A, int lda, long long sA,
+                                                   const double2* __restrict__ B, int ldb, long long sB,
+                                                   double2* __restrict__ C, int ldc, long long sC,
+                                                   double alpha, int splits, int kchunk, long long sP) {
   __shared__ double2 As[ZBK][ZBM];
   __shared__ double2 Bs[ZBK][ZBN];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, tid = threadIdx.x;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, tid = threadIdx.x;
   const int m0 = blockIdx.y * ZBM, n0 = blockIdx.x * ZBN;
   const int b = blockIdx.z / splits, split = blockIdx.z - b * splits;
   A += (size_t)b * sA;
   B += (size_t)b * sB;
   C += (size_t)b * sC + (size_t)split * sP;
   const int kbeg = split * kchunk, kend = min(K, kbeg + kchunk);
-  double cr[4][4], ci[4][4];
+  double cr[2][2] = {}, ci[2][2] = {};
+  double2 ra[2], rb[2];                          // the next K block, loaded ahead
+  const double2 zero = make_double2(0.0, 0.0);
+  auto load = [&](int k0) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) cr[i][j] = ci[i][j] = 0.0;
-
+    for (int t = 0; t < 2; ++t) {
+      const int e = tid + 64 * t;
+      const int gr = m0 + (e >> 3), gk = k0 + (e & 7);          // A: 16 rows x 8 k
+      ra[t] = (gr < M && gk < kend) ? A[(size_t)gr * lda + gk] : zero;
+      const int hk = k0 + (e >> 4), gc = n0 + (e & 15);         // B: 8 k x 16 columns
+      rb[t] = (hk < kend && gc < N) ? B[(size_t)hk * ldb + gc] : zero;
+    }
+  };
+  load(kbeg);
   for (int k0 = kbeg; k0 < kend; k0 += ZBK) {
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const int e = tid + 256 * t;
-      const int ar = e >> 4, ak = e & 15;          // A tile: 64 rows x 16 k
-      const int gr = m0 + ar, gk = k0 + ak;
-      As[ak][ar] = (gr < M && gk < kend) ? A[(size_t)gr * lda + gk] : make_double2(0.0, 0.0);
-      const int bk = e >> 6, bc = e & 63;          // B tile: 16 k x 64 cols
-      const int hk = k0 + bk, gc = n0 + bc;
-      Bs[bk][bc] = (hk < kend && gc < N) ? B[(size_t)hk * ldb + gc] : make_double2(0.0, 0.0);
+    for (int t = 0; t < 2; ++t) {
+      const int e = tid + 64 * t;
+      As[e & 7][e >> 3] = ra[t];
+      Bs[e >> 4][e & 15] = rb[t];
     }
     __syncthreads();
-#pragma unroll 4
+    if (k0 + ZBK < kend) load(k0 + ZBK);
+#pragma unroll
     for (int k = 0; k < ZBK; ++k) {
-      double2 a[4], b[4];
+      double2 a[2], bb[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[k][ty + 16 * i];
+      for (int i = 0; i < 2; ++i) a[i] = As[k][ty + 8 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[k][tx + 16 * j];
+      for (int j = 0; j < 2; ++j) bb[j] = Bs[k][tx + 8 * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          cr[i][j] = fma(a[i].x, b[j].x, cr[i][j]);
-          cr[i][j] = fma(-a[i].y, b[j].y, cr[i][j]);
-          ci[i][j] = fma(a[i].x, b[j].y, ci[i][j]);
-          ci[i][j] = fma(a[i].y, b[j].x, ci[i][j]);
+        for (int j = 0; j < 2; ++j) {
+          cr[i][j] = fma(a[i].x, bb[j].x, cr[i][j]);
+          cr[i][j] = fma(-a[i].y, bb[j].y, cr[i][j]);
+          ci[i][j] = fma(a[i].x, bb[j].y, ci[i][j]);
+          ci[i][j] = fma(a[i].y, bb[j].x, ci[i][j]);
         }
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = m0 + ty + 16 * i;
+  for (int i = 0; i < 2; ++i) {
+    const int r = m0 + ty + 8 * i;
     if (r >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = n0 + tx + 16 * j;
+    for (int j = 0; j < 2; ++j) {
+      const int c = n0 + tx + 8 * j;
       if (c < N) C[(size_t)r * ldc + c] = make_double2(alpha * cr[i][j], alpha * ci[i][j]);
     }
   }
@@ -115,11 +125,11 @@ static void keep_pool_memory() {
   done[dev] = true;
 }
 
-// A launch of fewer tiles than SMs would leave the FP64 pipes of most SMs
-// idle (a 256 x 256 output is 16 tiles; each SM retires about two FP64 FMAs
-// a clock), so such a launch splits K over up to 16 CTAs per tile, each
-// writing a partial product to scratch (the caller's, or stream-ordered pool
-// memory), and a second kernel sums the partials in split order.
+// A launch of fewer than two tiles per SM would leave FP64 pipes idle (a
+// 64 x 64 output is 16 tiles), so such a launch splits K over up to 16 CTAs
+// per tile, each writing a partial product to scratch (the caller's, or
+// stream-ordered pool memory), and a second kernel sums the partials in split
+// order.
 int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, const double2* B,
                  int ldb, long long sB, double2* C, int ldc, long long sC, int batch, double alpha,
                  cudaStream_t s, const ZgemmScratch* scratch) {
@@ -128,8 +138,8 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
   const long long tiles = (long long)cdiv(N, ZBN) * cdiv(M, ZBM) * batch;
   const int sms = sm_count();
   int splits = 1;
-  if (tiles < sms && K > 2 * ZBK)
-    splits = (int)std::min<long long>({(2LL * sms + tiles - 1) / tiles, (long long)cdiv(K, 2 * ZBK), 16LL,
+  if (tiles < 2LL * sms && K > ZBK)
+    splits = (int)std::min<long long>({(2LL * sms + tiles - 1) / tiles, (long long)cdiv(K, ZBK), 16LL,
                                        65535LL / batch});
   const long long sP = (long long)batch * M * N;          // one split's partials
   const size_t part_bytes = (size_t)sP * sizeof(double2);
@@ -141,7 +151,7 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
   }
   if (splits <= 1) {
     dim3 grid(cdiv(N, ZBN), cdiv(M, ZBM), batch);
-    zgemm_kernel<<<grid, 256, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, alpha, 1, K, 0);
+    zgemm_kernel<<<grid, 64, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, alpha, 1, K, 0);
     LGB_CUDA(cudaGetLastError());
     return LGB_OK;
   }
@@ -155,7 +165,7 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
     LGB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&P), (size_t)splits * part_bytes, s));
   }
   dim3 grid(cdiv(N, ZBN), cdiv(M, ZBM), batch * splits);
-  zgemm_kernel<<<grid, 256, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, P, N, (long long)M * N, 1.0,
+  zgemm_kernel<<<grid, 64, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, P, N, (long long)M * N, 1.0,
                                     splits, kchunk, sP);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) {

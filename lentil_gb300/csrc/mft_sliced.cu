@@ -306,14 +306,15 @@ bool sliced_left(int m, int n, int M, int N) {
   return (double)M * m * n + (double)M * n * N <= (double)m * n * N + (double)M * m * N;
 }
 
-// Where the sliced form is taken: both contractions at least 32 long, and work
-// beyond which its launches cost less than the plain GEMMs.  Device time of one
-// transform from a plan, plain -> sliced: 96^2 to 96^2 273 -> 35 us, 256^2
-// 278 -> 39, 512^2 2330 -> 90, 1019 x 941 to 1024^2 15800 -> 373, (32 x 1024)
-// to (1024 x 32) 399 -> 37.  Operands longer than 16384 would leave the 64-bit
-// sums too few fraction bits.
+// Where the sliced form is taken: where its five launches cost less than the
+// plain GEMMs' two to four.  Device time of one transform from a plan, plain
+// and sliced: 64^2 to 64^2 20 and 33 us, 96^2 29 and 33, 112^2 39 and 35, 256^2
+// 270 and 38, (8 x 8) to 512^2 27 and 38, (16 x 512) to 512^2 86 and 43,
+// (16 x 1024) to (16 x 1024) 171 and 39: the line is one of multiply-adds, just
+// below the crossing at about 102^2.
+// Operands longer than 16384 would leave the 64-bit sums too few fraction bits.
 bool sliced_applies(int m, int n, int M, int N) {
-  if (std::min(std::min(m, n), std::min(M, N)) < 32 || std::max(m, n) > 16384 ||
+  if (std::min(std::min(m, n), std::min(M, N)) < 8 || std::max(m, n) > 16384 ||
       std::max(M, N) > 32768)
     return false;
   const double left = (double)M * m * n + (double)M * n * N, right = (double)m * n * N + (double)M * m * N;

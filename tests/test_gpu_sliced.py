@@ -16,9 +16,9 @@ pytestmark = pytest.mark.gpu
 
 # (m, n, M, N): 48-column and 128-row tiles, 32-entry K stages, and their
 # neighbours; the smallest shapes of the rule; wide and tall transforms (the
-# right and the left product order)
+# right and the left product order); all of them take the sliced form
 SHAPES = [(96, 96, 96, 96), (97, 129, 95, 96), (127, 128, 129, 144), (160, 95, 47, 260),
-          (33, 257, 190, 193), (300, 64, 49, 128), (64, 300, 128, 49), (32, 400, 400, 33),
+          (33, 257, 190, 193), (300, 64, 97, 128), (64, 300, 128, 97), (32, 800, 400, 49), (8, 1040, 8, 260), (8, 9, 600, 600),
           (255, 256, 257, 241)]
 
 
@@ -89,6 +89,23 @@ def test_non_finite_input(cuda_device, bad, shape):
     assert torch.equal(a.isnan(), b.isnan())
     assert torch.equal(a[~a.isnan()], b[~b.isnan()])          # signed infinities
     assert torch.equal(F[0], F[2]) and bool(torch.view_as_real(F[0]).isfinite().all())
+
+
+@pytest.mark.parametrize('shape', [(1, 1, 1, 1), (5, 3, 2, 7), (15, 17, 16, 33), (64, 8, 9, 130),
+                                   (7, 300, 300, 7), (100, 90, 80, 70)])
+def test_plain_small_shapes(cuda_device, shape):
+    # the plain form's 16 x 16 tiles and 8-entry K blocks, split and whole,
+    # against the oracle; a batch splits K differently, to rounding
+    from oracle import lentil_oracle as lo
+    m, n, M, N = shape
+    alpha = (0.7 / max(m, M), 0.6 / max(n, N))
+    f = _field(m, n, 8)
+    ref = lo.dft2(f.cpu().numpy(), alpha, shape=(M, N), **ARGS)
+    for k in range(2):
+        F = lg.fourier.dft2(f, alpha, shape=(M, N), **ARGS)
+        assert lo.peak_normalised_error(F.cpu().numpy(), ref) < 1e-13
+    Fs = lg.fourier.dft2_batch(torch.stack([f] * 40), alpha, shape=(M, N), **ARGS)
+    assert float((Fs - F).abs().max()) <= 1e-14 * float(F.abs().max())
 
 
 def test_rule_is_by_shape(cuda_device):
