@@ -16,8 +16,9 @@
 //     for s <= 3: the FP32 accumulators hold it exactly, whatever order or
 //     rounding the tensor core uses.  Groups 4 to 6 share an accumulator
 //     (their rounding is below 2^-56 of the operands);
-//   - every 64 K entries the accumulators are drained into 64-bit integers in
-//     registers, in units of 2^-(16 + S): exact for groups 0-3.  Integer sums
+//   - every 64 K entries (256 for group 0, 128 for group 1: their sums have the
+//     room) the accumulators are drained into 64-bit integers in registers, in
+//     units of 2^-(16 + S): exact for groups 0-3.  Integer sums
 //     do not depend on their order, so dealing K out over CTAs gives the same
 //     bits.
 // What is left is the rounding of the operands, the products left out, and one
@@ -126,6 +127,17 @@ __device__ __forceinline__ Segment segment_at(const GemmParams& p, int pos, int 
   return s;
 }
 
+// Which chains of a segment (r = 0, 1, ...) start and end a sum of group g:
+// groups 0 and 1 run over four and two chains, at most 4 * 64 2^16 = 2 * 2 * 64
+// 2^16 = 2^24.  (Draining every group after every chain left the MMA waiting
+// 16 % of the time for the last ones of 20 drains in four chains; these are 15.)
+__device__ __forceinline__ bool starts(int g, int r) {
+  return g == 0 ? (r & 3) == 0 : g == 1 ? (r & 1) == 0 : true;
+}
+__device__ __forceinline__ bool drains(int g, int r, int count) {
+  return g == 0 ? (r & 3) == 3 || r == count - 1 : g == 1 ? (r & 1) == 1 || r == count - 1 : true;
+}
+
 // The digit products A_i B_j of one sum i + j, two k-steps each, added to the
 // accumulator d (started afresh when `fresh`).  The operand descriptors are
 // one 64-bit base each plus constants, and the warp stays converged around
@@ -229,21 +241,22 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     };
     constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                                ((uint32_t)(BM >> 4) << 24);       // FP32 += BF16 . BF16
-    int it = 0, c = 0;                         // stages and chains issued
+    int it = 0;                                // stages issued
+    int n[GROUPS] = {};                        // drains asked for, by group
     bool ok = true;
     for (int pos = begin; ok && pos < end;) {
       const Segment w = segment_at<REAL>(p, pos, end);
       pos += w.count;
       for (int st = 0; ok && st < 2 * w.count; ++st, ++it) {
-        const int s = it % STAGES;
-        const bool first = (st & 1) == 0, last = !first;
+        const int s = it % STAGES, r = st >> 1;
         if (!wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
         const uint64_t da = smem_desc_sw64(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw64(base + s * STAGE_BYTES + A_STAGE);
 #pragma unroll
         for (int g = GROUPS - 1; g >= 0; --g) {
-          // this accumulator's previous chain has been drained
-          if (first && !wait(acc_empty(g), (c & 1) ^ 1)) { ok = false; break; }
+          const bool first = (st & 1) == 0 && starts(g, r), last = (st & 1) == 1 && drains(g, r, w.count);
+          // this accumulator's previous sum has been drained
+          if (first && !wait(acc_empty(g), (n[g] & 1) ^ 1)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d = tmem + g * BN;
           if (g == 4) {                        // small products first
@@ -255,10 +268,12 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           if (g == 2) mma_sum<NA, NB, 2>(on, d, da, db, idesc, first);
           if (g == 1) mma_sum<NA, NB, 1>(on, d, da, db, idesc, first);
           if (g == 0) mma_sum<NA, NB, 0>(on, d, da, db, idesc, first);
-          if (last) mma_commit_cta(on, acc_full(g));
+          if (last) {
+            mma_commit_cta(on, acc_full(g));
+            ++n[g];
+          }
         }
         if (ok) mma_commit_cta(on, empty_bar(s));
-        if (last) ++c;
       }
     }
     mma_commit_cta(on, drain_bar);
@@ -269,7 +284,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     const uint32_t trow = tmem + ((uint32_t)(q4 * 32) << 16) + ch * RUN;
     const float unit4 = ldexpf(1.f, p.S);
     const int m1 = 1 << (p.S - BETA), m2 = 1 << (p.S - 2 * BETA), m3 = 1 << (p.S - 3 * BETA);
-    int c = 0;                                 // chains drained
+    int n[GROUPS] = {};                        // drains done, by group
     bool ok = true;
     for (int pos = begin; ok && pos < end;) {
       const Segment w = segment_at<REAL>(p, pos, end);
@@ -277,11 +292,13 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       long long acc[2 * RUN];                  // RUN real parts, RUN imaginary parts (or 2 RUN columns)
 #pragma unroll
       for (int j = 0; j < 2 * RUN; ++j) acc[j] = 0;
-      for (int k = 0; ok && k < w.count; ++k, ++c) {
+      for (int k = 0; ok && k < w.count; ++k) {
 #pragma unroll
         for (int g = GROUPS - 1; g >= 0; --g) {
-          ok = __all_sync(0xffffffffu, mbar_wait(acc_full(g), c & 1, p.err, p.wait_ns));
+          if (!drains(g, k, w.count)) continue;
+          ok = __all_sync(0xffffffffu, mbar_wait(acc_full(g), n[g] & 1, p.err, p.wait_ns));
           if (!ok) break;
+          ++n[g];
           tc_fence_after();
           uint32_t r[2 * RUN];
 #pragma unroll
