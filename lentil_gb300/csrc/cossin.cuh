@@ -1,0 +1,80 @@
+// cos and sin of a fixed-point phase, in fixed point.
+//
+// The DFT matrices need 53-bit cosines and sines of phases that are exact
+// 64-bit fractions of a cycle (phase_fixed, common.cuh).  Double-precision
+// sincospi holds this part's FP64 pipe (17 clocks a value per SM measured in the
+// phasor kernel); the integer pipes give the same in about two: the nearest of 512 points of the
+// circle from a table, and a rotation by the rest, |d| < 2^-7.3, with the
+// Taylor series of cos d and sin d in 64-bit fixed point, cut where the terms
+// fall below 2^-63.  The error is below 2^-60 (2.4 units of 2^-62 at most over
+// thousands of phases against 60-digit values).
+#pragma once
+
+#include <stdint.h>
+
+namespace lgb {
+
+// round(2^62 cos(2 pi i / 512)), i = 0 .. 128
+__device__ static const unsigned long long COS_TABLE[129] = {
+    0x4000000000000000, 0x3ffec42d3725b6af, 0x3ffb10c1099a1976, 0x3ff4e5dffdeeb93a,
+    0x3fec43c6f2dafbc7, 0x3fe12acb1ce35a81, 0x3fd39b5a0310742a, 0x3fc395f97ab61234,
+    0x3fb11b47a24a4b3c, 0x3f9c2bfadb4cf5a9, 0x3f84c8e1c33fa68f, 0x3f6af2e32bae8247,
+    0x3f4eaafe114a2d43, 0x3f2ff2499213350f, 0x3f0ec9f4e297526b, 0x3eeb33474240eec2,
+    0x3ec52f9feeb96056, 0x3e9cc076165e599c, 0x3e71e758c9cb118a, 0x3e44a5eeec75b370,
+    0x3e14fdf72461ae55, 0x3de2f147c8e784b2, 0x3dae81ced092c67a, 0x3d77b191be16e872,
+    0x3d3e82ad8c5bb4bb, 0x3d02f75699a2198c, 0x3cc511d891c223dd, 0x3c84d4965782fcd4,
+    0x3c424209ed0dc97f, 0x3bfd5cc45b7c5557, 0x3bb6276d998478c2, 0x3b6ca4c471413595,
+    0x3b20d79e651a8c51, 0x3ad2c2e793cd1586, 0x3a8269a29b927359, 0x3a2fcee87c6bb7ef,
+    0x39daf5e8798ee5e2, 0x3983e1e7f9f8b879, 0x392a96426823e9ed, 0x38cf166910e7363b,
+    0x387165e3017b61a4, 0x3811884ce4aa921b, 0x37af8158df2a533f, 0x374b54ce6b21a4bf,
+    0x36e5068a32dc7b22, 0x367c9a7deaae230a, 0x361214b02a03ff37, 0x35a5793c43aa215c,
+    0x3536cc521d434606, 0x34c6123605f5c386, 0x34534f408c4f03bb, 0x33de87de535f286c,
+    0x3367c08fe70e8168, 0x32eefde98fae8375, 0x3274449324c7f69f, 0x31f79947df2819d2,
+    0x317900d62a2e816a, 0x30f8801f745d7d69, 0x30761c17ff2edba4, 0x2ff1d9c6ae2ee132,
+    0x2f6bbe44d55f5dbc, 0x2ee3cebe06e4c257, 0x2e5a106fdfff2c87, 0x2dce88a9d5515d12,
+    0x2d413cccfe779921, 0x2cb2324be0f07ae2, 0x2c216eaa3a59bdb7, 0x2b8ef77cca031883,
+    0x2afad26919d93f45, 0x2a65052546ab2b98, 0x29cd9577c7cbd228, 0x293489373612716c,
+    0x2899e64a123bac30, 0x27fdb2a68aada89b, 0x275ff45240a17279, 0x26c0b1620cb3e570,
+    0x261feff9c2e069c2, 0x257db64bf5e7d3ef, 0x24da0a99ba25bd51, 0x2434f33267d6b163,
+    0x238e76735cd190d9, 0x22e69ac7bdb69141, 0x223d66a836964508, 0x2192e09abb131d39,
+    0x20e70f3245ffdb2d, 0x2039f90e987d6db3, 0x1f8ba4dbf89ab9fb, 0x1edc1952ef78d589,
+    0x1e2b5d3806f63b1e, 0x1d79775b86e38955, 0x1cc66e9931c45e17, 0x1c1249d8011ee6a0,
+    0x1b5d1009e15cc02b, 0x1aa6c82b6d3fc98b, 0x19ef7943a8ed8a2e, 0x19372a63bc93d72d,
+    0x187de2a6aea962d2, 0x17c3a9311dcce702, 0x17088530fa459eaf, 0x164c7ddd3f27c611,
+    0x158f9a75ab1fdcfe, 0x14d1e24278e76a25, 0x14135c9417660143, 0x135410c2e18151b1,
+    0x1294062ed59f05a9, 0x11d3443f4cdb3dd2, 0x1111d262b1f67761, 0x104fb80e37fdadff,
+    0x0f8cfcbd90af8d58, 0x0ec9a7f2a2a188af, 0x0e05c1353f27b17e, 0x0d415012d802284f,
+    0x0c7c5c1e34d3055b, 0x0bb6ecef285f98a4, 0x0af10a22459fe32a, 0x0a2abb58949f2ced,
+    0x0964083747309d11, 0x089cf8676d7abb56, 0x07d59395aa5cc38d, 0x070de171e7b0b53d,
+    0x0645e9af0a6d0af8, 0x057db402a6a90630, 0x04b54824b3867d73, 0x03ecadcf3f041bfe,
+    0x0323ecbe21bb027d, 0x025b0caeb28ab9a3, 0x0192155f7a3667e0, 0x00c90e8fe6f63c23,
+    0x0000000000000000,
+};
+
+// (cos, sin)(2 pi ph / 2^64) in units of 2^-62; table: COS_TABLE or a copy.
+__device__ __forceinline__ longlong2 cossin_q62(uint64_t ph, const unsigned long long* table) {
+  const uint32_t at = (uint32_t)((ph + (1ull << 54)) >> 55) & 511u;      // nearest table point
+  const int64_t r = (int64_t)(ph - ((uint64_t)at << 55));               // |r| <= 2^54
+  const uint64_t ar = (uint64_t)(r < 0 ? -r : r);
+  const uint64_t d = __umul64hi(ar << 8, 7244019458077122842ull);                      // |d|, Q68, < 2^60.7
+  const uint64_t d2 = __umul64hi(d << 1, d << 1);                        // d^2, Q74, < 2^59.4
+  const uint32_t y = (uint32_t)(d2 >> 28);                               // d^2, Q46
+  // 1 - cos d = d^2 (1/2 - d^2/24 + d^4/720)
+  const uint32_t w = 2863311531u - __umulhi(y, 5825u);         // 1/24 - d^2/720, Q36
+  const uint64_t a = __umul64hi(d2, (1ull << 61) - ((uint64_t)__umulhi(y, w) << 12));   // Q72, < 2^56.4
+  // sin d = d (1 - d^2 (1/6 - d^2/120))
+  const uint64_t q6 = 768614336404564650ull - ((uint64_t)__umulhi(y, 2290649225u) << 10); // Q62
+  const uint64_t u = __umul64hi(d2, q6);                                 // Q72, < 2^54.8
+  const uint64_t sd = (d << 2) - (__umul64hi(d, u << 8) >> 14);          // Q70, < 2^62.7
+  const int j = at & 127;
+  const uint64_t c = table[j], s = table[128 - j];
+  const int64_t ca = (int64_t)(__umul64hi(c, a << 6) >> 14), sa = (int64_t)(__umul64hi(s, a << 6) >> 14);
+  int64_t cs = (int64_t)(__umul64hi(c, sd) >> 6), ss = (int64_t)(__umul64hi(s, sd) >> 6);
+  if (r < 0) { cs = -cs; ss = -ss; }
+  int64_t x = (int64_t)c - ca - ss, yv = (int64_t)s - sa + cs;           // cos, sin of the first quadrant's angle
+  if (at & 128) { const int64_t t = x; x = -yv; yv = t; }
+  if (at & 256) { x = -x; yv = -yv; }
+  return make_longlong2(x, yv);
+}
+
+}  // namespace lgb

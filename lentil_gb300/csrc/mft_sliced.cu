@@ -10,23 +10,33 @@
 // A field with a NaN gives NaN everywhere (each output sums every entry); one
 // with infinities, or a device-side wait that ran out, makes `finish`
 // evaluate that transform in plain FP64 instead.
+#include "cossin.cuh"
 #include "sliced.cuh"
 
 namespace lgb {
 namespace {
 
+// x * 2^-62 as a 53-bit fraction, rounded
+__device__ __forceinline__ long long unit53(long long x) { return (x + 256) >> 9; }
+
 // DFT-matrix digits: vector j < L (output index) over the input index; matrix
-// z's axis is axes[z], or ax when there is one.
+// z's axis is axes[z], or ax when there is one.  Bound by the 24 or 36 bytes
+// written per entry (6.9 us for a 512^2 operand B); the cosines are integer
+// arithmetic because sincospi alone would take the FP64 pipe longer than that.
 __global__ void __launch_bounds__(128) matrix_digits_kernel(PhaseAxis ax, const PhaseAxis* __restrict__ axes,
                                                             int len_in, DigitRows out) {
+  __shared__ unsigned long long table[129];
+  for (int i = threadIdx.x; i < 129; i += 128) table[i] = COS_TABLE[i];
+  __syncthreads();
   if (axes) ax = axes[blockIdx.z];
   out.base += (size_t)blockIdx.z * NE * out.plane();
   const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x), j = blockIdx.y;
   if (k >= out.kp) return;
-  const double2 zero = make_double2(0.0, 0.0);
-  const double2 e0 = k < len_in ? expm2pi_fixed_f64(phase_fixed(ax, k, j)) : zero;
-  const double2 e1 = k + 1 < len_in ? expm2pi_fixed_f64(phase_fixed(ax, k + 1, j)) : zero;
-  store_digits<NE>(out, j, k, unit53(e0.x), unit53(e0.y), unit53(e1.x), unit53(e1.y));
+  const uint64_t ph = phase_fixed(ax, k, j);
+  longlong2 e0 = make_longlong2(0, 0), e1 = e0;                 // (cos, sin): E = cos - i sin
+  if (k < len_in) e0 = cossin_q62(ph, table);
+  if (k + 1 < len_in) e1 = cossin_q62(ph + phase_step_in(ax, j), table);
+  store_digits<NE>(out, j, k, unit53(e0.x), -unit53(e0.y), unit53(e1.x), -unit53(e1.y));
 }
 
 // f's rows (one block each) -> digits, vectors of n entries.
@@ -105,36 +115,47 @@ __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
 }
 
 // Row r of the first product (entry a in units of 2^(expA[a] - 16 - S)) ->
-// its digits as an operand of the second.  A thread keeps its first
-// 2 KEEP entries between the two passes (rows up to 2048 entries are read once).
+// its digits as an operand of the second.  The first 2 KEEP entries of a thread
+// stay in registers between the two passes (rows of up to 1024 are read once).
 __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<longlong2> q,
                                                             const int* __restrict__ expA, int S,
                                                             DigitRows out, int* __restrict__ exps) {
-  constexpr int KEEP = 4;
-  constexpr int NONE = -(1 << 28);
+  constexpr int KEEP = 2, NONE = -(1 << 28);
   const int r = blockIdx.x, b = blockIdx.y;
-  const longlong2* P = q.P + (size_t)b * q.item_stride;
+  const longlong2* P = q.P + (size_t)b * q.item_stride + (size_t)r * q.ld;
+  const size_t sP = (size_t)q.rows * q.ld;
   const int* ea = expA + (size_t)b * q.cols;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ int se[8];
   count_parts(q, b, r, parts);
-  longlong2 kept[2 * KEEP];
+  longlong2 kept[2 * KEEP], rest[2];
   int e = NONE;
-  auto look = [&](int a) {
-    longlong2 v = make_longlong2(0, 0);
-    if (a < q.cols) {
-      v = entry(q, P, parts, r, a);
-      if (v.x | v.y) e = max(e, ea[a] + max(bit_length(v.x), bit_length(v.y)));
-    }
-    return v;
+  auto note = [&](int a, longlong2 v) {
+    if (v.x | v.y) e = max(e, ea[a] + max(bit_length(v.x), bit_length(v.y)));
   };
+  {
+    size_t at[2 * KEEP];
+    int n[2 * KEEP];
 #pragma unroll
-  for (int i = 0; i < KEEP; ++i) {
-    const int k = 2 * threadIdx.x + 512 * i;
-    kept[2 * i] = look(k);
-    kept[2 * i + 1] = look(k + 1);
+    for (int i = 0; i < 2 * KEEP; ++i) {
+      const int k = 2 * threadIdx.x + 512 * (i >> 1) + (i & 1);
+      at[i] = k;
+      n[i] = k < q.cols ? parts[k / BM] : 0;
+    }
+    sum_parts<2 * KEEP>(P, sP, at, n, kept);
+#pragma unroll
+    for (int i = 0; i < 2 * KEEP; ++i) note((int)at[i], kept[i]);
   }
-  for (int k = 512 * KEEP + threadIdx.x; k < q.cols; k += 256) look(k);
+  auto fetch = [&](int k) {                     // entries k, k + 1 -> rest
+    const size_t at[2] = {(size_t)k, (size_t)k + 1};
+    const int n[2] = {k < q.cols ? parts[k / BM] : 0, k + 1 < q.cols ? parts[(k + 1) / BM] : 0};
+    sum_parts<2>(P, sP, at, n, rest);
+  };
+  for (int k = 512 * KEEP + 2 * threadIdx.x; k < q.cols; k += 512) {
+    fetch(k);
+    note(k, rest[0]);
+    note(k + 1, rest[1]);
+  }
   e = __reduce_max_sync(0xffffffffu, e);
   if ((threadIdx.x & 31) == 0) se[threadIdx.x >> 5] = e;
   __syncthreads();
@@ -153,8 +174,8 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<lo
     if (k < out.kp) put(k, kept[2 * i], kept[2 * i + 1]);
   }
   for (int k = 512 * KEEP + 2 * threadIdx.x; k < out.kp; k += 512) {
-    const longlong2 z = make_longlong2(0, 0);
-    put(k, k < q.cols ? entry(q, P, parts, r, k) : z, k + 1 < q.cols ? entry(q, P, parts, r, k + 1) : z);
+    fetch(k);
+    put(k, rest[0], rest[1]);
   }
 }
 
@@ -213,35 +234,44 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
   __syncthreads();
 }
 
-// F = P's entries, scaled.  Bound by reading P from L2 and by the
-// FP64 pipe's two conversions and two multiplications an entry.
+constexpr int FIN_ROWS = 4;                  // rows per finish block
+
+// F = P's entries, scaled.  Bound by reading P from L2 and writing F (32 bytes
+// an entry).  With conversions and both scalings on the FP64 pipe and a row per
+// block it took 24.7 us at 1024^2 (cold caches); put together from bits, the
+// parts of four rows in flight at once, 17.3.
 __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
-  const int u = blockIdx.y, b = blockIdx.z;
-  const int flag = p.flags[b];
+  const int b = blockIdx.z, flag = p.flags[b];
   if (*p.err != 0 || (flag & FLAG_INF && !(flag & FLAG_NAN))) {
     if (blockIdx.x != 0) return;
-    for (int q = u; q < (p.left ? p.M : p.N); q += p.M) plain_line(p, b, q);
+    for (int q = blockIdx.y; q < (p.left ? p.M : p.N); q += gridDim.y) plain_line(p, b, q);
     return;
   }
-  __shared__ uint8_t parts[MAX_TILES_A];
-  count_parts(p.q, b, u, parts);
-  const int v = blockIdx.x * 256 + threadIdx.x;
+  const int v = blockIdx.x * 256 + threadIdx.x, u0 = blockIdx.y * FIN_ROWS;
   if (v >= p.N) return;
-  double2* F = p.F + ((size_t)b * p.M + u) * p.N + v;
+  double2* F = p.F + ((size_t)b * p.M + u0) * p.N + v;
+  const int rows = min(FIN_ROWS, p.M - u0);
   if (flag) {
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
-    *F = make_double2(nan, nan);
+    for (int i = 0; i < rows; ++i) F[(size_t)i * p.N] = make_double2(nan, nan);
     return;
   }
-  const longlong2 z = entry(p.q, p.q.P + (size_t)b * p.q.item_stride, parts, u, v);
-  const int e = (p.left ? p.exps[(size_t)b * p.M + u] : p.exps[(size_t)b * p.N + v]) - 16 - p.S;
-  const double x = (double)z.x * p.scale, y = (double)z.y * p.scale;
-  if (e > -960 && e < 960) {                    // 2^e is a normal number
-    const double c = __longlong_as_double((long long)(e + 1023) << 52);
-    *F = make_double2(x * c, y * c);
-  } else {
-    *F = make_double2(scalbn(x, e), scalbn(y, e));
+  const int* exps = p.exps + (p.left ? (size_t)b * p.M + u0 : (size_t)b * p.N + v);
+  longlong2 z[FIN_ROWS];
+  size_t at[FIN_ROWS];
+  int n[FIN_ROWS], e[FIN_ROWS];
+#pragma unroll
+  for (int i = 0; i < FIN_ROWS; ++i) {
+    const int tile = (b * p.q.deal.tilesB + (u0 + i) / BC) * p.q.deal.tilesA + v / BM;
+    at[i] = (size_t)(u0 + i) * p.q.ld + v;
+    n[i] = i < rows ? p.q.deal.parts(tile) : 0;
+    e[i] = i < rows ? exps[p.left ? i : 0] - 16 - p.S : 0;
   }
+  sum_parts<FIN_ROWS>(p.q.P + (size_t)b * p.q.item_stride, (size_t)p.M * p.q.ld, at, n, z);
+#pragma unroll
+  for (int i = 0; i < FIN_ROWS; ++i)
+    if (i < rows)
+      F[(size_t)i * p.N] = make_double2(scaled(z[i].x, e[i], p.scale), scaled(z[i].y, e[i], p.scale));
 }
 
 // Shapes of one sliced transform and its workspace.
@@ -381,7 +411,7 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     p.scratch = t.P;
     p.flags = t.flags;
     p.err = t.err;
-    finish_kernel<<<dim3(cdiv(q.N, 256), q.M, items), 256, 0, s>>>(p);
+    finish_kernel<<<dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s>>>(p);
     LGB_CUDA(cudaGetLastError());
     if (own) {
       e1.base += (size_t)items * NE * e1.plane();

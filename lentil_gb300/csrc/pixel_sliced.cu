@@ -69,33 +69,47 @@ __global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out
 }
 
 // Row r of a product (entry a in units of 2^(ea[a] + eb[r] - 16 - S)) ->
-// digits.  A thread keeps its first 2 KEEP entries between the two passes.
+// digits.  The first 2 KEEP entries of a thread stay in registers between the
+// two passes.
 __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSums<long long> q,
                                                                  const int* __restrict__ ea,
                                                                  const int* __restrict__ eb, int S,
                                                                  DigitRows out, int* __restrict__ exps) {
   constexpr int KEEP = 4, NONE = -(1 << 28);
   const int r = blockIdx.x;
+  const long long* P = q.P + (size_t)r * q.ld;
+  const size_t sP = (size_t)q.rows * q.ld;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ int se[8];
   count_parts(q, 0, r, parts);
-  long long kept[2 * KEEP];
+  long long kept[2 * KEEP], rest[2];
   int e = NONE;
-  auto look = [&](int a) {
-    long long v = 0;
-    if (a < q.cols) {
-      v = entry(q, q.P, parts, r, a);
-      if (v) e = max(e, ea[a] + bit_length(v));
-    }
-    return v;
+  auto note = [&](int a, long long v) {
+    if (v) e = max(e, ea[a] + bit_length(v));
   };
+  {
+    size_t at[2 * KEEP];
+    int n[2 * KEEP];
 #pragma unroll
-  for (int i = 0; i < KEEP; ++i) {
-    const int k = 2 * threadIdx.x + 512 * i;
-    kept[2 * i] = look(k);
-    kept[2 * i + 1] = look(k + 1);
+    for (int i = 0; i < 2 * KEEP; ++i) {
+      const int k = 2 * threadIdx.x + 512 * (i >> 1) + (i & 1);
+      at[i] = k;
+      n[i] = k < q.cols ? parts[k / BM] : 0;
+    }
+    sum_parts<2 * KEEP>(P, sP, at, n, kept);
+#pragma unroll
+    for (int i = 0; i < 2 * KEEP; ++i) note((int)at[i], kept[i]);
   }
-  for (int k = 512 * KEEP + threadIdx.x; k < q.cols; k += 256) look(k);
+  auto fetch = [&](int k) {
+    const size_t at[2] = {(size_t)k, (size_t)k + 1};
+    const int n[2] = {k < q.cols ? parts[k / BM] : 0, k + 1 < q.cols ? parts[(k + 1) / BM] : 0};
+    sum_parts<2>(P, sP, at, n, rest);
+  };
+  for (int k = 512 * KEEP + 2 * threadIdx.x; k < q.cols; k += 512) {
+    fetch(k);
+    note(k, rest[0]);
+    note(k + 1, rest[1]);
+  }
   e = __reduce_max_sync(0xffffffffu, e);
   if ((threadIdx.x & 31) == 0) se[threadIdx.x >> 5] = e;
   __syncthreads();
@@ -111,15 +125,26 @@ __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSu
     const int k = 2 * threadIdx.x + 512 * i;
     if (k < out.kp) put(k, kept[2 * i], kept[2 * i + 1]);
   }
-  for (int k = 512 * KEEP + 2 * threadIdx.x; k < out.kp; k += 512)
-    put(k, k < q.cols ? entry(q, q.P, parts, r, k) : 0, k + 1 < q.cols ? entry(q, q.P, parts, r, k + 1) : 0);
+  for (int k = 512 * KEEP + 2 * threadIdx.x; k < out.kp; k += 512) {
+    fetch(k);
+    put(k, rest[0], rest[1]);
+  }
 }
 
-// v * 2^e
-__device__ __forceinline__ double scaled(long long v, int e) {
-  const double x = (double)v;
-  if (e > -960 && e < 960) return x * __longlong_as_double((long long)(e + 1023) << 52);
-  return scalbn(x, e);
+constexpr int FIN_COLS = 4;                  // columns per thread of a finish pass
+
+// Entries k of row r at l = l0 + 256 i of a product.
+__device__ __forceinline__ void row_entries(const PartialSums<long long>& q, const uint8_t* parts, int r, int l0,
+                                            long long (&v)[FIN_COLS]) {
+  size_t at[FIN_COLS];
+  int n[FIN_COLS];
+#pragma unroll
+  for (int i = 0; i < FIN_COLS; ++i) {
+    const int l = l0 + 256 * i;
+    at[i] = l;
+    n[i] = l < q.cols ? parts[l / BM] : 0;
+  }
+  sum_parts<FIN_COLS>(q.P + (size_t)r * q.ld, (size_t)q.rows * q.ld, at, n, v);
 }
 
 __device__ __forceinline__ double block_sum(double v, double* sm) {      // 256 threads; thread 0 has the sum
@@ -164,18 +189,25 @@ __global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, c
   }
   double s = 0.0, sd = 0.0;
   const int Nd = N / os;
-  for (int l = threadIdx.x; l < N; l += 256) {
-    double v = 0.0;
-    if (plain)
-      for (int j = 0; j < N; ++j) v = fma(T[j], c[j >= l ? j - l : j - l + N], v);
-    else
-      v = scaled(entry(p.q, p.q.P, parts, k, l), p.ea[l] + p.eb[k] - 16 - p.S);
-    v = fabs(v);
-    if (p.out) p.out[(size_t)k * N + l] = v;
-    s += v;
-    if (d && k % os == 0 && l % os == 0) {
-      d[(size_t)(k / os) * Nd + l / os] = v;
-      sd += v;
+  for (int l0 = threadIdx.x; l0 < N; l0 += 256 * FIN_COLS) {
+    long long z[FIN_COLS];
+    if (!plain) row_entries(p.q, parts, k, l0, z);
+#pragma unroll
+    for (int i = 0; i < FIN_COLS; ++i) {
+      const int l = l0 + 256 * i;
+      if (l >= N) break;
+      double v = 0.0;
+      if (plain)
+        for (int j = 0; j < N; ++j) v = fma(T[j], c[j >= l ? j - l : j - l + N], v);
+      else
+        v = scaled(z[i], p.ea[l] + p.eb[k] - 16 - p.S, 1.0);
+      v = fabs(v);
+      if (p.out) p.out[(size_t)k * N + l] = v;
+      s += v;
+      if (d && k % os == 0 && l % os == 0) {
+        d[(size_t)(k / os) * Nd + l / os] = v;
+        sd += v;
+      }
     }
   }
   s = block_sum(s, sm);
@@ -196,20 +228,28 @@ __global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p
   const bool plain = p.status[0] != 0 || p.status[1] != 0;
   count_parts(p.q, 0, k, parts);
   double s = 0.0;
-  for (int l = threadIdx.x; l < S; l += 256) {
-    double v = 0.0;
-    if (plain) {
-      const int nk = min(RS_BW, N - q0[k]), nl = min(RS_BW, N - q0[l]);
-      for (int a = 0; a < nk; ++a) {
-        double t = 0.0;
-        for (int b = 0; b < nl; ++b) t = fma(Gt[(size_t)b * S + l], img[(size_t)(q0[k] + a) * N + q0[l] + b], t);
-        v = fma(Gt[(size_t)a * S + k], t, v);
+  for (int l0 = threadIdx.x; l0 < S; l0 += 256 * FIN_COLS) {
+    long long z[FIN_COLS];
+    if (!plain) row_entries(p.q, parts, k, l0, z);
+#pragma unroll
+    for (int i = 0; i < FIN_COLS; ++i) {
+      const int l = l0 + 256 * i;
+      if (l >= S) break;
+      double v = 0.0;
+      if (plain) {
+        const int nk = min(RS_BW, N - q0[k]), nl = min(RS_BW, N - q0[l]);
+        for (int a = 0; a < nk; ++a) {
+          double t = 0.0;
+          for (int b = 0; b < nl; ++b)
+            t = fma(Gt[(size_t)b * S + l], img[(size_t)(q0[k] + a) * N + q0[l] + b], t);
+          v = fma(Gt[(size_t)a * S + k], t, v);
+        }
+      } else {
+        v = scaled(z[i], p.ea[l] + p.eb[k] - 16 - p.S, 1.0);
       }
-    } else {
-      v = scaled(entry(p.q, p.q.P, parts, k, l), p.ea[l] + p.eb[k] - 16 - p.S);
+      p.out[(size_t)k * S + l] = v;
+      s += v;
     }
-    p.out[(size_t)k * S + l] = v;
-    s += v;
   }
   s = block_sum(s, sm);
   if (threadIdx.x == 0) atomicAdd(p.sum, s);

@@ -347,22 +347,40 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---------------------------------------------------------------- digits ---
-// A small integer as a float without the conversion pipe (16 lanes a clock)
-__device__ __forceinline__ float small_float(int t) {
-  return __int_as_float(0x4B400000 + t) - 12582912.f;
-}
-
 // The N digits of X, |X| <= 2^(9 N - 1), as bf16 bits in the high half of a
-// word; digit i carries 2^(-9 i).
+// word; digit i carries 2^(-9 i).  A bias of 256 in every place turns the
+// signed digits into bit fields; a field under the exponent of 1.5 2^23 is a
+// float, and one FMA takes bias and offset off and scales (exactly): three
+// instructions a digit, none of them on the conversion or 64-bit paths.
 template <int N>
 __device__ __forceinline__ void digits_of(long long X, uint32_t (&d)[N]) {
+  constexpr unsigned long long ones = 0x0040201008040201ull;          // sum of 2^(9 i), i < 7
+  constexpr unsigned long long bias = 256ull * (ones & ((1ull << (BETA * (N - 1))) - 1));
+  const unsigned long long Y = (unsigned long long)X + bias;
 #pragma unroll
-  for (int i = N - 1; i > 0; --i) {
-    const int t = (int)((X + 256) & 511) - 256;
-    X = (X - t) >> BETA;
-    d[i] = __float_as_uint(small_float(t) * (1.f / (float)(1ull << (BETA * i))));
+  for (int i = 0; i < N; ++i) {
+    const int sh = BETA * (N - 1 - i);
+    const float s = 1.f / (float)(1ull << (BETA * i));
+    // the leading digit is signed: 512 more keep its field positive
+    const uint32_t u = (uint32_t)(Y >> sh) + (i == 0 ? 512u : 0u);
+    const float f = __uint_as_float((u & (i == 0 ? 1023u : 511u)) | 0x4B400000u);
+    d[i] = __float_as_uint(fmaf(f, s, -(12582912.f + (i == 0 ? 512.f : 256.f)) * s));
   }
-  d[0] = __float_as_uint(small_float((int)X));
+}
+
+// v * 2^e * scale as a double: v * 2^e, rounded to nearest even, is put together
+// from its bits (a conversion from 64-bit integers holds the FP64 pipe).
+__device__ __forceinline__ double scaled(long long v, int e, double scale) {
+  if (v == 0) return 0.0;
+  const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+  const int lz = __clzll((long long)m), exp = 63 - lz + e + 1023;
+  if (exp < 1 || exp > 2045) return scalbn((double)v * scale, e);
+  const unsigned long long t = m << lz;
+  const uint32_t low = (uint32_t)t & 0x7FFu;
+  unsigned long long q = t >> 11;                        // 53 bits, the leading one set
+  q += low > 0x400u || (low == 0x400u && (q & 1));
+  q += (unsigned long long)(exp - 1) << 52;              // a carry goes into the exponent
+  return scale * __longlong_as_double((long long)(q | ((unsigned long long)v & 0x8000000000000000ull)));
 }
 
 constexpr int XBITS = BETA * ND - 1;         // a data entry is |X| < 2^62 of its vector's scale
@@ -377,17 +395,6 @@ __device__ __forceinline__ long long fixed_data(double x, int e) {
   const int sh = e - E;                      // m < 2^53 has XBITS - 53 bits of room
   if (sh <= XBITS - 53) m <<= XBITS - 53 - sh;
   else m = sh > XBITS + 1 ? 0 : (m + (1ll << (sh - (XBITS - 53) - 1))) >> (sh - (XBITS - 53));
-  return (long long)u < 0 ? -m : m;
-}
-
-// E of modulus <= 1 as E * 2^53, rounded
-__device__ __forceinline__ long long unit53(double x) {
-  const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-  const int E = (int)(u >> 52) & 0x7FF;
-  if (E == 0) return 0;
-  long long m = (long long)((u & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 1;    // 54 bits
-  const int sh = 1023 - E;
-  if (sh > 0) m = sh > 55 ? 0 : (m + (1ll << (sh - 1))) >> sh;
   return (long long)u < 0 ? -m : m;
 }
 
@@ -453,17 +460,27 @@ __device__ __forceinline__ void count_parts(const PartialSums<V>& q, int item, i
   __syncthreads();
 }
 
-// Entry a of row r (P: the item's).
 __device__ __forceinline__ void add_to(long long& a, long long b) { a += b; }
 __device__ __forceinline__ void add_to(longlong2& a, longlong2 b) { a.x += b.x; a.y += b.y; }
-template <typename V>
-__device__ __forceinline__ V entry(const PartialSums<V>& q, const V* __restrict__ P,
-                                           const uint8_t* parts, int r, int a) {
-  const size_t sP = (size_t)q.rows * q.ld;
-  const V* p = P + (size_t)r * q.ld + a;
-  V v = *p;
-  for (int k = parts[a / BM] - 1; k > 0; --k) add_to(v, *(p += sP));
-  return v;
+
+// v[i] = the sum of n[i] parts (0: none) of the entry at offset at[i], i < COUNT.
+// The parts go in the outer loop, so that COUNT loads are in flight.
+template <int COUNT, typename V>
+__device__ __forceinline__ void sum_parts(const V* __restrict__ P, size_t part_stride, const size_t (&at)[COUNT],
+                                          const int (&n)[COUNT], V (&v)[COUNT]) {
+  int most = 0;
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) {
+    most = max(most, n[i]);
+    v[i] = V{};
+  }
+  for (int k = 0; k < most; ++k, P += part_stride) {
+    V w[COUNT];
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) w[i] = k < n[i] ? P[at[i]] : V{};
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) add_to(v[i], w[i]);
+  }
 }
 
 __device__ __forceinline__ int bit_length(long long v) { return 64 - __clzll(v < 0 ? -v : v); }
