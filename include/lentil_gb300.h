@@ -284,12 +284,17 @@ int lgb_zernike_eval(const double* rho, const double* theta, const double* mask,
  *   then q = dft2(Hc, alpha, shape=(m, n), shift=-offset, offset=-shift)
  *   (the adjoint MFT: E1^T conj(H) E2^T), and
  *   lgb_phasor_adjoint:    grad_opd[r0+i, c0+j] += -(4 pi / lambda) Im(q f)
+ *   lgb_phasor_adjoint_stack: the same for a stack q, f [count][m][n], written
+ *     to whole planes grad_opd [count][H][W] (zero outside the slice)
  * ---------------------------------------------------------------------- */
 int lgb_abs2(const lgb_c128* F, double* I, size_t count, lgb_stream stream);
 int lgb_intensity_adjoint(const lgb_c128* F, const double* grad_I, lgb_c128* Hc, size_t count,
                           lgb_stream stream);
 int lgb_phasor_adjoint(const lgb_c128* q, const lgb_c128* f, int m, int n, double wavelength,
                        double* grad_opd, int ld, int r0, int c0, lgb_stream stream);
+int lgb_phasor_adjoint_stack(const lgb_c128* q, const lgb_c128* f, int count, int m, int n,
+                             double wavelength, double* grad_opd, int H, int W, int r0, int c0,
+                             lgb_stream stream);
 /* Modal OPD for phase retrieval: out[p] = sum_k coeffs[k] basis[k][p] and
  * its adjoint out[k] = sum_p basis[k][p] grad[p] (deterministic sums), with
  * an FP32 basis [K][P] (K <= 1024): both stream the basis once.  Workspace of

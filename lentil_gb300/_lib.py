@@ -118,6 +118,8 @@ SIGNATURES = {
     'lgb_intensity_adjoint': (c_int, [c_void_p, c_void_p, c_void_p, c_size_t, c_void_p]),
     'lgb_phasor_adjoint': (c_int, [c_void_p, c_void_p, c_int, c_int, c_double, c_void_p, c_int,
                                    c_int, c_int, c_void_p]),
+    'lgb_phasor_adjoint_stack': (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_double,
+                                         c_void_p, c_int, c_int, c_int, c_int, c_void_p]),
     'lgb_psf_plan_create': (c_int, [ctypes.POINTER(PsfDesc), ctypes.POINTER(c_void_p), c_void_p]),
     'lgb_psf_plan_bytes': (c_size_t, [c_void_p]),
     'lgb_psf_plan_size': (c_size_t, [ctypes.POINTER(PsfDesc)]),

@@ -4,8 +4,9 @@ lentil, which has no gradients).
 ``mft_intensity(opd, amp, ...)`` is lentil's monochromatic PSF
 (``propagate_dft(Wavefront(lam) * Pupil(amp, opd)).intensity``, one field,
 no tilt) as a ``torch.autograd.Function`` of the OPD map.  Forward: phasor
-kernel, MFT (complex128 or split tensor-core), |F|^2.  Backward, with the
-field recomputed instead of stored: dL/dF* = dL/dI * F, the adjoint MFT
+kernel, MFT (complex128 or split tensor-core), |F|^2.  Backward, from the
+field f and its transform F kept by the forward pass (recomputing them was a
+third of an evaluation's transforms): dL/dF* = dL/dI * F, the adjoint MFT
 (a dft2 of its conjugate with offset and shift swapped and negated), and
 dL/dopd = (2 pi / lambda) 2 Im(g conj(f)) from the phasor-adjoint kernel.
 """
@@ -76,18 +77,17 @@ class MFTIntensity(torch.autograd.Function):
         opd = opd.detach().to(torch.float64).contiguous()
         opd = opd.unsqueeze(0) if single else opd
         amp = amp.detach().to(torch.float64).contiguous()
-        _, F = _forward_field(amp, opd, g)
+        f, F = _forward_field(amp, opd, g)
         I = torch.empty(F.shape, dtype=torch.float64, device=F.device)
         _lib.call('lgb_abs2', F.data_ptr(), I.data_ptr(), F.numel(), dv.stream_ptr())
-        ctx.save_for_backward(opd, amp)
+        ctx.save_for_backward(f, F)
         ctx.g, ctx.single = g, single
         return I[0] if single else I
 
     @staticmethod
     def backward(ctx, grad_I):
-        opd, amp = ctx.saved_tensors
+        f, F = ctx.saved_tensors
         g = ctx.g
-        f, F = _forward_field(amp, opd, g)                 # recomputed, not stored
         gI = grad_I.detach().to(torch.float64).contiguous().reshape(F.shape)
         Hc = torch.empty_like(F)
         _lib.call('lgb_intensity_adjoint', F.data_ptr(), gI.data_ptr(), Hc.data_ptr(), F.numel(),
@@ -96,10 +96,10 @@ class MFTIntensity(torch.autograd.Function):
         q = fourier.dft2_batch(Hc, g.alpha, shape=(m, n), shift=(-g.offset[0], -g.offset[1]),
                                offset=(-g.shift[0], -g.shift[1]), unitary=True,
                                precision=g.precision)
-        grad = torch.zeros_like(opd)
-        for k in range(opd.shape[0]):
-            _lib.call('lgb_phasor_adjoint', q[k].data_ptr(), f[k].data_ptr(), m, n, g.wavelength,
-                      grad[k].data_ptr(), g.plane[1], r0, c0, dv.stream_ptr())
+        H, W = g.plane
+        grad = torch.empty((f.shape[0], H, W), dtype=torch.float64, device=F.device)
+        _lib.call('lgb_phasor_adjoint_stack', q.data_ptr(), f.data_ptr(), f.shape[0], m, n,
+                  g.wavelength, grad.data_ptr(), H, W, r0, c0, dv.stream_ptr())
         return (grad[0] if ctx.single else grad), None, None
 
 

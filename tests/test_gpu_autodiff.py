@@ -284,3 +284,25 @@ def test_stacked_opd_matches_broadcast_add(cuda_device):
     (s1 * G).sum().backward()
     (s2 * G).sum().backward()
     assert float((c1.grad - c2.grad).abs().max()) <= 1e-6 * float(c2.grad.abs().max())
+
+
+def test_phasor_adjoint_stack(cuda_device):
+    # whole planes of a stack against the one-plane form: the same values
+    # inside the slice, zeros outside (which may hold anything before)
+    from lentil_gb300 import _lib
+    rng = np.random.default_rng(18)
+    s = torch.cuda.current_stream().cuda_stream
+    for K, H, W, r0, c0, m, n in ((3, 40, 130, 2, 5, 31, 120), (1, 7, 9, 0, 0, 7, 9), (2, 5, 4, 4, 3, 1, 1)):
+        mk = lambda: torch.as_tensor(rng.normal(size=(K, m, n)) + 1j * rng.normal(size=(K, m, n)), device='cuda')
+        q, f = mk(), mk()
+        out = torch.full((K, H, W), float('nan'), dtype=torch.float64, device='cuda')
+        _lib.call('lgb_phasor_adjoint_stack', q.data_ptr(), f.data_ptr(), K, m, n, 633e-9,
+                  out.data_ptr(), H, W, r0, c0, s)
+        ref = torch.zeros_like(out)
+        for k in range(K):
+            _lib.call('lgb_phasor_adjoint', q[k].data_ptr(), f[k].data_ptr(), m, n, 633e-9,
+                      ref[k].data_ptr(), W, r0, c0, s)
+        assert torch.equal(out, ref)
+    with pytest.raises(ValueError):
+        _lib.call('lgb_phasor_adjoint_stack', q.data_ptr(), f.data_ptr(), 2, 2, 2, 633e-9,
+                  out.data_ptr(), 5, 4, 4, 3, s)
