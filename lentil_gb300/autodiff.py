@@ -65,6 +65,13 @@ def _forward_field(amp, opd, g):
     return f, F
 
 
+def _f64(x):
+    """x as a contiguous float64 tensor (x itself when it is one)."""
+    if x.dtype == torch.float64 and x.is_contiguous():
+        return x
+    return x.to(torch.float64).contiguous()
+
+
 class MFTIntensity(torch.autograd.Function):
     """I = |dft2(amp exp(2 pi i opd / lambda))|^2, differentiable in opd.
     ``opd`` is one map [H, W] or a stack [K, H, W] sharing ``amp`` and the
@@ -74,9 +81,9 @@ class MFTIntensity(torch.autograd.Function):
     @staticmethod
     def forward(ctx, opd, amp, g):
         single = opd.dim() == 2
-        opd = opd.detach().to(torch.float64).contiguous()
+        opd = _f64(opd.detach())
         opd = opd.unsqueeze(0) if single else opd
-        amp = amp.detach().to(torch.float64).contiguous()
+        amp = _f64(amp.detach())
         f, F = _forward_field(amp, opd, g)
         I = torch.empty(F.shape, dtype=torch.float64, device=F.device)
         _lib.call('lgb_abs2', F.data_ptr(), I.data_ptr(), F.numel(), dv.stream_ptr())
@@ -88,7 +95,7 @@ class MFTIntensity(torch.autograd.Function):
     def backward(ctx, grad_I):
         f, F = ctx.saved_tensors
         g = ctx.g
-        gI = grad_I.detach().to(torch.float64).contiguous().reshape(F.shape)
+        gI = _f64(grad_I.detach()).reshape(F.shape)
         Hc = torch.empty_like(F)
         _lib.call('lgb_intensity_adjoint', F.data_ptr(), gI.data_ptr(), Hc.data_ptr(), F.numel(),
                   dv.stream_ptr())
@@ -116,7 +123,7 @@ class _BasisOPD(torch.autograd.Function):
     @staticmethod
     def forward(ctx, coeffs, basis32):
         K, P = int(basis32.shape[0]), int(basis32[0].numel())
-        c = coeffs.detach().to(torch.float64).contiguous()
+        c = _f64(coeffs.detach())
         out = torch.empty(tuple(basis32.shape[1:]), dtype=torch.float64, device=c.device)
         _lib.call('lgb_basis_expand', basis32.data_ptr(), c.data_ptr(), K, P, out.data_ptr(),
                   dv.stream_ptr())
@@ -127,7 +134,7 @@ class _BasisOPD(torch.autograd.Function):
     def backward(ctx, grad):
         (basis32,) = ctx.saved_tensors
         K, P = int(basis32.shape[0]), int(basis32[0].numel())
-        g = grad.detach().to(torch.float64).contiguous()
+        g = _f64(grad.detach())
         out = torch.empty(K, dtype=torch.float64, device=g.device)
         nb = _lib.load().lgb_basis_project_workspace_size(K)
         ws = dv.workspace(nb)
@@ -146,8 +153,8 @@ class _StackedOPD(torch.autograd.Function):
     def forward(ctx, coeffs, basis32, add):
         K, P = int(basis32.shape[0]), int(basis32[0].numel())
         n = int(add.shape[0])
-        c = coeffs.detach().to(torch.float64).contiguous()
-        d = add.detach().to(torch.float64).contiguous()
+        c = _f64(coeffs.detach())
+        d = _f64(add.detach())
         out = torch.empty((n,) + tuple(basis32.shape[1:]), dtype=torch.float64, device=c.device)
         _lib.call('lgb_basis_expand_stack', basis32.data_ptr(), c.data_ptr(), K, P, d.data_ptr(),
                   n, out.data_ptr(), dv.stream_ptr())
@@ -159,7 +166,7 @@ class _StackedOPD(torch.autograd.Function):
     def backward(ctx, grad):
         (basis32,) = ctx.saved_tensors
         K, P = int(basis32.shape[0]), int(basis32[0].numel())
-        g = grad.detach().to(torch.float64).contiguous()
+        g = _f64(grad.detach())
         out = torch.empty(K, dtype=torch.float64, device=g.device)
         nb = _lib.load().lgb_basis_project_workspace_size(K)
         ws = dv.workspace(nb)
@@ -177,8 +184,8 @@ class _SquaredError(torch.autograd.Function):
     def forward(ctx, I, T):
         if I.shape != T.shape:
             raise ValueError(f'images {tuple(I.shape)} and targets {tuple(T.shape)} differ')
-        I = I.to(torch.float64).contiguous()
-        T = T.to(torch.float64).contiguous()
+        I = _f64(I)
+        T = _f64(T)
         loss = torch.empty((), dtype=torch.float64, device=I.device)
         ws = torch.empty(_lib.load().lgb_sq_error_workspace_size(), dtype=torch.uint8,
                          device=I.device)
@@ -190,7 +197,7 @@ class _SquaredError(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         I, T = ctx.saved_tensors
-        g = grad.to(torch.float64).contiguous()
+        g = _f64(grad)
         dI = torch.empty_like(I)
         _lib.call('lgb_sq_error_grad', I.data_ptr(), T.data_ptr(), I.numel(), g.data_ptr(),
                   dI.data_ptr(), dv.stream_ptr())

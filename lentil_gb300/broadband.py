@@ -27,7 +27,7 @@ import torch
 from . import _device as dv
 from . import _lib
 from . import util
-from .propagate import plan_fields
+from .propagate import _dft_alpha, plan_fields
 
 
 class _ProbeField:
@@ -127,6 +127,8 @@ class PSFPlan:
         if nbytes == 0:                  # an invalid description: the size call recorded why
             _lib.check(_lib.EINVAL)
         self._home = torch.cuda.current_stream()
+        self._home_ptr = self._home.cuda_stream
+        self._split = d.precision != _lib.FP64
         self._foreign = set()
         self._mem = dv.workspace(nbytes)
         h = ctypes.c_void_p()
@@ -245,21 +247,21 @@ class PSFPlan:
         if out is None:
             out = torch.empty((count,) + self.image_shape, dtype=torch.float64, device=dev)
             accumulate = False
-        cur = torch.cuda.current_stream()
-        if cur != self._home and not torch.cuda.is_current_stream_capturing():
+        sp = dv.stream_ptr()
+        if sp != self._home_ptr and not torch.cuda.is_current_stream_capturing():
+            cur = torch.cuda.current_stream()
             cur.wait_event(self._built)
-            if cur.cuda_stream not in self._foreign:
+            if sp not in self._foreign:
                 self._mem.record_stream(cur)
-                self._foreign.add(cur.cuda_stream)
+                self._foreign.add(sp)
         if workspace is not None:
             if lam_idx is not None and (lam_idx.dtype != torch.int32 or not lam_idx.is_cuda):
                 raise TypeError('lam_idx must be an int32 CUDA tensor')
             _lib.call('lgb_psf_execute_ws', self._h, count, dv.ptr(lam_idx), n_sel,
                       amp.data_ptr(), opd.data_ptr(), weights.data_ptr(), out.data_ptr(),
-                      int(bool(accumulate)), workspace.data_ptr(), workspace.numel(),
-                      dv.stream_ptr())
+                      int(bool(accumulate)), workspace.data_ptr(), workspace.numel(), sp)
             if check:
-                _lib.call('lgb_dft2_status', workspace.data_ptr(), dv.stream_ptr())
+                _lib.call('lgb_dft2_status', workspace.data_ptr(), sp)
             return out
         if lam_idx is not None and (lam_idx.dtype != torch.int32 or not lam_idx.is_cuda):
             raise TypeError('lam_idx must be an int32 CUDA tensor')
@@ -277,9 +279,10 @@ class PSFPlan:
                           amp.data_ptr(), opd.data_ptr(), weights.data_ptr(), out.data_ptr(),
                           int(bool(accumulate)), cur.cuda_stream)
             if not capturing:
-                self._own_done = torch.cuda.Event()
+                if self._own_done is None:
+                    self._own_done = torch.cuda.Event()
                 self._own_done.record(cur)
-            if check:
+            if check and self._split:      # (complex128 executes have no status to wait for)
                 _lib.call('lgb_psf_plan_status', self._h, cur.cuda_stream)
         return out
 
@@ -441,10 +444,17 @@ def plan_geometry(plane_shape, s, tilts, dx, focal_length, ptype, wavelengths, d
     g.plane_shape, g.fslice, g.offset = tuple(plane_shape), (r0, c0, m, n), off
     g.alphas, g.shifts, g.keep = [], [], []
     window, shape_out = None, None
-    for i, lam in enumerate(np.atleast_1d(wavelengths)):
+    lams = np.atleast_1d(wavelengths)
+    for i, lam in enumerate(lams):
+        if i and not tilts:               # without tilts only the sampling depends on the wavelength
+            if window is not None:
+                g.keep.append(i)
+                g.alphas.append(tuple(float(a) for a in _dft_alpha(dx, du2, lam, focal_length, oversample)))
+                g.shifts.append(g.shifts[0])
+            continue
         probe = _ProbeWavefront(lam, dx, focal_length, plane_shape,
                                 [_ProbeField(off, (m, n), list(tilts))], ptype)
-        _, shape_out, _, jobs = plan_fields(probe, du, shape, prop_shape, oversample, mask)
+        _, shape_out, du2, jobs = plan_fields(probe, du, shape, prop_shape, oversample, mask)
         if not jobs:
             continue
         j = jobs[0]

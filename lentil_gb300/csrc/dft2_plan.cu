@@ -140,6 +140,7 @@ struct ExecSpace {
   float* maxabs;
   uint16_t *fh, *fl, *gh, *gl;
   double2* T;
+  ZgemmScratch partials;       // plain FP64: no pool allocations per execute
 };
 
 size_t exec_carve(const lgb_dft2_plan_s* P, int count, void* base, ExecSpace* s) {
@@ -155,6 +156,12 @@ size_t exec_carve(const lgb_dft2_plan_s* P, int count, void* base, ExecSpace* s)
   } else {
     t.T = c.take<double2>((size_t)count *
                           std::max((size_t)P->M * P->n, (size_t)P->m * P->N));
+    t.partials.bytes = P->left ? std::max(zgemm_partial_bytes(P->M, P->n, P->m, count),
+                                          zgemm_partial_bytes(P->M, P->N, P->n, count))
+                               : std::max(zgemm_partial_bytes(P->m, P->N, P->n, count),
+                                          zgemm_partial_bytes(P->M, P->N, P->m, count));
+    if (t.partials.bytes > ((size_t)256 << 20)) t.partials.bytes = 0;      // do not split
+    t.partials.ptr = c.take<char>(t.partials.bytes);
   }
   if (s) *s = t;
   return std::max<size_t>(c.used, 256);
@@ -387,12 +394,12 @@ extern "C" int lgb_dft2_plan_execute(lgb_dft2_plan P, const lgb_c128* f, int cou
     const long long sf = (long long)m * n, sF = (long long)M * N;
     if (P->left) {
       const long long sT = (long long)M * n;
-      if ((st = launch_zgemm(M, n, m, P->E1, m, 0, fin, n, sf, w.T, n, sT, count, 1.0, s))) return st;
-      return launch_zgemm(M, N, n, w.T, n, sT, P->E2, N, 0, Fout, N, sF, count, P->scale, s);
+      if ((st = launch_zgemm(M, n, m, P->E1, m, 0, fin, n, sf, w.T, n, sT, count, 1.0, s, &w.partials))) return st;
+      return launch_zgemm(M, N, n, w.T, n, sT, P->E2, N, 0, Fout, N, sF, count, P->scale, s, &w.partials);
     }
     const long long sT = (long long)m * N;
-    if ((st = launch_zgemm(m, N, n, fin, n, sf, P->E2, N, 0, w.T, N, sT, count, 1.0, s))) return st;
-    return launch_zgemm(M, N, m, P->E1, m, 0, w.T, N, sT, Fout, N, sF, count, P->scale, s);
+    if ((st = launch_zgemm(m, N, n, fin, n, sf, P->E2, N, 0, w.T, N, sT, count, 1.0, s, &w.partials))) return st;
+    return launch_zgemm(M, N, m, P->E1, m, 0, w.T, N, sT, Fout, N, sF, count, P->scale, s, &w.partials);
   }
   const bool bf16 = P->precision == LGB_SPLIT_BF16;
   float* const maxabs = bf16 ? nullptr : w.maxabs;     // bf16: no per-field scale

@@ -127,6 +127,8 @@ struct ZgemmScratch {
 int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA,
                  const double2* B, int ldb, long long sB, double2* C, int ldc, long long sC,
                  int batch, double alpha, cudaStream_t s, const ZgemmScratch* scratch = nullptr);
+// Bytes of the split-K partials launch_zgemm would use (0: it does not split)
+size_t zgemm_partial_bytes(int M, int N, int K, int batch);
 // Bytes of lgb_dft2's workspace on the plain FP64 path (plan.cu)
 size_t plain_dft2_workspace(int m, int n, int M, int N);
 // lgb_dft2_batch's body (plan.cu), with the FP64 GEMMs' split-K partials

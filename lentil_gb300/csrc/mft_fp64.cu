@@ -125,6 +125,20 @@ static void keep_pool_memory() {
   done[dev] = true;
 }
 
+// K splits of a launch (1: whole): see launch_zgemm.
+static int zgemm_splits(int M, int N, int K, int batch) {
+  const long long tiles = (long long)cdiv(N, ZBN) * cdiv(M, ZBM) * batch;
+  const int sms = sm_count();
+  if (tiles >= 2LL * sms || K <= ZBK) return 1;
+  return (int)std::min<long long>({(2LL * sms + tiles - 1) / tiles, (long long)cdiv(K, ZBK), 16LL,
+                                   65535LL / batch});
+}
+
+size_t zgemm_partial_bytes(int M, int N, int K, int batch) {
+  const int splits = zgemm_splits(M, N, K, batch);
+  return splits > 1 ? (size_t)splits * batch * M * N * sizeof(double2) : 0;
+}
+
 // A launch of fewer than two tiles per SM would leave FP64 pipes idle (a
 // 64 x 64 output is 16 tiles), so such a launch splits K over up to 16 CTAs
 // per tile, each writing a partial product to scratch (the caller's, or
@@ -135,12 +149,7 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
                  cudaStream_t s, const ZgemmScratch* scratch) {
   if (M <= 0 || N <= 0 || batch <= 0) return LGB_OK;
   LGB_REQUIRE(batch <= 65535, LGB_EINVAL, "zgemm: batch too large");
-  const long long tiles = (long long)cdiv(N, ZBN) * cdiv(M, ZBM) * batch;
-  const int sms = sm_count();
-  int splits = 1;
-  if (tiles < 2LL * sms && K > ZBK)
-    splits = (int)std::min<long long>({(2LL * sms + tiles - 1) / tiles, (long long)cdiv(K, ZBK), 16LL,
-                                       65535LL / batch});
+  int splits = zgemm_splits(M, N, K, batch);
   const long long sP = (long long)batch * M * N;          // one split's partials
   const size_t part_bytes = (size_t)sP * sizeof(double2);
   if (scratch) {                                          // as many splits as fit

@@ -13,6 +13,7 @@ import torch
 from . import _device as dv
 from . import _lib
 from . import extent as ext
+from . import util
 
 
 class Field:
@@ -74,7 +75,7 @@ class Field:
         x, y = 0, 0
         for t in self.tilt:
             x, y = t.__shift__(xs=x, ys=y, z=z, wavelength=wavelength)
-        ps = np.broadcast_to(pixelscale, (2,))
+        ps = util.pair(pixelscale)
         out = x / ps[0] * oversample, y / ps[1] * oversample
         if indexing == 'ij':
             out = -out[1], out[0]

@@ -19,6 +19,7 @@ import torch
 
 from . import _device as dv
 from . import _lib
+from . import util
 
 # Device-resident DFT matrices of recently used geometries (lgb_dft2_plan_*):
 # a repeated transform of one geometry builds no matrices and copies nothing
@@ -37,7 +38,9 @@ class _Dft2Plan:
         self.nbytes = int(lib.lgb_dft2_plan_size(m, n, M, N, prec))
         self._mem = dv.workspace(self.nbytes)
         self._home = torch.cuda.current_stream()
+        self._home_ptr = self._home.cuda_stream
         self._foreign = set()
+        self._ws_bytes = {}           # batch count -> workspace bytes
         h = ctypes.c_void_p()
         _lib.call('lgb_dft2_plan_create_in', m, n, M, N, ar, ac, sr, sc, orow, ocol, unitary, prec,
                   self._mem.data_ptr(), self.nbytes, dv.stream_ptr(), ctypes.byref(h))
@@ -52,17 +55,20 @@ class _Dft2Plan:
         """fd: [count, m, n] contiguous complex128 CUDA tensor -> [count, M, N].
         A device-side failure of an earlier execute is raised here."""
         count = int(fd.shape[0])
-        s = torch.cuda.current_stream()
-        if s != self._home and not torch.cuda.is_current_stream_capturing():
+        sp = dv.stream_ptr()
+        if sp != self._home_ptr and not torch.cuda.is_current_stream_capturing():
+            s = torch.cuda.current_stream()
             s.wait_event(self._built)         # the matrices are built before s reads them
-            if s.cuda_stream not in self._foreign:
+            if sp not in self._foreign:
                 self._mem.record_stream(s)    # keep the matrices until s is done with them
-                self._foreign.add(s.cuda_stream)
+                self._foreign.add(sp)
         F = torch.empty((count,) + self.shape_out, dtype=torch.complex128, device=fd.device)
-        nbytes = self._lib.lgb_dft2_plan_workspace_size(self._h, count)
-        ws = dv.workspace(nbytes)
+        nbytes = self._ws_bytes.get(count)
+        if nbytes is None:
+            nbytes = self._ws_bytes[count] = self._lib.lgb_dft2_plan_workspace_size(self._h, count)
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=fd.device)
         _lib.call('lgb_dft2_plan_execute', self._h, fd.data_ptr(), count, F.data_ptr(),
-                  ws.data_ptr(), nbytes, dv.stream_ptr())
+                  ws.data_ptr(), nbytes, sp)
         return F
 
     def status(self):
@@ -85,7 +91,7 @@ def _plan(m, n, M, N, ar, ac, sr, sc, orow, ocol, unitary, prec):
     """The cached plan of a geometry, created on its second use (None on the
     first: a one-off transform builds its matrices in its own workspace)."""
     key = (m, n, M, N, ar, ac, sr, sc, orow, ocol, int(bool(unitary)), prec,
-           torch.cuda.current_device())
+           dv.index())
     with _plans_lock:
         p = _plans.get(key)
         if p is not None:
@@ -212,6 +218,11 @@ def _transform(fd, M, N, alpha, shift, offset, unitary, precision):
 
 
 def _pair(x, name):
+    t = type(x)
+    if t is float or t is int:
+        return float(x), float(x)
+    if t is tuple and len(x) == 2 and isinstance(x[0], (int, float)) and isinstance(x[1], (int, float)):
+        return float(x[0]), float(x[1])
     v = np.broadcast_to(np.asarray(x, dtype=float), (2,))
     return float(v[0]), float(v[1])
 
@@ -223,7 +234,7 @@ def _shape(shape, npix, f_shape):
         shape = npix
     if shape is None:
         return int(f_shape[0]), int(f_shape[1])
-    M, N = np.broadcast_to(np.asarray(shape), (2,))
+    M, N = util.pair(shape)
     return int(M), int(N)
 
 

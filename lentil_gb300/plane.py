@@ -187,7 +187,7 @@ class Plane(_PlaneBase):
         if mask is not None:
             self._mask = _asarray(mask)
         if pixelscale is not None:
-            self._pixelscale = np.broadcast_to(pixelscale, (2,))
+            self._pixelscale = util.pair(pixelscale)
         if diameter is not None:
             self._diameter = diameter
         if ptype is not None:
@@ -327,8 +327,8 @@ class Plane(_PlaneBase):
 
 def _mul_pixelscale(a, b):
     """lentil/plane.py:614-629."""
-    a = None if a is None else np.broadcast_to(a, (2,))
-    b = None if b is None else np.broadcast_to(b, (2,))
+    a = None if a is None else util.pair(a)
+    b = None if b is None else util.pair(b)
     if a is None:
         return b
     if b is None:

@@ -58,8 +58,8 @@ def plan_fields(wavefront, pixelscale, shape=None, prop_shape=None, oversample=2
     Returns (ptype_out, shape_out, du, jobs); a field whose window misses the
     output produces no job, as in lentil."""
     ptype_out = _propagate_ptype(wavefront.ptype, method='fraunhofer')
-    shape = np.asarray(wavefront.shape) if shape is None else np.broadcast_to(shape, (2,))
-    prop_shape = np.asarray(shape) if prop_shape is None else np.broadcast_to(prop_shape, (2,))
+    shape = np.asarray(wavefront.shape) if shape is None else util.pair(shape)
+    prop_shape = np.asarray(shape) if prop_shape is None else util.pair(prop_shape)
     shape_out = shape * oversample
     prop_shape_out = prop_shape * oversample
     if mask is not None:
@@ -71,7 +71,7 @@ def plan_fields(wavefront, pixelscale, shape=None, prop_shape=None, oversample=2
     else:
         out_extent = ext.array_extent(shape_out, shift=(0, 0))
     dx = wavefront.pixelscale
-    du = np.broadcast_to(pixelscale, (2,))
+    du = util.pair(pixelscale)
     z = wavefront.focal_length
     jobs = []
     for field in wavefront.data:
@@ -198,7 +198,7 @@ def propagate_fft(wavefront, pixelscale, shape=None, oversample=2, scratch=None,
         raise NotImplementedError('propagate_fft does not support Wavefronts with fitted tilt. '
                                   'Use propagate_dft instead.')
     ptype_out = _propagate_ptype(wavefront.ptype, method='fraunhofer')
-    pixelscale = np.broadcast_to(pixelscale, (2,))
+    pixelscale = util.pair(pixelscale)
     fft_shape, prop_wavelength = _fft_shape(wavefront.pixelscale, pixelscale,
                                             wavefront.focal_length, wavefront.wavelength,
                                             oversample)

@@ -4,6 +4,23 @@ never touch the GPU."""
 import numpy as np
 
 
+_SCALARS = (int, float, np.float64, np.int64)
+
+
+def pair(x):
+    """``np.broadcast_to(x, (2,))``, at a fraction of its cost for the usual
+    arguments (a number, two numbers, an array of two)."""
+    t = type(x)
+    if t in _SCALARS:
+        return np.array((x, x))
+    if t is np.ndarray:
+        if x.shape == (2,):
+            return x
+    elif t in (tuple, list) and len(x) == 2 and type(x[0]) in _SCALARS and type(x[1]) in _SCALARS:
+        return np.array(x)
+    return np.broadcast_to(x, (2,))
+
+
 def mesh(shape, shift=(0, 0), angle=0):
     """Centred (row, col) coordinate grids, optionally rotated by ``angle``
     degrees (lentil/helper.py:7-17)."""
@@ -18,16 +35,18 @@ def mesh(shape, shift=(0, 0), angle=0):
 def boundary(x, threshold=0):
     """(rmin, rmax, cmin, cmax) of the entries above ``threshold``
     (lentil/util.py:190-218)."""
-    x = np.asarray(x) > threshold
+    x = np.asarray(x)
+    if x.dtype != bool or threshold != 0:
+        x = x > threshold
     rows = np.flatnonzero(x.any(axis=1))
-    cols = np.flatnonzero(x.any(axis=0))
+    cols = np.flatnonzero(x[rows[0]:rows[-1] + 1].any(axis=0))
     return rows[0], rows[-1], cols[0], cols[-1]
 
 
 def boundary_slice(x, threshold=0, pad=(0, 0)):
     """Bounding box of ``x > threshold`` as a slice pair
     (lentil/helper.py:27-62)."""
-    pad = np.broadcast_to(np.asarray(pad), (2,))
+    pad = pair(pad)
     rmin, rmax, cmin, cmax = boundary(x, threshold)
     return np.s_[max(rmin - pad[0], 0):min(rmax + pad[0] + 1, x.shape[0]),
                  max(cmin - pad[1], 0):min(cmax + pad[1] + 1, x.shape[1])]

@@ -5,6 +5,7 @@ import torch
 
 from . import _device as dv
 from . import field as fld
+from . import util
 from .field import Field
 from .ptype import ptype as _ptype, none, pupil, image
 
@@ -15,20 +16,20 @@ class Wavefront:
     CUDA tensors (then CUDA tensors); ``.insert`` updates ``out`` in place."""
 
     def __init__(self, wavelength, pixelscale=None, diameter=None, focal_length=None,
-                 tilt=None, ptype=None):
+                 tilt=None, ptype=None, _unit=True):
         from .plane import Tilt
         self.focal_length = focal_length if focal_length else None
         self.diameter = diameter
         self.shape = ()
         self._wavelength = wavelength
-        self._pixelscale = None if pixelscale is None else np.broadcast_to(pixelscale, (2,))
+        self._pixelscale = None if pixelscale is None else util.pair(pixelscale)
         self.ptype = ptype
         self._tensor_io = False
         if tilt is not None:
             if len(tilt) != 2:
                 raise ValueError('tilt must be specified as [rx, ry]')
             tilt = [Tilt(x=tilt[0], y=tilt[1])]
-        self.data = [Field(data=np.array(1, dtype=complex), offset=None, tilt=tilt)]
+        self.data = [Field(data=np.array(1, dtype=complex), offset=None, tilt=tilt)] if _unit else []
 
     def __mul__(self, plane):
         return plane.__mul__(self)
@@ -87,7 +88,8 @@ class Wavefront:
               shape=None, ptype=None):
         """Wavefront with no fields (lentil/wavefront.py:127-142)."""
         w = cls(wavelength=wavelength, pixelscale=pixelscale, diameter=diameter,
-                focal_length=focal_length, tilt=tilt, ptype=ptype)
+                focal_length=focal_length, tilt=tilt, ptype=ptype,
+                **({'_unit': False} if cls is Wavefront else {}))
         w.data = []
         w.shape = () if shape is None else shape
         return w
