@@ -440,55 +440,59 @@ split_mft_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_consta
         mbar_wait_issued(full_bar(k % STAGES), (k / STAGES) & 1, p.wait_ns);
   } else if (warp == 1) {
     // ------------------------------------------------------- MMA issuer
-    // (even CTA) the whole warp walks the items (the live K-block set is a
-    // warp collective); lane 0 issues the MMAs and the commits
+    // (even CTA) the whole warp walks the items and the K blocks, converged: the
+    // live K-block set is a warp collective, and the operands of the MMAs stay
+    // in uniform registers.  Issued from a loop that one lane ran alone, an MMA
+    // took about 95 clocks: hidden behind a 256-wide MMA's 128 except where the
+    // pipe was to catch up, but not behind a 128-wide one's 64 (broadband
+    // 1024^2 x 64 at that width 2450 -> 1730 us, three 512^2 fields 61 -> 51).
+    // One elected lane issues the MMAs and the commits.
     if (leader) {
+      const uint32_t on = elect_one();
+      auto wait = [&](uint32_t bar, uint32_t parity) {
+        return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.err, p.wait_ns)) != 0;
+      };
       uint32_t it = 0;                       // K blocks issued (stage ring)
       uint32_t gi = 0;                       // accumulator groups issued (accumulator uses)
       bool ok = true;
       for (int i = pair; ok && i < p.n_items; i += npairs) {
         const Item w = decode(p, i);
         const Live lv = live_kblocks<BN>(p, w);
-        if (lane == 0) {
-          const uint32_t idesc = (p.idesc & ~(0x3Fu << 17)) |
-                                 ((uint32_t)(tile_n<BN>(p, w.tn) >> 3) << 17);
-          int j = 0;                         // live K blocks of this item issued
-          for (int kb = 0; kb < p.kblocks; ++kb) {
-            if (!is_live(lv, kb)) continue;
-            const int s = it % STAGES, xb = gi & 1;
-            const bool first = j % KB == 0;
-            const bool last = j % KB == KB - 1 || j == lv.n - 1;
-            if (!mbar_wait(full_bar(s), (it / STAGES) & 1, p.err, p.wait_ns)) { ok = false; break; }
-            // accumulator xb was drained by both CTAs (its previous group, gi - 2)
-            if (first && !mbar_wait(acc_empty(xb), ((gi >> 1) & 1) ^ 1, p.err, p.wait_ns)) { ok = false; break; }
-            tc_fence_after();
-            const uint32_t sa = base + s * STAGE_BYTES, X = tmem + xb * ACC_COLS;
+        const uint32_t idesc = (p.idesc & ~(0x3Fu << 17)) |
+                               ((uint32_t)(tile_n<BN>(p, w.tn) >> 3) << 17);
+        int j = 0;                           // live K blocks of this item issued
+        for (int kb = 0; kb < p.kblocks; ++kb) {
+          if (!is_live(lv, kb)) continue;
+          const int s = it % STAGES, xb = gi & 1;
+          const bool first = j % KB == 0;
+          const bool last = j % KB == KB - 1 || j == lv.n - 1;
+          if (!wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
+          // accumulator xb was drained by both CTAs (its previous group, gi - 2)
+          if (first && !wait(acc_empty(xb), ((gi >> 1) & 1) ^ 1)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = base + s * STAGE_BYTES, X = tmem + xb * ACC_COLS;
+          const uint64_t a_hi = smem_desc(sa), a_lo = smem_desc(sa + A_BYTES);
+          const uint64_t b_hi = smem_desc(sa + 2 * A_BYTES), b_lo = smem_desc(sa + 2 * A_BYTES + B_BYTES);
 #pragma unroll
-            for (int k = 0; k < KSTEPS; ++k) {   // hi.lo + lo.hi: small terms first
-              mma_f16(X, smem_desc(sa + k * 32), smem_desc(sa + 2 * A_BYTES + B_BYTES + k * 32),
-                      idesc, (first && k == 0) ? 0u : 1u);
-              mma_f16(X, smem_desc(sa + A_BYTES + k * 32), smem_desc(sa + 2 * A_BYTES + k * 32),
-                      idesc, 1u);
-            }
-#pragma unroll
-            for (int k = 0; k < KSTEPS; ++k)     // hi.hi last
-              mma_f16(X, smem_desc(sa + k * 32), smem_desc(sa + 2 * A_BYTES + k * 32), idesc, 1u);
-            mma_commit_pair(empty_bar(s));       // both CTAs' stage s free once these retire
-            if (last) {
-              mma_commit_pair(acc_full(xb));     // accumulator xb ready for the epilogues
-              ++gi;
-            }
-            ++j;
-            ++it;
+          for (int k = 0; k < KSTEPS; ++k) {   // hi.lo + lo.hi: small terms first
+            mma_f16(on, X, a_hi + 2 * k, b_lo + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+            mma_f16(on, X, a_lo + 2 * k, b_hi + 2 * k, idesc, 1u);
           }
+#pragma unroll
+          for (int k = 0; k < KSTEPS; ++k)     // hi.hi last
+            mma_f16(on, X, a_hi + 2 * k, b_hi + 2 * k, idesc, 1u);
+          mma_commit_pair(on, empty_bar(s));   // both CTAs' stage s free once these retire
+          if (last) {
+            mma_commit_pair(on, acc_full(xb)); // accumulator xb ready for the epilogues
+            ++gi;
+          }
+          ++j;
+          ++it;
         }
-        ok = __shfl_sync(0xffffffffu, ok, 0) != 0;
       }
       // all issued MMAs have retired before TMEM is released
-      if (lane == 0) {
-        mma_commit_pair(drain_bar);
-        mbar_wait_issued(drain_bar, 0, p.wait_ns);
-      }
+      mma_commit_pair(on, drain_bar);
+      mbar_wait_issued(drain_bar, 0, p.wait_ns);
       __syncwarp();
     }
   } else {
@@ -771,10 +775,10 @@ static int run_split_mft(const SplitMftProblem& q, cudaEvent_t* ev, cudaStream_t
 // stage over the resident CTA pairs, capped at 8 (launches of eight or more
 // waves behave alike).
 //
-// The occupancy model below prices both widths.  Where it separates them by
-// TUNE_DECISIVE or more (many waves: the 256-wide tile; a launch far below
-// one wave: the 128-wide one) its choice is final.  In between, measure mode
-// (the default) tunes the class online, on the caller's own launches: the
+// The occupancy model below prices both widths.  For launches of eight or more
+// waves in both stages its choice is final: the 256-wide tile is 3-4 % faster
+// there, less than a trial tells apart.  Below, where a width can win by up to
+// 1.35x, measure mode (the default) tunes the class online, on the caller's own launches: the
 // next TUNE_TRIALS launches alternate the two widths, the model's first, each
 // bracketed by CUDA events on its stream; a later launch of the class finds
 // them all finished (cudaEventQuery, no host wait), compares the fastest run
@@ -786,7 +790,7 @@ static int run_split_mft(const SplitMftProblem& q, cudaEvent_t* ev, cudaStream_t
 // nothing.  Model mode takes the model's choice at once; a forced width
 // overrides everything.
 constexpr int TUNE_TRIALS = 4;
-constexpr double TUNE_DECISIVE = 1.4;
+constexpr int TUNE_WAVES = 8;        // waves a class key counts up to
 
 struct Trial {
   int width = 0;
@@ -823,17 +827,17 @@ static TuneKey tune_key(const SplitMftProblem& q) {
   const int pairs = std::max(1, sm_count() / 2);
   StageShape sh[2];
   stage_shapes(q, 128, sh);
-  auto waves = [&](long long items) { return (int)std::min<long long>(8, (items + pairs - 1) / pairs); };
+  auto waves = [&](long long items) { return (int)std::min<long long>(TUNE_WAVES, (items + pairs - 1) / pairs); };
   return {q.bf16 ? 1 : 0, q.m, q.n, q.M, q.N, q.epilogue, waves(sh[0].items), waves(sh[1].items)};
 }
 
 // Cost of each width: waves of work items over the resident CTA pairs times
-// K blocks, a 128-wide item costing 0.78 of a 256-wide one (measured on the
-// broadband workload: twice the items took 1.56x the time at full
-// occupancy).  Either width holds one CTA per SM, so the pairs are taken as
+// K blocks, a 128-wide item costing 0.52 of a 256-wide one (measured on the
+// broadband workload: twice the items took 1.04x the time at full occupancy;
+// 0.78 and 1.47x while one lane alone issued the MMAs).  Either width holds one CTA per SM, so the pairs are taken as
 // half the SMs: no occupancy query, which keeps the model usable inside a
-// stream capture.  Returns the cheaper width; *ratio = dearer / cheaper.
-static int model_tile(const SplitMftProblem& q, double* ratio = nullptr) {
+// stream capture.  Returns the cheaper width.
+static int model_tile(const SplitMftProblem& q) {
   double cost[2];
   const int bns[2] = {256, 128};
   const int pairs = std::max(1, sm_count() / 2);
@@ -842,9 +846,8 @@ static int model_tile(const SplitMftProblem& q, double* ratio = nullptr) {
     stage_shapes(q, bns[c], sh);
     cost[c] = 0.0;
     for (const StageShape& x : sh) cost[c] += (double)((x.items + pairs - 1) / pairs) * x.kblocks;
-    cost[c] *= bns[c] == 256 ? 1.0 : 0.78;
+    cost[c] *= bns[c] == 256 ? 1.0 : 0.52;
   }
-  if (ratio) *ratio = std::max(cost[0], cost[1]) / std::max(1e-30, std::min(cost[0], cost[1]));
   return cost[1] < cost[0] ? 128 : 256;
 }
 
@@ -872,15 +875,14 @@ static int choose_tile(const SplitMftProblem& q, cudaStream_t s, int* bn, cudaEv
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   LGB_CUDA(cudaStreamIsCapturing(s, &cap));
   *key = tune_key(q);
-  double ratio = 1.0;
-  const int model = model_tile(q, &ratio);
+  const int model = model_tile(q);
   std::lock_guard<std::mutex> lock(T.mu);
   if (T.forced) { *bn = T.forced; return LGB_OK; }
   auto it = T.table.find(*key);
   if (it != T.table.end() && it->second.best) { *bn = it->second.best; return LGB_OK; }
   *bn = model;
   if (cap != cudaStreamCaptureStatusNone) return LGB_OK;
-  if (T.mode == LGB_TUNE_MODEL || ratio >= TUNE_DECISIVE) {
+  if (T.mode == LGB_TUNE_MODEL || ((*key)[6] == TUNE_WAVES && (*key)[7] == TUNE_WAVES)) {
     T.table[*key].best = model;
     return LGB_OK;
   }

@@ -160,21 +160,26 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
 }
 // D[256 x 256] (+)= A[256 x 16] . B[256 x 16]^T over the CTA pair: each CTA
 // supplies 128 rows of A and 128 rows of B at the same shared-memory offset.
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                        uint32_t accumulate) {
+// Issued by the lane with `on`: the whole warp runs the code around it, so the
+// operands stay in uniform registers.
+__device__ __forceinline__ void mma_f16(uint32_t on, uint32_t d_tmem, uint64_t a, uint64_t b,
+                                        uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on));
 }
 // arrive once on the barrier at this offset in both CTAs when the MMAs
-// issued so far have completed
-__device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
+// issued so far by the lane with `on` have completed
+__device__ __forceinline__ void mma_commit_pair(uint32_t on, uint32_t bar) {
   const uint16_t both = 3;
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], %1;" ::"r"(bar), "h"(both)
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
+      " [%0], %1;\n\t}" ::"r"(bar), "h"(both), "r"(on)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
