@@ -127,8 +127,8 @@ size_t plan_carve(lgb_dft2_plan_s* P, void* base) {
     P->e2h = c.take<uint16_t>(nrows2 * 2 * P->kp2);
     P->e2l = c.take<uint16_t>(nrows2 * 2 * P->kp2);
   } else if (P->sliced) {
-    P->d1 = c.take<uint16_t>(sliced_matrix_entries(P->m, P->M, true));
-    P->d2 = c.take<uint16_t>(sliced_matrix_entries(P->n, P->N, !P->left));
+    P->d1 = c.take<uint16_t>(sliced_matrix_entries(P->m, P->M));
+    P->d2 = c.take<uint16_t>(sliced_matrix_entries(P->n, P->N));
   } else {
     P->E1 = c.take<double2>((size_t)P->M * P->m);
     P->E2 = c.take<double2>((size_t)P->n * P->N);
@@ -259,8 +259,8 @@ int plan_build(lgb_dft2_plan_s* P, const PhaseAxis* ax, cudaStream_t s) {
     return st;
   }
   if (P->sliced) {
-    int st = launch_matrix_digits(ax[0], nullptr, 1, P->m, P->M, true, P->d1, s);
-    return st ? st : launch_matrix_digits(ax[1], nullptr, 1, P->n, P->N, !P->left, P->d2, s);
+    int st = launch_matrix_digits(ax[0], nullptr, 1, P->m, P->M, P->d1, s);
+    return st ? st : launch_matrix_digits(ax[1], nullptr, 1, P->n, P->N, P->d2, s);
   }
   int st = launch_dft_matrix_c128(ax[0], P->m, P->M, P->E1, true, s);
   if (!st) st = launch_dft_matrix_c128(ax[1], P->n, P->N, P->E2, false, s);

@@ -142,9 +142,8 @@ int dft2_batch(const double2* f, int count, int m, int n, double2* F, int M, int
 struct SlicedDft2 {
   int count, m, n, M, N;
   bool left;                 // product order: (E1 f) E2, else E1 (f E2)
-  // launch_matrix_digits of the row axis (m -> M), an operand B, and of the
-  // column axis (n -> N), an operand A when left, else B; one matrix for all
-  // items, or one per item when axes is set
+  // launch_matrix_digits of the row axis (m -> M) and of the column axis
+  // (n -> N); one matrix for all items, or one per item when axes is set
   const uint16_t *e1, *e2;
   PhaseAxis ar, ac;          // the axes ...
   const PhaseAxis* axes;     // ... or, on the device, item i's: axes[i] (rows) and axes[cols + i]
@@ -156,10 +155,10 @@ struct SlicedDft2 {
 // the order that needs fewer flops; (E1 f) E2, lentil's, when they are equal
 bool sliced_left(int m, int n, int M, int N);
 bool sliced_applies(int m, int n, int M, int N);
-size_t sliced_matrix_entries(int len_in, int len_out, bool operand_b);    // 16-bit entries of one matrix
+size_t sliced_matrix_entries(int len_in, int len_out);    // 16-bit entries of one matrix
 // the digits of `count` matrices: the axes on the device, or (count 1, null) `ax`
 int launch_matrix_digits(const PhaseAxis& ax, const PhaseAxis* axes, int count, int len_in, int len_out,
-                         bool operand_b, uint16_t* out, cudaStream_t s);
+                         uint16_t* out, cudaStream_t s);
 size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left);
 int launch_sliced_dft2(const SlicedDft2& q, void* workspace, cudaStream_t s);
 

@@ -16,27 +16,28 @@
 namespace lgb {
 namespace {
 
-// x * 2^-62 as a 53-bit fraction, rounded
-__device__ __forceinline__ long long unit53(long long x) { return (x + 256) >> 9; }
-
 // DFT-matrix digits: vector j < L (output index) over the input index; matrix
-// z's axis is axes[z], or ax when there is one.  Bound by the 24 or 36 bytes
-// written per entry (6.9 us for a 512^2 operand B); the cosines are integer
-// arithmetic because sincospi alone would take the FP64 pipe longer than that.
+// z's axis is axes[z], or ax when there is one.  Bound by the 42 bytes written
+// per entry (17.5 us for 1019 x 1024, cold caches); the cosines are integer arithmetic because
+// sincospi alone would take the FP64 pipe longer than that.
 __global__ void __launch_bounds__(128) matrix_digits_kernel(PhaseAxis ax, const PhaseAxis* __restrict__ axes,
                                                             int len_in, DigitRows out) {
   __shared__ unsigned long long table[129];
   for (int i = threadIdx.x; i < 129; i += 128) table[i] = COS_TABLE[i];
   __syncthreads();
   if (axes) ax = axes[blockIdx.z];
-  out.base += (size_t)blockIdx.z * NE * out.plane();
+  out.base += (size_t)blockIdx.z * ND * out.plane();
   const int k = 2 * (blockIdx.x * blockDim.x + threadIdx.x), j = blockIdx.y;
   if (k >= out.kp) return;
   const uint64_t ph = phase_fixed(ax, k, j);
   longlong2 e0 = make_longlong2(0, 0), e1 = e0;                 // (cos, sin): E = cos - i sin
   if (k < len_in) e0 = cossin_q62(ph, table);
   if (k + 1 < len_in) e1 = cossin_q62(ph + phase_step_in(ax, j), table);
-  store_digits<NE>(out, j, k, unit53(e0.x), -unit53(e0.y), unit53(e1.x), -unit53(e1.y));
+  store_digits3(out, j, k, make_longlong2(e0.x, -e0.y), make_longlong2(e1.x, -e1.y));
+}
+
+__device__ __forceinline__ longlong2 fixed_entry(double2 z, int e) {
+  return make_longlong2(fixed_data(z.x, e), fixed_data(z.y, e));
 }
 
 // f's rows (one block each) -> digits, vectors of n entries.
@@ -67,8 +68,7 @@ __global__ void __launch_bounds__(128) slice_rows_kernel(const double2* __restri
   const double2 zero = make_double2(0.0, 0.0);
   for (int k = 2 * threadIdx.x; k < out.kp; k += 256) {
     const double2 z0 = k < n ? src[k] : zero, z1 = k + 1 < n ? src[k + 1] : zero;
-    store_digits<ND>(out, i, k, fixed_data(z0.x, e), fixed_data(z0.y, e), fixed_data(z1.x, e),
-                     fixed_data(z1.y, e));
+    store_digits3(out, i, k, fixed_entry(z0, e), fixed_entry(z1, e));
   }
 }
 
@@ -109,25 +109,24 @@ __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
   for (int k = 2 * (part * 32 + lane); k < out.kp; k += 64 * PARTS) {
     const double2 z0 = k < m ? src[(size_t)k * n] : zero;
     const double2 z1 = k + 1 < m ? src[(size_t)(k + 1) * n] : zero;
-    store_digits<ND>(out, j, k, fixed_data(z0.x, e), fixed_data(z0.y, e), fixed_data(z1.x, e),
-                     fixed_data(z1.y, e));
+    store_digits3(out, j, k, fixed_entry(z0, e), fixed_entry(z1, e));
   }
 }
 
 // Row r of the first product (entry a in units of 2^(expA[a] - 16 - S)) ->
 // its digits as an operand of the second.  The first 2 KEEP entries of a thread
 // stay in registers between the two passes (rows of up to 1024 are read once).
-__global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<longlong2> q,
+__global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
                                                             const int* __restrict__ expA, int S,
                                                             DigitRows out, int* __restrict__ exps) {
   constexpr int KEEP = 2, NONE = -(1 << 28);
   const int r = blockIdx.x, b = blockIdx.y;
-  const longlong2* P = q.P + (size_t)b * q.item_stride + (size_t)r * q.ld;
-  const size_t sP = (size_t)q.rows * q.ld;
+  const long long* P = q.P + (size_t)b * 3 * q.stride + (size_t)r * q.ld;
+  const int tiles = q.deal.tilesA;
   const int* ea = expA + (size_t)b * q.cols;
-  __shared__ uint8_t parts[MAX_TILES_A];
+  __shared__ uint8_t parts[3 * MAX_TILES_A];
   __shared__ int se[8];
-  count_parts(q, b, r, parts);
+  count_parts<3>(q, 3 * b, r, parts);
   longlong2 kept[2 * KEEP], rest[2];
   int e = NONE;
   auto note = [&](int a, longlong2 v) {
@@ -135,21 +134,27 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<lo
   };
   {
     size_t at[2 * KEEP];
-    int n[2 * KEEP];
+    int n[3][2 * KEEP];
 #pragma unroll
     for (int i = 0; i < 2 * KEEP; ++i) {
       const int k = 2 * threadIdx.x + 512 * (i >> 1) + (i & 1);
       at[i] = k;
-      n[i] = k < q.cols ? parts[k / BM] : 0;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) n[c][i] = k < q.cols ? parts[c * tiles + k / BM] : 0;
     }
-    sum_parts<2 * KEEP>(P, sP, at, n, kept);
+    sum_parts3<2 * KEEP>(P, q.stride, q.part(), at, n, kept);
 #pragma unroll
     for (int i = 0; i < 2 * KEEP; ++i) note((int)at[i], kept[i]);
   }
   auto fetch = [&](int k) {                     // entries k, k + 1 -> rest
     const size_t at[2] = {(size_t)k, (size_t)k + 1};
-    const int n[2] = {k < q.cols ? parts[k / BM] : 0, k + 1 < q.cols ? parts[(k + 1) / BM] : 0};
-    sum_parts<2>(P, sP, at, n, rest);
+    int n[3][2];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      n[c][0] = k < q.cols ? parts[c * tiles + k / BM] : 0;
+      n[c][1] = k + 1 < q.cols ? parts[c * tiles + (k + 1) / BM] : 0;
+    }
+    sum_parts3<2>(P, q.stride, q.part(), at, n, rest);
   };
   for (int k = 512 * KEEP + 2 * threadIdx.x; k < q.cols; k += 512) {
     fetch(k);
@@ -165,8 +170,8 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<lo
   out.base += (size_t)b * ND * out.plane();
   auto put = [&](int k, longlong2 v0, longlong2 v1) {
     const int s0 = k < q.cols ? ea[k] - e + XBITS : 0, s1 = k + 1 < q.cols ? ea[k + 1] - e + XBITS : 0;
-    store_digits<ND>(out, r, k, shift_round(v0.x, s0), shift_round(v0.y, s0), shift_round(v1.x, s1),
-                     shift_round(v1.y, s1));
+    store_digits3(out, r, k, make_longlong2(shift_round(v0.x, s0), shift_round(v0.y, s0)),
+                  make_longlong2(shift_round(v1.x, s1), shift_round(v1.y, s1)));
   };
 #pragma unroll
   for (int i = 0; i < KEEP; ++i) {
@@ -181,7 +186,7 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums<lo
 
 // ---------------------------------------------------------------- finish ---
 struct FinishParams {
-  PartialSums<longlong2> q;             // rows M, cols N
+  PartialSums q;             // rows M, cols N
   int M, N, S;
   const int* exps;           // [item][M] (left) or [item][N]: exponent of the sliced product
   int left;                  // (E1 f) E2, else E1 (f E2)
@@ -193,7 +198,7 @@ struct FinishParams {
   PhaseAxis ar, ac;
   const PhaseAxis* axes;     // per item, or null: ar, ac
   int cols;
-  longlong2* scratch;        // P again: the item's intermediate rows
+  long long* scratch;        // P again: the item's intermediate rows
   const int* flags;
   const int* err;
 };
@@ -212,7 +217,7 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
   const double2* f = p.f + (size_t)b * p.m * p.n;
   double2* F = p.F + (size_t)b * p.M * p.N;
   const int len = p.left ? p.n : p.m, inner = p.left ? p.m : p.n;
-  double2* T = reinterpret_cast<double2*>(p.scratch + (size_t)b * p.q.item_stride) + (size_t)q * len;
+  double2* T = reinterpret_cast<double2*>(p.scratch + (size_t)b * 3 * p.q.stride) + (size_t)q * len;
   for (int a = threadIdx.x; a < len; a += blockDim.x) {
     double2 t = make_double2(0.0, 0.0);
     for (int k = 0; k < inner; ++k) {
@@ -236,10 +241,10 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
 
 constexpr int FIN_ROWS = 4;                  // rows per finish block
 
-// F = P's entries, scaled.  Bound by reading P from L2 and writing F (32 bytes
-// an entry).  With conversions and both scalings on the FP64 pipe and a row per
-// block it took 24.7 us at 1024^2 (cold caches); put together from bits, the
-// parts of four rows in flight at once, 17.3.
+// F = P's entries, scaled.  Bound by reading P from L2 and writing F (40 bytes
+// an entry and a part; 21 us at 1024^2, cold caches).  Results are put together
+// from bits and four rows' parts are in flight at once: with conversions and
+// both scalings on the FP64 pipe and a row per block it took half as long again.
 __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
   const int b = blockIdx.z, flag = p.flags[b];
   if (*p.err != 0 || (flag & FLAG_INF && !(flag & FLAG_NAN))) {
@@ -259,15 +264,20 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
   const int* exps = p.exps + (p.left ? (size_t)b * p.M + u0 : (size_t)b * p.N + v);
   longlong2 z[FIN_ROWS];
   size_t at[FIN_ROWS];
-  int n[FIN_ROWS], e[FIN_ROWS];
+  int n[3][FIN_ROWS], e[FIN_ROWS];
+  static_assert(BN % FIN_ROWS == 0, "the rows lie in one tile");
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const int parts = p.q.parts(3 * b + c, u0, v);
+#pragma unroll
+    for (int i = 0; i < FIN_ROWS; ++i) n[c][i] = i < rows ? parts : 0;
+  }
 #pragma unroll
   for (int i = 0; i < FIN_ROWS; ++i) {
-    const int tile = (b * p.q.deal.tilesB + (u0 + i) / BC) * p.q.deal.tilesA + v / BM;
     at[i] = (size_t)(u0 + i) * p.q.ld + v;
-    n[i] = i < rows ? p.q.deal.parts(tile) : 0;
     e[i] = i < rows ? exps[p.left ? i : 0] - 16 - p.S : 0;
   }
-  sum_parts<FIN_ROWS>(p.q.P + (size_t)b * p.q.item_stride, (size_t)p.M * p.q.ld, at, n, z);
+  sum_parts3<FIN_ROWS>(p.q.P + (size_t)b * 3 * p.q.stride, p.q.stride, p.q.part(), at, n, z);
 #pragma unroll
   for (int i = 0; i < FIN_ROWS; ++i)
     if (i < rows)
@@ -282,10 +292,10 @@ struct Layout {
   int rows1;                 // rows of the intermediate (K2 entries each)
   int chunk, ld1, ld2;
   Deal deal1, deal2;
-  long long item_stride;     // P entries per item
+  long long stride;          // P entries per product
   int *err, *flags, *exp1, *exp2;
   DigitRows d1, d2;          // digits of f (operand A) and of the intermediate
-  longlong2* P;
+  long long* P;
   size_t bytes;
 };
 
@@ -298,8 +308,8 @@ Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
   t.K2 = t.left ? n : m;
   t.vecs1 = t.left ? n : m;
   t.rows1 = t.left ? M : N;
-  t.d1 = DigitRows{nullptr, t.vecs1, round_up(t.K1, BK), 0};
-  t.d2 = DigitRows{nullptr, t.rows1, round_up(t.K2, BK), t.left ? 1 : 0};
+  t.d1 = DigitRows{nullptr, t.vecs1, round_up(t.K1, BK), 3};
+  t.d2 = DigitRows{nullptr, t.rows1, round_up(t.K2, BK), 3};
   // first GEMM: A = vectors of f, B = the first matrix; second: P's rows are
   // F's rows, its contiguous index F's columns
   t.ld1 = round_up(t.vecs1, BM);
@@ -307,11 +317,11 @@ Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
   const size_t p1 = (size_t)t.rows1 * t.ld1, p2 = (size_t)M * t.ld2;              // one partial sum
   const size_t b1 = 2 * ND * t.d1.plane(), b2 = 2 * ND * t.d2.plane();
   t.chunk = (int)std::min<long long>(
-      count, std::max<long long>(1, (long long)(CHUNK_BYTES / (b1 + b2 + sizeof(longlong2) * std::max(p1, p2)))));
+      count, std::max<long long>(1, (long long)(CHUNK_BYTES / (b1 + b2 + 3 * sizeof(long long) * std::max(p1, p2)))));
   t.chunk = cdiv(count, cdiv(count, t.chunk));                                    // even chunks
-  t.deal1 = deal_of(t.vecs1, t.rows1, BC, cdiv(t.K1, BK), t.chunk);
-  t.deal2 = deal_of(N, M, BC, cdiv(t.K2, BK), t.chunk);
-  t.item_stride = (long long)std::max(p1 * max_parts(t.deal1), p2 * max_parts(t.deal2));
+  t.deal1 = deal_of(t.vecs1, t.rows1, cdiv(t.K1, 2 * BK), 3 * t.chunk);
+  t.deal2 = deal_of(N, M, cdiv(t.K2, 2 * BK), 3 * t.chunk);
+  t.stride = (long long)std::max(p1 * max_parts(t.deal1), p2 * max_parts(t.deal2));
   size_t off = 0;
   auto take = [&](size_t bytes) {
     off = align_up(off, 256);
@@ -325,7 +335,7 @@ Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
   t.exp2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.rows1));
   t.d1.base = reinterpret_cast<uint16_t*>(take(b1 * t.chunk));
   t.d2.base = reinterpret_cast<uint16_t*>(take(b2 * t.chunk));
-  t.P = reinterpret_cast<longlong2*>(take(sizeof(longlong2) * (size_t)t.item_stride * t.chunk));
+  t.P = reinterpret_cast<long long*>(take(sizeof(long long) * (size_t)t.stride * 3 * t.chunk));
   t.bytes = off;
   return t;
 }
@@ -338,10 +348,10 @@ bool sliced_left(int m, int n, int M, int N) {
 
 // Where the sliced form is taken: where its five launches cost less than the
 // plain GEMMs' two to four.  Device time of one transform from a plan, plain
-// and sliced: 64^2 to 64^2 20 and 33 us, 96^2 29 and 33, 112^2 39 and 35, 256^2
-// 270 and 38, (8 x 8) to 512^2 27 and 38, (16 x 512) to 512^2 86 and 43,
-// (16 x 1024) to (16 x 1024) 171 and 39: the line is one of multiply-adds, just
-// below the crossing at about 102^2.
+// and sliced: 64^2 to 64^2 20 and 33 us, 96^2 29 and 35, 112^2 39 and 37, 256^2
+// 270 and 39, (8 x 8) to 512^2 27 and 33, (16 x 512) to 512^2 86 and 37,
+// (16 x 1024) to (16 x 1024) 171 and 45: the line is one of multiply-adds, just
+// below the crossing at about 105^2.
 // Operands longer than 16384 would leave the 64-bit sums too few fraction bits.
 bool sliced_applies(int m, int n, int M, int N) {
   if (std::min(std::min(m, n), std::min(M, N)) < 8 || std::max(m, n) > 16384 ||
@@ -351,13 +361,15 @@ bool sliced_applies(int m, int n, int M, int N) {
   return std::min(left, right) >= 2.0 * 96 * 96 * 96;
 }
 
-size_t sliced_matrix_entries(int len_in, int len_out, bool operand_b) {
-  return NE * DigitRows{nullptr, len_out, round_up(len_in, BK), operand_b ? 1 : 0}.plane();
+static DigitRows matrix_rows(const uint16_t* digits, int len_in, int len_out) {
+  return DigitRows{const_cast<uint16_t*>(digits), len_out, round_up(len_in, BK), 3};
 }
 
+size_t sliced_matrix_entries(int len_in, int len_out) { return ND * matrix_rows(nullptr, len_in, len_out).plane(); }
+
 int launch_matrix_digits(const PhaseAxis& ax, const PhaseAxis* axes, int count, int len_in, int len_out,
-                         bool operand_b, uint16_t* out, cudaStream_t s) {
-  const DigitRows d{out, len_out, round_up(len_in, BK), operand_b ? 1 : 0};
+                         uint16_t* out, cudaStream_t s) {
+  const DigitRows d = matrix_rows(out, len_in, len_out);
   matrix_digits_kernel<<<dim3(cdiv(d.kp, 256), len_out, count), 128, 0, s>>>(ax, axes, len_in, d);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
@@ -370,9 +382,8 @@ size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left) {
 int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   const Layout t = layout(q.count, q.m, q.n, q.M, q.N, q.left, ws);
   const bool own = q.axes != nullptr;
-  DigitRows e1{const_cast<uint16_t*>(q.e1), q.M, round_up(q.m, BK), 1};
-  DigitRows e2{const_cast<uint16_t*>(q.e2), q.N, round_up(q.n, BK), t.left ? 0 : 1};
-  const int S1 = unit_shift(t.K1), S2 = unit_shift(t.K2);
+  DigitRows e1 = matrix_rows(q.e1, q.m, q.M), e2 = matrix_rows(q.e2, q.n, q.N);
+  const int S1 = unit_shift(t.K1, 3), S2 = unit_shift(t.K2, 3);
   int st;
   for (int b0 = 0; b0 < q.count; b0 += t.chunk) {
     const int items = std::min(t.chunk, q.count - b0);
@@ -384,16 +395,19 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     else
       slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.flags);
     LGB_CUDA(cudaGetLastError());
-    if ((st = launch_gemm<ND, NE, false>(t.d1, items, t.left ? e1 : e2, own ? items : 1, items, t.deal1, Band{}, S1, t.P, t.item_stride, t.ld1, t.err, s)))
+    const int own_items = own ? items : 1;
+    if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, Band{}, S1, t.P,
+                          t.stride, t.ld1, t.err, s)))
       return st;
     slice_product_kernel<<<dim3(t.rows1, items), 256, 0, s>>>(
-        PartialSums<longlong2>{t.P, t.item_stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2);
+        PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2);
     LGB_CUDA(cudaGetLastError());
-    st = t.left ? launch_gemm<NE, ND, false>(e2, own ? items : 1, t.d2, items, items, t.deal2, Band{}, S2, t.P, t.item_stride, t.ld2, t.err, s)
-                : launch_gemm<ND, NE, false>(t.d2, items, e1, own ? items : 1, items, t.deal2, Band{}, S2, t.P, t.item_stride, t.ld2, t.err, s);
-    if (st) return st;
+    if ((st = launch_gemm(t.left ? e2 : t.d2, t.left ? own_items : items, t.left ? t.d2 : e1,
+                          t.left ? items : own_items, items, t.K2, t.deal2, Band{}, S2, t.P, t.stride, t.ld2, t.err,
+                          s)))
+      return st;
     FinishParams p{};
-    p.q = PartialSums<longlong2>{t.P, t.item_stride, t.ld2, q.M, q.N, t.deal2};
+    p.q = PartialSums{t.P, t.stride, t.ld2, q.M, q.N, t.deal2};
     p.M = q.M;
     p.N = q.N;
     p.S = S2;
@@ -414,8 +428,8 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     finish_kernel<<<dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s>>>(p);
     LGB_CUDA(cudaGetLastError());
     if (own) {
-      e1.base += (size_t)items * NE * e1.plane();
-      e2.base += (size_t)items * NE * e2.plane();
+      e1.base += (size_t)items * ND * e1.plane();
+      e2.base += (size_t)items * ND * e2.plane();
     }
   }
   return LGB_OK;

@@ -34,16 +34,6 @@ struct BandedRows {                          // G[r][q0[r] + b] = Gt[b][r]
   }
 };
 
-__device__ __forceinline__ void store_real_digits(const DigitRows& o, int r, int k, long long v0, long long v1) {
-  uint16_t* p = o.base + (size_t)r * o.kp + k;
-  uint32_t a[ND], c[ND];
-  digits_of(v0, a);
-  digits_of(v1, c);
-#pragma unroll
-  for (int i = 0; i < ND; ++i)
-    *reinterpret_cast<uint32_t*>(p + i * o.plane()) = __byte_perm(a[i], c[i], 0x7632);
-}
-
 // Row r (one block) of a real matrix -> digits and exponent.
 template <typename Rows>
 __global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out, int* __restrict__ exps,
@@ -64,24 +54,23 @@ __global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out
   }
   if (bad) return;
   for (int k = 2 * threadIdx.x; k < out.kp; k += 512)
-    store_real_digits(out, r, k, k < K ? fixed_data(src.at(r, k), e) : 0,
+    store_digits(out, 0, r, k, k < K ? fixed_data(src.at(r, k), e) : 0,
                       k + 1 < K ? fixed_data(src.at(r, k + 1), e) : 0);
 }
 
 // Row r of a product (entry a in units of 2^(ea[a] + eb[r] - 16 - S)) ->
 // digits.  The first 2 KEEP entries of a thread stay in registers between the
 // two passes.
-__global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSums<long long> q,
+__global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSums q,
                                                                  const int* __restrict__ ea,
                                                                  const int* __restrict__ eb, int S,
                                                                  DigitRows out, int* __restrict__ exps) {
   constexpr int KEEP = 4, NONE = -(1 << 28);
   const int r = blockIdx.x;
   const long long* P = q.P + (size_t)r * q.ld;
-  const size_t sP = (size_t)q.rows * q.ld;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ int se[8];
-  count_parts(q, 0, r, parts);
+  count_parts<1>(q, 0, r, parts);
   long long kept[2 * KEEP], rest[2];
   int e = NONE;
   auto note = [&](int a, long long v) {
@@ -96,14 +85,14 @@ __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSu
       at[i] = k;
       n[i] = k < q.cols ? parts[k / BM] : 0;
     }
-    sum_parts<2 * KEEP>(P, sP, at, n, kept);
+    sum_parts<2 * KEEP>(P, q.part(), at, n, kept);
 #pragma unroll
     for (int i = 0; i < 2 * KEEP; ++i) note((int)at[i], kept[i]);
   }
   auto fetch = [&](int k) {
     const size_t at[2] = {(size_t)k, (size_t)k + 1};
     const int n[2] = {k < q.cols ? parts[k / BM] : 0, k + 1 < q.cols ? parts[(k + 1) / BM] : 0};
-    sum_parts<2>(P, sP, at, n, rest);
+    sum_parts<2>(P, q.part(), at, n, rest);
   };
   for (int k = 512 * KEEP + 2 * threadIdx.x; k < q.cols; k += 512) {
     fetch(k);
@@ -117,7 +106,7 @@ __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSu
   for (int w = 0; w < 8; ++w) e = max(e, se[w]);
   if (threadIdx.x == 0) exps[r] = e == NONE ? 0 : e + eb[r] - 16 - S;
   auto put = [&](int k, long long v0, long long v1) {
-    store_real_digits(out, r, k, k < q.cols ? shift_round(v0, ea[k] - e + XBITS) : 0,
+    store_digits(out, 0, r, k, k < q.cols ? shift_round(v0, ea[k] - e + XBITS) : 0,
                       k + 1 < q.cols ? shift_round(v1, ea[k + 1] - e + XBITS) : 0);
   };
 #pragma unroll
@@ -134,7 +123,7 @@ __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSu
 constexpr int FIN_COLS = 4;                  // columns per thread of a finish pass
 
 // Entries k of row r at l = l0 + 256 i of a product.
-__device__ __forceinline__ void row_entries(const PartialSums<long long>& q, const uint8_t* parts, int r, int l0,
+__device__ __forceinline__ void row_entries(const PartialSums& q, const uint8_t* parts, int r, int l0,
                                             long long (&v)[FIN_COLS]) {
   size_t at[FIN_COLS];
   int n[FIN_COLS];
@@ -144,7 +133,7 @@ __device__ __forceinline__ void row_entries(const PartialSums<long long>& q, con
     at[i] = l;
     n[i] = l < q.cols ? parts[l / BM] : 0;
   }
-  sum_parts<FIN_COLS>(q.P + (size_t)r * q.ld, (size_t)q.rows * q.ld, at, n, v);
+  sum_parts<FIN_COLS>(q.P + (size_t)r * q.ld, q.part(), at, n, v);
 }
 
 __device__ __forceinline__ double block_sum(double v, double* sm) {      // 256 threads; thread 0 has the sum
@@ -158,7 +147,7 @@ __device__ __forceinline__ double block_sum(double v, double* sm) {      // 256 
 }
 
 struct FinishReal {
-  PartialSums<long long> q;
+  PartialSums q;
   const int *ea, *eb;
   int S;
   const int* status;         // [0] expired wait, [1] non-finite input
@@ -178,7 +167,7 @@ __global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, c
   __shared__ double sm[8];
   const bool plain = p.status[0] != 0 || p.status[1] != 0;
   double* T = scratch + (size_t)k * N;       // plain: row k of C img (P's memory)
-  count_parts(p.q, 0, k, parts);
+  count_parts<1>(p.q, 0, k, parts);
   if (plain) {
     for (int j = threadIdx.x; j < N; j += 256) {
       double t = 0.0;
@@ -226,7 +215,7 @@ __global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ double sm[8];
   const bool plain = p.status[0] != 0 || p.status[1] != 0;
-  count_parts(p.q, 0, k, parts);
+  count_parts<1>(p.q, 0, k, parts);
   double s = 0.0;
   for (int l0 = threadIdx.x; l0 < S; l0 += 256 * FIN_COLS) {
     long long z[FIN_COLS];
@@ -256,7 +245,7 @@ __global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p
 }
 
 // ------------------------------------------------------------------ host ---
-DigitRows real_rows(uint16_t* base, int L, int K) { return DigitRows{base, L, round_up(K, BK), -1}; }
+DigitRows real_rows(uint16_t* base, int L, int K) { return DigitRows{base, L, round_up(K, BK), 1}; }
 
 // Two products of one sandwich: X is p x q (rows of K = q), R has rows r of
 // length q, L rows r of length p (both sides have the same operator here).
@@ -271,8 +260,8 @@ struct Sandwich {
     band.step = step;
     band.total = total;
     band.count = step ? std::min(total, (96 * step + 68) / 64 + 2) : total;
-    deal1 = deal_of(p, r, BN, band.count, 1);                 // A: X's rows, B: operator rows
-    deal2 = deal_of(r, r, BN, band.count, 1);                 // A: rows of the first product
+    deal1 = deal_of(p, r, band.count, 1);                 // A: X's rows, B: operator rows
+    deal2 = deal_of(r, r, band.count, 1);                 // A: rows of the first product
     ld1 = round_up(p, BM);
     ld2 = round_up(r, BM);
     P_entries = std::max((size_t)r * ld1 * max_parts(deal1), (size_t)r * ld2 * max_parts(deal2));
@@ -312,18 +301,18 @@ Space carve(const Sandwich& w, void* ws) {
 
 template <typename Rows>
 int run_sandwich(const Sandwich& w, const Space& t, const double* X, const Rows& op, cudaStream_t s) {
-  const int S = unit_shift(w.q);
+  const int S = unit_shift(w.q, 1);
   const DigitRows dX = real_rows(t.dX, w.p, w.q), dR = real_rows(t.dR, w.r, w.q), dT = real_rows(t.dT, w.r, w.p);
   LGB_CUDA(cudaMemsetAsync(t.status, 0, 2 * sizeof(int), s));
   slice_real_kernel<<<w.p, 256, 0, s>>>(DenseRows{X, w.q}, dX, t.eX, t.status + 1);
   slice_real_kernel<<<w.r, 256, 0, s>>>(op, dR, t.eR, t.status + 1);
   LGB_CUDA(cudaGetLastError());
-  int st = launch_gemm<ND, ND, true>(dX, 1, dR, 1, 1, w.deal1, w.band, S, t.P, 0, w.ld1, t.status, s);
+  int st = launch_gemm(dX, 1, dR, 1, 1, w.q, w.deal1, w.band, S, t.P, 0, w.ld1, t.status, s);
   if (st) return st;
-  slice_real_product_kernel<<<w.r, 256, 0, s>>>(PartialSums<long long>{t.P, 0, w.ld1, w.r, w.p, w.deal1}, t.eX,
+  slice_real_product_kernel<<<w.r, 256, 0, s>>>(PartialSums{t.P, 0, w.ld1, w.r, w.p, w.deal1}, t.eX,
                                                 t.eR, S, dT, t.eT);
   LGB_CUDA(cudaGetLastError());
-  return launch_gemm<ND, ND, true>(dT, 1, dR, 1, 1, w.deal2, w.band, S, t.P, 0, w.ld2, t.status, s);
+  return launch_gemm(dT, 1, dR, 1, 1, w.q, w.deal2, w.band, S, t.P, 0, w.ld2, t.status, s);
 }
 
 }  // namespace
@@ -336,7 +325,7 @@ int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, dou
   const Space t = carve(w, ws);
   const int st = run_sandwich(w, t, img, CirculantRows{c, N}, s);
   if (st) return st;
-  const FinishReal f{PartialSums<long long>{t.P, 0, w.ld2, N, N, w.deal2}, t.eT, t.eR, unit_shift(N), t.status,
+  const FinishReal f{PartialSums{t.P, 0, w.ld2, N, N, w.deal2}, t.eT, t.eR, unit_shift(N, 1), t.status,
                      P, sums};
   finish_pixel_kernel<<<N, 256, 0, s>>>(f, img, c, reinterpret_cast<double*>(t.P), os, d, sums + 1);
   LGB_CUDA(cudaGetLastError());
@@ -351,7 +340,7 @@ int launch_resample_sliced(const double* P, int N, int os, int S, const double* 
   const Space t = carve(w, ws);
   const int st = run_sandwich(w, t, P, BandedRows{Gt, q0, N, S}, s);
   if (st) return st;
-  const FinishReal f{PartialSums<long long>{t.P, 0, w.ld2, S, S, w.deal2}, t.eT, t.eR, unit_shift(N), t.status,
+  const FinishReal f{PartialSums{t.P, 0, w.ld2, S, S, w.deal2}, t.eT, t.eR, unit_shift(N, 1), t.status,
                      raw, sum};
   finish_resample_kernel<<<S, 256, 0, s>>>(f, P, Gt, q0, N);
   LGB_CUDA(cudaGetLastError());

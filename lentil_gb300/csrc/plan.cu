@@ -63,8 +63,8 @@ static size_t carve_sliced(void* ws, int count, int m, int n, int M, int N, Dft2
   Carve c(ws);
   Dft2SlicedSpace t;
   t.ws = c.take<char>(sliced_dft2_workspace(count, m, n, M, N, sliced_left(m, n, M, N)));
-  t.e1 = c.take<uint16_t>(sliced_matrix_entries(m, M, true));
-  t.e2 = c.take<uint16_t>(sliced_matrix_entries(n, N, !sliced_left(m, n, M, N)));
+  t.e1 = c.take<uint16_t>(sliced_matrix_entries(m, M));
+  t.e2 = c.take<uint16_t>(sliced_matrix_entries(n, N));
   if (s) *s = t;
   return c.used;
 }
@@ -160,8 +160,8 @@ int lgb::dft2_batch(const double2* fin, int count, int m, int n, double2* Fout, 
     q.scale = scale;
     q.f = fin;
     q.F = Fout;
-    if ((st = launch_matrix_digits(ar, nullptr, 1, m, M, true, w.e1, s))) return st;
-    if ((st = launch_matrix_digits(ac, nullptr, 1, n, N, !q.left, w.e2, s))) return st;
+    if ((st = launch_matrix_digits(ar, nullptr, 1, m, M, w.e1, s))) return st;
+    if ((st = launch_matrix_digits(ac, nullptr, 1, n, N, w.e2, s))) return st;
     return launch_sliced_dft2(q, w.ws, s);
   }
   if (precision == LGB_FP64) {
@@ -366,8 +366,8 @@ static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
   } else {
     const size_t Q = (size_t)B * L;
     if (P->sliced) {
-      P->d1 = c.take<uint16_t>(L * sliced_matrix_entries(d.m, d.M, true));
-      P->d2 = c.take<uint16_t>(L * sliced_matrix_entries(d.n, d.N, false));
+      P->d1 = c.take<uint16_t>(L * sliced_matrix_entries(d.m, d.M));
+      P->d2 = c.take<uint16_t>(L * sliced_matrix_entries(d.n, d.N));
       P->sliced_ws = c.take<char>(sliced_dft2_workspace(L, d.m, d.n, d.M, d.N, true));
     } else {
       P->E1 = c.take<double2>((size_t)L * d.M * d.m);
@@ -477,8 +477,8 @@ static int build_plan(lgb_psf_plan_s* P, cudaStream_t s, lgb_psf_plan* plan) {
     st = launch_e1_block_split(P->axes, L, d.m, d.M, P->kp1, cdiv(d.M, 64) * 128, bf16, P->e1h, P->e1l, s);
     if (!st) st = launch_e2_block_split(P->axes + L, L, d.n, d.N, P->kp2, cdiv(d.N, 128) * 256, bf16, P->e2h, P->e2l, s);
   } else if (P->sliced) {
-    st = launch_matrix_digits(PhaseAxis{}, P->axes, L, d.m, d.M, true, P->d1, s);
-    if (!st) st = launch_matrix_digits(PhaseAxis{}, P->axes + L, L, d.n, d.N, false, P->d2, s);
+    st = launch_matrix_digits(PhaseAxis{}, P->axes, L, d.m, d.M, P->d1, s);
+    if (!st) st = launch_matrix_digits(PhaseAxis{}, P->axes + L, L, d.n, d.N, P->d2, s);
   } else {
     for (int l = 0; l < L && !st; ++l) {
       st = launch_dft_matrix_c128(axes[l], d.m, d.M, P->E1 + (size_t)l * d.M * d.m, true, s);

@@ -8,9 +8,8 @@
 //   - every vector of a contraction (a column of f, a row of E1, ...) is
 //     scaled by a power of two above its largest entry and cut into signed
 //     digits of 9 bits, |d| <= 256, each exact in bf16; digit i is stored as
-//     d 2^(-9 i).  Data has ND = 7 digits (62 bits below the vector's largest
-//     entry: with 54, fields with isolated spikes lost a factor of two against
-//     FP64), a DFT matrix NE = 6 (its entries are 53-bit numbers of modulus 1);
+//     d 2^(-9 i).  Seven digits hold 62 bits below the vector's largest entry
+//     (with six, fields with isolated spikes lost a factor of two against FP64);
 //   - the products of digits with i + j <= 6 are kept, grouped by s = i + j.  A
 //     group's sum over 64 K entries is at most (s + 1) 64 2^16 <= 2^24 units
 //     for s <= 3: the FP32 accumulators hold it exactly, whatever order or
@@ -24,12 +23,13 @@
 // What is left is the rounding of the operands, the products left out, and one
 // rounding per stored result; an FP64 accumulation rounds at every K step.
 //
-// A complex product needs no complex arithmetic on the way: operand B holds
-// the row sets [-im | re | im], operand A the sets [re | im], and a tile's
-// columns are 48 real and the same 48 imaginary parts,
-//     A re rows x (B re, B im rows)  +  A im rows x (B -im, B re rows),
-// so that the accumulators hold the complex sums.  Real operands have one set
-// and a tile 96 columns.
+// A complex product is three real ones (Gauss): operands hold the row sets re,
+// im and h = (re + im) / 2, the products of like sets are
+//     P0 = Ar Br,  P1 = Ai Bi,  P2 = 2 Ah Bh,
+// and readers form re = P0 - P1, im = 2 P2 - P0 - P1 in integers, which loses
+// nothing.  That is 84 digit products where four real products took 108 (a DFT
+// matrix had six digits then): 1019 x 941 to 1024^2 went from 337 to 300 us,
+// 512^2 from 82 to 76.
 #pragma once
 
 #include <algorithm>
@@ -45,31 +45,28 @@ namespace {
 
 using namespace tc;
 
-
-constexpr int ND = 7;                        // digits of a data operand (f, the intermediate)
-constexpr int NE = 6;                        // digits of a DFT matrix (|E| <= 1, 53-bit entries)
+constexpr int ND = 7;                        // digits per entry
 constexpr int BETA = 9;                      // bits per digit
-constexpr int BM = 128, BC = 48, BK = 32;    // tile: A rows, complex B rows, K per stage
-constexpr int BN = 2 * BC;                   // MMA columns
+constexpr int BM = 128, BN = 96, BK = 32;    // tile: A rows, B rows, K per stage
 constexpr int STAGES = 2;
 constexpr int GROUPS = 5;                    // accumulators: s = 0, 1, 2, 3, and 4 to 6 together
 constexpr uint32_t A_SLICE = BM * BK * 2, B_SLICE = BN * BK * 2;
-constexpr uint32_t stage_bytes(int na, int nb) { return na * A_SLICE + nb * B_SLICE; }
+constexpr uint32_t A_STAGE = ND * A_SLICE, STAGE_BYTES = ND * (A_SLICE + B_SLICE);
 constexpr int EPI_WARPS = 8;
 constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t BAR_BYTES = 256;
-constexpr uint32_t smem_bytes(int na, int nb) { return STAGES * stage_bytes(na, nb) + BAR_BYTES + 1024; }
-constexpr int RUN = BC / 2;                  // tile columns per epilogue warp, of either half
+constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
+constexpr int RUN = BN / 2;                  // tile columns per epilogue warp
 constexpr unsigned long long WAIT_NS = 2000000000ull;
-static_assert(smem_bytes(ND, ND) <= 232448, "shared memory per CTA");
-static_assert(GROUPS * BN <= 512 && RUN == 24, "tensor memory columns; the drain loads 3 x 8 of them");
+static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
+static_assert(GROUPS * BN <= 512 && RUN == 48, "tensor memory columns; the drain loads 3 x 16 of them");
 
-// How a launch's work is dealt out: the chains (two stages of one tile: 32
-// complex K entries, or 64 real ones) of all tiles in a row, `per` of them to
-// each CTA.  A tile's chains then lie in
-// one CTA or in a few neighbouring ones, which write a partial sum each.
+// How a launch's work is dealt out: the chains (64 K entries of one tile) of all
+// tiles of all products in a row, `per` of them to each CTA.  A tile's chains
+// then lie in one CTA or in a few neighbouring ones, which write a partial sum
+// each.
 struct Deal {
-  int tilesA, tilesB;        // tiles of one item: A rows (fastest), B rows
+  int tilesA, tilesB;        // tiles of one product: A rows (fastest), B rows
   int chains;                // per tile
   int per;                   // chains per CTA
   __host__ __device__ int first_cta(int tile) const { return tile * chains / per; }
@@ -78,7 +75,7 @@ struct Deal {
   }
 };
 
-// Which chains of a real contraction a column tile takes: all, or, for a
+// Which chains of a contraction a column tile takes: all, or, for a
 // banded operand B whose row k covers K entries around k * step, a window.
 struct Band {
   int step;                  // 0: all chains
@@ -92,37 +89,38 @@ struct Band {
 
 struct GemmParams {
   Deal deal;
-  Band band;                 // real contractions
-  int total;                 // chains of all tiles of all items
-  int rowsB;                 // complex
+  Band band;
+  int total;                 // chains of all tiles of all products
+  int sets;                  // products per item
+  int stages;                // of BK along K
+  int rowsB;
   int ld;                    // P row pitch (entries)
   int dA, dB;                // digit planes between items (0: shared by all items)
-  int S;                     // P unit: 2^-(16 + S) of the scaled operands
-  void* P;                   // [item][part][rowsB][ld] longlong2 (re, im), or long long
-  long long item_stride;     // entries between items
+  int S;                     // P unit: 2^-(16 + S) of the scaled operands, half that for P2
+  long long* P;              // [product][part][rowsB][ld]
+  long long stride;          // entries between products
   int* err;
   unsigned long long wait_ns;
 };
 
 // One CTA's run of chains of one tile.
 struct Segment {
-  int item, m0, n0;          // tile origin: complex A row, B row
+  int product, m0, n0;       // tile origin: A row, B row
   int chain, count;
   int part;                  // which of the tile's partial sums
 };
-template <bool REAL>
 __device__ __forceinline__ Segment segment_at(const GemmParams& p, int pos, int end) {
   Segment s;
   const int tile = pos / p.deal.chains;
   s.chain = pos - tile * p.deal.chains;
   s.count = min(p.deal.chains - s.chain, end - pos);
   const int tiles = p.deal.tilesA * p.deal.tilesB;
-  s.item = tile / tiles;
-  const int t = tile - s.item * tiles;
+  s.product = tile / tiles;
+  const int t = tile - s.product * tiles;
   const int tb = t / p.deal.tilesA;
   s.m0 = (t - tb * p.deal.tilesA) * BM;
-  s.n0 = tb * (REAL ? BN : BC);
-  if (REAL) s.chain += p.band.first(tb);
+  s.n0 = tb * BN;
+  s.chain += p.band.first(tb);
   s.part = (int)blockIdx.x - p.deal.first_cta(tile);
   return s;
 }
@@ -135,7 +133,8 @@ __device__ __forceinline__ bool starts(int g, int r) {
   return g == 0 ? (r & 3) == 0 : g == 1 ? (r & 1) == 0 : true;
 }
 __device__ __forceinline__ bool drains(int g, int r, int count) {
-  return g == 0 ? (r & 3) == 3 || r == count - 1 : g == 1 ? (r & 1) == 1 || r == count - 1 : true;
+  if (r == count - 1) return true;
+  return g == 0 ? (r & 3) == 3 : g == 1 ? (r & 1) == 1 : true;
 }
 
 // The digit products A_i B_j of one sum i + j, two k-steps each, added to the
@@ -143,39 +142,35 @@ __device__ __forceinline__ bool drains(int g, int r, int count) {
 // one 64-bit base each plus constants, and the warp stays converged around
 // them: with descriptors worked out per MMA, or in a loop that one lane runs
 // alone, the issuing warp was the limit, at 95 to 100 clk an MMA.
-template <int NA, int NB, int SUM>
+template <int SUM>
 __device__ __forceinline__ void mma_sum(uint32_t on, uint32_t d, uint64_t da, uint64_t db, uint32_t idesc,
                                         bool fresh) {
 #pragma unroll
-  for (int i = 0; i < NA; ++i) {
-    const int j = SUM - i;
-    if (j < 0 || j >= NB) continue;
+  for (int i = 0; i <= SUM; ++i) {
 #pragma unroll
-    for (int k = 0; k < BK / 16; ++k) {
-      const bool start = fresh && k == 0 && (i == 0 || SUM - i == NB - 1);   // the first one issued
-      mma_f16_cta(on, d, da + ((i * A_SLICE + k * 32) >> 4), db + ((j * B_SLICE + k * 32) >> 4), idesc,
-                  start ? 0u : 1u);
-    }
+    for (int k = 0; k < BK / 16; ++k)
+      mma_f16_cta(on, d, da + ((i * A_SLICE + k * 32) >> 4), db + (((SUM - i) * B_SLICE + k * 32) >> 4), idesc,
+                  fresh && i == 0 && k == 0 ? 0u : 1u);
   }
 }
 
 // P over this CTA's chains.
 //
-// Bound by the tensor pipe: 108 MMAs (27 digit products x 4 k-steps; 112 for
-// two data operands) of 128 x 96 x 16 per chain.  96 columns is the widest tile whose five
+// Bound by the tensor pipe: 112 MMAs (28 digit products x 4 k-steps) of
+// 128 x 96 x 16 per chain.  96 columns is the widest tile whose five
 // accumulators fit the 512 TMEM columns; the MMA then reads 7 KB of shared
 // memory per 48 clocks (149 B/clk against the 128 B/clk port), so it runs at
-// 56 clk at best.  Roles: warp 0 TMA (two stages of 32 K entries, all digits),
+// 56 clk at best; the 98 KB that TMA writes per stage share that port, which
+// makes it 3900 clk a stage (1019 x 941 to 1024^2: 92 us of MMAs at 56 clk in
+// 119).  Roles: warp 0 TMA (two stages of 32 K entries, all digits),
 // warp 1 MMA issue, warps 2..9 drain (lane quadrant w % 4, column half
 // (w - 2) / 4).  The groups are drained one by one, in the order they are
 // issued, while the next ones run.  One CTA per SM takes its share of the
 // chains (Deal), so the pipeline fills once per launch and no wave is partly
 // empty.
-template <int NA, int NB, bool REAL>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const GemmParams p) {
-  constexpr uint32_t A_STAGE = NA * A_SLICE, STAGE_BYTES = stage_bytes(NA, NB);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -220,15 +215,17 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       int it = 0;
       bool ok = true;
       for (int pos = begin; ok && pos < end;) {
-        const Segment w = segment_at<REAL>(p, pos, end);
+        const Segment w = segment_at(p, pos, end);
         pos += w.count;
-        for (int st = 2 * w.chain; st < 2 * (w.chain + w.count); ++st, ++it) {
-          const int s = it % STAGES, im = st & 1, k = (REAL ? st : st >> 1) * BK;
+        const int item = w.product / p.sets, set = w.product - item * p.sets;
+        const int last = min(p.stages, 2 * (w.chain + w.count));
+        for (int st = 2 * w.chain; st < last; ++st, ++it) {
+          const int s = it % STAGES;
           if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, p.err, p.wait_ns)) { ok = false; break; }
           mbar_expect_tx(full_bar(s), STAGE_BYTES);
           const uint32_t sa = base + s * STAGE_BYTES;
-          tma_load_4d_cta(sa, &tmA, full_bar(s), k, w.m0, REAL ? 0 : im, w.item * p.dA);
-          tma_load_4d_cta(sa + A_STAGE, &tmB, full_bar(s), k, w.n0, REAL ? 0 : 1 - im, w.item * p.dB);
+          tma_load_4d_cta(sa, &tmA, full_bar(s), st * BK, w.m0, set, item * p.dA);
+          tma_load_4d_cta(sa + A_STAGE, &tmB, full_bar(s), st * BK, w.n0, set, item * p.dB);
         }
       }
       for (int k = max(0, it - STAGES); k < it; ++k)       // issued copies land before exit
@@ -245,29 +242,31 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     int n[GROUPS] = {};                        // drains asked for, by group
     bool ok = true;
     for (int pos = begin; ok && pos < end;) {
-      const Segment w = segment_at<REAL>(p, pos, end);
+      const Segment w = segment_at(p, pos, end);
       pos += w.count;
-      for (int st = 0; ok && st < 2 * w.count; ++st, ++it) {
+      const int stages = min(p.stages - 2 * w.chain, 2 * w.count);
+      for (int st = 0; ok && st < stages; ++st, ++it) {
         const int s = it % STAGES, r = st >> 1;
+        const bool ends = (st & 1) == 1 || st == stages - 1;      // of a chain
         if (!wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
         const uint64_t da = smem_desc_sw64(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw64(base + s * STAGE_BYTES + A_STAGE);
 #pragma unroll
         for (int g = GROUPS - 1; g >= 0; --g) {
-          const bool first = (st & 1) == 0 && starts(g, r), last = (st & 1) == 1 && drains(g, r, w.count);
+          const bool first = (st & 1) == 0 && starts(g, r), last = ends && drains(g, r, w.count);
           // this accumulator's previous sum has been drained
           if (first && !wait(acc_empty(g), (n[g] & 1) ^ 1)) { ok = false; break; }
           tc_fence_after();
           const uint32_t d = tmem + g * BN;
           if (g == 4) {                        // small products first
-            mma_sum<NA, NB, 6>(on, d, da, db, idesc, first);
-            mma_sum<NA, NB, 5>(on, d, da, db, idesc, false);
-            mma_sum<NA, NB, 4>(on, d, da, db, idesc, false);
+            mma_sum<6>(on, d, da, db, idesc, first);
+            mma_sum<5>(on, d, da, db, idesc, false);
+            mma_sum<4>(on, d, da, db, idesc, false);
           }
-          if (g == 3) mma_sum<NA, NB, 3>(on, d, da, db, idesc, first);
-          if (g == 2) mma_sum<NA, NB, 2>(on, d, da, db, idesc, first);
-          if (g == 1) mma_sum<NA, NB, 1>(on, d, da, db, idesc, first);
-          if (g == 0) mma_sum<NA, NB, 0>(on, d, da, db, idesc, first);
+          if (g == 3) mma_sum<3>(on, d, da, db, idesc, first);
+          if (g == 2) mma_sum<2>(on, d, da, db, idesc, first);
+          if (g == 1) mma_sum<1>(on, d, da, db, idesc, first);
+          if (g == 0) mma_sum<0>(on, d, da, db, idesc, first);
           if (last) {
             mma_commit_cta(on, acc_full(g));
             ++n[g];
@@ -282,16 +281,17 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   } else {
     const int q4 = warp & 3, ch = (warp - 2) >> 2;
     const uint32_t trow = tmem + ((uint32_t)(q4 * 32) << 16) + ch * RUN;
-    const float unit4 = ldexpf(1.f, p.S);
-    const int m1 = 1 << (p.S - BETA), m2 = 1 << (p.S - 2 * BETA), m3 = 1 << (p.S - 3 * BETA);
     int n[GROUPS] = {};                        // drains done, by group
     bool ok = true;
     for (int pos = begin; ok && pos < end;) {
-      const Segment w = segment_at<REAL>(p, pos, end);
+      const Segment w = segment_at(p, pos, end);
       pos += w.count;
-      long long acc[2 * RUN];                  // RUN real parts, RUN imaginary parts (or 2 RUN columns)
+      const int S = p.S + (w.product % p.sets == 2);
+      const float unit4 = ldexpf(1.f, S);
+      const int m1 = 1 << (S - BETA), m2 = 1 << (S - 2 * BETA), m3 = 1 << (S - 3 * BETA);
+      long long acc[RUN];
 #pragma unroll
-      for (int j = 0; j < 2 * RUN; ++j) acc[j] = 0;
+      for (int j = 0; j < RUN; ++j) acc[j] = 0;
       for (int k = 0; ok && k < w.count; ++k) {
 #pragma unroll
         for (int g = GROUPS - 1; g >= 0; --g) {
@@ -300,41 +300,31 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           if (!ok) break;
           ++n[g];
           tc_fence_after();
-          uint32_t r[2 * RUN];
+          uint32_t r[RUN];
 #pragma unroll
-          for (int h = 0; h < 6; ++h) tmem_ld8(trow + g * BN + (h / 3) * BC + (h % 3) * 8, r + h * 8);
+          for (int h = 0; h < RUN / 16; ++h) tmem_ld16(trow + g * BN + h * 16, r + h * 16);
           tmem_ld_wait();
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(acc_empty(g));
 #pragma unroll
-          for (int j = 0; j < 2 * RUN; ++j) {
+          for (int j = 0; j < RUN; ++j) {
             const float v = __uint_as_float(r[j]);
             if (g == 4) acc[j] += (long long)__float2int_rn(v * unit4);
             else if (g == 3) acc[j] += (long long)__float2int_rn(v * 0x1p27f) * m3;
             else if (g == 2) acc[j] += (long long)__float2int_rn(v * 0x1p18f) * m2;
             else if (g == 1) acc[j] += (long long)__float2int_rn(v * 0x1p9f) * m1;
-            else acc[j] += (long long)__float2int_rn(v) << p.S;
+            else acc[j] += (long long)__float2int_rn(v) << S;
           }
         }
       }
       if (!ok) break;
       const int n0 = w.n0 + ch * RUN;
-      const size_t at = (size_t)w.item * p.item_stride + ((size_t)w.part * p.rowsB + n0) * p.ld + w.m0 +
-                        q4 * 32 + lane;
-      if (REAL) {
-        long long* out = static_cast<long long*>(p.P) + at;
+      long long* out = p.P + (size_t)w.product * p.stride + ((size_t)w.part * p.rowsB + n0) * p.ld + w.m0 +
+                       q4 * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < 2 * RUN; ++j) {
-          const int col = j < RUN ? j : BC + j - RUN;
-          if (n0 + col < p.rowsB) out[(size_t)col * p.ld] = acc[j];
-        }
-      } else {
-        longlong2* out = static_cast<longlong2*>(p.P) + at;
-#pragma unroll
-        for (int j = 0; j < RUN; ++j)
-          if (n0 + j < p.rowsB) out[(size_t)j * p.ld] = make_longlong2(acc[j], acc[RUN + j]);
-      }
+      for (int j = 0; j < RUN; ++j)
+        if (n0 + j < p.rowsB) out[(size_t)j * p.ld] = acc[j];
     }
   }
 
@@ -347,19 +337,16 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---------------------------------------------------------------- digits ---
-// The N digits of X, |X| <= 2^(9 N - 1), as bf16 bits in the high half of a
-// word; digit i carries 2^(-9 i).  A bias of 256 in every place turns the
+// The digits of X, |X| <= 2^62, as bf16 bits in the high half of a word; digit i carries 2^(-9 i).  A bias of 256 in every place turns the
 // signed digits into bit fields; a field under the exponent of 1.5 2^23 is a
 // float, and one FMA takes bias and offset off and scales (exactly): three
 // instructions a digit, none of them on the conversion or 64-bit paths.
-template <int N>
-__device__ __forceinline__ void digits_of(long long X, uint32_t (&d)[N]) {
-  constexpr unsigned long long ones = 0x0040201008040201ull;          // sum of 2^(9 i), i < 7
-  constexpr unsigned long long bias = 256ull * (ones & ((1ull << (BETA * (N - 1))) - 1));
+__device__ __forceinline__ void digits_of(long long X, uint32_t (&d)[ND]) {
+  constexpr unsigned long long bias = 256ull * 0x0000201008040201ull;   // 256 sum of 2^(9 i), i < 6
   const unsigned long long Y = (unsigned long long)X + bias;
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const int sh = BETA * (N - 1 - i);
+  for (int i = 0; i < ND; ++i) {
+    const int sh = BETA * (ND - 1 - i);
     const float s = 1.f / (float)(1ull << (BETA * i));
     // the leading digit is signed: 512 more keep its field positive
     const uint32_t u = (uint32_t)(Y >> sh) + (i == 0 ? 512u : 0u);
@@ -383,7 +370,7 @@ __device__ __forceinline__ double scaled(long long v, int e, double scale) {
   return scale * __longlong_as_double((long long)(q | ((unsigned long long)v & 0x8000000000000000ull)));
 }
 
-constexpr int XBITS = BETA * ND - 1;         // a data entry is |X| < 2^62 of its vector's scale
+constexpr int XBITS = BETA * ND - 1;         // an entry is |X| <= 2^62 of its vector's scale
 
 // x / 2^(e - 1022) * 2^XBITS rounded to nearest, for |x| < 2^(e - 1022); e is
 // a biased exponent >= 1 that is no smaller than x's.
@@ -398,34 +385,34 @@ __device__ __forceinline__ long long fixed_data(double x, int e) {
   return (long long)u < 0 ? -m : m;
 }
 
-// Digit operand of L vectors, [digit][set][L][kp] 16-bit entries: the sets of
-// complex vectors are re, im (operand A, b = 0), or -im, re, im (operand B,
-// b = 1); real ones have one (b = -1).
+// Digit operand of L vectors, [digit][set][L][kp] 16-bit entries.  Complex
+// vectors have three sets (re, im, (re + im) / 2), real ones one.
 struct DigitRows {
   uint16_t* base;
-  int L, kp, b;
+  int L, kp, sets;
   __host__ __device__ size_t set() const { return (size_t)L * kp; }
-  __host__ __device__ size_t plane() const { return (2 + b) * set(); }
+  __host__ __device__ size_t plane() const { return sets * set(); }
 };
-// Entries k, k + 1 of vector j.
-template <int N>
-__device__ __forceinline__ void store_digits(const DigitRows& o, int j, int k, long long re0, long long im0,
-                                             long long re1, long long im1) {
-  uint16_t* p = o.base + (size_t)j * o.kp + k;
-  uint32_t a[N], c[N];
-  digits_of(im0, a);
-  digits_of(im1, c);
+// Entries k, k + 1 of vector j in one set.
+__device__ __forceinline__ void store_digits(const DigitRows& o, int set, int j, int k, long long v0,
+                                             long long v1) {
+  uint16_t* p = o.base + set * o.set() + (size_t)j * o.kp + k;
+  uint32_t a[ND], c[ND];
+  digits_of(v0, a);
+  digits_of(v1, c);
 #pragma unroll
-  for (int i = 0; i < N; ++i) {
-    const uint32_t w = __byte_perm(a[i], c[i], 0x7632);
-    *reinterpret_cast<uint32_t*>(p + i * o.plane() + (1 + o.b) * o.set()) = w;
-    if (o.b) *reinterpret_cast<uint32_t*>(p + i * o.plane()) = w ^ 0x80008000u;
-  }
-  digits_of(re0, a);
-  digits_of(re1, c);
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    *reinterpret_cast<uint32_t*>(p + i * o.plane() + o.b * o.set()) = __byte_perm(a[i], c[i], 0x7632);
+  for (int i = 0; i < ND; ++i)
+    *reinterpret_cast<uint32_t*>(p + i * o.plane()) = __byte_perm(a[i], c[i], 0x7632);
+}
+// (a + b) / 2, to even: a rounding to one side would add up
+__device__ __forceinline__ long long half_sum(long long a, long long b) {
+  const long long h = (a >> 1) + (b >> 1) + (a & b & 1);
+  return h + ((a ^ b) & h & 1);
+}
+__device__ __forceinline__ void store_digits3(const DigitRows& o, int j, int k, longlong2 z0, longlong2 z1) {
+  store_digits(o, 0, j, k, z0.x, z1.x);
+  store_digits(o, 1, j, k, z0.y, z1.y);
+  store_digits(o, 2, j, k, half_sum(z0.x, z0.y), half_sum(z1.x, z1.y));
 }
 
 constexpr int FLAG_INF = 1, FLAG_NAN = 2;
@@ -439,48 +426,78 @@ __device__ __forceinline__ void note_exponent(double x, int& e, int& flag) {
     e = max(e, E);
 }
 
-// A product's rows as their readers see them.
-template <typename V>
+// A GEMM's products as their readers see them.
 struct PartialSums {
-  const V* P;                // [item][part][rows][ld]
-  long long item_stride;
+  const long long* P;        // [product][part][rows][ld]
+  long long stride;          // entries between products
   int ld, rows, cols;
   Deal deal;
+  __device__ __forceinline__ int parts(int product, int r, int a) const {
+    return deal.parts((product * deal.tilesB + r / BN) * deal.tilesA + a / BM);
+  }
+  __device__ __forceinline__ size_t part() const { return (size_t)rows * ld; }     // entries between parts
 };
 
 constexpr int MAX_TILES_A = 256;             // 128-row tiles of the longest A operand (32768 rows)
 
-// How many partial sums the tiles under row r of an item have, [tilesA] in
-// shared memory (ends with a block barrier).
-template <typename V>
-__device__ __forceinline__ void count_parts(const PartialSums<V>& q, int item, int r, uint8_t* parts) {
-  constexpr int width = sizeof(V) == 16 ? BC : BN;           // rows of a tile
-  for (int t = threadIdx.x; t < q.deal.tilesA; t += blockDim.x)
-    parts[t] = (uint8_t)q.deal.parts((item * q.deal.tilesB + r / width) * q.deal.tilesA + t);
+// How many partial sums the tiles under row r have, in COUNT products from the
+// given one: [COUNT][tilesA] in shared memory (ends with a block barrier).
+template <int COUNT>
+__device__ __forceinline__ void count_parts(const PartialSums& q, int product, int r, uint8_t* parts) {
+  for (int t = threadIdx.x; t < COUNT * q.deal.tilesA; t += blockDim.x) {
+    const int c = t / q.deal.tilesA;
+    parts[t] = (uint8_t)q.parts(product + c, r, (t - c * q.deal.tilesA) * BM);
+  }
   __syncthreads();
 }
 
-__device__ __forceinline__ void add_to(long long& a, long long b) { a += b; }
-__device__ __forceinline__ void add_to(longlong2& a, longlong2 b) { a.x += b.x; a.y += b.y; }
-
 // v[i] = the sum of n[i] parts (0: none) of the entry at offset at[i], i < COUNT.
 // The parts go in the outer loop, so that COUNT loads are in flight.
-template <int COUNT, typename V>
-__device__ __forceinline__ void sum_parts(const V* __restrict__ P, size_t part_stride, const size_t (&at)[COUNT],
-                                          const int (&n)[COUNT], V (&v)[COUNT]) {
+template <int COUNT>
+__device__ __forceinline__ void sum_parts(const long long* __restrict__ P, size_t part, const size_t (&at)[COUNT],
+                                          const int (&n)[COUNT], long long (&v)[COUNT]) {
   int most = 0;
 #pragma unroll
   for (int i = 0; i < COUNT; ++i) {
     most = max(most, n[i]);
-    v[i] = V{};
+    v[i] = 0;
   }
-  for (int k = 0; k < most; ++k, P += part_stride) {
-    V w[COUNT];
+  for (int k = 0; k < most; ++k, P += part) {
+    long long w[COUNT];
 #pragma unroll
-    for (int i = 0; i < COUNT; ++i) w[i] = k < n[i] ? P[at[i]] : V{};
+    for (int i = 0; i < COUNT; ++i) w[i] = k < n[i] ? P[at[i]] : 0;
 #pragma unroll
-    for (int i = 0; i < COUNT; ++i) add_to(v[i], w[i]);
+    for (int i = 0; i < COUNT; ++i) v[i] += w[i];
   }
+}
+
+// The same for complex entries: n[c][i] parts of product c, 3 COUNT loads in
+// flight.  2 P2 may wrap, what is left of it does not.
+template <int COUNT>
+__device__ __forceinline__ void sum_parts3(const long long* __restrict__ P, size_t stride, size_t part,
+                                           const size_t (&at)[COUNT], const int (&n)[3][COUNT],
+                                           longlong2 (&v)[COUNT]) {
+  int most = 0;
+  unsigned long long re[COUNT], im[COUNT];
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) {
+    most = max(most, max(n[0][i], max(n[1][i], n[2][i])));
+    re[i] = im[i] = 0;
+  }
+  for (int k = 0; k < most; ++k, P += part) {
+    long long w[3][COUNT];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int i = 0; i < COUNT; ++i) w[c][i] = k < n[c][i] ? P[c * stride + at[i]] : 0;
+#pragma unroll
+    for (int i = 0; i < COUNT; ++i) {
+      re[i] += (unsigned long long)w[0][i] - (unsigned long long)w[1][i];
+      im[i] += 2 * (unsigned long long)w[2][i] - (unsigned long long)w[0][i] - (unsigned long long)w[1][i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < COUNT; ++i) v[i] = make_longlong2((long long)re[i], (long long)im[i]);
 }
 
 __device__ __forceinline__ int bit_length(long long v) { return 64 - __clzll(v < 0 ? -v : v); }
@@ -499,33 +516,36 @@ __device__ __forceinline__ long long shift_round(long long v, int sh) {
 constexpr int GPU_SMS = 152;                 // GB300
 
 // Chains per CTA: an even share, one CTA per SM.
-inline Deal deal_of(int rowsA, int rowsB, int width, int chains, int items) {
+inline Deal deal_of(int rowsA, int rowsB, int chains, int products) {
   Deal d;
   d.tilesA = cdiv(rowsA, BM);
-  d.tilesB = cdiv(rowsB, width);
+  d.tilesB = cdiv(rowsB, BN);
   d.chains = chains;
-  d.per = (int)(((long long)items * d.tilesA * d.tilesB * d.chains + GPU_SMS - 1) / GPU_SMS);
+  d.per = (int)(((long long)products * d.tilesA * d.tilesB * d.chains + GPU_SMS - 1) / GPU_SMS);
   return d;
 }
 
 // Partial sums of a tile at most, whichever chain of a CTA it starts at.
 inline int max_parts(const Deal& d) { return std::min(d.chains, (d.chains + d.per - 2) / d.per + 1); }
 
-inline int unit_shift(int K) {
+// S for a contraction of K entries: sums reach K 2^16 (times sqrt 2 for im).
+// P2 has half that unit: |h| <= 2^7.5 in a DFT matrix leaves it the room, and
+// it counts four times.
+inline int unit_shift(int K, int sets) {
   int lg = 0;
   while ((1 << lg) < K) ++lg;
-  return std::min(36, 46 - lg);
+  return std::min(sets == 3 ? 38 : 39, 46 - lg);            // 2^(S + 1 - 9) is an int
 }
 
 // Tensor map of a digit operand seen as [items x digits][sets][L][kp], box
-// {32, box_rows, box_sets, digits}, 64-byte swizzle.
-inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int digits, int items, int box_rows, int box_sets) {
+// {32, box_rows, 1, digits}, 64-byte swizzle.
+inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int items, int box_rows) {
   auto enc = encode_fn();
   LGB_REQUIRE(enc, LGB_ECUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t row = (cuuint64_t)d.kp * 2, set = row * d.L;
-  cuuint64_t dims[4] = {(cuuint64_t)d.kp, (cuuint64_t)d.L, (cuuint64_t)(2 + d.b), (cuuint64_t)digits * items};
-  cuuint64_t strides[3] = {row, set, set * (2 + d.b)};
-  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)box_rows, (cuuint32_t)box_sets, (cuuint32_t)digits};
+  cuuint64_t dims[4] = {(cuuint64_t)d.kp, (cuuint64_t)d.L, (cuuint64_t)d.sets, (cuuint64_t)ND * items};
+  cuuint64_t strides[3] = {row, set, set * d.sets};
+  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1, (cuuint32_t)ND};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult res = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, d.base, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
@@ -535,35 +555,37 @@ inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int digits, int 
   return LGB_OK;
 }
 
-// One GEMM: A's and B's digits hold itemsA and itemsB items (1: shared by all).
-template <int NA, int NB, bool REAL>
-int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int itemsB, int items, const Deal& deal,
-                const Band& band, int S, void* P, long long item_stride, int ld, int* err, cudaStream_t s) {
+// The products of A's and B's sets over K entries, for `items` items; the
+// operands hold itemsA and itemsB of them (1: shared by all).
+inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int itemsB, int items, int K,
+                       const Deal& deal, const Band& band, int S, long long* P, long long stride, int ld,
+                       int* err, cudaStream_t s) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(sliced_gemm_kernel<NA, NB, REAL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem_bytes(NA, NB));
+    attr = cudaFuncSetAttribute(sliced_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
   });
   LGB_CUDA(attr);
   CUtensorMap a, b;
   int st;
-  if ((st = make_digit_map(&a, A, NA, itemsA, BM, 1))) return st;
-  if ((st = make_digit_map(&b, B, NB, itemsB, REAL ? BN : BC, REAL ? 1 : 2))) return st;
+  if ((st = make_digit_map(&a, A, itemsA, BM))) return st;
+  if ((st = make_digit_map(&b, B, itemsB, BN))) return st;
   GemmParams p{};
   p.deal = deal;
   p.band = band;
-  p.total = items * deal.tilesA * deal.tilesB * deal.chains;
+  p.sets = A.sets;
+  p.total = items * p.sets * deal.tilesA * deal.tilesB * deal.chains;
+  p.stages = cdiv(K, BK);
   p.rowsB = B.L;
   p.ld = ld;
-  p.dA = itemsA > 1 ? NA : 0;
-  p.dB = itemsB > 1 ? NB : 0;
+  p.dA = itemsA > 1 ? ND : 0;
+  p.dB = itemsB > 1 ? ND : 0;
   p.S = S;
   p.P = P;
-  p.item_stride = item_stride;
+  p.stride = stride;
   p.err = err;
   p.wait_ns = WAIT_NS;
-  sliced_gemm_kernel<NA, NB, REAL><<<cdiv(p.total, deal.per), NUM_THREADS, smem_bytes(NA, NB), s>>>(a, b, p);
+  sliced_gemm_kernel<<<cdiv(p.total, deal.per), NUM_THREADS, SMEM_BYTES, s>>>(a, b, p);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }
