@@ -114,6 +114,19 @@ __device__ __forceinline__ double2 expm2pi_fixed_f64(uint64_t ph) {
   return make_double2(c, -s);
 }
 
+// v * 2^e, rounded to nearest even, put together from its bits (a conversion
+// from 64-bit integers holds the FP64 pipe).
+__device__ __forceinline__ double assembled(uint64_t v, int e) {
+  if (v == 0) return 0.0;
+  const int lz = __clzll((long long)v), exp = 63 - lz + e + 1023;
+  if (exp < 1) return ldexp((double)v, e);
+  const uint64_t t = v << lz;
+  const uint32_t low = (uint32_t)t & 0x7FFu;
+  uint64_t q = t >> 11;                                  // 53 bits, the leading one set
+  q += low > 0x400u || (low == 0x400u && (q & 1));
+  return __longlong_as_double((long long)(q + ((uint64_t)(exp - 1) << 52)));   // a carry goes into the exponent
+}
+
 // exp(-2*pi*i*phase) in single precision from the fixed-point phase.
 __device__ __forceinline__ float2 expm2pi_fixed_f32(uint64_t ph) {
   const float x = (float)(int32_t)(ph >> 32) * 0x1p-31f;

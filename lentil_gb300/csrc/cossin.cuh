@@ -1,16 +1,18 @@
 // cos and sin of a fixed-point phase, in fixed point.
 //
-// The DFT matrices need 53-bit cosines and sines of phases that are exact
-// 64-bit fractions of a cycle (phase_fixed, common.cuh).  Double-precision
-// sincospi holds this part's FP64 pipe (17 clocks a value per SM measured in the
-// phasor kernel); the integer pipes give the same in about two: the nearest of 512 points of the
-// circle from a table, and a rotation by the rest, |d| < 2^-7.3, with the
-// Taylor series of cos d and sin d in 64-bit fixed point, cut where the terms
-// fall below 2^-63.  The error is below 2^-60 (2.4 units of 2^-62 at most over
+// DFT matrices and phasors need cosines and sines of phases that are exact
+// 64-bit fractions of a cycle (phase_fixed, common.cuh; x mod 2).  Double-
+// precision sincospi holds this part's FP64 pipe (17 clocks a value per SM
+// measured in the phasor kernel); the integer pipes give the same in about two:
+// the nearest of 512 points of the circle from a table, and a rotation by the
+// rest, |d| < 2^-7.3, with the Taylor series of cos d and sin d in 64-bit fixed
+// point, cut where the terms fall below 2^-63.  The error is below 2^-60 (2.4 units of 2^-62 at most over
 // thousands of phases against 60-digit values).
 #pragma once
 
 #include <stdint.h>
+
+#include "common.cuh"
 
 namespace lgb {
 
@@ -51,12 +53,23 @@ __device__ static const unsigned long long COS_TABLE[129] = {
     0x0000000000000000,
 };
 
-// (cos, sin)(2 pi ph / 2^64) in units of 2^-62; table: COS_TABLE or a copy.
-__device__ __forceinline__ longlong2 cossin_q62(uint64_t ph, const unsigned long long* table) {
-  const uint32_t at = (uint32_t)((ph + (1ull << 54)) >> 55) & 511u;      // nearest table point
-  const int64_t r = (int64_t)(ph - ((uint64_t)at << 55));               // |r| <= 2^54
-  const uint64_t ar = (uint64_t)(r < 0 ? -r : r);
-  const uint64_t d = __umul64hi(ar << 8, 7244019458077122842ull);                      // |d|, Q68, < 2^60.7
+// The nearest of the table's points to a phase, and the rest |r| <= 2^54.
+struct TablePoint {
+  uint32_t at;
+  bool neg;
+  uint64_t ar;
+};
+__device__ __forceinline__ TablePoint table_point(uint64_t ph) {
+  const uint32_t at = (uint32_t)((ph + (1ull << 54)) >> 55) & 511u;
+  const int64_t r = (int64_t)(ph - ((uint64_t)at << 55));
+  return TablePoint{at, r < 0, (uint64_t)(r < 0 ? -r : r)};
+}
+
+// (cos, sin) of a phase's angle less its quadrant (at & 384), in units of
+// 2^-62, and u = 1 - sin d / d of the rest d, Q72.
+__device__ __forceinline__ longlong2 first_quadrant_q62(const TablePoint& p, const unsigned long long* table,
+                                                        uint64_t& u) {
+  const uint64_t d = __umul64hi(p.ar << 8, 7244019458077122842ull);                    // |d|, Q68, < 2^60.7
   const uint64_t d2 = __umul64hi(d << 1, d << 1);                        // d^2, Q74, < 2^59.4
   const uint32_t y = (uint32_t)(d2 >> 28);                               // d^2, Q46
   // 1 - cos d = d^2 (1/2 - d^2/24 + d^4/720)
@@ -64,17 +77,57 @@ __device__ __forceinline__ longlong2 cossin_q62(uint64_t ph, const unsigned long
   const uint64_t a = __umul64hi(d2, (1ull << 61) - ((uint64_t)__umulhi(y, w) << 12));   // Q72, < 2^56.4
   // sin d = d (1 - d^2 (1/6 - d^2/120))
   const uint64_t q6 = 768614336404564650ull - ((uint64_t)__umulhi(y, 2290649225u) << 10); // Q62
-  const uint64_t u = __umul64hi(d2, q6);                                 // Q72, < 2^54.8
+  u = __umul64hi(d2, q6);                                                // Q72, < 2^54.8
   const uint64_t sd = (d << 2) - (__umul64hi(d, u << 8) >> 14);          // Q70, < 2^62.7
-  const int j = at & 127;
+  const int j = p.at & 127;
   const uint64_t c = table[j], s = table[128 - j];
   const int64_t ca = (int64_t)(__umul64hi(c, a << 6) >> 14), sa = (int64_t)(__umul64hi(s, a << 6) >> 14);
   int64_t cs = (int64_t)(__umul64hi(c, sd) >> 6), ss = (int64_t)(__umul64hi(s, sd) >> 6);
-  if (r < 0) { cs = -cs; ss = -ss; }
-  int64_t x = (int64_t)c - ca - ss, yv = (int64_t)s - sa + cs;           // cos, sin of the first quadrant's angle
-  if (at & 128) { const int64_t t = x; x = -yv; yv = t; }
-  if (at & 256) { x = -x; yv = -yv; }
-  return make_longlong2(x, yv);
+  if (p.neg) { cs = -cs; ss = -ss; }
+  return make_longlong2((int64_t)c - ca - ss, (int64_t)s - sa + cs);
+}
+
+// (cos, sin)(2 pi ph / 2^64) in units of 2^-62; table: COS_TABLE or a copy.
+__device__ __forceinline__ longlong2 cossin_q62(uint64_t ph, const unsigned long long* table) {
+  const TablePoint p = table_point(ph);
+  uint64_t u;
+  longlong2 z = first_quadrant_q62(p, table, u);
+  if (p.at & 128) z = make_longlong2(-z.y, z.x);
+  return p.at & 256 ? make_longlong2(-z.x, -z.y) : z;
+}
+
+// (cos, sin)(pi x) as doubles, each within 1.2 units of its last place: x 2^63
+// mod 2^64 is the phase, exactly (below |x| = 2^-11 up to its last place).
+// Next to an axis (at & 127 = 0) the small one of the two is sin d from d's
+// leading 64 bits, wherever they lie.
+__device__ __forceinline__ double2 cossinpi_f64(double x, const unsigned long long* table) {
+  const uint64_t bits = (uint64_t)__double_as_longlong(x);
+  int E = (int)(bits >> 52) & 0x7FF;
+  if (E == 0x7FF) return make_double2(x - x, x - x);                     // NaN
+  uint64_t m = bits & 0xFFFFFFFFFFFFFull;
+  if (E == 0) E = 1; else m |= 1ull << 52;
+  const int sh = E - 1012;                                               // x 2^63 = m 2^sh
+  uint64_t ph = sh >= 64 || sh <= -64 ? 0 : sh >= 0 ? m << sh : m >> -sh;
+  if (bits >> 63) ph = 0 - ph;
+  TablePoint p = table_point(ph);
+  if (sh < 0) p.neg = bits >> 63;
+  uint64_t u;
+  const longlong2 z = first_quadrant_q62(p, table, u);
+  uint64_t big = (uint64_t)z.x, v = (uint64_t)z.y;                       // cos, sin of the first quadrant's angle
+  int e = -62;
+  bool neg = false;
+  if ((p.at & 127) == 0) {
+    const uint64_t r = sh < 0 ? m : p.ar;
+    const int lz = __clzll((long long)r);
+    const uint64_t dn = __umul64hi(lz < 64 ? r << lz : 0, 14488038916154245685ull);    // d 2^(61 + lz)
+    v = dn - __umul64hi(dn, u >> 8);
+    e = -61 - lz + (sh < 0 ? sh : 0);
+    neg = p.neg;
+  }
+  double c = assembled(big, -62), s = assembled(v, e);
+  if (neg) s = -s;
+  if (p.at & 128) { const double t = c; c = -s; s = t; }
+  return p.at & 256 ? make_double2(-c, -s) : make_double2(c, s);
 }
 
 }  // namespace lgb

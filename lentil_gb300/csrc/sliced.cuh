@@ -337,10 +337,11 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---------------------------------------------------------------- digits ---
-// The digits of X, |X| <= 2^62, as bf16 bits in the high half of a word; digit i carries 2^(-9 i).  A bias of 256 in every place turns the
-// signed digits into bit fields; a field under the exponent of 1.5 2^23 is a
-// float, and one FMA takes bias and offset off and scales (exactly): three
-// instructions a digit, none of them on the conversion or 64-bit paths.
+// The digits of X, |X| <= 2^62, as bf16 bits in the high half of a word; digit
+// i carries 2^(-9 i).  A bias of 256 in every place turns the signed digits into
+// bit fields; a field under the exponent of 1.5 2^23 is a float, and one FMA
+// takes bias and offset off and scales (exactly): three instructions a digit,
+// none of them on the conversion or 64-bit paths.
 __device__ __forceinline__ void digits_of(long long X, uint32_t (&d)[ND]) {
   constexpr unsigned long long bias = 256ull * 0x0000201008040201ull;   // 256 sum of 2^(9 i), i < 6
   const unsigned long long Y = (unsigned long long)X + bias;
@@ -355,19 +356,13 @@ __device__ __forceinline__ void digits_of(long long X, uint32_t (&d)[ND]) {
   }
 }
 
-// v * 2^e * scale as a double: v * 2^e, rounded to nearest even, is put together
-// from its bits (a conversion from 64-bit integers holds the FP64 pipe).
+// v * 2^e * scale as a double
 __device__ __forceinline__ double scaled(long long v, int e, double scale) {
-  if (v == 0) return 0.0;
   const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
-  const int lz = __clzll((long long)m), exp = 63 - lz + e + 1023;
-  if (exp < 1 || exp > 2045) return scalbn((double)v * scale, e);
-  const unsigned long long t = m << lz;
-  const uint32_t low = (uint32_t)t & 0x7FFu;
-  unsigned long long q = t >> 11;                        // 53 bits, the leading one set
-  q += low > 0x400u || (low == 0x400u && (q & 1));
-  q += (unsigned long long)(exp - 1) << 52;              // a carry goes into the exponent
-  return scale * __longlong_as_double((long long)(q | ((unsigned long long)v & 0x8000000000000000ull)));
+  const int exp = 63 - __clzll((long long)m) + e + 1023;
+  if (m != 0 && (exp < 1 || exp > 2045)) return scalbn((double)v * scale, e);
+  const double r = scale * assembled(m, e);
+  return v < 0 ? -r : r;
 }
 
 constexpr int XBITS = BETA * ND - 1;         // an entry is |X| <= 2^62 of its vector's scale
