@@ -52,14 +52,14 @@ constexpr int STAGES = 2;
 constexpr int GROUPS = 5;                    // accumulators: s = 0, 1, 2, 3, and 4 to 6 together
 constexpr uint32_t A_SLICE = BM * BK * 2, B_SLICE = BN * BK * 2;
 constexpr uint32_t A_STAGE = ND * A_SLICE, STAGE_BYTES = ND * (A_SLICE + B_SLICE);
-constexpr int EPI_WARPS = 8;
+constexpr int EPI_WARPS = 16;
 constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t BAR_BYTES = 256;
 constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
-constexpr int RUN = BN / 2;                  // tile columns per epilogue warp
+constexpr int RUN = 4 * BN / EPI_WARPS;      // tile columns per epilogue warp
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
-static_assert(GROUPS * BN <= 512 && RUN == 48, "tensor memory columns; the drain loads 3 x 16 of them");
+static_assert(GROUPS * BN <= 512 && RUN == 24, "tensor memory columns; the drain loads 3 x 8 of them");
 
 // How a launch's work is dealt out: the chains (64 K entries of one tile) of all
 // tiles of all products in a row, `per` of them to each CTA.  A tile's chains
@@ -137,37 +137,46 @@ __device__ __forceinline__ bool drains(int g, int r, int count) {
   return g == 0 ? (r & 3) == 3 : g == 1 ? (r & 1) == 1 : true;
 }
 
-// The digit products A_i B_j of one sum i + j, two k-steps each, added to the
-// accumulator d (started afresh when `fresh`).  The operand descriptors are
-// one 64-bit base each plus constants, and the warp stays converged around
-// them: with descriptors worked out per MMA, or in a loop that one lane runs
-// alone, the issuing warp was the limit, at 95 to 100 clk an MMA.
-template <int SUM>
-__device__ __forceinline__ void mma_sum(uint32_t on, uint32_t d, uint64_t da, uint64_t db, uint32_t idesc,
-                                        bool fresh) {
+// The products of digit i of A with digits j0 >= j >= j1 of B, two k-steps, into
+// the accumulators of i + j (4 to 6: the last one); the first of them starts its
+// sum afresh when `fresh`.  A's tile stays in the MMA's collector for the run,
+// else shared memory is read more slowly than the tensor core computes.  The
+// operand descriptors are one 64-bit base each plus constants, and the warp
+// stays converged around them: with descriptors worked out per MMA, or in a
+// loop that one lane runs alone, the issuing warp was the limit, at 95 to 100
+// clk an MMA.
+__device__ __forceinline__ void mma_run(int i, int j0, int j1, uint32_t on, uint32_t tmem, uint64_t da,
+                                        uint64_t db, uint32_t idesc, bool fresh) {
 #pragma unroll
-  for (int i = 0; i <= SUM; ++i) {
+  for (int k = 0; k < BK / 16; ++k) {
 #pragma unroll
-    for (int k = 0; k < BK / 16; ++k)
-      mma_f16_cta(on, d, da + ((i * A_SLICE + k * 32) >> 4), db + (((SUM - i) * B_SLICE + k * 32) >> 4), idesc,
-                  fresh && i == 0 && k == 0 ? 0u : 1u);
+    for (int j = j0; j >= j1; --j) {
+      const int g = i + j < GROUPS ? i + j : GROUPS - 1;
+      mma_f16_cta(on, tmem + g * BN, da + ((i * A_SLICE + k * 32) >> 4), db + ((j * B_SLICE + k * 32) >> 4),
+                  idesc, k == 0 && j == j1 && fresh ? 0u : 1u, j != j0, j != j1);
+    }
   }
 }
 
 // P over this CTA's chains.
 //
 // Bound by the tensor pipe: 112 MMAs (28 digit products x 4 k-steps) of
-// 128 x 96 x 16 per chain.  96 columns is the widest tile whose five
-// accumulators fit the 512 TMEM columns; the MMA then reads 7 KB of shared
-// memory per 48 clocks (149 B/clk against the 128 B/clk port), so it runs at
-// 56 clk at best; the 98 KB that TMA writes per stage share that port, which
-// makes it 3900 clk a stage (1019 x 941 to 1024^2: 92 us of MMAs at 56 clk in
-// 119).  Roles: warp 0 TMA (two stages of 32 K entries, all digits),
-// warp 1 MMA issue, warps 2..9 drain (lane quadrant w % 4, column half
-// (w - 2) / 4).  The groups are drained one by one, in the order they are
-// issued, while the next ones run.  One CTA per SM takes its share of the
-// chains (Deal), so the pipeline fills once per launch and no wave is partly
-// empty.
+// 128 x 96 x 16 per chain, 48 clk each; 96 columns is the widest tile whose five
+// accumulators fit the 512 TMEM columns.  An MMA that reads both operands from
+// shared memory (7 KB) takes 56 clk, and the 98 KB that TMA writes per stage
+// share the port: in the order of the sums i + j, with nothing kept, a stage
+// took 3900 clk.  Runs over B's digits with A's in the collector read 4.6 KB and
+// run at 49: 1019 x 941 to 1024^2 went from 121 to 110 us per GEMM (transform
+// 300 -> 283), 512^2 from 76 to 71.5.  What is left above the 81 us of MMAs: the
+// first loads and the last sums (6 us), loads (830 MB from L2 in all, 12 %) and
+// drains (9 %) that the MMAs wait for.
+//
+// Roles: warp 0 TMA (two stages of 32 K entries; digits 4 to 6 of a stage are
+// done with, and loaded anew, while its sums 0 to 3 run), warp 1 MMA issue,
+// warps 2..17 drain (lane quadrant w % 4, 24 columns each).  A drain takes some
+// 800 clk, most of it the conversions (16 a clock).  One CTA per SM takes its
+// share of the chains (Deal), so the pipeline fills once per launch and no wave
+// is partly empty.
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const GemmParams p) {
@@ -176,19 +185,21 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const uint32_t base = (raw + 1023u) & ~1023u;
   const uint32_t bars = base + STAGES * STAGE_BYTES;
   auto full_bar = [&](int s) { return bars + 8u * s; };
-  auto empty_bar = [&](int s) { return bars + 16u + 8u * s; };
+  auto low_empty = [&](int s) { return bars + 16u + 8u * s; };       // digits 4 to 6
+  auto high_empty = [&](int s) { return bars + 144u + 8u * s; };     // digits 0 to 3
   auto acc_full = [&](int g) { return bars + 32u + 8u * g; };
   auto acc_empty = [&](int g) { return bars + 80u + 8u * g; };
   const uint32_t drain_bar = bars + 128u;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 136);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 160);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = blockIdx.x * p.deal.per, end = min(p.total, begin + p.deal.per);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
-      mbar_init(full_bar(s), 1);
-      mbar_init(empty_bar(s), 1);
+      mbar_init(full_bar(s), 2);
+      mbar_init(low_empty(s), 1);
+      mbar_init(high_empty(s), 1);
     }
     for (int g = 0; g < GROUPS; ++g) {
       mbar_init(acc_full(g), 1);
@@ -221,11 +232,18 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         const int last = min(p.stages, 2 * (w.chain + w.count));
         for (int st = 2 * w.chain; st < last; ++st, ++it) {
           const int s = it % STAGES;
-          if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, p.err, p.wait_ns)) { ok = false; break; }
-          mbar_expect_tx(full_bar(s), STAGE_BYTES);
-          const uint32_t sa = base + s * STAGE_BYTES;
-          tma_load_4d_cta(sa, &tmA, full_bar(s), st * BK, w.m0, set, item * p.dA);
-          tma_load_4d_cta(sa + A_STAGE, &tmB, full_bar(s), st * BK, w.n0, set, item * p.dB);
+          const uint32_t sa = base + s * STAGE_BYTES, parity = ((it / STAGES) & 1) ^ 1;
+          auto load = [&](uint32_t empty, int d0, int d1) {
+            if (!mbar_wait(empty, parity, p.err, p.wait_ns)) return false;
+            mbar_expect_tx(full_bar(s), (d1 - d0) * (A_SLICE + B_SLICE));
+            for (int d = d0; d < d1; ++d) {
+              tma_load_4d_cta(sa + d * A_SLICE, &tmA, full_bar(s), st * BK, w.m0, set, item * p.dA + d);
+              tma_load_4d_cta(sa + A_STAGE + d * B_SLICE, &tmB, full_bar(s), st * BK, w.n0, set, item * p.dB + d);
+            }
+            return true;
+          };
+          ok = load(low_empty(s), GROUPS - 1, ND) && load(high_empty(s), 0, GROUPS - 1);
+          if (!ok) break;
         }
       }
       for (int k = max(0, it - STAGES); k < it; ++k)       // issued copies land before exit
@@ -251,28 +269,33 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (!wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
         const uint64_t da = smem_desc_sw64(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw64(base + s * STAGE_BYTES + A_STAGE);
-#pragma unroll
-        for (int g = GROUPS - 1; g >= 0; --g) {
-          const bool first = (st & 1) == 0 && starts(g, r), last = ends && drains(g, r, w.count);
-          // this accumulator's previous sum has been drained
-          if (first && !wait(acc_empty(g), (n[g] & 1) ^ 1)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t d = tmem + g * BN;
-          if (g == 4) {                        // small products first
-            mma_sum<6>(on, d, da, db, idesc, first);
-            mma_sum<5>(on, d, da, db, idesc, false);
-            mma_sum<4>(on, d, da, db, idesc, false);
-          }
-          if (g == 3) mma_sum<3>(on, d, da, db, idesc, first);
-          if (g == 2) mma_sum<2>(on, d, da, db, idesc, first);
-          if (g == 1) mma_sum<1>(on, d, da, db, idesc, first);
-          if (g == 0) mma_sum<0>(on, d, da, db, idesc, first);
-          if (last) {
+        // groups 4 to 6 first: their accumulator is drained while the others run
+        const bool begins = (st & 1) == 0;
+        auto done = [&](int g) {
+          if (ends && drains(g, r, w.count)) {
             mma_commit_cta(on, acc_full(g));
             ++n[g];
           }
+        };
+#pragma unroll
+        for (int i = ND - 1; i >= -4 && ok; --i) {
+          const int g = i >= 0 ? GROUPS - 1 : i + 4;              // whose sum this run may start
+          const bool fresh = (i == ND - 1 || i < 0) && begins && starts(g, r);
+          // this accumulator's previous sum has been drained
+          if (fresh) ok = wait(acc_empty(g), (n[g] & 1) ^ 1);
+          if (!ok) break;
+          tc_fence_after();
+          if (i >= 0) mma_run(i, ND - 1 - i, max(4 - i, 0), on, tmem, da, db, idesc, fresh);
+          else mma_run(i + 4, -1 - i, 0, on, tmem, da, db, idesc, fresh);
+          if (i == 0) {
+            done(GROUPS - 1);
+            mma_commit_cta(on, low_empty(s));
+          }
         }
-        if (ok) mma_commit_cta(on, empty_bar(s));
+        if (!ok) break;
+#pragma unroll
+        for (int g = GROUPS - 2; g >= 0; --g) done(g);
+        mma_commit_cta(on, high_empty(s));
       }
     }
     mma_commit_cta(on, drain_bar);
@@ -302,7 +325,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           tc_fence_after();
           uint32_t r[RUN];
 #pragma unroll
-          for (int h = 0; h < RUN / 16; ++h) tmem_ld16(trow + g * BN + h * 16, r + h * 16);
+          for (int h = 0; h < RUN / 8; ++h) tmem_ld8(trow + g * BN + h * 8, r + h * 8);
           tmem_ld_wait();
           tc_fence_before();
           __syncwarp();
@@ -314,7 +337,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             else if (g == 3) acc[j] += (long long)__float2int_rn(v * 0x1p27f) * m3;
             else if (g == 2) acc[j] += (long long)__float2int_rn(v * 0x1p18f) * m2;
             else if (g == 1) acc[j] += (long long)__float2int_rn(v * 0x1p9f) * m1;
-            else acc[j] += (long long)__float2int_rn(v) << S;
+            else acc[j] += (long long)((unsigned long long)((uint32_t)__float2int_rn(v) << (S - 32)) << 32);
           }
         }
       }
@@ -525,7 +548,7 @@ inline int max_parts(const Deal& d) { return std::min(d.chains, (d.chains + d.pe
 
 // S for a contraction of K entries: sums reach K 2^16 (times sqrt 2 for im).
 // P2 has half that unit: |h| <= 2^7.5 in a DFT matrix leaves it the room, and
-// it counts four times.
+// it counts four times.  K <= 16384, so S >= 32.
 inline int unit_shift(int K, int sets) {
   int lg = 0;
   while ((1 << lg) < K) ++lg;
@@ -533,14 +556,14 @@ inline int unit_shift(int K, int sets) {
 }
 
 // Tensor map of a digit operand seen as [items x digits][sets][L][kp], box
-// {32, box_rows, 1, digits}, 64-byte swizzle.
+// {32, box_rows, 1, 1}, 64-byte swizzle.
 inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int items, int box_rows) {
   auto enc = encode_fn();
   LGB_REQUIRE(enc, LGB_ECUDA, "cuTensorMapEncodeTiled is unavailable");
   const cuuint64_t row = (cuuint64_t)d.kp * 2, set = row * d.L;
   cuuint64_t dims[4] = {(cuuint64_t)d.kp, (cuuint64_t)d.L, (cuuint64_t)d.sets, (cuuint64_t)ND * items};
   cuuint64_t strides[3] = {row, set, set * d.sets};
-  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1, (cuuint32_t)ND};
+  cuuint32_t box[4] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1, 1};
   cuuint32_t estr[4] = {1, 1, 1, 1};
   CUresult res = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, d.base, dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,

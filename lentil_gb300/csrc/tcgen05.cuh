@@ -234,15 +234,23 @@ __device__ __forceinline__ uint32_t elect_one() {
 }
 // D[128 x N] (+)= A[128 x 16] . B[N x 16]^T in this CTA, issued by the lane
 // with `on`: the whole warp runs the code around it, so the operands stay in
-// uniform registers.
+// uniform registers.  have_a takes A's tile from the collector, where the MMA
+// before left it; keep_a leaves it there for the next one.  (Both constants.)
 __device__ __forceinline__ void mma_f16_cta(uint32_t on, uint32_t d_tmem, uint64_t a, uint64_t b,
-                                            uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "setp.ne.b32 q, %5, 0;\n\t"
-      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on));
+                                            uint32_t idesc, uint32_t accumulate, bool have_a, bool keep_a) {
+#define LGB_MMA(collector)                                                                     \
+  asm volatile(                                                                                \
+      "{\n\t.reg .pred p, q;\n\t"                                                             \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                             \
+      "setp.ne.b32 q, %5, 0;\n\t"                                                             \
+      "@q tcgen05.mma.cta_group::1.kind::f16.collector::a::" collector                         \
+      " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),                                             \
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on))
+  if (have_a && keep_a) LGB_MMA("use");
+  else if (have_a) LGB_MMA("lastuse");
+  else if (keep_a) LGB_MMA("fill");
+  else LGB_MMA("discard");
+#undef LGB_MMA
 }
 // arrive once on the barrier when the MMAs issued so far by the lane with
 // `on` have completed
@@ -254,12 +262,11 @@ __device__ __forceinline__ void mma_commit_cta(uint32_t on, uint32_t bar) {
       "r"(on)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, "
-      "%8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
       : "r"(taddr));
 }
 
