@@ -48,6 +48,31 @@ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
 inline int round_up(int a, int b) { return cdiv(a, b) * b; }
 
+// A chain of kernels on one stream.  Each calls next_may_start first, so that
+// the next one's blocks are scheduled as soon as all of its own have begun, and
+// previous_done before it touches memory: launch and prologue of a kernel then
+// run under the one before.  (What it reads is not declared __restrict__: loads
+// of constants may be moved up past the wait.)
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void previous_done() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// kernel<<<grid, block, smem, s>>>(args...) in the chain of the kernel before it
+template <typename... Params, typename... Args>
+cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                        const Args&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &attr;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, kernel, Params(args)...);
+}
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 

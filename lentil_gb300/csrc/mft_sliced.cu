@@ -7,6 +7,8 @@
 //   slice_rows    P's rows, scaled to their largest entry -> digits
 //   sliced_gemm   P = the second product
 //   finish        P -> F, scaled
+// chained (launch_next): 512^2 takes 61.5 us, and took 71.5 launched one by one
+// with the flags cleared beforehand.
 // A field with a NaN gives NaN everywhere (each output sums every entry); one
 // with infinities, or a device-side wait that ran out, makes `finish`
 // evaluate that transform in plain FP64 instead.
@@ -36,6 +38,13 @@ __global__ void __launch_bounds__(128) matrix_digits_kernel(PhaseAxis ax, const 
   store_digits3(out, j, k, make_longlong2(e0.x, -e0.y), make_longlong2(e1.x, -e1.y));
 }
 
+// in place of a vector's exponent: it has infinities, or NaN
+constexpr int EXP_INF = 1 << 20, EXP_NAN = 1 << 21;
+
+__device__ __forceinline__ int exponent_or_flag(int e, int flag) {
+  return flag & FLAG_NAN ? EXP_NAN : flag ? EXP_INF : e - 1022;
+}
+
 __device__ __forceinline__ longlong2 fixed_entry(double2 z, int e) {
   return make_longlong2(fixed_data(z.x, e), fixed_data(z.y, e));
 }
@@ -43,8 +52,10 @@ __device__ __forceinline__ longlong2 fixed_entry(double2 z, int e) {
 // f's rows (one block each) -> digits, vectors of n entries.
 __global__ void __launch_bounds__(128) slice_rows_kernel(const double2* __restrict__ f, int m, int n,
                                                          DigitRows out, int* __restrict__ exps,
-                                                         int* __restrict__ flags) {
+                                                         int* __restrict__ err) {
+  next_may_start();
   const int i = blockIdx.x, b = blockIdx.y;
+  if (i == 0 && b == 0 && threadIdx.x == 0) *err = 0;
   const double2* src = f + ((size_t)b * m + i) * n;
   __shared__ int se[4], sf[4];
   int e = 1, flag = 0;
@@ -59,10 +70,7 @@ __global__ void __launch_bounds__(128) slice_rows_kernel(const double2* __restri
   __syncthreads();
   e = max(max(se[0], se[1]), max(se[2], se[3]));
   flag = sf[0] | sf[1] | sf[2] | sf[3];
-  if (threadIdx.x == 0) {
-    exps[(size_t)b * m + i] = e - 1022;
-    if (flag) atomicOr(flags + b, flag);
-  }
+  if (threadIdx.x == 0) exps[(size_t)b * m + i] = exponent_or_flag(e, flag);
   if (flag) return;                                       // this transform does not use its digits
   out.base += (size_t)b * ND * out.plane();
   const double2 zero = make_double2(0.0, 0.0);
@@ -78,7 +86,9 @@ constexpr int SC_COLS = 4, SC_WARPS = 16;    // columns and warps per block of s
 // block (a 64-byte piece of each row), SC_WARPS / SC_COLS warps per column.
 __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
     const double2* __restrict__ f, int m, int n, DigitRows out, int* __restrict__ exps,
-    int* __restrict__ flags) {
+    int* __restrict__ err) {
+  next_may_start();
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = warp % SC_COLS, part = warp / SC_COLS;
   constexpr int PARTS = SC_WARPS / SC_COLS;
@@ -99,10 +109,7 @@ __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
 #pragma unroll
   for (int q = 0; q < PARTS; ++q) { e = max(e, se[q * SC_COLS + c]); flag |= sf[q * SC_COLS + c]; }
   if (j >= n) return;
-  if (part == 0 && lane == 0) {
-    exps[(size_t)b * n + j] = e - 1022;
-    if (flag) atomicOr(flags + b, flag);
-  }
+  if (part == 0 && lane == 0) exps[(size_t)b * n + j] = exponent_or_flag(e, flag);
   if (flag) return;
   out.base += (size_t)b * ND * out.plane();
   const double2 zero = make_double2(0.0, 0.0);
@@ -116,9 +123,11 @@ __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
 // Row r of the first product (entry a in units of 2^(expA[a] - 16 - S)) ->
 // its digits as an operand of the second.  The first 2 KEEP entries of a thread
 // stay in registers between the two passes (rows of up to 1024 are read once).
+// A vector of f that is not finite marks every row.
 __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
-                                                            const int* __restrict__ expA, int S,
+                                                            const int* expA, int S,
                                                             DigitRows out, int* __restrict__ exps) {
+  next_may_start();
   constexpr int KEEP = 2, NONE = -(1 << 28);
   const int r = blockIdx.x, b = blockIdx.y;
   const long long* P = q.P + (size_t)b * 3 * q.stride + (size_t)r * q.ld;
@@ -127,10 +136,12 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
   __shared__ uint8_t parts[3 * MAX_TILES_A];
   __shared__ int se[8];
   count_parts<3>(q, 3 * b, r, parts);
+  previous_done();
   longlong2 kept[2 * KEEP], rest[2];
   int e = NONE;
   auto note = [&](int a, longlong2 v) {
-    if (v.x | v.y) e = max(e, ea[a] + max(bit_length(v.x), bit_length(v.y)));
+    const int x = a < q.cols ? ea[a] : NONE;
+    if (v.x | v.y || x >= EXP_INF) e = max(e, x + max(bit_length(v.x), bit_length(v.y)));
   };
   {
     size_t at[2 * KEEP];
@@ -166,7 +177,9 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < 8; ++w) e = max(e, se[w]);
-  if (threadIdx.x == 0) exps[(size_t)b * q.rows + r] = e == NONE ? 0 : e - 16 - S;
+  const int bad = e >= EXP_NAN ? EXP_NAN : e >= EXP_INF ? EXP_INF : 0;
+  if (threadIdx.x == 0) exps[(size_t)b * q.rows + r] = bad ? bad : e == NONE ? 0 : e - 16 - S;
+  if (bad) return;
   out.base += (size_t)b * ND * out.plane();
   auto put = [&](int k, longlong2 v0, longlong2 v1) {
     const int s0 = k < q.cols ? ea[k] - e + XBITS : 0, s1 = k + 1 < q.cols ? ea[k + 1] - e + XBITS : 0;
@@ -199,7 +212,6 @@ struct FinishParams {
   const PhaseAxis* axes;     // per item, or null: ar, ac
   int cols;
   long long* scratch;        // P again: the item's intermediate rows
-  const int* flags;
   const int* err;
 };
 
@@ -246,8 +258,9 @@ constexpr int FIN_ROWS = 4;                  // rows per finish block
 // from bits and four rows' parts are in flight at once: with conversions and
 // both scalings on the FP64 pipe and a row per block it took half as long again.
 __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
-  const int b = blockIdx.z, flag = p.flags[b];
-  if (*p.err != 0 || (flag & FLAG_INF && !(flag & FLAG_NAN))) {
+  previous_done();
+  const int b = blockIdx.z, flag = p.exps[(size_t)b * (p.left ? p.M : p.N)];      // all of them, if one is
+  if (*p.err != 0 || flag == EXP_INF) {
     if (blockIdx.x != 0) return;
     for (int q = blockIdx.y; q < (p.left ? p.M : p.N); q += gridDim.y) plain_line(p, b, q);
     return;
@@ -256,7 +269,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
   if (v >= p.N) return;
   double2* F = p.F + ((size_t)b * p.M + u0) * p.N + v;
   const int rows = min(FIN_ROWS, p.M - u0);
-  if (flag) {
+  if (flag == EXP_NAN) {
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
     for (int i = 0; i < rows; ++i) F[(size_t)i * p.N] = make_double2(nan, nan);
     return;
@@ -293,7 +306,7 @@ struct Layout {
   int chunk, ld1, ld2;
   Deal deal1, deal2;
   long long stride;          // P entries per product
-  int *err, *flags, *exp1, *exp2;
+  int *err, *exp1, *exp2;
   DigitRows d1, d2;          // digits of f (operand A) and of the intermediate
   long long* P;
   size_t bytes;
@@ -329,8 +342,7 @@ Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
     off += bytes;
     return q;
   };
-  t.err = reinterpret_cast<int*>(take(16 + sizeof(int) * t.chunk));
-  t.flags = t.err ? t.err + 4 : nullptr;
+  t.err = reinterpret_cast<int*>(take(16));
   t.exp1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.vecs1));
   t.exp2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.rows1));
   t.d1.base = reinterpret_cast<uint16_t*>(take(b1 * t.chunk));
@@ -348,10 +360,10 @@ bool sliced_left(int m, int n, int M, int N) {
 
 // Where the sliced form is taken: where its five launches cost less than the
 // plain GEMMs' two to four.  Device time of one transform from a plan, plain
-// and sliced: 64^2 to 64^2 20 and 33 us, 96^2 29 and 35, 112^2 39 and 37, 256^2
-// 270 and 39, (8 x 8) to 512^2 27 and 33, (16 x 512) to 512^2 86 and 37,
-// (16 x 1024) to (16 x 1024) 171 and 45: the line is one of multiply-adds, just
-// below the crossing at about 105^2.
+// and sliced: 64^2 to 64^2 20 and 29 us, 96^2 29 and 31, 112^2 39 and 33, 256^2
+// 270 and 37, (8 x 8) to 512^2 27 and 29, (16 x 512) to 512^2 86 and 35,
+// (16 x 1024) to (16 x 1024) 171 and 41: the line is one of multiply-adds, just
+// below the crossing at about 100^2.
 // Operands longer than 16384 would leave the 64-bit sums too few fraction bits.
 bool sliced_applies(int m, int n, int M, int N) {
   if (std::min(std::min(m, n), std::min(M, N)) < 8 || std::max(m, n) > 16384 ||
@@ -388,20 +400,18 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   for (int b0 = 0; b0 < q.count; b0 += t.chunk) {
     const int items = std::min(t.chunk, q.count - b0);
     const double2* f = q.f + (size_t)b0 * q.m * q.n;
-    LGB_CUDA(cudaMemsetAsync(t.err, 0, 16 + sizeof(int) * items, s));
     if (t.left)
       slice_cols_kernel<<<dim3(cdiv(q.n, SC_COLS), items), 32 * SC_WARPS, 0, s>>>(f, q.m, q.n, t.d1, t.exp1,
-                                                                                 t.flags);
+                                                                                 t.err);
     else
-      slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.flags);
+      slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.err);
     LGB_CUDA(cudaGetLastError());
     const int own_items = own ? items : 1;
     if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, Band{}, S1, t.P,
                           t.stride, t.ld1, t.err, s)))
       return st;
-    slice_product_kernel<<<dim3(t.rows1, items), 256, 0, s>>>(
-        PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2);
-    LGB_CUDA(cudaGetLastError());
+    LGB_CUDA(launch_next(slice_product_kernel, dim3(t.rows1, items), 256, 0, s,
+                         PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2));
     if ((st = launch_gemm(t.left ? e2 : t.d2, t.left ? own_items : items, t.left ? t.d2 : e1,
                           t.left ? items : own_items, items, t.K2, t.deal2, Band{}, S2, t.P, t.stride, t.ld2, t.err,
                           s)))
@@ -423,10 +433,8 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     p.axes = own ? q.axes + b0 : nullptr;
     p.cols = q.cols;
     p.scratch = t.P;
-    p.flags = t.flags;
     p.err = t.err;
-    finish_kernel<<<dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s>>>(p);
-    LGB_CUDA(cudaGetLastError());
+    LGB_CUDA(launch_next(finish_kernel, dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s, p));
     if (own) {
       e1.base += (size_t)items * ND * e1.plane();
       e2.base += (size_t)items * ND * e2.plane();

@@ -5,6 +5,8 @@
 // Each product is: digits of X's rows and of R's rows; GEMM (its output's
 // contiguous index runs over X's rows, so the transposed product comes out
 // row by row); digits of those rows; GEMM with L's digits; finish.
+// The launches are chained (launch_next): 1000^2 by 3 takes 214 us, and took 246
+// one by one.
 // Non-finite images, and a device-side wait that ran out, are evaluated in
 // plain FP64 by the finishing kernels.
 #include "pixelate.cuh"
@@ -34,11 +36,10 @@ struct BandedRows {                          // G[r][q0[r] + b] = Gt[b][r]
   }
 };
 
-// Row r (one block) of a real matrix -> digits and exponent.
+// Row r of a real matrix -> digits and exponent, by one block.
 template <typename Rows>
-__global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out, int* __restrict__ exps,
-                                                         int* __restrict__ flag) {
-  const int r = blockIdx.x, K = src.K;
+__device__ __forceinline__ void slice_real_row(const Rows& src, int r, const DigitRows& out, int* exps, int* flag) {
+  const int K = src.K;
   __shared__ int se[8], sf[8];
   int e = 1, bad = 0;
   for (int k = threadIdx.x; k < K; k += 256) note_exponent(src.at(r, k), e, bad);
@@ -58,19 +59,33 @@ __global__ void __launch_bounds__(256) slice_real_kernel(Rows src, DigitRows out
                       k + 1 < K ? fixed_data(src.at(r, k + 1), e) : 0);
 }
 
+// The rows of X, then those of the operator.
+template <typename Rows>
+__global__ void __launch_bounds__(256) slice_real_kernel(DenseRows X, int rows, DigitRows dX, int* __restrict__ eX,
+                                                         Rows op, DigitRows dR, int* __restrict__ eR,
+                                                         int* __restrict__ flag) {
+  next_may_start();
+  previous_done();
+  const int r = blockIdx.x;
+  if (r < rows) slice_real_row(X, r, dX, eX, flag);
+  else slice_real_row(op, r - rows, dR, eR, flag);
+}
+
 // Row r of a product (entry a in units of 2^(ea[a] + eb[r] - 16 - S)) ->
 // digits.  The first 2 KEEP entries of a thread stay in registers between the
 // two passes.
 __global__ void __launch_bounds__(256) slice_real_product_kernel(const PartialSums q,
-                                                                 const int* __restrict__ ea,
-                                                                 const int* __restrict__ eb, int S,
+                                                                 const int* ea,
+                                                                 const int* eb, int S,
                                                                  DigitRows out, int* __restrict__ exps) {
+  next_may_start();
   constexpr int KEEP = 4, NONE = -(1 << 28);
   const int r = blockIdx.x;
   const long long* P = q.P + (size_t)r * q.ld;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ int se[8];
   count_parts<1>(q, 0, r, parts);
+  previous_done();
   long long kept[2 * KEEP], rest[2];
   int e = NONE;
   auto note = [&](int a, long long v) {
@@ -157,17 +172,19 @@ struct FinishReal {
 
 // Row k of |C img C^T|: its entries, their sum, and, when d is set, the
 // samples on the detector grid with their sum.
-__global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, const double* __restrict__ img,
-                                                           const double* __restrict__ c,
+__global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, const double* img,
+                                                           const double* c,
                                                            double* __restrict__ scratch, int os,
                                                            double* __restrict__ d,
                                                            double* __restrict__ sum_d) {
+  next_may_start();
   const int N = p.q.rows, k = blockIdx.x;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ double sm[8];
+  count_parts<1>(p.q, 0, k, parts);
+  previous_done();
   const bool plain = p.status[0] != 0 || p.status[1] != 0;
   double* T = scratch + (size_t)k * N;       // plain: row k of C img (P's memory)
-  count_parts<1>(p.q, 0, k, parts);
   if (plain) {
     for (int j = threadIdx.x; j < N; j += 256) {
       double t = 0.0;
@@ -208,14 +225,16 @@ __global__ void __launch_bounds__(256) finish_pixel_kernel(const FinishReal p, c
 }
 
 // Row k of G p G^T and its sum.
-__global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p, const double* __restrict__ img,
-                                                              const double* __restrict__ Gt,
-                                                              const int* __restrict__ q0, int N) {
+__global__ void __launch_bounds__(256) finish_resample_kernel(const FinishReal p, const double* img,
+                                                              const double* Gt,
+                                                              const int* q0, int N) {
+  next_may_start();
   const int S = p.q.rows, k = blockIdx.x;
   __shared__ uint8_t parts[MAX_TILES_A];
   __shared__ double sm[8];
-  const bool plain = p.status[0] != 0 || p.status[1] != 0;
   count_parts<1>(p.q, 0, k, parts);
+  previous_done();
+  const bool plain = p.status[0] != 0 || p.status[1] != 0;
   double s = 0.0;
   for (int l0 = threadIdx.x; l0 < S; l0 += 256 * FIN_COLS) {
     long long z[FIN_COLS];
@@ -271,7 +290,6 @@ struct Sandwich {
 size_t digit_entries(int L, int K) { return ND * real_rows(nullptr, L, K).plane(); }
 
 struct Space {
-  int* status;               // [0] expired wait, [1] non-finite
   int *eX, *eR, *eT;
   uint16_t *dX, *dR, *dT;
   long long* P;
@@ -287,7 +305,6 @@ Space carve(const Sandwich& w, void* ws) {
     off += bytes;
     return q;
   };
-  t.status = reinterpret_cast<int*>(take(2 * sizeof(int)));
   t.eX = reinterpret_cast<int*>(take(sizeof(int) * w.p));
   t.eR = reinterpret_cast<int*>(take(sizeof(int) * w.r));
   t.eT = reinterpret_cast<int*>(take(sizeof(int) * w.r));
@@ -300,50 +317,45 @@ Space carve(const Sandwich& w, void* ws) {
 }
 
 template <typename Rows>
-int run_sandwich(const Sandwich& w, const Space& t, const double* X, const Rows& op, cudaStream_t s) {
+int run_sandwich(const Sandwich& w, const Space& t, const double* X, const Rows& op, int* status, cudaStream_t s) {
   const int S = unit_shift(w.q, 1);
   const DigitRows dX = real_rows(t.dX, w.p, w.q), dR = real_rows(t.dR, w.r, w.q), dT = real_rows(t.dT, w.r, w.p);
-  LGB_CUDA(cudaMemsetAsync(t.status, 0, 2 * sizeof(int), s));
-  slice_real_kernel<<<w.p, 256, 0, s>>>(DenseRows{X, w.q}, dX, t.eX, t.status + 1);
-  slice_real_kernel<<<w.r, 256, 0, s>>>(op, dR, t.eR, t.status + 1);
-  LGB_CUDA(cudaGetLastError());
-  int st = launch_gemm(dX, 1, dR, 1, 1, w.q, w.deal1, w.band, S, t.P, 0, w.ld1, t.status, s);
+  LGB_CUDA(launch_next(slice_real_kernel<Rows>, w.p + w.r, 256, 0, s, DenseRows{X, w.q}, w.p, dX, t.eX, op, dR, t.eR,
+                       status + 1));
+  int st = launch_gemm(dX, 1, dR, 1, 1, w.q, w.deal1, w.band, S, t.P, 0, w.ld1, status, s);
   if (st) return st;
-  slice_real_product_kernel<<<w.r, 256, 0, s>>>(PartialSums{t.P, 0, w.ld1, w.r, w.p, w.deal1}, t.eX,
-                                                t.eR, S, dT, t.eT);
-  LGB_CUDA(cudaGetLastError());
-  return launch_gemm(dT, 1, dR, 1, 1, w.q, w.deal2, w.band, S, t.P, 0, w.ld2, t.status, s);
+  LGB_CUDA(launch_next(slice_real_product_kernel, w.r, 256, 0, s, PartialSums{t.P, 0, w.ld1, w.r, w.p, w.deal1}, t.eX,
+                       t.eR, S, dT, t.eT));
+  return launch_gemm(dT, 1, dR, 1, 1, w.q, w.deal2, w.band, S, t.P, 0, w.ld2, status, s);
 }
 
 }  // namespace
 
 size_t pixel_sliced_workspace(int N) { return carve(Sandwich(N, N, N, 0), nullptr).bytes; }
 
-int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, double* P, double* sums, int os,
-                        double* d, cudaStream_t s) {
+int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, int* status, double* P, double* sums,
+                        int os, double* d, cudaStream_t s) {
   const Sandwich w(N, N, N, 0);
   const Space t = carve(w, ws);
-  const int st = run_sandwich(w, t, img, CirculantRows{c, N}, s);
+  const int st = run_sandwich(w, t, img, CirculantRows{c, N}, status, s);
   if (st) return st;
-  const FinishReal f{PartialSums{t.P, 0, w.ld2, N, N, w.deal2}, t.eT, t.eR, unit_shift(N, 1), t.status,
+  const FinishReal f{PartialSums{t.P, 0, w.ld2, N, N, w.deal2}, t.eT, t.eR, unit_shift(N, 1), status,
                      P, sums};
-  finish_pixel_kernel<<<N, 256, 0, s>>>(f, img, c, reinterpret_cast<double*>(t.P), os, d, sums + 1);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(finish_pixel_kernel, N, 256, 0, s, f, img, c, reinterpret_cast<double*>(t.P), os, d, sums + 1));
   return LGB_OK;
 }
 
 size_t resample_sliced_workspace(int N, int os, int S) { return carve(Sandwich(N, N, S, os), nullptr).bytes; }
 
 int launch_resample_sliced(const double* P, int N, int os, int S, const double* Gt, const int* q0, void* ws,
-                           double* raw, double* sum, cudaStream_t s) {
+                           int* status, double* raw, double* sum, cudaStream_t s) {
   const Sandwich w(N, N, S, os);
   const Space t = carve(w, ws);
-  const int st = run_sandwich(w, t, P, BandedRows{Gt, q0, N, S}, s);
+  const int st = run_sandwich(w, t, P, BandedRows{Gt, q0, N, S}, status, s);
   if (st) return st;
-  const FinishReal f{PartialSums{t.P, 0, w.ld2, S, S, w.deal2}, t.eT, t.eR, unit_shift(N, 1), t.status,
+  const FinishReal f{PartialSums{t.P, 0, w.ld2, S, S, w.deal2}, t.eT, t.eR, unit_shift(N, 1), status,
                      raw, sum};
-  finish_resample_kernel<<<S, 256, 0, s>>>(f, P, Gt, q0, N);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(finish_resample_kernel, S, 256, 0, s, f, P, Gt, q0, N));
   return LGB_OK;
 }
 

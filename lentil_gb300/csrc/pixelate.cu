@@ -214,6 +214,7 @@ __global__ void transpose_c128_kernel(const double2* __restrict__ in, double2* _
 // computed once per call (FP64 sinpi is slow on this part's FP64 pipe; the
 // N^2 products below only read)
 __global__ void sinc_table_kernel(int N, double os, double* __restrict__ s, double* __restrict__ tab) {
+  next_may_start();
   const int i = blockIdx.x * blockDim.x + threadIdx.x, k = i < N ? i : i - N;
   if (i < N) s[k] = sinc_os(k, N, os);
   else if (tab && k < N) tab[k] = cospi(2.0 * (double)k / N);
@@ -223,13 +224,15 @@ __global__ void sinc_table_kernel(int N, double os, double* __restrict__ s, doub
 // c[k] = (1/N) sum_f s_f cos(2 pi f k / N), one block per tap, the cosines
 // from the table at the exact phase index f k mod N.  (One thread per tap,
 // each with N cospi of its own, took 1.59 ms at N = 1000 on 8 CTAs.)
-__global__ void __launch_bounds__(128) pixel_taps_kernel(int N, const double* __restrict__ sinc,
-                                                         const double* __restrict__ tab,
+__global__ void __launch_bounds__(128) pixel_taps_kernel(int N, const double* sinc,
+                                                         const double* tab,
                                                          double* __restrict__ c) {
+  next_may_start();
   const int k = blockIdx.x;
   __shared__ double sm[4];
   int ph = (int)(((long long)threadIdx.x * k) % N);
   const int step = (int)((128ll * k) % N);
+  previous_done();
   double acc = 0.0;
   for (int f = threadIdx.x; f < N; f += 128) {
     acc = fma(sinc[f], tab[ph], acc);
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(4 * RS_BW) resample_operator_kernel(int N, int
                                                                       double* __restrict__ Gt,
                                                                       int* __restrict__ q0,
                                                                       double* __restrict__ pos) {
+  next_may_start();
   __shared__ double h[RS_TAPS + 1];
   if (threadIdx.x <= RS_TAPS) {                 // sqrt(3) z^t by squaring
     double p = sqrt(3.0) - 2.0, v = sqrt(3.0);
@@ -414,6 +418,7 @@ __global__ void __launch_bounds__(4 * RS_BW) resample_operator_kernel(int N, int
     q0[k] = start;
     pos[k] = x;
   }
+  previous_done();                              // reads nothing of the kernels before it; the next ones do
 }
 
 constexpr int RS_ROWS = 8;        // image rows per thread in the row pass
@@ -473,11 +478,12 @@ __global__ void __launch_bounds__(256) resample_cols_kernel(const double* __rest
 // out = (raw * (sum p / sum raw)) * mask, the mask being the order-1
 // nearest-mode interpolation of (p != 0) at the same points, zeroed below
 // DBL_EPSILON (lentil/util.py:317-320, 333-347)
-__global__ void __launch_bounds__(256) resample_finish_kernel(const double* __restrict__ raw,
-                                                              const double* __restrict__ p, int N, int S,
-                                                              const double* __restrict__ pos,
-                                                              const double* __restrict__ sums,
+__global__ void __launch_bounds__(256) resample_finish_kernel(const double* raw,
+                                                              const double* p, int N, int S,
+                                                              const double* pos,
+                                                              const double* sums,
                                                               double* __restrict__ out) {
+  previous_done();
   const int k = blockIdx.y, l = blockIdx.x * 256 + threadIdx.x;
   __shared__ double ratio;
   if (threadIdx.x == 0) ratio = sums[0] / sums[2];
@@ -524,6 +530,7 @@ static bool sliced_size(int N) { return N >= 64 && N <= 16384; }
 
 struct PixelSpace {
   double* sums;          // [0] sum p, [1] sum of the grid samples, [2] sum of the resampled
+  int* status;           // behind sums: two words each of the tensor-core products
   double* sinc;          // [N] sinc(fftfreq * os)
   double* d;
   // GEMM path
@@ -548,7 +555,8 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
   int logN;
   const size_t NN = (size_t)N * N;
   const int Nd = N / std::max(os, 1);
-  t.sums = static_cast<double*>(take(4 * sizeof(double)));
+  t.sums = static_cast<double*>(take(4 * sizeof(double) + 4 * sizeof(int)));
+  t.status = reinterpret_cast<int*>(t.sums + 4);
   t.sinc = static_cast<double*>(take((size_t)N * sizeof(double)));
   t.d = static_cast<double*>(take((size_t)Nd * Nd * sizeof(double)));
   const bool fft = fft_size(N, &logN);
@@ -585,7 +593,7 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
 // to sums[0]; with d, every os-th sample and their sum (sums[1]).
 static int run_pixel(const double* img, int N, int os_mtf, PixelSpace* w, double* P, int os, double* d,
                      cudaStream_t s) {
-  LGB_CUDA(cudaMemsetAsync(w->sums, 0, 4 * sizeof(double), s));
+  LGB_CUDA(cudaMemsetAsync(w->sums, 0, 4 * sizeof(double) + 4 * sizeof(int), s));
   sinc_table_kernel<<<cdiv(2 * N, 128), 128, 0, s>>>(N, (double)os_mtf, w->sinc, w->tab);
   int logN;
   const double* src;
@@ -609,9 +617,8 @@ static int run_pixel(const double* img, int N, int os_mtf, PixelSpace* w, double
     transpose_f64_kernel<<<tgrid, tblock, 0, s>>>(R, RT, N);
     src = RT;
   } else {
-    pixel_taps_kernel<<<N, 128, 0, s>>>(N, w->sinc, w->tab, w->c);
-    LGB_CUDA(cudaGetLastError());
-    if (sliced_size(N)) return launch_pixel_sliced(img, N, w->c, w->sliced, P, w->sums, os, d, s);
+    LGB_CUDA(launch_next(pixel_taps_kernel, N, 128, 0, s, N, w->sinc, w->tab, w->c));
+    if (sliced_size(N)) return launch_pixel_sliced(img, N, w->c, w->sliced, w->status, P, w->sums, os, d, s);
     circulant_kernel<<<dim3(cdiv(N, 128), N), 128, 0, s>>>(N, w->c, w->C);
     dim3 grid(cdiv(N, DBN), cdiv(N, DBM));
     dgemm_kernel<<<grid, 256, 0, s>>>(N, w->C, img, w->T);      // T = C . img
@@ -791,18 +798,18 @@ extern "C" int lgb_pixelate(const double* img, int rows, int cols, int oversampl
   int logN;
   double* const P = fft_size(N, &logN) ? reinterpret_cast<double*>(w.Y) : w.P;
   if ((st = run_pixel(img, N, os, &w, P, 1, nullptr, s))) return st;
-  resample_operator_kernel<<<S, 4 * RS_BW, 0, s>>>(N, os, S, w.Gt, w.q0, w.pos);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(resample_operator_kernel, S, 4 * RS_BW, 0, s, N, os, S, w.Gt, w.q0, w.pos));
   if (sliced_size(N)) {
-    if ((st = launch_resample_sliced(P, N, os, S, w.Gt, w.q0, w.sliced, w.raw, w.sums + 2, s))) return st;
+    if ((st = launch_resample_sliced(P, N, os, S, w.Gt, w.q0, w.sliced, w.status + 2, w.raw, w.sums + 2,
+                                     s)))
+      return st;
   } else {
     resample_rows_kernel<<<dim3(cdiv(S, 64), cdiv(N, 4 * RS_ROWS)), dim3(64, 4), 0, s>>>(
         P, N, S, w.Gt, w.q0, w.Tm);
     resample_cols_kernel<<<dim3(cdiv(S, 64), cdiv(S, 4 * RS_OUT)), dim3(64, 4), 0, s>>>(
         w.Tm, N, S, w.Gt, w.q0, w.raw, w.sums);
   }
-  resample_finish_kernel<<<dim3(cdiv(S, 256), S), 256, 0, s>>>(w.raw, P, N, S, w.pos, w.sums, out);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(resample_finish_kernel, dim3(cdiv(S, 256), S), 256, 0, s, w.raw, P, N, S, w.pos, w.sums, out));
   return LGB_OK;
 }
 

@@ -16,12 +16,13 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // |C img C^T| for the circulant C of the taps c[N]: P[N][N] (may be null), its
 // sum added to sums[0]; with d, every os-th sample and their sum (sums[1])
+// status: two words, zero: [0] an expired wait, [1] non-finite input
 size_t pixel_sliced_workspace(int N);
-int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, double* P, double* sums, int os,
-                        double* d, cudaStream_t s);
+int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, int* status, double* P, double* sums,
+                        int os, double* d, cudaStream_t s);
 // raw = G P G^T for the banded operator (Gt[RS_BW][S], q0[S]), its sum added to *sum
 size_t resample_sliced_workspace(int N, int os, int S);
 int launch_resample_sliced(const double* P, int N, int os, int S, const double* Gt, const int* q0, void* ws,
-                           double* raw, double* sum, cudaStream_t s);
+                           int* status, double* raw, double* sum, cudaStream_t s);
 
 }  // namespace lgb

@@ -192,6 +192,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const uint32_t drain_bar = bars + 128u;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 160);
 
+  next_may_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = blockIdx.x * p.deal.per, end = min(p.total, begin + p.deal.per);
 
@@ -218,6 +219,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  previous_done();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -603,8 +605,7 @@ inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int i
   p.stride = stride;
   p.err = err;
   p.wait_ns = WAIT_NS;
-  sliced_gemm_kernel<<<cdiv(p.total, deal.per), NUM_THREADS, SMEM_BYTES, s>>>(a, b, p);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(sliced_gemm_kernel, cdiv(p.total, deal.per), NUM_THREADS, SMEM_BYTES, s, a, b, p));
   return LGB_OK;
 }
 
