@@ -133,10 +133,10 @@ __device__ __forceinline__ void ft_store_4d(const CUtensorMap* map, uint32_t src
 }
 
 // a read-once stream: no L1 allocation (the block's wavelength loop keeps
-// the values in registers)
+// the values in registers); volatile, to stay behind previous_done
 __device__ __forceinline__ double ld_stream(const double* p) {
   double v;
-  asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  asm volatile("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(v) : "l"(p));
   return v;
 }
 
@@ -152,6 +152,8 @@ __global__ void __launch_bounds__(256, BF16 ? 5 : 4) split_field_T_kernel(SplitF
                                                             const __grid_constant__ CUtensorMap map_lo) {
   extern __shared__ uint8_t ft_smem_raw[];
   __shared__ int warp_nz[8];
+  next_may_start();
+  previous_done();
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(ft_smem_raw);
   const uint32_t tiles = (raw + 1023u) & ~1023u;                          // 1024-byte aligned
   uint8_t* const tile = ft_smem_raw + (tiles - raw);
@@ -318,8 +320,7 @@ int launch_split_field_T(const SplitFieldArgs& a, bool bf16, cudaStream_t s) {
   }
   groups = cdiv(L, cdiv(L, groups));                 // no empty trailing group
   dim3 grid(cdiv(a.kp, TR) * groups, cdiv(a.n, TC), psfs);
-  kfn<<<grid, 256, FT_SMEM_BYTES, s>>>(a, groups, map_hi, map_lo);
-  LGB_CUDA(cudaGetLastError());
+  LGB_CUDA(launch_next(kfn, grid, 256, FT_SMEM_BYTES, s, a, groups, map_hi, map_lo));
   return LGB_OK;
 }
 
@@ -334,6 +335,7 @@ __device__ __forceinline__ float warp_max(float v) {
 
 __global__ void maxabs_amp_kernel(const double* __restrict__ amp, int H, int W, int r0, int c0,
                                   int m, int n, float* __restrict__ out) {
+  next_may_start();
   const int b = blockIdx.y;
   float v = 0.f;
   const size_t total = (size_t)m * n;
@@ -347,6 +349,7 @@ __global__ void maxabs_amp_kernel(const double* __restrict__ amp, int H, int W, 
 }
 
 __global__ void maxabs_c128_kernel(const double2* __restrict__ f, int count, float* __restrict__ out) {
+  next_may_start();
   float v = 0.f;
   f += (size_t)blockIdx.y * count;                 // field blockIdx.y of a batch
   out += blockIdx.y;

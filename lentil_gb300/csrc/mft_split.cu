@@ -196,8 +196,8 @@ __device__ __forceinline__ Live live_kblocks(const Params& p, const Item& w) {
     bool nz = false;
     if (u < U) {
       const uint8_t* fu = f + (size_t)u * p.kf_pitch;
-      nz = BN == 256 ? __ldg(reinterpret_cast<const unsigned long long*>(fu)) != 0ull
-                     : __ldg(reinterpret_cast<const unsigned int*>(fu)) != 0u;
+      nz = BN == 256 ? *reinterpret_cast<const unsigned long long*>(fu) != 0ull
+                     : *reinterpret_cast<const unsigned int*>(fu) != 0u;
     }
     unit[g] = __ballot_sync(0xffffffffu, nz);
   }
@@ -368,6 +368,7 @@ split_mft_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_consta
   const uint32_t drain_bar = bars + 96u;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + (bars - base) + 112);
 
+  next_may_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
@@ -396,6 +397,7 @@ split_mft_kernel(const __grid_constant__ CUtensorMap tmA_hi, const __grid_consta
   cluster_sync();                        // both CTAs' barriers and TMEM are ready
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  previous_done();
 
   if (warp == 0) {
     // ------------------------------------------------------ TMA producer
@@ -588,13 +590,15 @@ static cudaLaunchConfig_t pair_config(uint32_t smem, cudaStream_t s, cudaLaunchA
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // as launch_next
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(2);
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cfg;
 }
 
@@ -620,7 +624,7 @@ static int max_pairs() {
   if (set_smem_attr<BF16, BN, KB>() != cudaSuccess) return 0;
   std::lock_guard<std::mutex> lock(mu);
   if (cached[dev] == 0) {
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     cudaLaunchConfig_t cfg = pair_config(TileCfg<BN>::SMEM_BYTES, 0, attr);
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, split_mft_kernel<BF16, BN, KB>, &cfg) != cudaSuccess) n = 0;
@@ -637,7 +641,7 @@ static int launch_one(const Params& p, const CUtensorMap& a_hi, const CUtensorMa
   if (p.n_items <= 0) return LGB_OK;
   const int pairs = max_pairs<BF16, BN, KB>();
   LGB_REQUIRE(pairs > 0, LGB_ECUDA, "split mft: no CTA pair of the tensor-core kernel fits on this GPU");
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cudaLaunchConfig_t cfg = pair_config(TileCfg<BN>::SMEM_BYTES, s, attr);
   cfg.gridDim = dim3(2 * std::min(p.n_items, pairs));
   LGB_CUDA(cudaLaunchKernelEx(&cfg, split_mft_kernel<BF16, BN, KB>, a_hi, a_lo, b_hi, b_lo, c0, c1, p));
