@@ -10,8 +10,9 @@
  * never aborts the process; lgb_last_error() returns the message of the
  * calling thread's last failure.
  *
- * Precision: LGB_FP64 computes in complex128 (the plain form, parity with
- * lentil within 1e-12 peak-normalised).  LGB_SPLIT_BF16 / LGB_SPLIT_FP16 run
+ * Precision: LGB_FP64 computes in complex128 (parity with lentil within 1e-12
+ * peak-normalised): exact digit products on the tensor cores, or the FP64
+ * units for small transforms.  LGB_SPLIT_BF16 / LGB_SPLIT_FP16 run
  * the contractions on the tcgen05 tensor cores with each operand split into
  * two 16-bit floats (hi + lo; three partial products, FP32 accumulation).
  */

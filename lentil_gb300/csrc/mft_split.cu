@@ -838,9 +838,9 @@ static TuneKey tune_key(const SplitMftProblem& q) {
 // Cost of each width: waves of work items over the resident CTA pairs times
 // K blocks, a 128-wide item costing 0.52 of a 256-wide one (measured on the
 // broadband workload: twice the items took 1.04x the time at full occupancy;
-// 0.78 and 1.47x while one lane alone issued the MMAs).  Either width holds one CTA per SM, so the pairs are taken as
-// half the SMs: no occupancy query, which keeps the model usable inside a
-// stream capture.  Returns the cheaper width.
+// 0.78 and 1.47x while one lane alone issued the MMAs).  Either width holds one
+// CTA per SM, so the pairs are taken as half the SMs: no occupancy query, which
+// keeps the model usable inside a stream capture.  Returns the cheaper width.
 static int model_tile(const SplitMftProblem& q) {
   double cost[2];
   const int bns[2] = {256, 128};

@@ -168,8 +168,8 @@ __device__ __forceinline__ void mma_run(int i, int j0, int j1, uint32_t on, uint
 // took 3900 clk.  Runs over B's digits with A's in the collector read 4.6 KB and
 // run at 49: 1019 x 941 to 1024^2 went from 121 to 110 us per GEMM (transform
 // 300 -> 283), 512^2 from 76 to 71.5.  What is left above the 81 us of MMAs: the
-// first loads and the last sums (6 us), loads (830 MB from L2 in all, 12 %) and
-// drains (9 %) that the MMAs wait for.
+// first loads and the last sums (6 us), loads (12 %, by latency: L2 runs at a
+// third of its rate) and drains (9 %) that the MMAs wait for.
 //
 // Roles: warp 0 TMA (two stages of 32 K entries; digits 4 to 6 of a stage are
 // done with, and loaded anew, while its sums 0 to 3 run), warp 1 MMA issue,

@@ -24,8 +24,11 @@ from . import util
 # Device-resident DFT matrices of recently used geometries (lgb_dft2_plan_*):
 # a repeated transform of one geometry builds no matrices and copies nothing
 # from the host.  Least recently used plans are destroyed beyond either bound.
+# (A complex128 matrix entry takes 42 bytes in digits, 16 as a number: 3 GiB hold
+# the plans that 1 GiB of the plain form did, a 3000-pixel transform and its
+# adjoint among them.)
 PLAN_CACHE_ENTRIES = 32
-PLAN_CACHE_BYTES = 1 << 30
+PLAN_CACHE_BYTES = 3 << 30
 
 
 class _Dft2Plan:
