@@ -251,12 +251,13 @@ __device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
   __syncthreads();
 }
 
-constexpr int FIN_ROWS = 4;                  // rows per finish block
+constexpr int FIN_ROWS = 4;                  // rows per finish block, of launches that fill the GPU
 
 // F = P's entries, scaled.  Bound by reading P from L2 and writing F (40 bytes
 // an entry and a part; 21 us at 1024^2, cold caches).  Results are put together
 // from bits and four rows' parts are in flight at once: with conversions and
 // both scalings on the FP64 pipe and a row per block it took half as long again.
+template <int ROWS>
 __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
   previous_done();
   const int b = blockIdx.z, flag = p.exps[(size_t)b * (p.left ? p.M : p.N)];      // all of them, if one is
@@ -265,34 +266,34 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
     for (int q = blockIdx.y; q < (p.left ? p.M : p.N); q += gridDim.y) plain_line(p, b, q);
     return;
   }
-  const int v = blockIdx.x * 256 + threadIdx.x, u0 = blockIdx.y * FIN_ROWS;
+  const int v = blockIdx.x * 256 + threadIdx.x, u0 = blockIdx.y * ROWS;
   if (v >= p.N) return;
   double2* F = p.F + ((size_t)b * p.M + u0) * p.N + v;
-  const int rows = min(FIN_ROWS, p.M - u0);
+  const int rows = min(ROWS, p.M - u0);
   if (flag == EXP_NAN) {
     const double nan = __longlong_as_double(0x7FF8000000000000ll);
     for (int i = 0; i < rows; ++i) F[(size_t)i * p.N] = make_double2(nan, nan);
     return;
   }
   const int* exps = p.exps + (p.left ? (size_t)b * p.M + u0 : (size_t)b * p.N + v);
-  longlong2 z[FIN_ROWS];
-  size_t at[FIN_ROWS];
-  int n[3][FIN_ROWS], e[FIN_ROWS];
-  static_assert(BN % FIN_ROWS == 0, "the rows lie in one tile");
+  longlong2 z[ROWS];
+  size_t at[ROWS];
+  int n[3][ROWS], e[ROWS];
+  static_assert(BN % ROWS == 0, "the rows lie in one tile");
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const int parts = p.q.parts(3 * b + c, u0, v);
 #pragma unroll
-    for (int i = 0; i < FIN_ROWS; ++i) n[c][i] = i < rows ? parts : 0;
+    for (int i = 0; i < ROWS; ++i) n[c][i] = i < rows ? parts : 0;
   }
 #pragma unroll
-  for (int i = 0; i < FIN_ROWS; ++i) {
+  for (int i = 0; i < ROWS; ++i) {
     at[i] = (size_t)(u0 + i) * p.q.ld + v;
     e[i] = i < rows ? exps[p.left ? i : 0] - 16 - p.S : 0;
   }
-  sum_parts3<FIN_ROWS>(p.q.P + (size_t)b * 3 * p.q.stride, p.q.stride, p.q.part(), at, n, z);
+  sum_parts3<ROWS>(p.q.P + (size_t)b * 3 * p.q.stride, p.q.stride, p.q.part(), at, n, z);
 #pragma unroll
-  for (int i = 0; i < FIN_ROWS; ++i)
+  for (int i = 0; i < ROWS; ++i)
     if (i < rows)
       F[(size_t)i * p.N] = make_double2(scaled(z[i].x, e[i], p.scale), scaled(z[i].y, e[i], p.scale));
 }
@@ -434,7 +435,14 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     p.cols = q.cols;
     p.scratch = t.P;
     p.err = t.err;
-    LGB_CUDA(launch_next(finish_kernel, dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s, p));
+    // four rows a block where that is a block per SM; below, one row (256^2: 64
+    // blocks of four rows, the transform 34.9 us, 256 of one, 31.3; 512^2: 256
+    // blocks of four, 57.7, 1024 of one, 60.6)
+    const int blocks = cdiv(q.N, 256) * cdiv(q.M, FIN_ROWS) * items;
+    if (blocks >= GPU_SMS)
+      LGB_CUDA(launch_next(finish_kernel<FIN_ROWS>, dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s, p));
+    else
+      LGB_CUDA(launch_next(finish_kernel<1>, dim3(cdiv(q.N, 256), q.M, items), 256, 0, s, p));
     if (own) {
       e1.base += (size_t)items * ND * e1.plane();
       e2.base += (size_t)items * ND * e2.plane();

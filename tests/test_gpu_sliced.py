@@ -143,3 +143,14 @@ def test_pixelate_of_non_finite_images(cuda_device, bad):
     p = lg.detector.pixel(img, 2)
     assert not np.isfinite(p).any()
     assert np.isfinite(lg.detector.pixelate(np.nan_to_num(img, posinf=1.0), 3)).all()
+
+
+@pytest.mark.parametrize('shape', [(120, 130, 602, 601), (120, 130, 301, 257), (120, 130, 97, 130)])
+def test_finish_rows(cuda_device, shape):
+    # results in groups of four rows (the last group partly filled) and row by row
+    m, n, M, N = shape
+    alpha = (0.7 / max(m, M), 0.6 / max(n, N))
+    f = _field(m, n, 9)
+    ref = _plain(f, M, N, alpha, ARGS['shift'], ARGS['offset'])
+    F = lg.fourier.dft2(f, alpha, shape=(M, N), **ARGS)
+    assert float((F - ref).abs().max()) <= 2 * max(m, n) * 2.0 ** -53 * float(ref.abs().max())
