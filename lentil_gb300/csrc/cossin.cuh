@@ -96,14 +96,19 @@ __device__ __forceinline__ longlong2 cossin_q62(uint64_t ph, const unsigned long
   return p.at & 256 ? make_longlong2(-z.x, -z.y) : z;
 }
 
-// (cos, sin)(pi x) as doubles, each within 1.2 units of its last place: x 2^63
-// mod 2^64 is the phase, exactly (below |x| = 2^-11 up to its last place).
-// Next to an axis (at & 127 = 0) the small one of the two is sin d from d's
-// leading 64 bits, wherever they lie.
-__device__ __forceinline__ double2 cossinpi_f64(double x, const unsigned long long* table) {
+// v 2^e, or its negative
+struct FixedValue {
+  uint64_t v;
+  int e;
+  bool neg;
+};
+
+// cos and sin of pi x, x finite: x 2^63 mod 2^64 is the phase, exactly (below
+// |x| = 2^-11 up to its last place).  Next to an axis (at & 127 = 0) the small
+// one of the two is sin d from d's leading 64 bits, wherever they lie.
+__device__ __forceinline__ void cossinpi(double x, const unsigned long long* table, FixedValue& c, FixedValue& s) {
   const uint64_t bits = (uint64_t)__double_as_longlong(x);
   int E = (int)(bits >> 52) & 0x7FF;
-  if (E == 0x7FF) return make_double2(x - x, x - x);                     // NaN
   uint64_t m = bits & 0xFFFFFFFFFFFFFull;
   if (E == 0) E = 1; else m |= 1ull << 52;
   const int sh = E - 1012;                                               // x 2^63 = m 2^sh
@@ -113,21 +118,46 @@ __device__ __forceinline__ double2 cossinpi_f64(double x, const unsigned long lo
   if (sh < 0) p.neg = bits >> 63;
   uint64_t u;
   const longlong2 z = first_quadrant_q62(p, table, u);
-  uint64_t big = (uint64_t)z.x, v = (uint64_t)z.y;                       // cos, sin of the first quadrant's angle
-  int e = -62;
-  bool neg = false;
+  c = FixedValue{(uint64_t)z.x, -62, false};                             // of the first quadrant's angle
+  s = FixedValue{(uint64_t)z.y, -62, false};
   if ((p.at & 127) == 0) {
     const uint64_t r = sh < 0 ? m : p.ar;
     const int lz = __clzll((long long)r);
     const uint64_t dn = __umul64hi(lz < 64 ? r << lz : 0, 14488038916154245685ull);    // d 2^(61 + lz)
-    v = dn - __umul64hi(dn, u >> 8);
-    e = -61 - lz + (sh < 0 ? sh : 0);
-    neg = p.neg;
+    s = FixedValue{dn - __umul64hi(dn, u >> 8), -61 - lz + (sh < 0 ? sh : 0), p.neg};
   }
-  double c = assembled(big, -62), s = assembled(v, e);
-  if (neg) s = -s;
-  if (p.at & 128) { const double t = c; c = -s; s = t; }
-  return p.at & 256 ? make_double2(-c, -s) : make_double2(c, s);
+  if (p.at & 128) {
+    const FixedValue t = c;
+    c = FixedValue{s.v, s.e, !s.neg};
+    s = t;
+  }
+  if (p.at & 256) {
+    c.neg = !c.neg;
+    s.neg = !s.neg;
+  }
+}
+
+// a exp(i pi x), each component within 1.3 units of its last place.  The
+// product with the amplitude is taken in integers too: a double-precision
+// multiply holds the FP64 pipe 16 clocks a warp.
+__device__ __forceinline__ double2 phasor_f64(double a, double x, const unsigned long long* table) {
+  if (((uint32_t)__double2hiint(x) & 0x7FF00000u) == 0x7FF00000u) return make_double2(x - x, x - x);   // NaN
+  const uint64_t bits = (uint64_t)__double_as_longlong(a);
+  if (bits << 1 == 0) return make_double2(0.0, 0.0);                     // outside the pupil
+  FixedValue c, s;
+  cossinpi(x, table, c, s);
+  const int E = (int)(bits >> 52) & 0x7FF;
+  if (E == 0 || E == 0x7FF) {                                            // subnormal, not finite
+    const double cv = assembled(c.v, c.e), sv = assembled(s.v, s.e);
+    return make_double2(a * (c.neg ? -cv : cv), a * (s.neg ? -sv : sv));
+  }
+  const uint64_t ma = bits << 11 | 1ull << 63;                           // |a| = ma 2^(E - 1086)
+  auto times = [&](const FixedValue& q) {
+    const int lz = __clzll((long long)q.v);
+    const double r = q.v ? assembled(__umul64hi(q.v << lz, ma), q.e - lz + E - 1022) : 0.0;
+    return q.neg != (bool)(bits >> 63) ? -r : r;
+  };
+  return make_double2(times(c), times(s));
 }
 
 }  // namespace lgb

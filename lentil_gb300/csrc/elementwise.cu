@@ -29,8 +29,7 @@ __global__ void phasor_c128_kernel(const double* __restrict__ amp, double amp_va
   double a = amp ? amp[p] : amp_value;
   if (mask) a *= mask[p];
   const double o = opd ? opd[p] : opd_value;
-  const double2 e = cossinpi_f64(o * two_over_lambda, COS_TABLE);     // exp(+2 pi i opd/lambda)
-  out[(size_t)i * n + j] = make_double2(a * e.x, a * e.y);
+  out[(size_t)i * n + j] = phasor_f64(a, o * two_over_lambda, COS_TABLE);   // a exp(+2 pi i opd/lambda)
 }
 
 // A stack of K phasors amp * exp(2 pi i opd_k / lambda) over one slice, for
@@ -50,7 +49,7 @@ __global__ void phasor_stack_kernel(const double* __restrict__ amp,
   const size_t p = (size_t)(r0 + i) * W + (c0 + j);
   const double a = amp[p];
   const double o = opd[(size_t)k * H * W + p];
-  double s, c;
+  double2 f;
   if (FAST) {
     const float oh = (float)o, ol = (float)(o - (double)oh);
     const float ph = oh * khalf.x;
@@ -59,18 +58,16 @@ __global__ void phasor_stack_kernel(const double* __restrict__ amp,
     const float x = (ph - 2.f * rintf(0.5f * ph)) + e;
     float sf, cf;
     sincospif(x, &sf, &cf);
-    s = sf;
-    c = cf;
+    f = make_double2(a * cf, a * sf);
   } else {
-    const double2 e = cossinpi_f64(o * two_over_lambda, COS_TABLE);
-    c = e.x;
-    s = e.y;
+    f = phasor_f64(a, o * two_over_lambda, COS_TABLE);
   }
-  out[((size_t)k * m + i) * n + j] = make_double2(a * c, a * s);
+  out[((size_t)k * m + i) * n + j] = f;
 }
 
-// Bound by the some 150 integer operations a value takes (33 MB written in 41 us):
-// 512^2 at 8 wavelengths took 117 us with sincospi.
+// Bound by the some 150 integer operations a value takes: 512 x 475 at 8
+// wavelengths took 117 us with sincospi, 41 with the amplitude multiplied on the
+// FP64 pipe and nothing skipped outside the pupil, 31 so.
 __global__ void phasor_batch_c128_kernel(const double* __restrict__ amp,
                                          const double* __restrict__ opd, int H, int W, int r0,
                                          int c0, int m, int n,
@@ -85,10 +82,8 @@ __global__ void phasor_batch_c128_kernel(const double* __restrict__ amp,
   if (j >= n || i >= m) return;
   const size_t p = ((size_t)b * H + r0 + i) * W + (c0 + j);
   const double a = amp[p], o = opd[p];
-  for (int l = 0; l < L; ++l) {
-    const double2 e = cossinpi_f64(o * two_over_lambda[l], table);
-    out[(((size_t)b * L + l) * m + i) * n + j] = make_double2(a * e.x, a * e.y);
-  }
+  for (int l = 0; l < L; ++l)
+    out[(((size_t)b * L + l) * m + i) * n + j] = phasor_f64(a, o * two_over_lambda[l], table);
 }
 
 int launch_phasor_batch_c128(const double* amp, const double* opd, int H, int W, int r0, int c0,

@@ -59,3 +59,21 @@ def test_phasor_non_finite(cuda_device):
               dv.stream_ptr())
     got = out.cpu().numpy()
     assert np.all(np.isnan(got[:3].real) & np.isnan(got[:3].imag)) and np.isfinite(got[3])
+
+
+@pytest.mark.parametrize('amp', [1.0, -0.7310585786300049, 3e300, 2e-290, 5e-324, 0.0, float('inf'), float('nan')])
+def test_phasor_amplitude(cuda_device, amp):
+    x = np.concatenate([_phases('axes'), _phases('near')[:500], _phases('table')[:500]])
+    opd = torch.as_tensor(x, device='cuda')
+    a = torch.full((len(x),), amp, dtype=torch.float64, device='cuda')
+    out = torch.empty(len(x), dtype=torch.complex128, device='cuda')
+    _lib.call('lgb_phasor', a.data_ptr(), 0.0, None, opd.data_ptr(), 0.0, 1, len(x), 0, 0, 1, len(x), 2.0,
+              out.data_ptr(), dv.stream_ptr())
+    got = out.cpu().numpy()
+    with np.errstate(all='ignore'):
+        for g, r in zip((got.real, got.imag), _reference(x)):
+            want = np.longdouble(amp) * r
+            ok = np.isfinite(want)
+            assert np.array_equal(np.isnan(g), np.isnan(want)) and np.array_equal(np.isinf(g), np.isinf(want))
+            # as above; subnormal results have an absolute last place
+            assert np.all(np.abs(g[ok] - want[ok]) <= 2.6e-16 * np.abs(want[ok]) + 5e-324)
