@@ -148,7 +148,7 @@ size_t exec_carve(const lgb_dft2_plan_s* P, int count, void* base, ExecSpace* s)
   PlanCarve c(base);
   ExecSpace t{};
   if (split_precision(P->precision)) {
-    t.maxabs = c.take<float>(std::max(count, 4));
+    t.maxabs = c.take<float>(maxabs_floats(count));
     t.fh = c.take<uint16_t>((size_t)count * P->n * 2 * P->kp1);
     t.fl = c.take<uint16_t>((size_t)count * P->n * 2 * P->kp1);
     t.gh = c.take<uint16_t>((size_t)count * P->M * 2 * P->kp2);

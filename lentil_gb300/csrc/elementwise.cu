@@ -127,6 +127,12 @@ __device__ __forceinline__ void ft_store_4d(const CUtensorMap* map, uint32_t src
       : "memory");
 }
 
+__device__ __forceinline__ float warp_max(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
 // a read-once stream: no L1 allocation (the block's wavelength loop keeps
 // the values in registers); volatile, to stay behind previous_done
 __device__ __forceinline__ double ld_stream(const double* p) {
@@ -156,7 +162,14 @@ __global__ void __launch_bounds__(256, BF16 ? 5 : 4) split_field_T_kernel(SplitF
   const int rtile = blockIdx.x / groups, g = blockIdx.x - rtile * groups;   // row tile, group
   const int rt = rtile * TR, ct = blockIdx.y * TC;
   const int b = blockIdx.z;                                                 // PSF
-  const float sf = a.maxabs ? pow2_scale_for(a.maxabs[b]) : 1.f;   // none: unscaled (bf16)
+  float sf = 1.f;                                                           // no maxima: unscaled (bf16)
+  if (a.maxabs) {
+    const float4 q = reinterpret_cast<const float4*>(a.maxabs + (a.batch + 3) / 4 * 4)[b * (MAXABS_PARTS / 4) +
+                                                                                    (tid & 31)];
+    const float v = warp_max(fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w)));
+    if (blockIdx.x == 0 && blockIdx.y == 0 && tid == 0) a.maxabs[b] = v;
+    sf = pow2_scale_for(v);
+  }
 
   // thread (w, lane) owns field column ct + lane and rows rt + 8w .. 8w+7:
   // each global load instruction reads 32 consecutive columns of one row,
@@ -319,56 +332,62 @@ int launch_split_field_T(const SplitFieldArgs& a, bool bf16, cudaStream_t s) {
   return LGB_OK;
 }
 
+// max |.| reductions feeding the power-of-two split scales: a partial maximum per
+// block, taken on the bits (conversions would hold the FP64 pipe), NaN ignored.
+// Nothing is cleared first (a memset and atomics, with the operand kernel waiting
+// for both, took 6 us more of the 58 of a (3, 512, 512) transform).
 // ---------------------------------------------------------------------------
-// max |.| reductions feeding the power-of-two split scales
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
+__device__ __forceinline__ void note_max(double x, uint64_t& v) {
+  const uint64_t bits = (uint64_t)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  if (bits <= 0x7FF0000000000000ull && bits > v) v = bits;
 }
 
-__global__ void maxabs_amp_kernel(const double* __restrict__ amp, int H, int W, int r0, int c0,
-                                  int m, int n, float* __restrict__ out) {
+__device__ __forceinline__ void store_block_max(uint64_t bits, float* out) {       // 256 threads
+  __shared__ float sm[8];
+  const float v = warp_max((float)__longlong_as_double((long long)bits));
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const float w = warp_max(threadIdx.x < 8 ? sm[threadIdx.x] : 0.f);
+    if (threadIdx.x == 0) *out = w;
+  }
+}
+
+__global__ void __launch_bounds__(256) maxabs_amp_kernel(const double* __restrict__ amp, int H, int W, int r0, int c0,
+                                                         int m, int n, float* __restrict__ part) {
   next_may_start();
   const int b = blockIdx.y;
-  float v = 0.f;
+  uint64_t v = 0;
   const size_t total = (size_t)m * n;
-  for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < total;
-       p += (size_t)gridDim.x * blockDim.x) {
+  for (size_t p = (size_t)blockIdx.x * 256 + threadIdx.x; p < total; p += (size_t)MAXABS_PARTS * 256) {
     const int i = (int)(p / n), j = (int)(p % n);
-    v = fmaxf(v, (float)fabs(amp[((size_t)b * H + r0 + i) * W + c0 + j]));
+    note_max(amp[((size_t)b * H + r0 + i) * W + c0 + j], v);
   }
-  v = warp_max(v);
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(out + b), __float_as_int(v));
+  store_block_max(v, part + b * MAXABS_PARTS + blockIdx.x);
 }
 
-__global__ void maxabs_c128_kernel(const double2* __restrict__ f, int count, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) maxabs_c128_kernel(const double2* __restrict__ f, int count,
+                                                          float* __restrict__ part) {
   next_may_start();
-  float v = 0.f;
+  uint64_t v = 0;
   f += (size_t)blockIdx.y * count;                 // field blockIdx.y of a batch
-  out += blockIdx.y;
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < count; p += gridDim.x * blockDim.x) {
+  for (int p = blockIdx.x * 256 + threadIdx.x; p < count; p += MAXABS_PARTS * 256) {
     const double2 z = f[p];
-    v = fmaxf(v, fmaxf((float)fabs(z.x), (float)fabs(z.y)));
+    note_max(z.x, v);
+    note_max(z.y, v);
   }
-  v = warp_max(v);
-  if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(out), __float_as_int(v));
+  store_block_max(v, part + blockIdx.y * MAXABS_PARTS + blockIdx.x);
 }
 
 int launch_maxabs_amp(const double* amp, int batch, int H, int W, int r0, int c0, int m, int n,
                       float* out, cudaStream_t s) {
-  LGB_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * batch, s));
-  const int blocks = (int)std::min<size_t>(2 * (size_t)sm_count(), cdiv(m * n, 256));
-  maxabs_amp_kernel<<<dim3(blocks > 0 ? blocks : 1, batch), 256, 0, s>>>(amp, H, W, r0, c0, m, n, out);
+  maxabs_amp_kernel<<<dim3(MAXABS_PARTS, batch), 256, 0, s>>>(amp, H, W, r0, c0, m, n, out + round_up(batch, 4));
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }
 
 int launch_maxabs_c128_batch(const double2* f, int count, int batch, float* out, cudaStream_t s) {
-  LGB_CUDA(cudaMemsetAsync(out, 0, sizeof(float) * batch, s));
-  const int blocks = std::max(1, std::min(2 * sm_count(), cdiv(count, 256)));
-  maxabs_c128_kernel<<<dim3(blocks, batch), 256, 0, s>>>(f, count, out);
+  maxabs_c128_kernel<<<dim3(MAXABS_PARTS, batch), 256, 0, s>>>(f, count, out + round_up(batch, 4));
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
 }

@@ -87,7 +87,7 @@ struct SplitFieldArgs {
   const double2* field;    // [batch][m][n] complex128 (L 1)
   // common
   int m, n, kp, L, batch;
-  const float* maxabs;     // [batch] max |component| of the field (device), or null: no scale
+  float* maxabs;           // launch_maxabs's result (device), or null: no scale
   uint16_t* hi;            // [batch*L][n][2*kp]
   uint16_t* lo;
   const int* lam_idx;      // optional [L] device: wavelength -> khalf slot
@@ -104,10 +104,13 @@ int launch_split_field_T(const SplitFieldArgs& a, bool bf16, cudaStream_t s);
 // at kp and n (mft_split.cu).
 int make_field_T_store_map(CUtensorMap* map, const uint16_t* ptr, bool bf16, int kp, int n, int Q);
 
-// max over the slice of |amp| (phasor mode) or max(|re|,|im|) (complex mode)
+// max over the slice of |amp| (phasor mode) or max(|re|,|im|) (complex mode) per
+// field, in maxabs_floats(batch) floats: partial maxima only; the operand kernel
+// (split_field_T) forms out[b] from them
+constexpr int MAXABS_PARTS = 128;
+inline size_t maxabs_floats(int batch) { return (size_t)round_up(batch, 4) * (1 + MAXABS_PARTS); }
 int launch_maxabs_amp(const double* amp, int batch, int H, int W, int r0, int c0, int m, int n,
                       float* out, cudaStream_t s);
-// per field b < batch of `count` entries each: out[b] = max(|re|, |im|)
 int launch_maxabs_c128_batch(const double2* f, int count, int batch, float* out, cudaStream_t s);
 
 // out[i,j] (+)= (re, im) scaled; generic complex128 copy/convert kernels

@@ -80,7 +80,7 @@ static size_t carve_split(void* ws, int count, int m, int n, int M, int N, Dft2S
   Dft2SplitSpace t;
   t.err = c.take<int>(4);
   t.axes = c.take<PhaseAxis>(2);
-  t.maxabs = c.take<float>(std::max(count, 4));
+  t.maxabs = c.take<float>(maxabs_floats(count));
   t.unit2 = c.take<double>(2);
   t.e1h = c.take<uint16_t>(mrows1 * 2 * kp1);
   t.e1l = c.take<uint16_t>(mrows1 * 2 * kp1);
@@ -294,7 +294,7 @@ static size_t carve_operands(void* base, const lgb_psf_desc& d, int kp1, int kp2
   SplitOperands t;
   const size_t Q = (size_t)B * L;
   t.err = c.take<int>(4);
-  t.maxabs = c.take<float>(B);
+  t.maxabs = c.take<float>(maxabs_floats(B));
   t.fh = c.take<uint16_t>(Q * d.n * 2 * kp1);
   t.fl = c.take<uint16_t>(Q * d.n * 2 * kp1);
   t.gh = c.take<uint16_t>(Q * d.M * 2 * kp2);
@@ -346,7 +346,7 @@ static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
   P->two_over_lambda = c.take<double>(L);
   P->khalf = c.take<float2>(L);
   P->axes = c.take<PhaseAxis>(2 * (size_t)L);
-  P->maxabs = c.take<float>(B);
+  P->maxabs = c.take<float>(maxabs_floats(B));
   if (is_split(d.precision)) {
     const size_t mrows1 = (size_t)cdiv(d.M, 64) * 128, nrows2 = (size_t)cdiv(d.N, 128) * 256;
     const size_t Q = (size_t)B * L;
