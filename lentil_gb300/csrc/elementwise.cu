@@ -332,6 +332,7 @@ int launch_split_field_T(const SplitFieldArgs& a, bool bf16, cudaStream_t s) {
   return LGB_OK;
 }
 
+// ---------------------------------------------------------------------------
 // max |.| reductions feeding the power-of-two split scales: a partial maximum per
 // block, taken on the bits (conversions would hold the FP64 pipe), NaN ignored.
 // Nothing is cleared first (a memset and atomics, with the operand kernel waiting
