@@ -443,6 +443,14 @@ int lgb_psf_plan_destroy(lgb_psf_plan plan);
  * ---------------------------------------------------------------------- */
 int lgb_test_stall_tma(int item, int kblock, double wait_ms);
 
+/* The same for the tensor-core products of LGB_FP64: after `launch` further
+ * launches of their GEMM in the process, the next one's first CTA issues no
+ * loads for its stage `stage` (32 K entries each), or, with `release`, does not
+ * give that stage's leading digits free for the loads two stages on, and every
+ * wait of that launch is bounded by wait_ms.  The launch gives up, and the
+ * kernels behind it evaluate its transforms in plain FP64. */
+int lgb_test_stall_sliced(int launch, int stage, int release, double wait_ms);
+
 /* ------------------------------------------------------------------------
  * Tile-shape autotuner of the split-precision MFT (extension: lentil has no
  * GPU path).  Every split launch (lgb_dft2/_batch/idft2 and plan executes)

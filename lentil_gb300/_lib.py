@@ -36,6 +36,7 @@ SIGNATURES = {
     'lgb_version': (c_int, []),
     'lgb_mempool_usage': (c_int, [c_int, c_int, ctypes.POINTER(ctypes.c_ulonglong)]),
     'lgb_test_stall_tma': (c_int, [c_int, c_int, c_double]),
+    'lgb_test_stall_sliced': (c_int, [c_int, c_int, c_int, c_double]),
     'lgb_dft2_matrices': (c_int, [c_int, c_int, c_int, c_int, c_double, c_double, c_double,
                                   c_double, c_double, c_double, c_void_p, c_void_p, c_void_p]),
     'lgb_dft2_workspace_size': (c_size_t, [c_int, c_int, c_int, c_int, c_int]),

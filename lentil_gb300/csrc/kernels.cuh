@@ -164,6 +164,14 @@ int launch_matrix_digits(const PhaseAxis& ax, const PhaseAxis* axes, int count, 
                          uint16_t* out, cudaStream_t s);
 size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left);
 int launch_sliced_dft2(const SlicedDft2& q, void* workspace, cudaStream_t s);
+// One-shot test of the sliced GEMM's bounded waits (lgb_test_stall_sliced): what
+// the launch that asks has to hold back, stage -1 for nothing.
+struct SlicedStall {
+  int stage = -1;
+  bool release = false;
+  unsigned long long wait_ns = 0;
+};
+SlicedStall take_sliced_stall();
 
 // out[b] += sum_l weights[b][l] * unit2[l] * |F[b][l]|^2 into a window (FP64)
 int launch_intensity_accum_c128(const double2* F, int M, int N, long long sF, int batch_inner,

@@ -12,6 +12,9 @@
 // A field with a NaN gives NaN everywhere (each output sums every entry); one
 // with infinities, or a device-side wait that ran out, makes `finish`
 // evaluate that transform in plain FP64 instead.
+#include <atomic>
+#include <mutex>
+
 #include "cossin.cuh"
 #include "sliced.cuh"
 
@@ -451,4 +454,30 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   return LGB_OK;
 }
 
+// The armed stall: launches to go by first, and what the one after them holds back.
+static std::mutex g_stall_mu;
+static std::atomic<int> g_stall_launches{-1};       // -1: none (the launches' only look at it)
+static SlicedStall g_stall;
+
+SlicedStall take_sliced_stall() {
+  SlicedStall none;
+  if (g_stall_launches.load(std::memory_order_relaxed) < 0) return none;
+  std::lock_guard<std::mutex> lock(g_stall_mu);
+  if (g_stall_launches < 0 || g_stall_launches-- > 0) return none;
+  return g_stall;
+}
+
 }  // namespace lgb
+
+using namespace lgb;
+
+extern "C" int lgb_test_stall_sliced(int launch, int stage, int release, double wait_ms) {
+  LGB_REQUIRE(launch >= 0 && stage >= 0, LGB_EINVAL, "test_stall_sliced: launch and stage must be >= 0");
+  LGB_REQUIRE(wait_ms > 0.0 && wait_ms <= 2000.0, LGB_EINVAL, "test_stall_sliced: wait_ms must lie in (0, 2000]");
+  std::lock_guard<std::mutex> lock(g_stall_mu);
+  g_stall.stage = stage;
+  g_stall.release = release != 0;
+  g_stall.wait_ns = (unsigned long long)(wait_ms * 1e6);
+  g_stall_launches = launch;
+  return LGB_OK;
+}

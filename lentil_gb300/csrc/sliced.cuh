@@ -101,6 +101,9 @@ struct GemmParams {
   long long stride;          // entries between products
   int* err;
   unsigned long long wait_ns;
+  // wait-expiry test (-1: none): CTA 0 issues no loads for its stage hold_loads,
+  // or does not release digits 0 to 3 of its stage hold_release
+  int hold_loads, hold_release;
 };
 
 // One CTA's run of chains of one tile.
@@ -191,12 +194,14 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   auto acc_empty = [&](int g) { return bars + 80u + 8u * g; };
   const uint32_t drain_bar = bars + 128u;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_raw + (bars - raw) + 160);
+  volatile int* half_loaded = reinterpret_cast<volatile int*>(smem_raw + (bars - raw) + 164);
 
   next_may_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int begin = blockIdx.x * p.deal.per, end = min(p.total, begin + p.deal.per);
 
   if (threadIdx.x == 0) {
+    *half_loaded = 0;
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full_bar(s), 2);
       mbar_init(low_empty(s), 1);
@@ -244,8 +249,19 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             }
             return true;
           };
-          ok = load(low_empty(s), GROUPS - 1, ND) && load(high_empty(s), 0, GROUPS - 1);
+          if (blockIdx.x == 0 && it == p.hold_loads) continue;
+          ok = load(low_empty(s), GROUPS - 1, ND);
           if (!ok) break;
+          ok = load(high_empty(s), 0, GROUPS - 1);
+          if (!ok) {
+            // half a stage is in flight: an arrival in place of the other half's
+            // lets its barrier complete when the copies land, for the wait below,
+            // and the MMA warp is told to leave the stage alone
+            *half_loaded = 1;
+            mbar_arrive(full_bar(s));
+            ++it;
+            break;
+          }
         }
       }
       for (int k = max(0, it - STAGES); k < it; ++k)       // issued copies land before exit
@@ -268,7 +284,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       for (int st = 0; ok && st < stages; ++st, ++it) {
         const int s = it % STAGES, r = st >> 1;
         const bool ends = (st & 1) == 1 || st == stages - 1;      // of a chain
-        if (!wait(full_bar(s), (it / STAGES) & 1)) { ok = false; break; }
+        if (!wait(full_bar(s), (it / STAGES) & 1) || *half_loaded) { ok = false; break; }
         const uint64_t da = smem_desc_sw64(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw64(base + s * STAGE_BYTES + A_STAGE);
         // groups 4 to 6 first: their accumulator is drained while the others run
@@ -297,7 +313,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (!ok) break;
 #pragma unroll
         for (int g = GROUPS - 2; g >= 0; --g) done(g);
-        mma_commit_cta(on, high_empty(s));
+        if (blockIdx.x != 0 || it != p.hold_release) mma_commit_cta(on, high_empty(s));
       }
     }
     mma_commit_cta(on, drain_bar);
@@ -605,6 +621,12 @@ inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int i
   p.stride = stride;
   p.err = err;
   p.wait_ns = WAIT_NS;
+  p.hold_loads = p.hold_release = -1;
+  const SlicedStall stall = take_sliced_stall();
+  if (stall.stage >= 0) {
+    (stall.release ? p.hold_release : p.hold_loads) = stall.stage;
+    p.wait_ns = stall.wait_ns;
+  }
   LGB_CUDA(launch_next(sliced_gemm_kernel, cdiv(p.total, deal.per), NUM_THREADS, SMEM_BYTES, s, a, b, p));
   return LGB_OK;
 }
