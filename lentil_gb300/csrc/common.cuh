@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/lentil_gb300.h"
+#include "per_device.cuh"
 #include <nvtx3/nvToolsExt.h>
 
 namespace lgb {
@@ -71,6 +72,17 @@ cudaError_t launch_next(void (*kernel)(Params...), dim3 grid, dim3 block, size_t
   c.attrs = &attr;
   c.numAttrs = 1;
   return cudaLaunchKernelEx(&c, kernel, Params(args)...);
+}
+
+// Raises the kernel's limit of dynamic shared memory on the current device.
+template <typename Kernel>
+cudaError_t allow_shared_memory(OncePerDevice& once, Kernel* kernel, size_t bytes) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  return once.run(dev, cudaSuccess, [&] {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  });
 }
 
 // Number of SMs of the current device (cached per device).

@@ -604,14 +604,8 @@ static cudaLaunchConfig_t pair_config(uint32_t smem, cudaStream_t s, cudaLaunchA
 
 template <bool BF16, int BN, int KB>
 static cudaError_t set_smem_attr() {
-  static std::once_flag once;
-  static cudaError_t err = cudaSuccess;
-  std::call_once(once, [] {
-    err = cudaFuncSetAttribute(split_mft_kernel<BF16, BN, KB>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)TileCfg<BN>::SMEM_BYTES);
-  });
-  return err;
+  static OncePerDevice once;
+  return allow_shared_memory(once, split_mft_kernel<BF16, BN, KB>, TileCfg<BN>::SMEM_BYTES);
 }
 
 // Largest number of CTA pairs of this kernel resident at once (per device).

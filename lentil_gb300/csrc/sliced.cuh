@@ -34,7 +34,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <mutex>
 
 #include "common.cuh"
 #include "kernels.cuh"
@@ -596,12 +595,8 @@ inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int items, int b
 inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int itemsB, int items, int K,
                        const Deal& deal, const Band& band, int S, long long* P, long long stride, int ld,
                        int* err, cudaStream_t s) {
-  static std::once_flag once;
-  static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] {
-    attr = cudaFuncSetAttribute(sliced_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-  });
-  LGB_CUDA(attr);
+  static OncePerDevice once;
+  LGB_CUDA(allow_shared_memory(once, sliced_gemm_kernel, SMEM_BYTES));
   CUtensorMap a, b;
   int st;
   if ((st = make_digit_map(&a, A, itemsA, BM))) return st;
