@@ -8,17 +8,19 @@ _SCALARS = (int, float, np.float64, np.int64)
 
 
 def pair(x):
-    """``np.broadcast_to(x, (2,))``, at a fraction of its cost for the usual
-    arguments (a number, two numbers, an array of two)."""
+    """``np.broadcast_to(x, (2,))``, read-only as that is, at a fraction of its
+    cost for the usual arguments (a number, two numbers, an array of two)."""
     t = type(x)
     if t in _SCALARS:
-        return np.array((x, x))
-    if t is np.ndarray:
-        if x.shape == (2,):
-            return x
+        v = np.array((x, x))
+    elif t is np.ndarray and x.shape == (2,):
+        v = x.view()
     elif t in (tuple, list) and len(x) == 2 and type(x[0]) in _SCALARS and type(x[1]) in _SCALARS:
-        return np.array(x)
-    return np.broadcast_to(x, (2,))
+        v = np.array(x)
+    else:
+        return np.broadcast_to(x, (2,))
+    v.flags.writeable = False
+    return v
 
 
 def mesh(shape, shift=(0, 0), angle=0):
