@@ -38,10 +38,12 @@ def boundary(x, threshold=0):
     """(rmin, rmax, cmin, cmax) of the entries above ``threshold``
     (lentil/util.py:190-218)."""
     x = np.asarray(x)
-    if x.dtype != bool or threshold != 0:
+    if x.dtype != bool or np.ndim(threshold) or threshold != 0:
         x = x > threshold
     rows = np.flatnonzero(x.any(axis=1))
-    cols = np.flatnonzero(x[rows[0]:rows[-1] + 1].any(axis=0))
+    if x.ndim == 2:                       # nothing is set outside these rows
+        x = x[rows[0]:rows[-1] + 1]
+    cols = np.flatnonzero(x.any(axis=0))
     return rows[0], rows[-1], cols[0], cols[-1]
 
 

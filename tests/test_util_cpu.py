@@ -25,3 +25,31 @@ def test_pixelscale_is_not_a_way_into_the_callers_array():
     assert mine.flags.writeable and mine[0] == 1e-3
     mine[1] = 3e-3                            # a view of it, as np.broadcast_to gives
     assert w.pixelscale[1] == 3e-3
+
+
+def _boundary(x, threshold):
+    x = np.asarray(x) > threshold
+    rows, cols = np.flatnonzero(x.any(axis=1)), np.flatnonzero(x.any(axis=0))
+    return rows[0], rows[-1], cols[0], cols[-1]
+
+
+@pytest.mark.parametrize('threshold', [0, 0.0, False, 0.5, True, float('nan'), np.array(0), np.array([[0], [1], [0]]),
+                                       np.array([0, 0, 0.5, 0])])
+@pytest.mark.parametrize('dtype', [bool, float, int])
+def test_boundary(dtype, threshold):
+    x = np.array([[0, 0, 0, 0], [0, 1, 0, 0], [0, 1, 1, 0]], dtype=dtype)
+    try:
+        want = _boundary(x, threshold)
+    except IndexError:                         # nothing above the threshold
+        with pytest.raises(IndexError):
+            util.boundary(x, threshold)
+        return
+    assert util.boundary(x, threshold) == want
+
+
+@pytest.mark.parametrize('dtype', [bool, float])
+def test_boundary_of_a_cube(dtype):
+    x = np.zeros((3, 5, 7), dtype=dtype)
+    x[1, 2:4, 3:6] = 1
+    x[0, 4, 1] = 1
+    assert util.boundary(x) == _boundary(x, 0)
