@@ -231,7 +231,8 @@ class PSFPlan:
         """amp (mask applied), opd: [n, H, W] float64 CUDA tensors (n <= batch);
         weights: [n, L] (or [n, len(lam_idx)]); returns out [n, rows, cols]
         float64.  ``lam_idx`` (int32 CUDA tensor) restricts the PSFs to those
-        of the plan's wavelengths."""
+        of the plan's wavelengths.  With ``check`` the call waits for the image
+        and raises what went wrong on the device."""
         dev = dv.device()
         amp = amp if amp.dtype == torch.float64 and amp.is_contiguous() else amp.double().contiguous()
         opd = opd if opd.dtype == torch.float64 and opd.is_contiguous() else opd.double().contiguous()
@@ -282,7 +283,8 @@ class PSFPlan:
                 if self._own_done is None:
                     self._own_done = torch.cuda.Event()
                 self._own_done.record(cur)
-            if check and self._split:      # (complex128 executes have no status to wait for)
+            # (a complex128 execute records no status: there the call waits for errors alone)
+            if check and (self._split or not capturing):
                 _lib.call('lgb_psf_plan_status', self._h, cur.cuda_stream)
         return out
 
@@ -422,7 +424,10 @@ def broadband_psf(pupil, wavelengths, weights, pixelscale, shape=None, prop_shap
         return _deliver(img, out, tensor_io)
     plan = _cached_plan(geo, precision)
     w = dv.to_device(weights[geo.keep], torch.float64).reshape(1, -1)
-    plan.execute(a, o, w, out=img.reshape((1,) + geo.shape_out), accumulate=True)
+    # complex128 products record no status to wait for (an expired wait is made
+    # good on the device), and this call returns as propagate_dft does: waiting
+    # took a loop of eight-wavelength 512^2 images from 420 to 607 us each
+    plan.execute(a, o, w, out=img.reshape((1,) + geo.shape_out), accumulate=True, check=plan._split)
     return _deliver(img, out, tensor_io)
 
 
