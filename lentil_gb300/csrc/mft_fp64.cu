@@ -17,7 +17,8 @@ namespace lgb {
 // work, and takes 4 us here; at 512^3 the two tiles cost the same.
 constexpr int ZBM = 16, ZBN = 16, ZBK = 8;
 
-// blockIdx.z = b * splits + split: problem b, K range [split * kchunk,
+// blockIdx.x counts the tiles (fields of more than 16 x 65535 rows have more
+// than y holds); blockIdx.z = b * splits + split: problem b, K range [split * kchunk,
 // (split + 1) * kchunk); with splits > 1 each split writes its own partial
 // product (C offset by split * sP) for zgemm_reduce_kernel to sum in order.
 __global__ void __launch_bounds__(64) zgemm_kernel(int M, int N, int K,
@@ -28,7 +29,8 @@ __global__ void __launch_bounds__(64) zgemm_kernel(int M, int N, int K,
   __shared__ double2 As[ZBK][ZBM];
   __shared__ double2 Bs[ZBK][ZBN];
   const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, tid = threadIdx.x;
-  const int m0 = blockIdx.y * ZBM, n0 = blockIdx.x * ZBN;
+  const int tiles_n = (N + ZBN - 1) / ZBN, tm = blockIdx.x / tiles_n;
+  const int m0 = tm * ZBM, n0 = ((int)blockIdx.x - tm * tiles_n) * ZBN;
   const int b = blockIdx.z / splits, split = blockIdx.z - b * splits;
   A += (size_t)b * sA;
   B += (size_t)b * sB;
@@ -159,7 +161,7 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
     splits = 1;
   }
   if (splits <= 1) {
-    dim3 grid(cdiv(N, ZBN), cdiv(M, ZBM), batch);
+    dim3 grid(cdiv(N, ZBN) * cdiv(M, ZBM), 1, batch);
     zgemm_kernel<<<grid, 64, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC, alpha, 1, K, 0);
     LGB_CUDA(cudaGetLastError());
     return LGB_OK;
@@ -173,7 +175,7 @@ int launch_zgemm(int M, int N, int K, const double2* A, int lda, long long sA, c
     keep_pool_memory();
     LGB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&P), (size_t)splits * part_bytes, s));
   }
-  dim3 grid(cdiv(N, ZBN), cdiv(M, ZBM), batch * splits);
+  dim3 grid(cdiv(N, ZBN) * cdiv(M, ZBM), 1, batch * splits);
   zgemm_kernel<<<grid, 64, 0, s>>>(M, N, K, A, lda, sA, B, ldb, sB, P, N, (long long)M * N, 1.0,
                                     splits, kchunk, sP);
   cudaError_t e = cudaGetLastError();
