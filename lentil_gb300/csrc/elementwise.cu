@@ -608,18 +608,21 @@ __global__ void phasor_adjoint_kernel(const double2* __restrict__ q, const doubl
 // The same for a stack, whole planes written: out[k][r][c] inside the slice,
 // zero outside (one launch in place of a clear and one per plane).
 __global__ void phasor_adjoint_stack_kernel(const double2* __restrict__ q, const double2* __restrict__ f,
-                                            int m, int n, double scale, double* __restrict__ out, int H,
-                                            int W, int r0, int c0) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y, k = blockIdx.z;
+                                            int count, int m, int n, double scale, double* __restrict__ out,
+                                            int H, int W, int r0, int c0) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, j = c - c0;
   if (c >= W) return;
-  const int i = r - r0, j = c - c0;
-  double v = 0.0;
-  if (i >= 0 && i < m && j >= 0 && j < n) {
-    const size_t p = ((size_t)k * m + i) * n + j;
-    const double2 a = q[p], b = f[p];
-    v += -2.0 * scale * (a.x * b.y + a.y * b.x);
-  }
-  out[((size_t)k * H + r) * W + c] = v;
+  for (int k = blockIdx.z; k < count; k += gridDim.z)         // (a grid holds 65535 rows and planes)
+    for (int r = blockIdx.y; r < H; r += gridDim.y) {
+      const int i = r - r0;
+      double v = 0.0;
+      if (i >= 0 && i < m && j >= 0 && j < n) {
+        const size_t p = ((size_t)k * m + i) * n + j;
+        const double2 a = q[p], b = f[p];
+        v += -2.0 * scale * (a.x * b.y + a.y * b.x);
+      }
+      out[((size_t)k * H + r) * W + c] = v;
+    }
 }
 
 static int grid_for(size_t count) {
@@ -670,12 +673,12 @@ extern "C" int lgb_phasor_adjoint_stack(const lgb_c128* q, const lgb_c128* f, in
   LGB_RANGE("lgb_phasor_adjoint_stack");
   LGB_REQUIRE(q && f && grad_opd, LGB_EINVAL, "phasor_adjoint: null pointer");
   LGB_REQUIRE(wavelength != 0.0, LGB_EINVAL, "phasor_adjoint: wavelength must be nonzero");
-  LGB_REQUIRE(count >= 1 && count <= 65535 && H >= 1 && H <= 65535 && W >= 1, LGB_EINVAL,
-              "phasor_adjoint: plane sizes out of range");
+  LGB_REQUIRE(count >= 1 && H >= 1 && W >= 1, LGB_EINVAL, "phasor_adjoint: sizes must be positive");
   LGB_REQUIRE(r0 >= 0 && c0 >= 0 && m >= 0 && n >= 0 && r0 + m <= H && c0 + n <= W, LGB_EINVAL,
               "phasor_adjoint: slice outside the plane");
-  phasor_adjoint_stack_kernel<<<dim3(cdiv(W, 128), H, count), 128, 0, as_stream(stream)>>>(
-      reinterpret_cast<const double2*>(q), reinterpret_cast<const double2*>(f), m, n,
+  const dim3 grid(cdiv(W, 128), std::min(H, 65535), std::min(count, 65535));
+  phasor_adjoint_stack_kernel<<<grid, 128, 0, as_stream(stream)>>>(
+      reinterpret_cast<const double2*>(q), reinterpret_cast<const double2*>(f), count, m, n,
       2.0 * M_PI / wavelength, grad_opd, H, W, r0, c0);
   LGB_CUDA(cudaGetLastError());
   return LGB_OK;
