@@ -13,21 +13,25 @@
 //   - the products of digits with i + j <= 6 are kept, grouped by s = i + j.  A
 //     group's sum over 64 K entries is at most (s + 1) 64 2^16 <= 2^24 units
 //     for s <= 3: the FP32 accumulators hold it exactly, whatever order or
-//     rounding the tensor core uses.  Groups 4 to 6 share an accumulator
-//     (their rounding is below 2^-56 of the operands);
+//     rounding the tensor core uses.  Groups 4 to 6 share an accumulator, which
+//     is cut off at its last place at every MMA: 2^-52 of the largest product
+//     when every digit is at its largest and of one sign (5 x 32 products of
+//     2^16 2^-36, an FP32 place of 2^-36), 2^-57 for digits at random;
 //   - every 64 K entries (256 for group 0, 128 for group 1: their sums have the
-//     room) the accumulators are drained into 64-bit integers in registers, in
-//     units of 2^-(16 + S): exact for groups 0-3.  Integer sums
-//     do not depend on their order, so dealing K out over CTAs gives the same
-//     bits.
-// What is left is the rounding of the operands, the products left out, and one
-// rounding per stored result; an FP64 accumulation rounds at every K step.
+//     room; 32 for groups 4 to 6) the accumulators are drained into 64-bit
+//     integers in registers, in units of 2^-(16 + S): exact for groups 0-3.
+//     Integer sums do not depend on their order, so dealing K out over CTAs
+//     gives the same bits.
+// What is left, all of it relative to the largest entries of the two vectors of
+// a sum: the rounding of the operands (2^-63), the products left out (2^-60), the
+// last places of groups 4 to 6 and their rounding to the unit; and one rounding
+// per stored result.  An FP64 accumulation rounds at every K step.
 //
 // A complex product is three real ones (Gauss): operands hold the row sets re,
 // im and h = (re + im) / 2, the products of like sets are
 //     P0 = Ar Br,  P1 = Ai Bi,  P2 = 2 Ah Bh,
-// and readers form re = P0 - P1, im = 2 P2 - P0 - P1 in integers, which loses
-// nothing.  That is 84 digit products where four real products took 108 (a DFT
+// and readers form re = P0 - P1, im = 2 P2 - P0 - P1 in integers, modulo 2^64,
+// which loses nothing.  That is 84 digit products where four real products took 108 (a DFT
 // matrix had six digits then): 1019 x 941 to 1024^2 went from 337 to 300 us,
 // 512^2 from 82 to 76.
 #pragma once
@@ -95,7 +99,7 @@ struct GemmParams {
   int rowsB;
   int ld;                    // P row pitch (entries)
   int dA, dB;                // digit planes between items (0: shared by all items)
-  int S;                     // P unit: 2^-(16 + S) of the scaled operands, half that for P2
+  int S;                     // P unit: 2^-(16 + S) of the scaled operands, a quarter of it for P2
   long long* P;              // [product][part][rowsB][ld]
   long long stride;          // entries between products
   int* err;
@@ -130,11 +134,16 @@ __device__ __forceinline__ Segment segment_at(const GemmParams& p, int pos, int 
 // Which chains of a segment (r = 0, 1, ...) start and end a sum of group g:
 // groups 0 and 1 run over four and two chains, at most 4 * 64 2^16 = 2 * 2 * 64
 // 2^16 = 2^24.  (Draining every group after every chain left the MMA waiting
-// 16 % of the time for the last ones of 20 drains in four chains; these are 15.)
+// 16 % of the time for the last ones of 20 drains in four chains.)  Groups 4 to 6
+// start and end one every stage: drained every chain, the shared accumulator was
+// cut off at group 4's last place for twice as long, and with the three groups in
+// the order of A's digits too, fields of a cross of ones over 1e-3 (333 x 257)
+// came out 1.27 times as far from exact as in plain FP64, amplitudes over ten
+// decades 1.18 times; now 0.93 and 1.00 (1019 x 941 to 1024^2 278 -> 293 us).
 __device__ __forceinline__ bool starts(int g, int r) {
   return g == 0 ? (r & 3) == 0 : g == 1 ? (r & 1) == 0 : true;
 }
-__device__ __forceinline__ bool drains(int g, int r, int count) {
+__device__ __forceinline__ bool drains(int g, int r, int count) {          // g < 4
   if (r == count - 1) return true;
   return g == 0 ? (r & 3) == 3 : g == 1 ? (r & 1) == 1 : true;
 }
@@ -169,9 +178,10 @@ __device__ __forceinline__ void mma_run(int i, int j0, int j1, uint32_t on, uint
 // share the port: in the order of the sums i + j, with nothing kept, a stage
 // took 3900 clk.  Runs over B's digits with A's in the collector read 4.6 KB and
 // run at 49: 1019 x 941 to 1024^2 went from 121 to 110 us per GEMM (transform
-// 300 -> 283), 512^2 from 76 to 71.5.  What is left above the 81 us of MMAs: the
-// first loads and the last sums (6 us), loads (12 %, by latency: L2 runs at a
-// third of its rate) and drains (9 %) that the MMAs wait for.
+// 300 -> 283), 512^2 from 76 to 71.5.  (Group 4's five products are runs of one.)
+// What is left above the 81 us of MMAs: the first loads and the last sums (6 us),
+// loads (12 %, by latency: L2 runs at a third of its rate) and drains that the
+// MMAs wait for.
 //
 // Roles: warp 0 TMA (two stages of 32 K entries; digits 4 to 6 of a stage are
 // done with, and loaded anew, while its sums 0 to 3 run), warp 1 MMA issue,
@@ -286,28 +296,38 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (!wait(full_bar(s), (it / STAGES) & 1) || *half_loaded) { ok = false; break; }
         const uint64_t da = smem_desc_sw64(base + s * STAGE_BYTES);
         const uint64_t db = smem_desc_sw64(base + s * STAGE_BYTES + A_STAGE);
-        // groups 4 to 6 first: their accumulator is drained while the others run
         const bool begins = (st & 1) == 0;
         auto done = [&](int g) {
-          if (ends && drains(g, r, w.count)) {
+          if (g == GROUPS - 1 || (ends && drains(g, r, w.count))) {
             mma_commit_cta(on, acc_full(g));
             ++n[g];
           }
         };
-#pragma unroll
-        for (int i = ND - 1; i >= -4 && ok; --i) {
-          const int g = i >= 0 ? GROUPS - 1 : i + 4;              // whose sum this run may start
-          const bool fresh = (i == ND - 1 || i < 0) && begins && starts(g, r);
-          // this accumulator's previous sum has been drained
-          if (fresh) ok = wait(acc_empty(g), (n[g] & 1) ^ 1);
-          if (!ok) break;
+        // whether group g's sum starts here, once its previous one has been drained
+        auto fresh = [&](int g) {
+          if (g < GROUPS - 1 && (!begins || !starts(g, r))) return false;
+          ok = wait(acc_empty(g), (n[g] & 1) ^ 1);
           tc_fence_after();
-          if (i >= 0) mma_run(i, ND - 1 - i, max(4 - i, 0), on, tmem, da, db, idesc, fresh);
-          else mma_run(i + 4, -1 - i, 0, on, tmem, da, db, idesc, fresh);
-          if (i == 0) {
-            done(GROUPS - 1);
-            mma_commit_cta(on, low_empty(s));
-          }
+          return true;
+        };
+        tc_fence_after();
+        // groups 4 to 6 first: their accumulator is drained while the others run.
+        // Of them 6 and 5, then 4, whose last place the sum keeps from then on.
+        const bool f4 = fresh(GROUPS - 1);
+        if (!ok) break;
+#pragma unroll
+        for (int i = ND - 1; i >= 0; --i)
+          mma_run(i, ND - 1 - i, max(GROUPS - i, 0), on, tmem, da, db, idesc, f4 && i == ND - 1);
+#pragma unroll
+        for (int i = GROUPS - 1; i >= 0; --i)
+          mma_run(i, GROUPS - 1 - i, GROUPS - 1 - i, on, tmem, da, db, idesc, false);
+        done(GROUPS - 1);
+        mma_commit_cta(on, low_empty(s));
+#pragma unroll
+        for (int g = GROUPS - 2; g >= 0; --g) {
+          const bool f = fresh(g);
+          if (!ok) break;
+          mma_run(g, GROUPS - 2 - g, 0, on, tmem, da, db, idesc, f);
         }
         if (!ok) break;
 #pragma unroll
@@ -326,18 +346,18 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     for (int pos = begin; ok && pos < end;) {
       const Segment w = segment_at(p, pos, end);
       pos += w.count;
-      const int S = p.S + (w.product % p.sets == 2);
+      const int S = p.S + (w.product % p.sets == 2 ? 2 : 0);
       const float unit4 = ldexpf(1.f, S);
-      const int m1 = 1 << (S - BETA), m2 = 1 << (S - 2 * BETA), m3 = 1 << (S - 3 * BETA);
-      long long acc[RUN];
+      // sums of groups 1 to 3 are whole multiples of 2^-9, 2^-18, 2^-27 below 2^24
+      // of them: three more bits leave the multipliers below 2^31
+      const int m1 = 1 << (S - BETA - 3), m2 = 1 << (S - 2 * BETA - 3), m3 = 1 << (S - 3 * BETA - 3);
+      unsigned long long acc[RUN];
 #pragma unroll
       for (int j = 0; j < RUN; ++j) acc[j] = 0;
       for (int k = 0; ok && k < w.count; ++k) {
-#pragma unroll
-        for (int g = GROUPS - 1; g >= 0; --g) {
-          if (!drains(g, k, w.count)) continue;
+        auto drain = [&](int g) {
           ok = __all_sync(0xffffffffu, mbar_wait(acc_full(g), n[g] & 1, p.err, p.wait_ns));
-          if (!ok) break;
+          if (!ok) return;
           ++n[g];
           tc_fence_after();
           uint32_t r[RUN];
@@ -351,12 +371,17 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           for (int j = 0; j < RUN; ++j) {
             const float v = __uint_as_float(r[j]);
             if (g == 4) acc[j] += (long long)__float2int_rn(v * unit4);
-            else if (g == 3) acc[j] += (long long)__float2int_rn(v * 0x1p27f) * m3;
-            else if (g == 2) acc[j] += (long long)__float2int_rn(v * 0x1p18f) * m2;
-            else if (g == 1) acc[j] += (long long)__float2int_rn(v * 0x1p9f) * m1;
-            else acc[j] += (long long)((unsigned long long)((uint32_t)__float2int_rn(v) << (S - 32)) << 32);
+            else if (g == 3) acc[j] += (long long)__float2int_rn(v * 0x1p30f) * m3;
+            else if (g == 2) acc[j] += (long long)__float2int_rn(v * 0x1p21f) * m2;
+            else if (g == 1) acc[j] += (long long)__float2int_rn(v * 0x1p12f) * m1;
+            else acc[j] += (unsigned long long)((uint32_t)__float2int_rn(v) << (S - 32)) << 32;
           }
-        }
+        };
+        const int last = min(p.stages - 2 * (w.chain + k), 2);
+        for (int st = 0; ok && st < last; ++st) drain(GROUPS - 1);
+#pragma unroll
+        for (int g = GROUPS - 2; g >= 0; --g)
+          if (ok && drains(g, k, w.count)) drain(g);
       }
       if (!ok) break;
       const int n0 = w.n0 + ch * RUN;
@@ -364,7 +389,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                        q4 * 32 + lane;
 #pragma unroll
       for (int j = 0; j < RUN; ++j)
-        if (n0 + j < p.rowsB) out[(size_t)j * p.ld] = acc[j];
+        if (n0 + j < p.rowsB) out[(size_t)j * p.ld] = (long long)acc[j];
     }
   }
 
@@ -507,7 +532,7 @@ __device__ __forceinline__ void sum_parts(const long long* __restrict__ P, size_
 }
 
 // The same for complex entries: n[c][i] parts of product c, 3 COUNT loads in
-// flight.  2 P2 may wrap, what is left of it does not.
+// flight.  4 P2, P2's sum in its units, may wrap; what is left of it does not.
 template <int COUNT>
 __device__ __forceinline__ void sum_parts3(const long long* __restrict__ P, size_t stride, size_t part,
                                            const size_t (&at)[COUNT], const int (&n)[3][COUNT],
@@ -528,7 +553,7 @@ __device__ __forceinline__ void sum_parts3(const long long* __restrict__ P, size
 #pragma unroll
     for (int i = 0; i < COUNT; ++i) {
       re[i] += (unsigned long long)w[0][i] - (unsigned long long)w[1][i];
-      im[i] += 2 * (unsigned long long)w[2][i] - (unsigned long long)w[0][i] - (unsigned long long)w[1][i];
+      im[i] += (unsigned long long)w[2][i] - (unsigned long long)w[0][i] - (unsigned long long)w[1][i];
     }
   }
 #pragma unroll
@@ -564,12 +589,14 @@ inline Deal deal_of(int rowsA, int rowsB, int chains, int products) {
 inline int max_parts(const Deal& d) { return std::min(d.chains, (d.chains + d.per - 2) / d.per + 1); }
 
 // S for a contraction of K entries: sums reach K 2^16 (times sqrt 2 for im).
-// P2 has half that unit: |h| <= 2^7.5 in a DFT matrix leaves it the room, and
-// it counts four times.  K <= 16384, so S >= 32.
+// P2 counts four times and has a quarter of the unit, so that its roundings
+// weigh no more than P0's and P1's (with half of it, fields with a cross of ones
+// over 1e-3 or ten decades of amplitudes came out up to 1.27 times further from
+// exact than the FP64 GEMM leaves them).  K <= 16384, so S >= 32.
 inline int unit_shift(int K, int sets) {
   int lg = 0;
   while ((1 << lg) < K) ++lg;
-  return std::min(sets == 3 ? 38 : 39, 46 - lg);            // 2^(S + 1 - 9) is an int
+  return std::min(sets == 3 ? 40 : 42, 46 - lg);            // group 4's sums are ints, below 2^(S - 11)
 }
 
 // Tensor map of a digit operand seen as [items x digits][sets][L][kp], box
