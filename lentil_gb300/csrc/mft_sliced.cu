@@ -399,7 +399,7 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   const Layout t = layout(q.count, q.m, q.n, q.M, q.N, q.left, ws);
   const bool own = q.axes != nullptr;
   DigitRows e1 = matrix_rows(q.e1, q.m, q.M), e2 = matrix_rows(q.e2, q.n, q.N);
-  const int S1 = unit_shift(t.K1, 3), S2 = unit_shift(t.K2, 3);
+  const int S1 = unit_shift(t.K1), S2 = unit_shift(t.K2);
   int st;
   for (int b0 = 0; b0 < q.count; b0 += t.chunk) {
     const int items = std::min(t.chunk, q.count - b0);
@@ -411,13 +411,13 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
       slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.err);
     LGB_CUDA(cudaGetLastError());
     const int own_items = own ? items : 1;
-    if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, Band{}, S1, t.P,
+    if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, S1, nullptr, t.P,
                           t.stride, t.ld1, t.err, s)))
       return st;
     LGB_CUDA(launch_next(slice_product_kernel, dim3(t.rows1, items), 256, 0, s,
                          PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2));
     if ((st = launch_gemm(t.left ? e2 : t.d2, t.left ? own_items : items, t.left ? t.d2 : e1,
-                          t.left ? items : own_items, items, t.K2, t.deal2, Band{}, S2, t.P, t.stride, t.ld2, t.err,
+                          t.left ? items : own_items, items, t.K2, t.deal2, S2, nullptr, t.P, t.stride, t.ld2, t.err,
                           s)))
       return st;
     FinishParams p{};

@@ -10,13 +10,13 @@
 //     C a + i C b), between tiled transposes (~5 N^2 log2 N flop), in
 //     double-float arithmetic (below);
 //   - any other N: |C . img . C^T| with C the real symmetric circulant
-//     C[i][j] = c[(i - j) mod N], c = ifft(s): two products on the tensor
-//     cores at FP64 accuracy (pixel_sliced.cu), or, where N is outside their
-//     range, two FP64 GEMMs.
+//     C[i][j] = c[(i - j) mod N], c = ifft(s): two products, near taps in FP64
+//     and the others on the tensor cores (pixel_sliced.cu), or, where N is
+//     outside their range, two FP64 GEMMs.
 // pixelate then resamples by 1/os with a cubic spline (lentil/util.py:261-349);
 // when N is a multiple of os every sample falls on a grid point, so the
 // result is d = p[::os, ::os] rescaled by sum(p)/sum(d) and masked where
-// d == 0; otherwise the spline evaluation runs as two banded products
+// d == 0; otherwise the spline evaluation runs as two banded FP64 passes
 // (the off-grid section below).
 //
 // The same FFT machinery also filters white noise for lgb_power_spectrum
@@ -350,8 +350,11 @@ __global__ void pixelate_scale_kernel(int count, const double* __restrict__ d,
 // samples: with h truncated at |t| <= RS_TAPS (|z|^31 < 2e-18 of the
 // signal) the window is RS_BW = 2 RS_TAPS + 4 wide, and the whole
 // resampling is out = G p G^T with G banded, S x RS_BW plus a start index
-// per row: two products on the tensor cores over the windows of 96 rows
-// (pixel_sliced.cu), or, outside their range, two FP64 passes.
+// per row.  Both passes are FP64 FMA over L2-resident operands.  (As digit
+// products on the tensor cores, 0.05 ms in place of 0.11 for 1000^2 by 3, samples
+// that are faint beside their row lost digits that the FP64 sums keep.)
+constexpr int RS_PAD = 12, RS_TAPS = 30, RS_BW = 2 * RS_TAPS + 4;
+
 __host__ __device__ __forceinline__ double rs_coord(int k, int S, int N, int os) {
   return ((double)k - S / 2.0) / (1.0 / os) + N / 2.0;
 }
@@ -522,20 +525,19 @@ static bool fft_size(int N, int* logN) {
 }
 
 // The tensor-core products (pixel_sliced.cu) take images of 64 to 16384 rows:
-// below, a contraction is too short to be worth cutting into digits (at
-// N = 75 the two forms cost the same), above, their 64-bit sums run out.
-// N = 1000: the two products 4.1 -> 0.1 ms; the resampling by 3 of them
-// 0.11 -> 0.05 ms.
+// below, a contraction is too short to be worth cutting into digits, above,
+// their 64-bit sums run out.  FP64 GEMMs and these, the whole MTF in us: 66^2 191
+// and 62, 300^2 669 and 87, 1000^2 4090 and 396, 3000^2 89900 and 7765.
 static bool sliced_size(int N) { return N >= 64 && N <= 16384; }
 
 struct PixelSpace {
   double* sums;          // [0] sum p, [1] sum of the grid samples, [2] sum of the resampled
-  int* status;           // behind sums: two words each of the tensor-core products
+  int* status;           // behind sums: two words of the tensor-core products
   double* sinc;          // [N] sinc(fftfreq * os)
   double* d;
   // GEMM path
   double *c, *tab, *C, *T, *P;
-  void* sliced;          // workspace of the tensor-core products (MTF, then resampling)
+  void* sliced;          // workspace of the tensor-core products
   // FFT path
   double2 *X, *Y, *tw;
   // off-grid resampling: operator and the two passes
@@ -555,7 +557,7 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
   int logN;
   const size_t NN = (size_t)N * N;
   const int Nd = N / std::max(os, 1);
-  t.sums = static_cast<double*>(take(4 * sizeof(double) + 4 * sizeof(int)));
+  t.sums = static_cast<double*>(take(4 * sizeof(double) + 2 * sizeof(int)));
   t.status = reinterpret_cast<int*>(t.sums + 4);
   t.sinc = static_cast<double*>(take((size_t)N * sizeof(double)));
   t.d = static_cast<double*>(take((size_t)Nd * Nd * sizeof(double)));
@@ -575,14 +577,12 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
   }
   const int S = resample_size(N, std::max(os, 1));
   const bool off_grid = !resample_on_grid(N, std::max(os, 1), S);
-  if (sliced_size(N) && (!fft || off_grid))
-    t.sliced = take(std::max(fft ? 0 : pixel_sliced_workspace(N),
-                             off_grid ? resample_sliced_workspace(N, std::max(os, 1), S) : 0));
+  if (sliced_size(N) && !fft) t.sliced = take(pixel_sliced_workspace(N));
   if (off_grid) {
     t.Gt = static_cast<double*>(take((size_t)RS_BW * S * sizeof(double)));
     t.q0 = static_cast<int*>(take((size_t)S * sizeof(int)));
     t.pos = static_cast<double*>(take((size_t)S * sizeof(double)));
-    if (!sliced_size(N)) t.Tm = static_cast<double*>(take((size_t)N * S * sizeof(double)));
+    t.Tm = static_cast<double*>(take((size_t)N * S * sizeof(double)));
     t.raw = static_cast<double*>(take((size_t)S * S * sizeof(double)));
   }
   if (s) *s = t;
@@ -593,7 +593,7 @@ static size_t pixel_space(void* ws, int N, int os, PixelSpace* s) {
 // to sums[0]; with d, every os-th sample and their sum (sums[1]).
 static int run_pixel(const double* img, int N, int os_mtf, PixelSpace* w, double* P, int os, double* d,
                      cudaStream_t s) {
-  LGB_CUDA(cudaMemsetAsync(w->sums, 0, 4 * sizeof(double) + 4 * sizeof(int), s));
+  LGB_CUDA(cudaMemsetAsync(w->sums, 0, 4 * sizeof(double) + 2 * sizeof(int), s));
   sinc_table_kernel<<<cdiv(2 * N, 128), 128, 0, s>>>(N, (double)os_mtf, w->sinc, w->tab);
   int logN;
   const double* src;
@@ -799,16 +799,10 @@ extern "C" int lgb_pixelate(const double* img, int rows, int cols, int oversampl
   double* const P = fft_size(N, &logN) ? reinterpret_cast<double*>(w.Y) : w.P;
   if ((st = run_pixel(img, N, os, &w, P, 1, nullptr, s))) return st;
   LGB_CUDA(launch_next(resample_operator_kernel, S, 4 * RS_BW, 0, s, N, os, S, w.Gt, w.q0, w.pos));
-  if (sliced_size(N)) {
-    if ((st = launch_resample_sliced(P, N, os, S, w.Gt, w.q0, w.sliced, w.status + 2, w.raw, w.sums + 2,
-                                     s)))
-      return st;
-  } else {
-    resample_rows_kernel<<<dim3(cdiv(S, 64), cdiv(N, 4 * RS_ROWS)), dim3(64, 4), 0, s>>>(
-        P, N, S, w.Gt, w.q0, w.Tm);
-    resample_cols_kernel<<<dim3(cdiv(S, 64), cdiv(S, 4 * RS_OUT)), dim3(64, 4), 0, s>>>(
-        w.Tm, N, S, w.Gt, w.q0, w.raw, w.sums);
-  }
+  resample_rows_kernel<<<dim3(cdiv(S, 64), cdiv(N, 4 * RS_ROWS)), dim3(64, 4), 0, s>>>(
+      P, N, S, w.Gt, w.q0, w.Tm);
+  resample_cols_kernel<<<dim3(cdiv(S, 64), cdiv(S, 4 * RS_OUT)), dim3(64, 4), 0, s>>>(
+      w.Tm, N, S, w.Gt, w.q0, w.raw, w.sums);
   LGB_CUDA(launch_next(resample_finish_kernel, dim3(cdiv(S, 256), S), 256, 0, s, w.raw, P, N, S, w.pos, w.sums, out));
   return LGB_OK;
 }

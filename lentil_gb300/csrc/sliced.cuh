@@ -78,21 +78,8 @@ struct Deal {
   }
 };
 
-// Which chains of a contraction a column tile takes: all, or, for a
-// banded operand B whose row k covers K entries around k * step, a window.
-struct Band {
-  int step;                  // 0: all chains
-  int total, count;          // chains of the whole contraction, of a window
-  __host__ __device__ int first(int tb) const {
-    if (step == 0) return 0;
-    const int c = (tb * BN * step - step - 34) / 64;         // rows start at most step / 2 + 33 before
-    return c < 0 ? 0 : (c < total - count ? c : total - count);
-  }
-};
-
 struct GemmParams {
   Deal deal;
-  Band band;
   int total;                 // chains of all tiles of all products
   int sets;                  // products per item
   int stages;                // of BK along K
@@ -100,6 +87,7 @@ struct GemmParams {
   int ld;                    // P row pitch (entries)
   int dA, dB;                // digit planes between items (0: shared by all items)
   int S;                     // P unit: 2^-(16 + S) of the scaled operands, a quarter of it for P2
+  const int* unit;           // S, found on the device (null: the above)
   long long* P;              // [product][part][rowsB][ld]
   long long stride;          // entries between products
   int* err;
@@ -126,7 +114,6 @@ __device__ __forceinline__ Segment segment_at(const GemmParams& p, int pos, int 
   const int tb = t / p.deal.tilesA;
   s.m0 = (t - tb * p.deal.tilesA) * BM;
   s.n0 = tb * BN;
-  s.chain += p.band.first(tb);
   s.part = (int)blockIdx.x - p.deal.first_cta(tile);
   return s;
 }
@@ -346,7 +333,7 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     for (int pos = begin; ok && pos < end;) {
       const Segment w = segment_at(p, pos, end);
       pos += w.count;
-      const int S = p.S + (w.product % p.sets == 2 ? 2 : 0);
+      const int S = (p.unit ? *p.unit : p.S) + (w.product % p.sets == 2 ? 2 : 0);
       const float unit4 = ldexpf(1.f, S);
       // sums of groups 1 to 3 are whole multiples of 2^-9, 2^-18, 2^-27 below 2^24
       // of them: three more bits leave the multipliers below 2^31
@@ -593,10 +580,10 @@ inline int max_parts(const Deal& d) { return std::min(d.chains, (d.chains + d.pe
 // weigh no more than P0's and P1's (with half of it, fields with a cross of ones
 // over 1e-3 or ten decades of amplitudes came out up to 1.27 times further from
 // exact than the FP64 GEMM leaves them).  K <= 16384, so S >= 32.
-inline int unit_shift(int K, int sets) {
+inline int unit_shift(int K) {
   int lg = 0;
   while ((1 << lg) < K) ++lg;
-  return std::min(sets == 3 ? 40 : 42, 46 - lg);            // group 4's sums are ints, below 2^(S - 11)
+  return std::min(40, 46 - lg);                // group 4's sums are ints: S + 2 <= 42
 }
 
 // Tensor map of a digit operand seen as [items x digits][sets][L][kp], box
@@ -620,7 +607,7 @@ inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int items, int b
 // The products of A's and B's sets over K entries, for `items` items; the
 // operands hold itemsA and itemsB of them (1: shared by all).
 inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int itemsB, int items, int K,
-                       const Deal& deal, const Band& band, int S, long long* P, long long stride, int ld,
+                       const Deal& deal, int S, const int* unit, long long* P, long long stride, int ld,
                        int* err, cudaStream_t s) {
   static OncePerDevice once;
   LGB_CUDA(allow_shared_memory(once, sliced_gemm_kernel, SMEM_BYTES));
@@ -630,7 +617,6 @@ inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int i
   if ((st = make_digit_map(&b, B, itemsB, BN))) return st;
   GemmParams p{};
   p.deal = deal;
-  p.band = band;
   p.sets = A.sets;
   p.total = items * p.sets * deal.tilesA * deal.tilesB * deal.chains;
   p.stages = cdiv(K, BK);
@@ -639,6 +625,7 @@ inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int i
   p.dA = itemsA > 1 ? ND : 0;
   p.dB = itemsB > 1 ? ND : 0;
   p.S = S;
+  p.unit = unit;
   p.P = P;
   p.stride = stride;
   p.err = err;
