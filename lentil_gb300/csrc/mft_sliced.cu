@@ -214,6 +214,7 @@ struct FinishParams {
   PhaseAxis ar, ac;
   const PhaseAxis* axes;     // per item, or null: ar, ac
   int cols;
+  const int* vec_exps;       // [item][vectors of f]: exponents, or that it has infinities
   long long* scratch;        // P again: the item's intermediate rows
   const int* err;
 };
@@ -225,31 +226,85 @@ __device__ __forceinline__ void cfma(double2& c, double2 a, double2 b) {
   c.y = fma(a.y, b.x, c.y);
 }
 
-// One output row u (left) or column v of a transform in plain FP64, by one
-// block: the intermediate row, then the output from it.
-__device__ __noinline__ void plain_line(const FinishParams& p, int b, int q) {
+constexpr int LINES = 4;                     // output rows or columns at once
+constexpr int LINE_K = 64;                   // entries of a sum staged at once
+
+__device__ __forceinline__ double2 matrix_entry(const PhaseAxis& ax, int i, int j) {
+  const longlong2 z = cossin_q62(phase_fixed(ax, i, j), COS_TABLE);
+  const double c = assembled((uint64_t)(z.x < 0 ? -z.x : z.x), -62), s = assembled((uint64_t)(z.y < 0 ? -z.y : z.y), -62);
+  return make_double2(z.x < 0 ? -c : c, z.y > 0 ? -s : s);
+}
+
+// Output rows (left) or columns q0 .. q0 + LINES - 1 of a transform in plain FP64,
+// by one block: their intermediate rows, then the output from those.  Of a field
+// with infinities (`some`) only the vectors that hold one count: what they add to
+// an output is not finite, and what the others add does not change it.  An entry
+// of the first matrix serves the whole block, one of the second LINES outputs.
+// One infinity in 1019 x 941, to 1024^2: 136 ms with every vector and a sincospi
+// for every multiply-add, 1.2 so; all of it, after an expired wait, 18 (the FP64
+// GEMMs: 15.8).
+__device__ __noinline__ void plain_lines(const FinishParams& p, int b, int q0, bool some) {
+  __shared__ double2 e[LINE_K][LINES];
   const PhaseAxis ar = p.axes ? p.axes[b] : p.ar, ac = p.axes ? p.axes[p.cols + b] : p.ac;
-  const double2* f = p.f + (size_t)b * p.m * p.n;
-  double2* F = p.F + (size_t)b * p.M * p.N;
+  const PhaseAxis &ax1 = p.left ? ar : ac, &ax2 = p.left ? ac : ar;
   const int len = p.left ? p.n : p.m, inner = p.left ? p.m : p.n;
-  double2* T = reinterpret_cast<double2*>(p.scratch + (size_t)b * 3 * p.q.stride) + (size_t)q * len;
-  for (int a = threadIdx.x; a < len; a += blockDim.x) {
-    double2 t = make_double2(0.0, 0.0);
-    for (int k = 0; k < inner; ++k) {
-      if (p.left) cfma(t, expm2pi_fixed_f64(phase_fixed(ar, k, q)), f[(size_t)k * p.n + a]);
-      else cfma(t, f[(size_t)a * p.n + k], expm2pi_fixed_f64(phase_fixed(ac, k, q)));
+  const double2* f = p.f + (size_t)b * p.m * p.n;
+  const size_t along = p.left ? p.n : 1, across = p.left ? 1 : p.n;      // strides of a vector, of the vectors
+  double2* F = p.F + (size_t)b * p.M * p.N;
+  const int lines = min(LINES, (p.left ? p.M : p.N) - q0), outs = p.left ? p.N : p.M;
+  double2* T = reinterpret_cast<double2*>(p.scratch + (size_t)b * 3 * p.q.stride) + (size_t)q0 * len;
+  const int* vec = p.vec_exps + (size_t)b * len;
+  auto counts = [&](int k) { return !some || vec[k] >= EXP_INF; };
+  for (int a0 = 0; a0 < len; a0 += blockDim.x) {
+    const int a = a0 + threadIdx.x;
+    const bool mine = a < len && counts(a);
+    if (!__syncthreads_or(mine)) continue;
+    double2 t[LINES] = {};
+    for (int k0 = 0; k0 < inner; k0 += LINE_K) {
+      const int ks = min(LINE_K, inner - k0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < LINES * LINE_K; i += blockDim.x) {
+        const int l = i % LINES, k = i / LINES;
+        if (k < ks) e[k][l] = matrix_entry(ax1, k0 + k, q0 + min(l, lines - 1));
+      }
+      __syncthreads();
+      if (mine) {
+        const double2* x = f + a * across + k0 * along;
+        for (int k = 0; k < ks; ++k, x += along) {
+          const double2 z = *x;
+#pragma unroll
+          for (int l = 0; l < LINES; ++l) cfma(t[l], e[k][l], z);
+        }
+      }
     }
-    T[a] = t;
+#pragma unroll
+    for (int l = 0; l < LINES; ++l)
+      if (l < lines && mine) T[(size_t)l * len + a] = t[l];
   }
-  __syncthreads();
-  const int outs = p.left ? p.N : p.M;
-  for (int o = threadIdx.x; o < outs; o += blockDim.x) {
-    double2 t = make_double2(0.0, 0.0);
-    for (int k = 0; k < len; ++k) {
-      if (p.left) cfma(t, T[k], expm2pi_fixed_f64(phase_fixed(ac, k, o)));
-      else cfma(t, expm2pi_fixed_f64(phase_fixed(ar, k, o)), T[k]);
+  for (int o0 = 0; o0 < outs; o0 += blockDim.x) {
+    const int o = o0 + threadIdx.x;
+    double2 t[LINES] = {};
+    for (int k0 = 0; k0 < len; k0 += LINE_K) {
+      const int ks = min(LINE_K, len - k0);
+      __syncthreads();                                   // T is written, e no longer read
+      for (int i = threadIdx.x; i < LINES * LINE_K; i += blockDim.x) {
+        const int l = i / LINE_K, k = i % LINE_K;
+        if (k < ks && counts(k0 + k)) e[k][l] = T[(size_t)min(l, lines - 1) * len + k0 + k];
+      }
+      __syncthreads();
+      for (int k = 0; k < ks; ++k) {
+        if (!counts(k0 + k)) continue;
+        const double2 w = matrix_entry(ax2, k0 + k, min(o, outs - 1));
+#pragma unroll
+        for (int l = 0; l < LINES; ++l) cfma(t[l], e[k][l], w);
+      }
     }
-    F[p.left ? (size_t)q * p.N + o : (size_t)o * p.N + q] = make_double2(p.scale * t.x, p.scale * t.y);
+    if (o >= outs) continue;
+#pragma unroll
+    for (int l = 0; l < LINES; ++l)
+      if (l < lines)
+        F[p.left ? (size_t)(q0 + l) * p.N + o : (size_t)o * p.N + q0 + l] =
+            make_double2(p.scale * t[l].x, p.scale * t[l].y);
   }
   __syncthreads();
 }
@@ -265,8 +320,8 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
   previous_done();
   const int b = blockIdx.z, flag = p.exps[(size_t)b * (p.left ? p.M : p.N)];      // all of them, if one is
   if (*p.err != 0 || flag == EXP_INF) {
-    if (blockIdx.x != 0) return;
-    for (int q = blockIdx.y; q < (p.left ? p.M : p.N); q += gridDim.y) plain_line(p, b, q);
+    const int first = LINES * (blockIdx.y * gridDim.x + blockIdx.x), step = LINES * gridDim.y * gridDim.x;
+    for (int q = first; q < (p.left ? p.M : p.N); q += step) plain_lines(p, b, q, *p.err == 0);
     return;
   }
   const int v = blockIdx.x * 256 + threadIdx.x, u0 = blockIdx.y * ROWS;
@@ -436,6 +491,7 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
     p.ac = q.ac;
     p.axes = own ? q.axes + b0 : nullptr;
     p.cols = q.cols;
+    p.vec_exps = t.exp1;
     p.scratch = t.P;
     p.err = t.err;
     // four rows a block where that is a block per SM; below, one row (256^2: 64
