@@ -151,6 +151,8 @@ struct SlicedDft2 {
   PhaseAxis ar, ac;          // the axes ...
   const PhaseAxis* axes;     // ... or, on the device, item i's: axes[i] (rows) and axes[cols + i]
   int cols;
+  bool build;                // e1, e2 hold sliced_dft2_chunk's items, whose matrices are built from the
+                             // axes here, chunk by chunk
   double scale;
   const double2* f;          // [count][m][n]
   double2* F;                // [count][M][N]
@@ -163,6 +165,7 @@ size_t sliced_matrix_entries(int len_in, int len_out);    // 16-bit entries of o
 int launch_matrix_digits(const PhaseAxis& ax, const PhaseAxis* axes, int count, int len_in, int len_out,
                          uint16_t* out, cudaStream_t s);
 size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left);
+int sliced_dft2_chunk(int count, int m, int n, int M, int N, bool left);   // items done at once
 int launch_sliced_dft2(const SlicedDft2& q, void* workspace, cudaStream_t s);
 // One-shot test of the sliced GEMM's bounded waits (lgb_test_stall_sliced): what
 // the launch that asks has to hold back, stage -1 for nothing.

@@ -450,6 +450,10 @@ size_t sliced_dft2_workspace(int count, int m, int n, int M, int N, bool left) {
   return layout(count, m, n, M, N, left, nullptr).bytes;
 }
 
+int sliced_dft2_chunk(int count, int m, int n, int M, int N, bool left) {
+  return layout(count, m, n, M, N, left, nullptr).chunk;
+}
+
 int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   const Layout t = layout(q.count, q.m, q.n, q.M, q.N, q.left, ws);
   const bool own = q.axes != nullptr;
@@ -459,6 +463,10 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
   for (int b0 = 0; b0 < q.count; b0 += t.chunk) {
     const int items = std::min(t.chunk, q.count - b0);
     const double2* f = q.f + (size_t)b0 * q.m * q.n;
+    if (q.build) {
+      if ((st = launch_matrix_digits(PhaseAxis{}, q.axes + b0, items, q.m, q.M, e1.base, s))) return st;
+      if ((st = launch_matrix_digits(PhaseAxis{}, q.axes + q.cols + b0, items, q.n, q.N, e2.base, s))) return st;
+    }
     if (t.left)
       slice_cols_kernel<<<dim3(cdiv(q.n, SC_COLS), items), 32 * SC_WARPS, 0, s>>>(f, q.m, q.n, t.d1, t.exp1,
                                                                                  t.err);
@@ -502,7 +510,7 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
       LGB_CUDA(launch_next(finish_kernel<FIN_ROWS>, dim3(cdiv(q.N, 256), cdiv(q.M, FIN_ROWS), items), 256, 0, s, p));
     else
       LGB_CUDA(launch_next(finish_kernel<1>, dim3(cdiv(q.N, 256), q.M, items), 256, 0, s, p));
-    if (own) {
+    if (own && !q.build) {
       e1.base += (size_t)items * ND * e1.plane();
       e2.base += (size_t)items * ND * e2.plane();
     }

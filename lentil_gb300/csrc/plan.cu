@@ -334,8 +334,16 @@ struct lgb_psf_plan_s {
   double2 *E1 = nullptr, *E2 = nullptr, *f = nullptr, *T = nullptr, *F = nullptr;
   bool sliced = false;             // FP64 on the tensor cores: digit matrices in place of E1, E2
   uint16_t *d1 = nullptr, *d2 = nullptr;
+  bool resident = true;            // ... of every wavelength, else of a chunk, built by each execute
   void* sliced_ws = nullptr;       // one PSF's wavelengths
 };
+
+// Digit matrices that a complex128 plan keeps at most.  An entry takes 42 bytes where
+// it took 16 as a number, and 32 wavelengths at 4096^2 held 45 GB of them, the plan 64
+// (43 with numbers, 21 without).  Building them for each chunk of wavelengths costs 3 %
+// there (17.1 -> 17.5 ms a wavelength), 6 % at 2048^2 and 10 % at 1024^2, where 195
+// wavelengths fit.
+constexpr size_t RESIDENT_BYTES = (size_t)16 << 30;
 
 static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
   const lgb_psf_desc& d = P->d;
@@ -366,8 +374,11 @@ static size_t plan_carve(lgb_psf_plan_s* P, void* base) {
   } else {
     const size_t Q = (size_t)B * L;
     if (P->sliced) {
-      P->d1 = c.take<uint16_t>(L * sliced_matrix_entries(d.m, d.M));
-      P->d2 = c.take<uint16_t>(L * sliced_matrix_entries(d.n, d.N));
+      const size_t e1 = sliced_matrix_entries(d.m, d.M), e2 = sliced_matrix_entries(d.n, d.N);
+      P->resident = 2 * L * (e1 + e2) <= RESIDENT_BYTES;
+      const int kept = P->resident ? L : sliced_dft2_chunk(L, d.m, d.n, d.M, d.N, true);
+      P->d1 = c.take<uint16_t>(kept * e1);
+      P->d2 = c.take<uint16_t>(kept * e2);
       P->sliced_ws = c.take<char>(sliced_dft2_workspace(L, d.m, d.n, d.M, d.N, true));
     } else {
       P->E1 = c.take<double2>((size_t)L * d.M * d.m);
@@ -477,8 +488,8 @@ static int build_plan(lgb_psf_plan_s* P, cudaStream_t s, lgb_psf_plan* plan) {
     st = launch_e1_block_split(P->axes, L, d.m, d.M, P->kp1, cdiv(d.M, 64) * 128, bf16, P->e1h, P->e1l, s);
     if (!st) st = launch_e2_block_split(P->axes + L, L, d.n, d.N, P->kp2, cdiv(d.N, 128) * 256, bf16, P->e2h, P->e2l, s);
   } else if (P->sliced) {
-    st = launch_matrix_digits(PhaseAxis{}, P->axes, L, d.m, d.M, P->d1, s);
-    if (!st) st = launch_matrix_digits(PhaseAxis{}, P->axes + L, L, d.n, d.N, P->d2, s);
+    if (P->resident) st = launch_matrix_digits(PhaseAxis{}, P->axes, L, d.m, d.M, P->d1, s);
+    if (P->resident && !st) st = launch_matrix_digits(PhaseAxis{}, P->axes + L, L, d.n, d.N, P->d2, s);
   } else {
     for (int l = 0; l < L && !st; ++l) {
       st = launch_dft_matrix_c128(axes[l], d.m, d.M, P->E1 + (size_t)l * d.M * d.m, true, s);
@@ -632,6 +643,7 @@ static int psf_execute_n(lgb_psf_plan P, int B, const int* lam_idx, int n_sel, c
       q.e1 = P->d1; q.e2 = P->d2;
       q.axes = P->axes;
       q.cols = L;
+      q.build = !P->resident;
       q.scale = 1.0;
       q.f = P->f + q0 * sf;
       q.F = P->F + q0 * sF;
