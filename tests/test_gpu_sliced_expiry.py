@@ -14,7 +14,9 @@ import time
 import pytest
 import torch
 
+import lentil_gb300 as lg
 from lentil_gb300 import _lib
+from lentil_gb300.broadband import PSFPlan
 
 pytestmark = pytest.mark.gpu
 
@@ -61,3 +63,46 @@ def test_withheld_stage(cuda_device, shape, release, stage, launch):
     again = sliced()
     assert int(word) == _lib.OK
     assert torch.equal(again, before)
+
+
+def _stalled(call, launch, release, stage):
+    _lib.check(_lib.load().lgb_test_stall_sliced(launch, stage, release, 1.0))
+    t0 = time.perf_counter()
+    out = call()
+    torch.cuda.synchronize()
+    assert time.perf_counter() - t0 < 1.0
+    return out
+
+
+@pytest.mark.parametrize('launch', [0, 1])
+@pytest.mark.parametrize('release,stage', [(0, 3), (1, 3)])
+def test_plan_with_matrices_by_wavelength(cuda_device, release, stage, launch):
+    n, waves = 384, 5
+    lam = [5e-7 + 5e-8 * k for k in range(waves)]
+    plan = PSFPlan((n, n), (0, 0, n, n), (0, 0), lam, [(0.5 * 5e-7 / l / n, 0.4 * 5e-7 / l / n) for l in lam],
+                   [(0.25, -0.5)] * waves, (n, n), (n, n), (0, 0), precision='fp64')
+    g = torch.Generator(device='cuda').manual_seed(9)
+    amp = torch.rand(1, n, n, generator=g, dtype=torch.float64, device='cuda')
+    opd = 1e-7 * torch.rand(1, n, n, generator=g, dtype=torch.float64, device='cuda')
+    w = torch.rand(1, waves, generator=g, dtype=torch.float64, device='cuda')
+    run = lambda: plan.execute(amp, opd, w, check=False)
+    before = run()
+    image = _stalled(run, launch, release, stage)
+    assert not torch.equal(image, before)              # in plain FP64: other roundings
+    # an |F| of at most amp.sum() is off by 4 n roundings of it
+    assert float((image - before).abs().max()) <= waves * 2 * 4 * n * 2.0 ** -53 * float(before.max())
+    assert torch.equal(run(), before)
+
+
+@pytest.mark.parametrize('launch', [0, 1])
+@pytest.mark.parametrize('release,stage', [(0, 2), (1, 2)])
+def test_pixel_products(cuda_device, release, stage, launch):
+    n = 700
+    g = torch.Generator(device='cuda').manual_seed(9)
+    img = torch.rand(n, n, generator=g, dtype=torch.float64, device='cuda')
+    run = lambda: lg.detector.pixel(img, 3)
+    before = run()
+    image = _stalled(run, launch, release, stage)
+    assert not torch.equal(image, before)
+    assert float((image - before).abs().max()) <= 4 * n * 2.0 ** -53 * float(before.max())
+    assert torch.equal(run(), before)
