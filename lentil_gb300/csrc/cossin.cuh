@@ -3,7 +3,7 @@
 // DFT matrices and phasors need cosines and sines of phases that are exact
 // 64-bit fractions of a cycle (phase_fixed, common.cuh; x mod 2).  Double-
 // precision sincospi holds this part's FP64 pipe (17 clocks a value per SM
-// measured in the phasor kernel); the integer pipes give the same in about two:
+// measured in the phasor kernel); the integer pipes give the same in about five:
 // the nearest of 512 points of the circle from a table, and a rotation by the
 // rest, |d| < 2^-7.3, with the Taylor series of cos d and sin d in 64-bit fixed
 // point, cut where the terms fall below 2^-63.  The error is below 2^-60 (2.4 units of 2^-62 at most over

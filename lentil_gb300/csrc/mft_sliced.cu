@@ -418,11 +418,12 @@ bool sliced_left(int m, int n, int M, int N) {
 }
 
 // Where the sliced form is taken: where its five launches cost less than the
-// plain GEMMs' two to four.  Device time of one transform from a plan, plain
-// and sliced: 64^2 to 64^2 20 and 29 us, 96^2 29 and 31, 112^2 39 and 33, 256^2
-// 270 and 37, (8 x 8) to 512^2 27 and 29, (16 x 512) to 512^2 86 and 35,
-// (16 x 1024) to (16 x 1024) 171 and 41: the line is one of multiply-adds, just
-// below the crossing at about 100^2.
+// plain GEMMs' two to four.  Device time of one transform from a plan, plain and
+// sliced (us): 64^2 to 64^2 16.8 and 25.5, 88^2 26.2 and 27.1, 96^2 26.3 and 27.4,
+// 104^2 35.1 and 27.5, 128^2 42.7 and 27.7, 256^2 267 and 30.8; (8 x 8) to 512^2 23.9
+// and 27.8, (8 x 9) to 600^2 31.8 and 31.4, (16 x 512) to (16 x 512) 57.7 and 24.8,
+// (32 x 800) to (400 x 49) 46.9 and 31.1.  The line is one of multiply-adds, near the
+// crossing: beside it the plain form is up to 4 us ahead or 16 behind, by shape.
 // Operands longer than 16384 would leave the 64-bit sums too few fraction bits.
 bool sliced_applies(int m, int n, int M, int N) {
   if (std::min(std::min(m, n), std::min(M, N)) < 8 || std::max(m, n) > 16384 ||

@@ -775,8 +775,9 @@ static int run_split_mft(const SplitMftProblem& q, cudaEvent_t* ev, cudaStream_t
 //
 // The occupancy model below prices both widths.  For launches of eight or more
 // waves in both stages its choice is final: the 256-wide tile is 3-4 % faster
-// there, less than a trial tells apart.  Below, where a width can win by up to
-// 1.35x, measure mode (the default) tunes the class online, on the caller's own launches: the
+// there, less than a trial tells apart.  Below, where the 128-wide tile wins by 1.41
+// to 1.56x (less than a wave) or either by up to 7 % (two waves and more), measure
+// mode (the default) tunes the class online, on the caller's own launches: the
 // next TUNE_TRIALS launches alternate the two widths, the model's first, each
 // bracketed by CUDA events on its stream; a later launch of the class finds
 // them all finished (cudaEventQuery, no host wait), compares the fastest run
