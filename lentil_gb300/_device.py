@@ -58,6 +58,8 @@ def to_device(x, dtype):
     copy on the current stream."""
     dev = device()
     if is_tensor(x):
+        if x.is_conj() or x.is_neg():          # lazy views: their memory holds other values
+            x = x.resolve_conj().resolve_neg()
         if x.dtype == dtype and x.device == dev and x.is_contiguous():
             return x
         t = x.to(device=dev, dtype=dtype)
