@@ -14,12 +14,14 @@ def pair(x):
     if t in _SCALARS:
         v = np.array((x, x))
     elif t is np.ndarray and x.shape == (2,):
+        if not x.flags.writeable:
+            return x
         v = x.view()
     elif t in (tuple, list) and len(x) == 2 and type(x[0]) in _SCALARS and type(x[1]) in _SCALARS:
         v = np.array(x)
     else:
         return np.broadcast_to(x, (2,))
-    v.flags.writeable = False
+    v.setflags(write=False)
     return v
 
 
