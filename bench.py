@@ -655,7 +655,7 @@ def run_gpu(args):
                          'peak_kind': 'cuBLAS complex128 GEMM measured in this run',
                          'measured_fp64_peaks': fp64_peaks,
                          'note': 'whole plan execute (phasor, both products, intensity), '
-                                 'algorithmic MFT flops; the products run as exact bf16 digit '
+                                 'algorithmic MFT flops; the products run as bf16 digit '
                                  'products on the tensor cores, so the rate is above the FP64 '
                                  "units' peak that it is set against"}},
         'roofline': roofline,

@@ -11,8 +11,10 @@
  * calling thread's last failure.
  *
  * Precision: LGB_FP64 computes in complex128 (parity with lentil within 1e-12
- * peak-normalised): exact digit products on the tensor cores, or the FP64
- * units for small transforms.  LGB_SPLIT_BF16 / LGB_SPLIT_FP16 run
+ * peak-normalised): products of 62-bit fixed-point operands in bf16 digits on
+ * the tensor cores (28 of 49 digit products, summed in integers; their errors
+ * are relative to the largest entries of the vectors of a sum), or the FP64 units
+ * for small transforms.  LGB_SPLIT_BF16 / LGB_SPLIT_FP16 run
  * the contractions on the tcgen05 tensor cores with each operand split into
  * two 16-bit floats (hi + lo; three partial products, FP32 accumulation).
  */
@@ -200,7 +202,9 @@ int lgb_field_multiply(const lgb_c128* a, int lda, int ar0, int ac0,
 /* ------------------------------------------------------------------------
  * Detector pixel MTF.  Replaces lentil/detector.py:167-222 (pixel):
  *   out = |ifft2(fft2(img) * outer(s, s))|,  s = sinc(fftfreq(N) * os),
- * evaluated as |C . img . C^T| with C the real circulant of ifft(s) (FP64).
+ * evaluated as |C . img . C^T| with C the real circulant of ifft(s): by FFTs for
+ * powers of two up to 8192, else in FP64, of sizes 64 to 16384 with the taps
+ * beyond N / 32 (at least 16) by digit products on the tensor cores.
  * img and out are N x N float64 (lentil defines it for square images only;
  * rows != cols -> LGB_EINVAL).  Workspace: lgb_pixel_workspace_size bytes.
  * ---------------------------------------------------------------------- */
@@ -448,7 +452,9 @@ int lgb_test_stall_tma(int item, int kblock, double wait_ms);
  * loads for its stage `stage` (32 K entries each), or, with `release`, does not
  * give that stage's leading digits free for the loads two stages on, and every
  * wait of that launch is bounded by wait_ms.  The launch gives up, and the
- * kernels behind it evaluate its transforms in plain FP64. */
+ * kernels behind it evaluate its transforms in plain FP64: the results are right.
+ * lgb_dft2_status of a one-off transform's workspace reports LGB_ETIMEOUT; plans
+ * and lgb_pixel keep no record. */
 int lgb_test_stall_sliced(int launch, int stage, int release, double wait_ms);
 
 /* ------------------------------------------------------------------------

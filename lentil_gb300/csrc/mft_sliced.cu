@@ -7,8 +7,8 @@
 //   slice_rows    P's rows, scaled to their largest entry -> digits
 //   sliced_gemm   P = the second product
 //   finish        P -> F, scaled
-// chained (launch_next): 512^2 takes 61.5 us, and took 71.5 launched one by one
-// with the flags cleared beforehand.
+// chained (launch_next): 512^2 took 71.5 us launched one by one with the flags
+// cleared beforehand, 61.5 so (63.5 with the GEMM's later changes).
 // A field with a NaN gives NaN everywhere (each output sums every entry); one
 // with infinities, or a device-side wait that ran out, makes `finish`
 // evaluate that transform in plain FP64 instead.
