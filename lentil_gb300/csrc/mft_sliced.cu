@@ -8,7 +8,7 @@
 //   sliced_gemm   P = the second product
 //   finish        P -> F, scaled
 // chained (launch_next): 512^2 took 71.5 us launched one by one with the flags
-// cleared beforehand, 61.5 so (63.5 with the GEMM's later changes).
+// cleared beforehand, 61.5 so (65.2 with the later changes to its sums).
 // A field with a NaN gives NaN everywhere (each output sums every entry); one
 // with infinities, or a device-side wait that ran out, makes `finish`
 // evaluate that transform in plain FP64 instead.
@@ -54,8 +54,8 @@ __device__ __forceinline__ longlong2 fixed_entry(double2 z, int e) {
 
 // f's rows (one block each) -> digits, vectors of n entries.
 __global__ void __launch_bounds__(128) slice_rows_kernel(const double2* __restrict__ f, int m, int n,
-                                                         DigitRows out, int* __restrict__ exps,
-                                                         int* __restrict__ err) {
+                                                         DigitRows out, int* __restrict__ exps, int S,
+                                                         int* __restrict__ limits, int* __restrict__ err) {
   next_may_start();
   const int i = blockIdx.x, b = blockIdx.y;
   if (i == 0 && b == 0 && threadIdx.x == 0) *err = 0;
@@ -73,14 +73,24 @@ __global__ void __launch_bounds__(128) slice_rows_kernel(const double2* __restri
   __syncthreads();
   e = max(max(se[0], se[1]), max(se[2], se[3]));
   flag = sf[0] | sf[1] | sf[2] | sf[3];
-  if (threadIdx.x == 0) exps[(size_t)b * m + i] = exponent_or_flag(e, flag);
+  if (threadIdx.x == 0) {
+    exps[(size_t)b * m + i] = exponent_or_flag(e, flag);
+    limits[(size_t)b * m + i] = S;
+  }
   if (flag) return;                                       // this transform does not use its digits
   out.base += (size_t)b * ND * out.plane();
   const double2 zero = make_double2(0.0, 0.0);
+  unsigned sum = 0;
   for (int k = 2 * threadIdx.x; k < out.kp; k += 256) {
-    const double2 z0 = k < n ? src[k] : zero, z1 = k + 1 < n ? src[k + 1] : zero;
-    store_digits3(out, i, k, fixed_entry(z0, e), fixed_entry(z1, e));
+    const longlong2 x0 = fixed_entry(k < n ? src[k] : zero, e), x1 = fixed_entry(k + 1 < n ? src[k + 1] : zero, e);
+    sum += magnitude(x0) + magnitude(x1);
+    store_digits3(out, i, k, x0, x1);
   }
+  __shared__ unsigned sums[4];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) limits[(size_t)b * m + i] = unit_limit(sums[0] + sums[1] + sums[2] + sums[3], n, S);
 }
 
 constexpr int SC_COLS = 4, SC_WARPS = 16;    // columns and warps per block of slice_cols
@@ -88,8 +98,8 @@ constexpr int SC_COLS = 4, SC_WARPS = 16;    // columns and warps per block of s
 // f's columns -> digits, vectors of m entries: SC_COLS neighbouring columns a
 // block (a 64-byte piece of each row), SC_WARPS / SC_COLS warps per column.
 __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
-    const double2* __restrict__ f, int m, int n, DigitRows out, int* __restrict__ exps,
-    int* __restrict__ err) {
+    const double2* __restrict__ f, int m, int n, DigitRows out, int* __restrict__ exps, int S,
+    int* __restrict__ limits, int* __restrict__ err) {
   next_may_start();
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *err = 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -111,25 +121,36 @@ __global__ void __launch_bounds__(32 * SC_WARPS) slice_cols_kernel(
   __syncthreads();
 #pragma unroll
   for (int q = 0; q < PARTS; ++q) { e = max(e, se[q * SC_COLS + c]); flag |= sf[q * SC_COLS + c]; }
-  if (j >= n) return;
-  if (part == 0 && lane == 0) exps[(size_t)b * n + j] = exponent_or_flag(e, flag);
-  if (flag) return;
-  out.base += (size_t)b * ND * out.plane();
-  const double2 zero = make_double2(0.0, 0.0);
-  for (int k = 2 * (part * 32 + lane); k < out.kp; k += 64 * PARTS) {
-    const double2 z0 = k < m ? src[(size_t)k * n] : zero;
-    const double2 z1 = k + 1 < m ? src[(size_t)(k + 1) * n] : zero;
-    store_digits3(out, j, k, fixed_entry(z0, e), fixed_entry(z1, e));
+  unsigned sum = 0;
+  if (j < n && !flag) {
+    out.base += (size_t)b * ND * out.plane();
+    const double2 zero = make_double2(0.0, 0.0);
+    for (int k = 2 * (part * 32 + lane); k < out.kp; k += 64 * PARTS) {
+      const longlong2 x0 = fixed_entry(k < m ? src[(size_t)k * n] : zero, e);
+      const longlong2 x1 = fixed_entry(k + 1 < m ? src[(size_t)(k + 1) * n] : zero, e);
+      sum += magnitude(x0) + magnitude(x1);
+      store_digits3(out, j, k, x0, x1);
+    }
+  }
+  __shared__ unsigned sums[SC_WARPS];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (lane == 0) sums[warp] = sum;
+  __syncthreads();
+  if (j < n && part == 0 && lane == 0) {
+    for (int q = 1; q < PARTS; ++q) sum += sums[q * SC_COLS + c];
+    exps[(size_t)b * n + j] = exponent_or_flag(e, flag);
+    limits[(size_t)b * n + j] = flag ? S : unit_limit(sum, m, S);
   }
 }
 
-// Row r of the first product (entry a in units of 2^(expA[a] - 16 - S)) ->
-// its digits as an operand of the second.  The first 2 KEEP entries of a thread
+// Row r of the first product (entry a in units of 2^(expA[a] - 16 - S), S of its
+// tile) -> its digits as an operand of the second.  The first 2 KEEP entries of a thread
 // stay in registers between the two passes (rows of up to 1024 are read once).
 // A vector of f that is not finite marks every row.
 __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
-                                                            const int* expA, int S,
-                                                            DigitRows out, int* __restrict__ exps) {
+                                                            const int* expA, DigitRows out,
+                                                            int* __restrict__ exps, int S2,
+                                                            int* __restrict__ limits) {
   next_may_start();
   constexpr int KEEP = 2, NONE = -(1 << 28);
   const int r = blockIdx.x, b = blockIdx.y;
@@ -138,13 +159,20 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
   const int* ea = expA + (size_t)b * q.cols;
   __shared__ uint8_t parts[3 * MAX_TILES_A];
   __shared__ int se[8];
+  __shared__ unsigned sums[8];
   count_parts<3>(q, 3 * b, r, parts);
   previous_done();
-  longlong2 kept[2 * KEEP], rest[2];
-  int e = NONE;
-  auto note = [&](int a, longlong2 v) {
+  // of entry a's units, less 16, or that its vector is not finite
+  auto exponent = [&](int a) {
     const int x = a < q.cols ? ea[a] : NONE;
-    if (v.x | v.y || x >= EXP_INF) e = max(e, x + max(bit_length(v.x), bit_length(v.y)));
+    return a < q.cols && x < EXP_INF ? x - q.S(b, r, a) : x;
+  };
+  longlong2 kept[2 * KEEP], rest[2];
+  int x[2 * KEEP], y[2];
+  int e = NONE;
+  auto note = [&](int x, longlong2 v) {
+    if (x >= EXP_INF) e = max(e, x);
+    else if (v.x | v.y) e = max(e, x + max(bit_length(v.x), bit_length(v.y)));
   };
   {
     size_t at[2 * KEEP];
@@ -153,16 +181,19 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
     for (int i = 0; i < 2 * KEEP; ++i) {
       const int k = 2 * threadIdx.x + 512 * (i >> 1) + (i & 1);
       at[i] = k;
+      x[i] = exponent(k);
 #pragma unroll
       for (int c = 0; c < 3; ++c) n[c][i] = k < q.cols ? parts[c * tiles + k / BM] : 0;
     }
     sum_parts3<2 * KEEP>(P, q.stride, q.part(), at, n, kept);
 #pragma unroll
-    for (int i = 0; i < 2 * KEEP; ++i) note((int)at[i], kept[i]);
+    for (int i = 0; i < 2 * KEEP; ++i) note(x[i], kept[i]);
   }
   auto fetch = [&](int k) {                     // entries k, k + 1 -> rest
     const size_t at[2] = {(size_t)k, (size_t)k + 1};
     int n[3][2];
+    y[0] = exponent(k);
+    y[1] = exponent(k + 1);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       n[c][0] = k < q.cols ? parts[c * tiles + k / BM] : 0;
@@ -172,8 +203,8 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
   };
   for (int k = 512 * KEEP + 2 * threadIdx.x; k < q.cols; k += 512) {
     fetch(k);
-    note(k, rest[0]);
-    note(k + 1, rest[1]);
+    note(y[0], rest[0]);
+    note(y[1], rest[1]);
   }
   e = __reduce_max_sync(0xffffffffu, e);
   if ((threadIdx.x & 31) == 0) se[threadIdx.x >> 5] = e;
@@ -181,29 +212,42 @@ __global__ void __launch_bounds__(256) slice_product_kernel(const PartialSums q,
 #pragma unroll
   for (int w = 0; w < 8; ++w) e = max(e, se[w]);
   const int bad = e >= EXP_NAN ? EXP_NAN : e >= EXP_INF ? EXP_INF : 0;
-  if (threadIdx.x == 0) exps[(size_t)b * q.rows + r] = bad ? bad : e == NONE ? 0 : e - 16 - S;
+  if (threadIdx.x == 0) {
+    exps[(size_t)b * q.rows + r] = bad ? bad : e == NONE ? 0 : e - 16;
+    limits[(size_t)b * q.rows + r] = S2;
+  }
   if (bad) return;
   out.base += (size_t)b * ND * out.plane();
-  auto put = [&](int k, longlong2 v0, longlong2 v1) {
-    const int s0 = k < q.cols ? ea[k] - e + XBITS : 0, s1 = k + 1 < q.cols ? ea[k + 1] - e + XBITS : 0;
-    store_digits3(out, r, k, make_longlong2(shift_round(v0.x, s0), shift_round(v0.y, s0)),
-                  make_longlong2(shift_round(v1.x, s1), shift_round(v1.y, s1)));
+  unsigned sum = 0;
+  auto put = [&](int k, int e0, int e1, longlong2 v0, longlong2 v1) {
+    const int s0 = max(e0 - e + XBITS, -64), s1 = max(e1 - e + XBITS, -64);      // (beyond the row: zeros)
+    const longlong2 x0 = make_longlong2(shift_round(v0.x, s0), shift_round(v0.y, s0));
+    const longlong2 x1 = make_longlong2(shift_round(v1.x, s1), shift_round(v1.y, s1));
+    sum += magnitude(x0) + magnitude(x1);
+    store_digits3(out, r, k, x0, x1);
   };
 #pragma unroll
   for (int i = 0; i < KEEP; ++i) {
     const int k = 2 * threadIdx.x + 512 * i;
-    if (k < out.kp) put(k, kept[2 * i], kept[2 * i + 1]);
+    if (k < out.kp) put(k, x[2 * i], x[2 * i + 1], kept[2 * i], kept[2 * i + 1]);
   }
   for (int k = 512 * KEEP + 2 * threadIdx.x; k < out.kp; k += 512) {
     fetch(k);
-    put(k, rest[0], rest[1]);
+    put(k, y[0], y[1], rest[0], rest[1]);
+  }
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) sum += sums[w];
+    limits[(size_t)b * q.rows + r] = unit_limit(sum, q.cols, S2);
   }
 }
 
 // ---------------------------------------------------------------- finish ---
 struct FinishParams {
   PartialSums q;             // rows M, cols N
-  int M, N, S;
+  int M, N;
   const int* exps;           // [item][M] (left) or [item][N]: exponent of the sliced product
   int left;                  // (E1 f) E2, else E1 (f E2)
   double scale;
@@ -334,6 +378,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
     return;
   }
   const int* exps = p.exps + (p.left ? (size_t)b * p.M + u0 : (size_t)b * p.N + v);
+  const int unit = 16 + p.q.S(b, u0, v);
   longlong2 z[ROWS];
   size_t at[ROWS];
   int n[3][ROWS], e[ROWS];
@@ -347,7 +392,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const FinishParams p) {
 #pragma unroll
   for (int i = 0; i < ROWS; ++i) {
     at[i] = (size_t)(u0 + i) * p.q.ld + v;
-    e[i] = i < rows ? exps[p.left ? i : 0] - 16 - p.S : 0;
+    e[i] = i < rows ? exps[p.left ? i : 0] - unit : 0;
   }
   sum_parts3<ROWS>(p.q.P + (size_t)b * 3 * p.q.stride, p.q.stride, p.q.part(), at, n, z);
 #pragma unroll
@@ -366,6 +411,7 @@ struct Layout {
   Deal deal1, deal2;
   long long stride;          // P entries per product
   int *err, *exp1, *exp2;
+  int *lim1, *lim2, *tile1, *tile2;            // units: limits of the data's vectors, S of the tiles
   DigitRows d1, d2;          // digits of f (operand A) and of the intermediate
   long long* P;
   size_t bytes;
@@ -404,6 +450,10 @@ Layout layout(int count, int m, int n, int M, int N, bool left, void* ws) {
   t.err = reinterpret_cast<int*>(take(16));
   t.exp1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.vecs1));
   t.exp2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.rows1));
+  t.lim1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.vecs1));
+  t.lim2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.rows1));
+  t.tile1 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * t.deal1.tilesA));
+  t.tile2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)t.chunk * (t.left ? t.deal2.tilesB : t.deal2.tilesA)));
   t.d1.base = reinterpret_cast<uint16_t*>(take(b1 * t.chunk));
   t.d2.base = reinterpret_cast<uint16_t*>(take(b2 * t.chunk));
   t.P = reinterpret_cast<long long*>(take(sizeof(long long) * (size_t)t.stride * 3 * t.chunk));
@@ -469,26 +519,26 @@ int launch_sliced_dft2(const SlicedDft2& q, void* ws, cudaStream_t s) {
       if ((st = launch_matrix_digits(PhaseAxis{}, q.axes + q.cols + b0, items, q.n, q.N, e2.base, s))) return st;
     }
     if (t.left)
-      slice_cols_kernel<<<dim3(cdiv(q.n, SC_COLS), items), 32 * SC_WARPS, 0, s>>>(f, q.m, q.n, t.d1, t.exp1,
-                                                                                 t.err);
+      slice_cols_kernel<<<dim3(cdiv(q.n, SC_COLS), items), 32 * SC_WARPS, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, S1,
+                                                                                 t.lim1, t.err);
     else
-      slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, t.err);
+      slice_rows_kernel<<<dim3(q.m, items), 128, 0, s>>>(f, q.m, q.n, t.d1, t.exp1, S1, t.lim1, t.err);
     LGB_CUDA(cudaGetLastError());
     const int own_items = own ? items : 1;
-    if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, S1, nullptr, t.P,
-                          t.stride, t.ld1, t.err, s)))
+    if ((st = launch_gemm(t.d1, items, t.left ? e1 : e2, own_items, items, t.K1, t.deal1, t.lim1, BM, t.tile1,
+                          t.P, t.stride, t.ld1, t.err, s)))
       return st;
     LGB_CUDA(launch_next(slice_product_kernel, dim3(t.rows1, items), 256, 0, s,
-                         PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1}, t.exp1, S1, t.d2, t.exp2));
+                         PartialSums{t.P, t.stride, t.ld1, t.rows1, t.vecs1, t.deal1, t.tile1, false}, t.exp1, t.d2,
+                         t.exp2, S2, t.lim2));
     if ((st = launch_gemm(t.left ? e2 : t.d2, t.left ? own_items : items, t.left ? t.d2 : e1,
-                          t.left ? items : own_items, items, t.K2, t.deal2, S2, nullptr, t.P, t.stride, t.ld2, t.err,
-                          s)))
+                          t.left ? items : own_items, items, t.K2, t.deal2, t.lim2, t.left ? BN : BM, t.tile2,
+                          t.P, t.stride, t.ld2, t.err, s)))
       return st;
     FinishParams p{};
-    p.q = PartialSums{t.P, t.stride, t.ld2, q.M, q.N, t.deal2};
+    p.q = PartialSums{t.P, t.stride, t.ld2, q.M, q.N, t.deal2, t.tile2, t.left};
     p.M = q.M;
     p.N = q.N;
-    p.S = S2;
     p.exps = t.exp2;
     p.left = t.left;
     p.scale = q.scale;

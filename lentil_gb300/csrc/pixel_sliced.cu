@@ -249,7 +249,7 @@ int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, int
   const DigitRows dX = real_rows(t.dX, N), dR = real_rows(t.dR, N);
   const int w = std::max(16, cdiv(N, 32));             // N <= 16384: at most MAX_NEAR
   Combine f{};
-  f.q = PartialSums{t.P, 0, t.ld, N, N, t.deal};
+  f.q = PartialSums{t.P, 0, t.ld, N, N, t.deal, nullptr, false};
   f.ea = t.eX;
   f.eb = t.eR;
   f.unit = t.unit;
@@ -263,7 +263,7 @@ int launch_pixel_sliced(const double* img, int N, const double* c, void* ws, int
     f.X = pass == 0 ? img : t.Y;
     LGB_CUDA(launch_next(slice_real_kernel, pass == 0 ? 2 * N : N, 256, 0, s, DenseRows{f.X, N}, dX, t.eX,
                          FarTaps{c, N, w}, dR, t.eR, status + 1, t.unit));
-    const int st = launch_gemm(dX, 1, dR, 1, 1, N, t.deal, 0, t.unit, t.P, 0, t.ld, status, s);
+    const int st = launch_gemm(dX, 1, dR, 1, 1, N, t.deal, t.unit, 0, nullptr, t.P, 0, t.ld, status, s);
     if (st) return st;
     if (pass == 0) {
       f.Y = t.Y;

@@ -31,7 +31,8 @@
 // im and h = (re + im) / 2, the products of like sets are
 //     P0 = Ar Br,  P1 = Ai Bi,  P2 = 2 Ah Bh,
 // and readers form re = P0 - P1, im = 2 P2 - P0 - P1 in integers, modulo 2^64,
-// which loses nothing.  That is 84 digit products where four real products took 108 (a DFT
+// which loses nothing.  P2 counts four times and has a quarter of the unit, so that
+// its roundings weigh no more than P0's and P1's.  That is 84 digit products where four real products took 108 (a DFT
 // matrix had six digits then): 1019 x 941 to 1024^2 went from 337 to 300 us,
 // 512^2 from 82 to 76.
 #pragma once
@@ -60,6 +61,7 @@ constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
 constexpr uint32_t BAR_BYTES = 256;
 constexpr uint32_t SMEM_BYTES = STAGES * STAGE_BYTES + BAR_BYTES + 1024;
 constexpr int RUN = 4 * BN / EPI_WARPS;      // tile columns per epilogue warp
+constexpr int MAX_S = 40;                    // group 4's sums are ints below 2^(S - 11), S + 2 for P2
 constexpr unsigned long long WAIT_NS = 2000000000ull;
 static_assert(SMEM_BYTES <= 232448, "shared memory per CTA");
 static_assert(GROUPS * BN <= 512 && RUN == 24, "tensor memory columns; the drain loads 3 x 8 of them");
@@ -86,8 +88,12 @@ struct GemmParams {
   int rowsB;
   int ld;                    // P row pitch (entries)
   int dA, dB;                // digit planes between items (0: shared by all items)
-  int S;                     // P unit: 2^-(16 + S) of the scaled operands, a quarter of it for P2
-  const int* unit;           // S, found on the device (null: the above)
+  // P unit: 2^-(16 + S) of the scaled operands, a quarter of it for P2.  S of a tile
+  // is the least of its vectors' limits (unit_limit) on one side
+  const int* limits;         // [item][limit_count]
+  int limit_count;
+  int limit_rows;            // BM: A's vectors, BN: B's; 0: one value for all
+  int* tile_S;               // out: [item][tiles of that side]
   long long* P;              // [product][part][rowsB][ld]
   long long stride;          // entries between products
   int* err;
@@ -333,7 +339,18 @@ sliced_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     for (int pos = begin; ok && pos < end;) {
       const Segment w = segment_at(p, pos, end);
       pos += w.count;
-      const int S = (p.unit ? *p.unit : p.S) + (w.product % p.sets == 2 ? 2 : 0);
+      const int item = w.product / p.sets;
+      int S = MAX_S;
+      if (p.limit_rows == 0) {
+        S = *p.limits;
+      } else {
+        const int first = p.limit_rows == BM ? w.m0 : w.n0, last = min(first + p.limit_rows, p.limit_count);
+        for (int i = first + lane; i < last; i += 32) S = min(S, p.limits[item * p.limit_count + i]);
+        S = __reduce_min_sync(0xffffffffu, S);
+        if (warp == 2 && lane == 0)
+          p.tile_S[item * ((p.limit_count + p.limit_rows - 1) / p.limit_rows) + first / p.limit_rows] = S;
+      }
+      if (w.product - item * p.sets == 2) S += 2;
       const float unit4 = ldexpf(1.f, S);
       // sums of groups 1 to 3 are whole multiples of 2^-9, 2^-18, 2^-27 below 2^24
       // of them: three more bits leave the multipliers below 2^31
@@ -462,6 +479,23 @@ __device__ __forceinline__ void store_digits3(const DigitRows& o, int j, int k, 
   store_digits(o, 2, j, k, half_sum(z0.x, z0.y), half_sum(z1.x, z1.y));
 }
 
+// What an entry adds to the sum of |re| + |im| of a vector, in units of 2^46 (at most
+// 2^17: 16384 of them fit a word).
+__device__ __forceinline__ unsigned magnitude(longlong2 z) {
+  return (unsigned)(((unsigned long long)(z.x < 0 ? -z.x : z.x) + (unsigned long long)(z.y < 0 ? -z.y : z.y)) >> 46);
+}
+
+// The S that a data vector of K entries allows: its sums with entries |E| <= 1 are at
+// most L 2^16, L the sum of its |re| + |im| over 2^62, below (sum + K) 2^-16, and
+// L 2^(16 + S) stays below 2^63 with 2^-32 of it for the sums' roundings.
+// Never less than S, which holds for any vector.  A vector with few large entries has
+// a unit of up to 2^-56 of them so, where the one for K = 1040 is 2^-51: amplitudes
+// over ten decades, (8 x 1040) to (8 x 260), came out 2.0 times as far from exact as in
+// plain FP64 with that one, 0.9 times so (1019 x 941 to 1024^2 292 -> 296 us).
+__device__ __forceinline__ int unit_limit(unsigned sum, int K, int S) {
+  return min(MAX_S, max(S, 63 - (32 - __clz((int)(sum + K)))));
+}
+
 constexpr int FLAG_INF = 1, FLAG_NAN = 2;
 
 __device__ __forceinline__ void note_exponent(double x, int& e, int& flag) {
@@ -479,6 +513,11 @@ struct PartialSums {
   long long stride;          // entries between products
   int ld, rows, cols;
   Deal deal;
+  const int* tile_S;         // the tiles' S: [item][tiles along one side]
+  bool by_row;               // of rows (the B side), else of columns
+  __device__ __forceinline__ int S(int item, int r, int a) const {
+    return by_row ? tile_S[item * deal.tilesB + r / BN] : tile_S[item * deal.tilesA + a / BM];
+  }
   __device__ __forceinline__ int parts(int product, int r, int a) const {
     return deal.parts((product * deal.tilesB + r / BN) * deal.tilesA + a / BM);
   }
@@ -575,15 +614,12 @@ inline Deal deal_of(int rowsA, int rowsB, int chains, int products) {
 // Partial sums of a tile at most, whichever chain of a CTA it starts at.
 inline int max_parts(const Deal& d) { return std::min(d.chains, (d.chains + d.per - 2) / d.per + 1); }
 
-// S for a contraction of K entries: sums reach K 2^16 (times sqrt 2 for im).
-// P2 counts four times and has a quarter of the unit, so that its roundings
-// weigh no more than P0's and P1's (with half of it, fields with a cross of ones
-// over 1e-3 or ten decades of amplitudes came out up to 1.27 times further from
-// exact than the FP64 GEMM leaves them).  K <= 16384, so S >= 32.
+// S of a contraction of K entries, whatever they are: sums reach K 2^16 (times sqrt 2
+// for im).  K <= 16384, so S >= 32.
 inline int unit_shift(int K) {
   int lg = 0;
   while ((1 << lg) < K) ++lg;
-  return std::min(40, 46 - lg);                // group 4's sums are ints: S + 2 <= 42
+  return std::min(MAX_S, 46 - lg);
 }
 
 // Tensor map of a digit operand seen as [items x digits][sets][L][kp], box
@@ -607,7 +643,8 @@ inline int make_digit_map(CUtensorMap* map, const DigitRows& d, int items, int b
 // The products of A's and B's sets over K entries, for `items` items; the
 // operands hold itemsA and itemsB of them (1: shared by all).
 inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int itemsB, int items, int K,
-                       const Deal& deal, int S, const int* unit, long long* P, long long stride, int ld,
+                       const Deal& deal, const int* limits, int limit_rows, int* tile_S, long long* P,
+                       long long stride, int ld,
                        int* err, cudaStream_t s) {
   static OncePerDevice once;
   LGB_CUDA(allow_shared_memory(once, sliced_gemm_kernel, SMEM_BYTES));
@@ -624,8 +661,10 @@ inline int launch_gemm(const DigitRows& A, int itemsA, const DigitRows& B, int i
   p.ld = ld;
   p.dA = itemsA > 1 ? ND : 0;
   p.dB = itemsB > 1 ? ND : 0;
-  p.S = S;
-  p.unit = unit;
+  p.limits = limits;
+  p.limit_rows = limit_rows;
+  p.limit_count = limit_rows == BM ? A.L : B.L;
+  p.tile_S = tile_S;
   p.P = P;
   p.stride = stride;
   p.err = err;

@@ -1,7 +1,7 @@
 """The complex128 tensor-core form leaves a transform no further from exact than
 the plain FP64 GEMMs (``lgb_dft2_noalloc``), on fields of one size of amplitude
-and on those that fixed-point digits suit least: a cross of ones over 1e-3, and
-amplitudes over ten decades.
+and on those that fixed-point digits suit least: a cross of ones over 1e-3, a line
+of ones over 1e-4 across the longer side, and amplitudes over ten decades.
 
 Exact: the same transform in extended precision (``np.longdouble``, at least 64
 bits of mantissa) over some of its rows.  Errors are root-mean-square over those
@@ -28,6 +28,10 @@ def _field(kind, m, n):
         f[m // 2, :] += 1
         f[:, n // 2] += 1
         return f
+    if kind == 'line':
+        f = 1e-4 * (r() + 1j * r())
+        f[(slice(None), n // 3) if m <= n else (m // 3, slice(None))] += 1
+        return f
     return r() * np.exp(6 * r()) + 1j * (r() * np.exp(6 * r()))
 
 
@@ -44,8 +48,9 @@ def _product(a, b):
     return a[0] @ b[0] - a[1] @ b[1], a[0] @ b[1] + a[1] @ b[0]
 
 
-@pytest.mark.parametrize('kind', ['random', 'cross', 'decades'])
-@pytest.mark.parametrize('shape', [(128, 128, 128, 128), (256, 256, 256, 256), (333, 257, 290, 301)])
+@pytest.mark.parametrize('kind', ['random', 'cross', 'decades', 'line'])
+@pytest.mark.parametrize('shape', [(128, 128, 128, 128), (256, 256, 256, 256), (333, 257, 290, 301),
+                                   (8, 1040, 8, 260), (1040, 8, 260, 8), (32, 800, 400, 49)])     # long sums
 def test_no_further_from_exact_than_fp64(cuda_device, shape, kind):
     m, n, M, N = shape
     alpha = (0.7 / max(m, M), 0.6 / max(n, N))
